@@ -130,3 +130,40 @@ def test_fp8_config3_full_size():
     assert torch.equal(run(vs * 2), out * 2)
     err = float((out.float() - ref.float()).norm() / ref.float().norm())
     assert err < 5e-2, err
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("d", [64, 128, 32])
+def test_quantizer_is_the_quotient_bit_by_bit(dtype, d):
+    # block edges (127 / 128 / 129 rows), empty sequences, more sequences than one step of the search
+    # covers, sub-normal results, zeros, and values placed on and next to rounding boundaries
+    g = torch.Generator().manual_seed(d)
+    lengths = torch.tensor([127, 0, 128, 129, 1, 0, 256, 257] + [1, 0, 3] * 40 + [0, 300, 0])
+    offs = torch.cat([torch.zeros(1, dtype=torch.int64), torch.cumsum(lengths, 0)])
+    L, H = int(offs[-1]), 3
+    x = torch.randn(L, H, d, generator=g)
+    x[::7] *= 2.0 ** torch.randint(-14, 3, (L, H, 1), generator=g)[::7]
+    x[5::11, :, ::3] = 0.0
+    # a block whose scale is 1: every e4m3 midpoint and the 16-bit values beside it
+    lo = int(offs[6])
+    grid = torch.cat([m * 2.0 ** torch.arange(-9.0, 9.0) for m in torch.arange(8.0, 17.0, 0.5) / 8])
+    grid = torch.cat([grid, grid * (1 + 2.0 ** -8), grid * (1 - 2.0 ** -9), torch.tensor([448.0])]).clamp(max=448.0)
+    flat = x[lo:lo + 128].reshape(128, -1)
+    flat[:, :] = grid.repeat(128 * H * d // len(grid) + 1)[:128 * H * d].view(128, H, d).reshape(128, -1)
+    flat.view(128, H, d)[0, :, 0] = 448.0
+    x[lo:lo + 128] = flat.view(128, H, d)
+    x[-7, 1, 3] = float("inf")   # that block's scale is infinite: zeros and one NaN
+    x = x.to(dtype)
+    x8, scale, blocks = G.quantize_e4m3_block(x.cuda(), offs.cuda())
+    assert int(blocks[-1]) == int(((lengths + 127) // 128).sum())
+    x8, scale, blocks = x8.cpu().view(torch.uint8), scale.cpu(), blocks.cpu()
+    for b, n in enumerate(lengths.tolist()):
+        for r in range(0, n, 128):
+            rows = x[offs[b] + r:offs[b] + min(n, r + 128)].float()
+            sc = rows.abs().amax(dim=(0, 2)).clamp(min=1e-12) / 448.0
+            i = int(blocks[b]) + r // 128
+            assert torch.equal(scale[i], sc)
+            want = (rows / sc[None, :, None]).to(torch.float8_e4m3fn).view(torch.uint8)
+            got = x8[offs[b] + r:offs[b] + min(n, r + 128)]
+            nan = (want & 127) == 127          # (the sign of a NaN is nobody's)
+            assert torch.equal(got & 127 == 127, nan) and torch.equal(got[~nan], want[~nan])
