@@ -1,11 +1,14 @@
 // CUDA-core (SIMT) jagged HSTU attention, forward and backward, fp32 accumulation.
 //
 // This is the path for fp32 tensors and for head dimensions the tensor-core kernels do not
-// cover (anything other than 64 / 128, or d_qk != d_v).  It is written for clarity and exact
-// mask semantics, not for peak throughput: 32x32 tiles, one CTA of 128 threads per
-// (query tile, head, sequence) in the forward and dQ kernels and per (kv tile, head, sequence)
-// in the dK/dV kernel.  The backward uses two kernels so that every gradient element has a
-// single owner: no atomics, no scratch, bit-reproducible.
+// cover (anything other than 64 / 128, or d_qk != d_v).  32x32 tiles, one CTA per (query tile, head,
+// sequence) in the forward and dQ kernels and per (kv tile, head, sequence) in the dK/dV kernel.
+// The backward uses two kernels so that every gradient element has a single owner: no atomics, no
+// scratch, bit-reproducible.
+//
+// Two forms with the same sums in the same order.  Head dimensions 32 / 64 / 128 (d_qk = d_v) on the
+// grid of four elements run the vector kernels below; any other shape runs the element-wise kernels
+// that come first.
 //
 // Math (generative_recommenders/ops/pytorch/pt_hstu_attention.py:146-187, backward as in
 // generative_recommenders/ops/triton/triton_hstu_attention.py:1905-2020):
@@ -123,7 +126,7 @@ __device__ __forceinline__ void zero_rows_beyond_grid(E *base, int64_t row_strid
                                                       int start, int len, int d) {
   if (blockIdx.x != gridDim.x - 1) return;
   int first = (int)gridDim.x * T;
-  for (int64_t idx = (int64_t)first * d + threadIdx.x; idx < (int64_t)len * d; idx += NTHREADS) {
+  for (int64_t idx = (int64_t)first * d + threadIdx.x; idx < (int64_t)len * d; idx += blockDim.x) {
     int i = (int)(idx / d), x = (int)(idx - (int64_t)i * d);
     base[(int64_t)(start + i) * row_stride + (int64_t)h * head_stride + x] = from_f32<E>(0.f);
   }
@@ -334,6 +337,378 @@ __global__ void __launch_bounds__(NTHREADS) attn_kv_stationary_bwd_kernel(SimtPa
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// vector form: D = d_qk = d_v in {32, 64, 128}, rows on the grid of four elements
+//
+// What bounds the element-wise form on small calls is latency: a CTA walks its tiles one after the
+// other, each a chain of scalar loads with an index division between them and of dot products with
+// nine shared-memory loads for eight products.  Here 256 threads fetch the next tile into registers
+// (16-byte loads) while the present one is computed, the tile of S is 2 x 2 per thread and its second
+// product 4 columns per thread, both on 16-byte shared loads.  Measured in fp32 on 16 sequences of up
+// to 256 rows, 2 heads x 32: forward 65 -> 21 us, dQ 52 -> 26, dK / dV 74 -> 36.
+// ---------------------------------------------------------------------------------------
+constexpr int VTHREADS = 256;
+constexpr int PLD = T + 4;   // leading dimension of the P / dS tiles
+
+template <typename E> struct Raw4 { using type = uint2; };       // four 16-bit elements
+template <> struct Raw4<float> { using type = float4; };
+
+template <typename E> __device__ __forceinline__ float4 widen4(const typename Raw4<E>::type &raw) {
+  const E *e = reinterpret_cast<const E *>(&raw);
+  return make_float4(to_f32(e[0]), to_f32(e[1]), to_f32(e[2]), to_f32(e[3]));
+}
+template <typename E> __device__ __forceinline__ void store_row4(E *dst, const float (&f)[4]) {
+  typename Raw4<E>::type raw;
+  E *e = reinterpret_cast<E *>(&raw);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) e[i] = from_f32<E>(f[i]);
+  *reinterpret_cast<typename Raw4<E>::type *>(dst) = raw;
+}
+
+// One 32 x D tile on its way from global to shared memory, held in registers in between.
+template <typename E, int D> struct TileRegs {
+  static constexpr int N = T * D / 4 / VTHREADS, VPR = D / 4, LD = D + 4;
+  typename Raw4<E>::type raw[N];
+  __device__ __forceinline__ void fetch(const E *src, int64_t row_stride, int row0, int nrows) {
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      const int idx = threadIdx.x + n * VTHREADS, r = idx / VPR, c = idx % VPR;
+      raw[n] = typename Raw4<E>::type{};
+      if (r < nrows)
+        raw[n] = *reinterpret_cast<const typename Raw4<E>::type *>(src + (int64_t)(row0 + r) * row_stride + 4 * c);
+    }
+  }
+  __device__ __forceinline__ void put(float *dst) const {
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      const int idx = threadIdx.x + n * VTHREADS, r = idx / VPR, c = idx % VPR;
+      *reinterpret_cast<float4 *>(dst + r * LD + 4 * c) = widen4<E>(raw[n]);
+    }
+  }
+};
+
+// s[ii][jj] = sum_x A[ty + 16 ii][x] * Bm[tx + 16 jj][x], x in ascending order
+template <int D>
+__device__ __forceinline__ void dot_tile(float (&s)[2][2], const float *A, const float *Bm, int ty, int tx) {
+  constexpr int LD = D + 4;
+#pragma unroll
+  for (int ii = 0; ii < 2; ++ii)
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj) s[ii][jj] = 0.f;
+#pragma unroll 8
+  for (int x = 0; x < D; x += 4) {
+    float4 a[2], bv[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      a[i] = *reinterpret_cast<const float4 *>(A + (ty + 16 * i) * LD + x);
+      bv[i] = *reinterpret_cast<const float4 *>(Bm + (tx + 16 * i) * LD + x);
+    }
+#pragma unroll
+    for (int ii = 0; ii < 2; ++ii)
+#pragma unroll
+      for (int jj = 0; jj < 2; ++jj) {
+        s[ii][jj] = fmaf(a[ii].x, bv[jj].x, s[ii][jj]);
+        s[ii][jj] = fmaf(a[ii].y, bv[jj].y, s[ii][jj]);
+        s[ii][jj] = fmaf(a[ii].z, bv[jj].z, s[ii][jj]);
+        s[ii][jj] = fmaf(a[ii].w, bv[jj].w, s[ii][jj]);
+      }
+  }
+}
+
+// acc[ii] += sum_j Pm[row ii][j] * Bm[j][4 cv ..], j in ascending order; a thread owns the rows
+// rg + ii * RSTEP and the four columns from 4 cv on
+template <int D> struct RowOwner {
+  static constexpr int VPR = D / 4, RSTEP = VTHREADS / VPR, R = T / RSTEP;
+};
+template <int D>
+__device__ __forceinline__ void accumulate_rows(float (&acc)[RowOwner<D>::R][4], const float *Pm, const float *Bm,
+                                                int rg, int cv) {
+  constexpr int LD = D + 4, R = RowOwner<D>::R, RSTEP = RowOwner<D>::RSTEP;
+#pragma unroll
+  for (int j = 0; j < T; j += 4) {
+    float pr[R][4];
+#pragma unroll
+    for (int ii = 0; ii < R; ++ii) {
+      const float4 t = *reinterpret_cast<const float4 *>(Pm + (rg + ii * RSTEP) * PLD + j);
+      pr[ii][0] = t.x; pr[ii][1] = t.y; pr[ii][2] = t.z; pr[ii][3] = t.w;
+    }
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+      const float4 v = *reinterpret_cast<const float4 *>(Bm + (j + jj) * LD + 4 * cv);
+#pragma unroll
+      for (int ii = 0; ii < R; ++ii) {
+        acc[ii][0] = fmaf(pr[ii][jj], v.x, acc[ii][0]);
+        acc[ii][1] = fmaf(pr[ii][jj], v.y, acc[ii][1]);
+        acc[ii][2] = fmaf(pr[ii][jj], v.z, acc[ii][2]);
+        acc[ii][3] = fmaf(pr[ii][jj], v.w, acc[ii][3]);
+      }
+    }
+  }
+}
+
+// forward (MODE 0) / dQ (MODE 1) of one query tile
+template <typename E, int D, int MODE>
+__device__ __forceinline__ void q_tile_vec(const SimtParams &p, float *smem) {
+  constexpr int LD = D + 4, R = RowOwner<D>::R, RSTEP = RowOwner<D>::RSTEP;
+  const int b = blockIdx.z, h = blockIdx.y, tile = (int)blockIdx.x;
+  const SeqGeom g = seq_geom(p, b);
+  const bool cached = MODE == 0 && p.delta > 0;
+  if (tile * T >= (cached ? p.delta : g.len)) return;
+  const int L = g.m.L;
+  // position of the tile's first query inside the sequence, and its row in the q / out tensors
+  const int m0 = tile * T + (cached ? L - p.delta : 0);
+  const int64_t qrow0 = cached ? (int64_t)b * p.delta + tile * T : (int64_t)g.start + m0;
+  float *Qs = smem, *Ks = Qs + T * LD, *Vs = Ks + T * LD;
+  float *Gs = Vs + T * LD;                               // (MODE 1)
+  float *Ps = Gs + (MODE == 1 ? T * LD : 0);             // [T][PLD]
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const int rg = threadIdx.x / RowOwner<D>::VPR, cv = threadIdx.x % RowOwner<D>::VPR;
+  float acc[R][4];
+#pragma unroll
+  for (int ii = 0; ii < R; ++ii)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[ii][c] = 0.f;
+  DropMask drop;
+  drop.init(p);
+  if (m0 < L) {
+    const E *kp = (const E *)p.k + (int64_t)g.start * p.k_rs + (int64_t)h * p.k_hs;
+    const E *vp = (const E *)p.v + (int64_t)g.start * p.v_rs + (int64_t)h * p.v_hs;
+    const KvRange range = kv_range_for_q_tile(g.m, g.len, g.nt, m0, T);
+    auto next_tile = [&](int n) {
+      while (n < L && !tiles_overlap(range, n)) n += T;
+      return n;
+    };
+    TileRegs<E, D> kr, vr;
+    int n0 = next_tile(0);
+    {
+      const int qrows = min(T, L - m0);
+      TileRegs<E, D> qr, gr;
+      qr.fetch((const E *)p.q + qrow0 * p.q_rs + (int64_t)h * p.q_hs, p.q_rs, 0, qrows);
+      if (MODE == 1)
+        gr.fetch((const E *)p.dout + (int64_t)g.start * p.do_rs + (int64_t)h * p.do_hs, p.do_rs, m0, qrows);
+      if (n0 < L) {
+        kr.fetch(kp, p.k_rs, n0, min(T, L - n0));
+        vr.fetch(vp, p.v_rs, n0, min(T, L - n0));
+      }
+      qr.put(Qs);
+      if (MODE == 1) gr.put(Gs);
+    }
+    int id_i[2];
+    float sc[2];
+#pragma unroll
+    for (int ii = 0; ii < 2; ++ii) {
+      const int i = m0 + ty + 16 * ii;
+      id_i[ii] = g.m.id(i);
+      sc[ii] = (i >= 0 && i < L) ? row_scale(p, (int64_t)g.start + i) : 0.f;
+    }
+    while (n0 < L) {
+      __syncthreads();   // the previous tile has been used
+      kr.put(Ks);
+      vr.put(Vs);
+      __syncthreads();
+      const int nn = next_tile(n0 + T);
+      if (nn < L) {
+        kr.fetch(kp, p.k_rs, nn, min(T, L - nn));
+        vr.fetch(vp, p.v_rs, nn, min(T, L - nn));
+      }
+      float s[2][2], dp[2][2];
+      dot_tile<D>(s, Qs, Ks, ty, tx);
+      if (MODE == 1) dot_tile<D>(dp, Gs, Vs, ty, tx);
+#pragma unroll
+      for (int ii = 0; ii < 2; ++ii)
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+          const int i = m0 + ty + 16 * ii, j = n0 + tx + 16 * jj;
+          const bool ok = i >= 0 && i < L && j < L && g.m.valid_ids(i, j, id_i[ii], g.m.id(j));
+          float x = s[ii][jj] * p.alpha;
+          if (p.bias != nullptr) {
+            const int dist = i > j ? i - j : j - i;
+            if (dist < p.bias_numel) x += p.bias[dist];
+          }
+          float val;
+          if (MODE == 0)
+            val = ok ? siluf_(x) * sc[ii] : 0.f;
+          else
+            val = ok ? dp[ii][jj] * dsiluf_(x) * sc[ii] : 0.f;   // dS; alpha is applied to the finished dQ row
+          if (ok && drop.on) val *= drop.factor(p, (int64_t)g.start + i, h, j);
+          Ps[(ty + 16 * ii) * PLD + tx + 16 * jj] = val;
+        }
+      __syncthreads();
+      if (MODE == 1 && p.dbias != nullptr && threadIdx.x < 2 * T - 1) {
+        // one thread per diagonal of the 32 x 32 tile: rows - columns = m
+        const int m = (int)threadIdx.x - (T - 1);
+        float sum = 0.f;
+        for (int rr = m > 0 ? m : 0; rr < T && rr - m < T; ++rr) sum += Ps[rr * PLD + rr - m];
+        int dist = m0 - n0 + m;
+        dist = dist < 0 ? -dist : dist;
+        if (sum != 0.f && dist < p.bias_numel) atomicAdd(p.dbias + dist, sum);
+      }
+      accumulate_rows<D>(acc, Ps, MODE == 0 ? Vs : Ks, rg, cv);
+      n0 = nn;
+    }
+  }
+  if (MODE == 0) {
+    if (!cached) zero_rows_beyond_grid((E *)p.out, p.o_rs, p.o_hs, h, g.start, g.len, D);
+  } else {
+    zero_rows_beyond_grid((E *)p.dq, p.dq_rs, p.dq_hs, h, g.start, g.len, D);
+  }
+#pragma unroll
+  for (int ii = 0; ii < R; ++ii) {
+    const int r = rg + ii * RSTEP, i = m0 + r;
+    if (i < 0 || i >= g.len) continue;
+    E *op;
+    if (MODE == 0) {
+      op = (E *)p.out + (qrow0 + r) * p.o_rs + (int64_t)h * p.o_hs;
+    } else {
+      op = (E *)p.dq + (int64_t)(g.start + i) * p.dq_rs + (int64_t)h * p.dq_hs;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[ii][c] *= p.alpha;
+    }
+    store_row4<E>(op + 4 * cv, acc[ii]);
+  }
+}
+
+// dK and dV of one kv tile
+template <typename E, int D>
+__device__ __forceinline__ void kv_tile_vec(const SimtParams &p, float *smem) {
+  constexpr int LD = D + 4, R = RowOwner<D>::R, RSTEP = RowOwner<D>::RSTEP;
+  const int b = blockIdx.z, h = blockIdx.y, n0 = (int)blockIdx.x * T;
+  const SeqGeom g = seq_geom(p, b);
+  if (n0 >= g.len) return;
+  float *Qs = smem, *Ks = Qs + T * LD, *Vs = Ks + T * LD, *Gs = Vs + T * LD;
+  float *Pt = Gs + T * LD;           // P transposed: [key][query], leading dimension PLD
+  float *St = Pt + T * PLD;          // dS transposed
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const int rg = threadIdx.x / RowOwner<D>::VPR, cv = threadIdx.x % RowOwner<D>::VPR;
+  float acc_dk[R][4], acc_dv[R][4];
+#pragma unroll
+  for (int ii = 0; ii < R; ++ii)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc_dk[ii][c] = acc_dv[ii][c] = 0.f;
+  const int L = g.m.L;
+  DropMask drop;
+  drop.init(p);
+  if (n0 < L) {
+    const E *qp = (const E *)p.q + (int64_t)g.start * p.q_rs + (int64_t)h * p.q_hs;
+    const E *gp = (const E *)p.dout + (int64_t)g.start * p.do_rs + (int64_t)h * p.do_hs;
+    auto next_tile = [&](int m) {
+      while (m < L && !tiles_overlap(kv_range_for_q_tile(g.m, g.len, g.nt, m, T), n0)) m += T;
+      return m;
+    };
+    TileRegs<E, D> qr, gr;
+    int m0 = next_tile(0);
+    {
+      const int krows = min(T, L - n0);
+      TileRegs<E, D> kr, vr;
+      kr.fetch((const E *)p.k + (int64_t)g.start * p.k_rs + (int64_t)h * p.k_hs, p.k_rs, n0, krows);
+      vr.fetch((const E *)p.v + (int64_t)g.start * p.v_rs + (int64_t)h * p.v_hs, p.v_rs, n0, krows);
+      if (m0 < L) {
+        qr.fetch(qp, p.q_rs, m0, min(T, L - m0));
+        gr.fetch(gp, p.do_rs, m0, min(T, L - m0));
+      }
+      kr.put(Ks);
+      vr.put(Vs);
+    }
+    while (m0 < L) {
+      __syncthreads();   // the previous tile has been used
+      qr.put(Qs);
+      gr.put(Gs);
+      __syncthreads();
+      const int mn = next_tile(m0 + T);
+      if (mn < L) {
+        qr.fetch(qp, p.q_rs, mn, min(T, L - mn));
+        gr.fetch(gp, p.do_rs, mn, min(T, L - mn));
+      }
+      float s[2][2], dp[2][2];
+      dot_tile<D>(s, Qs, Ks, ty, tx);
+      dot_tile<D>(dp, Gs, Vs, ty, tx);
+#pragma unroll
+      for (int ii = 0; ii < 2; ++ii) {
+        const int i = m0 + ty + 16 * ii;
+        const int id_i = g.m.id(i);
+        const float sc = i < L ? row_scale(p, (int64_t)g.start + i) : 0.f;
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+          const int j = n0 + tx + 16 * jj;
+          const bool ok = i < L && j < L && g.m.valid_ids(i, j, id_i, g.m.id(j));
+          float x = s[ii][jj] * p.alpha;
+          if (p.bias != nullptr) {
+            const int dist = i > j ? i - j : j - i;
+            if (dist < p.bias_numel) x += p.bias[dist];
+          }
+          const float keep = (ok && drop.on) ? drop.factor(p, (int64_t)g.start + i, h, j) : 1.f;
+          const int at = (tx + 16 * jj) * PLD + ty + 16 * ii;
+          Pt[at] = ok ? siluf_(x) * sc * keep : 0.f;
+          St[at] = ok ? dp[ii][jj] * dsiluf_(x) * sc * p.alpha * keep : 0.f;
+        }
+      }
+      __syncthreads();
+      accumulate_rows<D>(acc_dv, Pt, Gs, rg, cv);
+      accumulate_rows<D>(acc_dk, St, Qs, rg, cv);
+      m0 = mn;
+    }
+  }
+  zero_rows_beyond_grid((E *)p.dk, p.dk_rs, p.dk_hs, h, g.start, g.len, D);
+  zero_rows_beyond_grid((E *)p.dv, p.dv_rs, p.dv_hs, h, g.start, g.len, D);
+#pragma unroll
+  for (int ii = 0; ii < R; ++ii) {
+    const int j = n0 + rg + ii * RSTEP;
+    if (j >= g.len) continue;
+    store_row4<E>((E *)p.dk + (int64_t)(g.start + j) * p.dk_rs + (int64_t)h * p.dk_hs + 4 * cv, acc_dk[ii]);
+    store_row4<E>((E *)p.dv + (int64_t)(g.start + j) * p.dv_rs + (int64_t)h * p.dv_hs + 4 * cv, acc_dv[ii]);
+  }
+}
+
+// PART 0: forward, 1: dQ, 2: dK and dV
+template <typename E, int D, int PART>
+__global__ void __launch_bounds__(VTHREADS, D == 128 ? 1 : 2) attn_vec_kernel(SimtParams p) {
+  extern __shared__ __align__(16) float smem[];
+  if constexpr (PART == 2)
+    kv_tile_vec<E, D>(p, smem);
+  else
+    q_tile_vec<E, D, PART>(p, smem);
+}
+
+template <typename E, int D, int PART>
+int launch_vec_part(const SimtParams &p, const b200_hstu_attn_args &a, cudaStream_t st) {
+  constexpr size_t smem = (size_t)((PART == 0 ? 3 : 4) * T * (D + 4) + (PART == 2 ? 2 : 1) * T * PLD) * sizeof(float);
+  auto kern = attn_vec_kernel<E, D, PART>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return check_cuda(e, "simt vector kernel smem attribute");
+  }
+  const int rows = PART == 0 && a.delta_size > 0 ? a.delta_size : a.max_seq_len;
+  kern<<<dim3((unsigned)((rows + T - 1) / T), (unsigned)a.H, (unsigned)a.B), VTHREADS, smem, st>>>(p);
+  count_launch();
+  B200_CHECK_LAUNCH("simt attention (vector form)");
+  return 0;
+}
+
+template <typename E, int D>
+int launch_vec(const SimtParams &p, const b200_hstu_attn_args &a, cudaStream_t st, bool bwd) {
+  if (!bwd) return launch_vec_part<E, D, 0>(p, a, st);
+  if (int rc = launch_vec_part<E, D, 1>(p, a, st)) return rc;
+  return launch_vec_part<E, D, 2>(p, a, st);
+}
+
+// The vector form takes every tensor by four elements: pointers and strides lie on that grid.
+template <typename E>
+bool vec_form_ok(const b200_hstu_attn_args &a, bool bwd) {
+  if (a.dqk != a.dv || (a.dqk != 32 && a.dqk != 64 && a.dqk != 128)) return false;
+  uintptr_t ptrs = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v;
+  int64_t strides = a.q_row_stride | a.q_head_stride | a.k_row_stride | a.k_head_stride | a.v_row_stride |
+                    a.v_head_stride;
+  if (bwd) {
+    ptrs |= (uintptr_t)a.dout | (uintptr_t)a.dq | (uintptr_t)a.dk | (uintptr_t)a.dv_;
+    strides |= a.do_row_stride | a.do_head_stride | a.dq_row_stride | a.dq_head_stride | a.dk_row_stride |
+               a.dk_head_stride | a.dv_row_stride | a.dv_head_stride;
+  } else {
+    ptrs |= (uintptr_t)a.out;
+    strides |= a.o_row_stride | a.o_head_stride;
+  }
+  return ptrs % (4 * sizeof(E)) == 0 && strides % 4 == 0;
+}
+
 SimtParams make_params(const b200_hstu_attn_args &a) {
   SimtParams p;
   p.q = a.q; p.k = a.k; p.v = a.v; p.dout = a.dout;
@@ -404,6 +779,12 @@ int launch_bwd(const b200_hstu_attn_args &a, cudaStream_t st) {
 
 template <typename E>
 int dispatch_d(const b200_hstu_attn_args &a, cudaStream_t st, bool bwd) {
+  if (vec_form_ok<E>(a, bwd)) {
+    const SimtParams p = make_params(a);
+    if (a.dqk == 32) return launch_vec<E, 32>(p, a, st, bwd);
+    if (a.dqk == 64) return launch_vec<E, 64>(p, a, st, bwd);
+    return launch_vec<E, 128>(p, a, st, bwd);
+  }
   int dmax = a.dqk > a.dv ? a.dqk : a.dv;
   if (dmax <= 32) return bwd ? launch_bwd<E, 32>(a, st) : launch_fwd<E, 32>(a, st);
   if (dmax <= 64) return bwd ? launch_bwd<E, 64>(a, st) : launch_fwd<E, 64>(a, st);

@@ -603,3 +603,46 @@ def test_drawn_shapes_forward_backward(batch, heads, max_len, dim, has_targets, 
     ref, rgrads = _oracle(q, k, v, offs, max_len, alpha, nt, window, ctx, full_tail, dout, scale=scale)
     name = ("drawn", batch, heads, max_len, dim, has_targets, ctx, window, full_tail, str(dtype), scalar_scale, seed)
     _check_all(name, out, grads, ref, rgrads, offs, f32=dtype == torch.float32)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("kw", [dict(), dict(contextual_seq_len=5, max_attn_len=33),
+                                dict(max_attn_len=40, min_full_attn_seq_len=20), dict(max_seq_len=96),
+                                dict(dropout_pr=0.2)])
+def test_cuda_core_vector_form_equals_element_wise(dtype, d, kw):
+    # tile edges (31 .. 33, 63 .. 65), empty and one-row sequences, rows beyond max_seq_len; the same
+    # numbers on storage shifted by one element take the element-wise kernels, which add in the same
+    # order: bit by bit the same but for contraction of a product into a sum (2 ulp of fp32)
+    kw = dict(kw)
+    g = torch.Generator().manual_seed(d)
+    lengths = torch.tensor([31, 32, 0, 33, 1, 64, 65, 130, 63])
+    nt = torch.tensor([3, 0, 0, 1, 0, 20, 40, 7, 2]).cuda()
+    offs = torch.cat([torch.zeros(1, dtype=torch.int64), torch.cumsum(lengths, 0)]).cuda()
+    L, H, N = int(lengths.sum()), 3, kw.pop("max_seq_len", 130)
+    src = [torch.randn(L, 2 * H, d, generator=g).to(dtype).cuda() for _ in range(3)]
+    dout = torch.randn(L, H, d, generator=g).to(dtype).cuda()
+    bias = torch.randn(100, generator=g).cuda() if "dropout_pr" not in kw else None
+    seed = torch.tensor([1234567], device="cuda") if "dropout_pr" in kw else None
+
+    def run(shift):
+        leaves = []
+        for t in src:
+            buf = torch.empty(t.numel() + shift, dtype=dtype, device="cuda")
+            buf[shift:].copy_(t.reshape(-1))
+            leaves.append(buf[shift:].view(L, 2 * H, d)[:, 1:1 + H].detach().requires_grad_())   # strided rows
+        b = None if bias is None else bias.clone().requires_grad_()
+        out = G.hstu_mha(N, 1.0 / d, *leaves, offs, num_targets=nt, bias_by_distance=b, dropout_seed=seed, **kw)
+        return (out.detach(),) + torch.autograd.grad(out, leaves + ([] if b is None else [b]), dout)
+
+    G.set_attention_impl("simt")
+    try:
+        fast, slow = run(0), run(1)
+    finally:
+        G.set_attention_impl("auto")
+    for i, (x, y) in enumerate(zip(fast, slow)):
+        if i == 4:       # the bias gradient is added up by atomics: any order
+            torch.testing.assert_close(x, y, rtol=1e-4, atol=1e-4 * float(y.abs().max()))
+        else:
+            eps = 2.0 ** -22 if dtype == torch.float32 else 2.0 ** -8   # (16 bits: one rounding may flip)
+            torch.testing.assert_close(x, y, rtol=eps, atol=eps * float(y.abs().max()))
