@@ -380,36 +380,40 @@ __global__ void __launch_bounds__(WARPS * 32, MAXV <= 2 ? 3 : (MAXV <= 4 ? 2 : 1
   }
 }
 
-// out[which][e] = sum_b partial[b][which][e]   (which in {0,1}).  A CTA takes 32 columns; its
-// eight warps split the partial rows (four loads in flight each) and are added up in a fixed
-// order, so the result does not depend on timing.
+// out[which][e] = sum_b partial[b][which][e]   (which in {0,1}).  A CTA takes 32 columns and what bounds
+// it is the latency of its loads: 32 warps split the partial rows (148 of them: five loads a lane, all
+// in flight: 4 us for 1024 columns, where eight warps with four in flight took 8) and are added up in a fixed order, so the result
+// does not depend on timing.
+constexpr int REDUCE_WARPS = 32;
 template <typename E>
-__global__ void __launch_bounds__(256) reduce_partial_kernel(const float *__restrict__ partial, int nblocks, int D,
-                                                             E *__restrict__ out0, E *__restrict__ out1) {
-  __shared__ float part[8][33];
+__global__ void __launch_bounds__(REDUCE_WARPS * 32)
+reduce_partial_kernel(const float *__restrict__ partial, int nblocks, int D, E *__restrict__ out0,
+                      E *__restrict__ out1) {
+  __shared__ float part[REDUCE_WARPS][33];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int e = blockIdx.x * 32 + lane;
   const int64_t stride = 2 * (int64_t)D;
   float s = 0.f;
   if (e < 2 * D) {
-    int b = g;
-    for (; b + 24 < nblocks; b += 32) {
-      const float v0 = partial[(int64_t)b * stride + e], v1 = partial[(int64_t)(b + 8) * stride + e];
-      const float v2 = partial[(int64_t)(b + 16) * stride + e], v3 = partial[(int64_t)(b + 24) * stride + e];
-      s += (v0 + v1) + (v2 + v3);
+    for (int b0 = g; b0 < nblocks; b0 += 5 * REDUCE_WARPS) {
+      float v[5];
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        const int b = b0 + i * REDUCE_WARPS;
+        v[i] = b < nblocks ? partial[(int64_t)b * stride + e] : 0.f;
+      }
+      s += ((v[0] + v[1]) + (v[2] + v[3])) + v[4];
     }
-    for (; b < nblocks; b += 8) s += partial[(int64_t)b * stride + e];
   }
   part[g][lane] = s;
   __syncthreads();
-  if (g == 0 && e < 2 * D) {
-    float t = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) t += part[i][lane];
-    if (e < D) {
-      if (out0) out0[e] = from_f32<E>(t);
+  const float t = warp_sum(part[lane][g]);   // warp g adds up column g
+  const int c = blockIdx.x * 32 + g;
+  if (lane == 0 && c < 2 * D) {
+    if (c < D) {
+      if (out0) out0[c] = from_f32<E>(t);
     } else {
-      if (out1) out1[e - D] = from_f32<E>(t);
+      if (out1) out1[c - D] = from_f32<E>(t);
     }
   }
 }
@@ -542,6 +546,35 @@ struct NormMulParams {
 // serves the eight 16-bit elements of a 16-byte vector, and the mask does not depend on the
 // element type or on how rows are spread over threads.
 // ---------------------------------------------------------------------------------------
+// Philox4x32-10 for N counters at once, round by round over all of them.  One call is a chain of ten
+// dependent multiplications and the kernels below run few warps; the round keys are shared as well.
+// Used where it measured faster (rows of 16-bit elements, dropout 0.3, 205 MB a tensor): forward with two
+// vectors per lane (D = 512) 290 -> 270 us, backward with one (D = 256) 480 -> 390 us.  The other forms are
+// bound by instruction issue, not by the chains, and lose by the registers it takes (forward D = 256
+// 304 -> 334, D = 1024 300 -> 390; backward D = 512 412 -> 414, D = 1024 427 -> 445): they go call by call.
+template <int N>
+__device__ __forceinline__ void philox_many(uint32_t k0, uint32_t k1, const uint64_t (&g)[N], uint32_t (&o)[N][4]) {
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    o[n][0] = (uint32_t)g[n];
+    o[n][1] = (uint32_t)(g[n] >> 32);
+    o[n][2] = o[n][3] = 0;
+  }
+#pragma unroll
+  for (int r = 0; r < 10; ++r) {
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      const uint64_t p0 = (uint64_t)0xD2511F53u * o[n][0], p1 = (uint64_t)0xCD9E8D57u * o[n][2];
+      o[n][0] = (uint32_t)(p1 >> 32) ^ o[n][1] ^ k0;
+      o[n][1] = (uint32_t)p1;
+      o[n][2] = (uint32_t)(p0 >> 32) ^ o[n][3] ^ k1;
+      o[n][3] = (uint32_t)p0;
+    }
+    k0 += 0x9E3779B9u;
+    k1 += 0xBB67AE85u;
+  }
+}
+
 struct Dropout {
   uint32_t k0, k1, thr;
   float scale;
@@ -560,15 +593,60 @@ struct Dropout {
     const uint32_t r = (o[j >> 1] >> (16 * (j & 1))) & 0xffffu;
     return r >= thr ? v * scale : 0.f;
   }
+  // one vector of eight elements with the generator's words for it; returns the keep bits
+  __device__ __forceinline__ uint32_t mask8(float (&v)[8], const uint32_t (&o)[4]) const {
+    // two pieces per word: the high one compares in place, the low one after a shift
+    const uint32_t thr_hi = thr << 16;
+    uint32_t kept = 0;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const bool lo = (o[w] << 16) >= thr_hi, hi = o[w] >= thr_hi;
+      v[2 * w] = lo ? v[2 * w] * scale : 0.f;
+      v[2 * w + 1] = hi ? v[2 * w + 1] * scale : 0.f;
+      if (lo) kept |= 1u << (2 * w);
+      if (hi) kept |= 2u << (2 * w);
+    }
+    return kept;
+  }
+  // Two parts of a row at once (rows of whole 8-element vectors): 2 MAXV chains of the generator side
+  // by side.  Vectors beyond the row are masked as well - they are never stored.
+  template <typename E, int MAXV>
+  __device__ __forceinline__ void apply_pair(Row<E, MAXV> &a, uint64_t base_a, Row<E, MAXV> &b, uint64_t base_b,
+                                             int lane) const {
+    uint64_t g[2 * MAXV];
+    uint32_t o[2 * MAXV][4];
+#pragma unroll
+    for (int k = 0; k < MAXV; ++k) {
+      g[2 * k] = (base_a + (uint64_t)((k * 32 + lane) * 8)) >> 3;
+      g[2 * k + 1] = (base_b + (uint64_t)((k * 32 + lane) * 8)) >> 3;
+    }
+    philox_many<2 * MAXV>(k0, k1, g, o);
+#pragma unroll
+    for (int k = 0; k < MAXV; ++k) {
+      mask8(a.v[k], o[2 * k]);
+      mask8(b.v[k], o[2 * k + 1]);
+    }
+  }
   // the D elements of one part of a row, whose first element has index `base` in the output matrix.
   // WHOLE: D is a multiple of the vector width, so that every vector is one aligned group of the
   // generator (no element-wise path in the code at all - it is most of the code otherwise, and these
   // kernels run few enough warps to feel the instruction cache).  STORE (only with WHOLE and 8-element
   // vectors, see norm_mul_mask_bytes): the keep bits of every vector also go to memory, one byte each.
-  template <bool WHOLE, bool STORE, typename E, int MAXV>
+  // JOINT: as apply_pair, the row's vectors side by side.
+  template <bool WHOLE, bool STORE, bool JOINT = false, typename E, int MAXV>
   __device__ __forceinline__ void apply(Row<E, MAXV> &r, uint64_t base, int D, int lane,
                                         uint8_t *mask_out = nullptr) const {
     constexpr int EV = VecInfo<E>::EV;
+    if constexpr (JOINT) {
+      uint64_t g[MAXV];
+      uint32_t o[MAXV][4];
+#pragma unroll
+      for (int k = 0; k < MAXV; ++k) g[k] = (base + (uint64_t)((k * 32 + lane) * 8)) >> 3;
+      philox_many<MAXV>(k0, k1, g, o);
+#pragma unroll
+      for (int k = 0; k < MAXV; ++k) mask8(r.v[k], o[k]);
+      return;
+    }
 #pragma unroll
     for (int k = 0; k < MAXV; ++k) {
       const int e0 = (k * 32 + lane) * EV;
@@ -579,19 +657,7 @@ struct Dropout {
         const uint64_t g = idx0 >> 3;
         philox4x32_10(k0, k1, (uint32_t)g, (uint32_t)(g >> 32), o);
         if constexpr (EV == 8) {
-          // two pieces per word: the high one compares in place, the low one after a shift
-          const uint32_t thr_hi = thr << 16;
-          uint32_t kept = 0;
-#pragma unroll
-          for (int w = 0; w < 4; ++w) {
-            const bool lo = (o[w] << 16) >= thr_hi, hi = o[w] >= thr_hi;
-            r.v[k][2 * w] = lo ? r.v[k][2 * w] * scale : 0.f;
-            r.v[k][2 * w + 1] = hi ? r.v[k][2 * w + 1] * scale : 0.f;
-            if (STORE) {
-              if (lo) kept |= 1u << (2 * w);
-              if (hi) kept |= 2u << (2 * w);
-            }
-          }
+          const uint32_t kept = mask8(r.v[k], o);
           if (STORE) mask_out[g] = (uint8_t)kept;
         } else {
           const int j0 = (int)(idx0 & 7);   // 0, or 4 for the second half of a group of 32-bit elements
@@ -657,6 +723,7 @@ struct MaskBytes {
 template <typename E, int MAXV, int DROPOUT>
 __global__ void __launch_bounds__(WARPS * 32, MAXV <= 2 ? 2 : 0) norm_mul_fwd_kernel(NormMulParams p) {
   constexpr bool WHOLE = DROPOUT >= 2, STORE = DROPOUT == 3 && VecInfo<E>::EV == 8;
+  constexpr bool JOINT = DROPOUT == 2 && VecInfo<E>::EV == 8 && MAXV == 2;
   constexpr int EV = VecInfo<E>::EV;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int D = p.H * p.V;
@@ -700,20 +767,31 @@ __global__ void __launch_bounds__(WARPS * 32, MAXV <= 2 ? 2 : 0) norm_mul_fwd_ke
     E *orow = (E *)p.out + row * p.out_rs;
     const uint64_t rbase = (uint64_t)row * (uint64_t)width;   // index of the row's first element
     int off = 0;
-    if (p.concat_u) {
+    bool paired = false;
+    if constexpr (JOINT) {
+      paired = p.concat_u && p.concat_x;
+      if (paired) {
+        Row<E, MAXV> du_ = ur, dx_ = xr;
+        drop.apply_pair(du_, rbase, dx_, rbase + D, lane);
+        du_.store(orow, D, lane, p.vec_ok);
+        dx_.store(orow + D, D, lane, p.vec_ok);
+        off = 2 * D;
+      }
+    }
+    if (!paired && p.concat_u) {
       if (DROPOUT) {
         Row<E, MAXV> du_ = ur;
-        drop.template apply<WHOLE, STORE>(du_, rbase, D, lane, p.mask);
+        drop.template apply<WHOLE, STORE, JOINT>(du_, rbase, D, lane, p.mask);
         du_.store(orow, D, lane, p.vec_ok);
       } else {
         ur.store(orow, D, lane, p.vec_ok);
       }
       off += D;
     }
-    if (p.concat_x) {
+    if (!paired && p.concat_x) {
       if (DROPOUT) {
         Row<E, MAXV> dx_ = xr;
-        drop.template apply<WHOLE, STORE>(dx_, rbase + off, D, lane, p.mask);
+        drop.template apply<WHOLE, STORE, JOINT>(dx_, rbase + off, D, lane, p.mask);
         dx_.store(orow + off, D, lane, p.vec_ok);
       } else {
         xr.store(orow + off, D, lane, p.vec_ok);
@@ -725,7 +803,7 @@ __global__ void __launch_bounds__(WARPS * 32, MAXV <= 2 ? 2 : 0) norm_mul_fwd_ke
 #pragma unroll
       for (int t = 0; t < EV; ++t)
         xr.v[k][t] = act_f(ur.v[k][t], p.act) * ((xr.v[k][t] - mean) * rstd * wr.v[k][t] + br.v[k][t]);
-    if (DROPOUT) drop.template apply<WHOLE, STORE>(xr, rbase + off, D, lane, p.mask);
+    if (DROPOUT) drop.template apply<WHOLE, STORE, JOINT>(xr, rbase + off, D, lane, p.mask);
     xr.store(orow + off, D, lane, p.vec_ok);
     if (lane == 0) {
       if (p.mean) p.mean[row] = mean;
@@ -836,6 +914,7 @@ template <typename E, int MAXV, int DROPOUT>
 __global__ void __launch_bounds__(WARPS * 32) norm_mul_bwd_kernel(NormMulParams p) {
   constexpr int EV = VecInfo<E>::EV;
   constexpr bool REGEN = DROPOUT == 1 || DROPOUT == 3, WHOLE = DROPOUT == 3;
+  constexpr bool JOINT = WHOLE && EV == 8 && MAXV == 1;   // (see philox_many)
   extern __shared__ float smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int D = p.H * p.V;
@@ -907,7 +986,7 @@ __global__ void __launch_bounds__(WARPS * 32) norm_mul_bwd_kernel(NormMulParams 
     }
     // the forward's mask, regenerated: the gradient of a dropped element is zero, of a kept one scaled
     const uint64_t rbase = (uint64_t)row * (uint64_t)width;
-    if (REGEN) drop.template apply<WHOLE, false>(gy, rbase + off_y, D, lane);
+    if (REGEN) drop.template apply<WHOLE, false, JOINT>(gy, rbase + off_y, D, lane);
     if constexpr (DROPOUT == 2) {
       if (PF && loaded) { if constexpr (PF) cmy.apply(gy, p.drop_scale); }
       else apply_stored_mask(gy, rbase + off_y, D, lane, p.mask, p.drop_scale);
@@ -938,13 +1017,29 @@ __global__ void __launch_bounds__(WARPS * 32) norm_mul_bwd_kernel(NormMulParams 
     for (int k = 0; k < MAXV; ++k)
 #pragma unroll
       for (int t = 0; t < EV; ++t) gy.v[k][t] = (gy.v[k][t] - c2 - xr.v[k][t] * c1) * rstd;
-    if (p.concat_u) {
+    bool paired = false;
+    if constexpr (JOINT) {
+      paired = loaded && p.concat_u && p.concat_x;
+      if (paired) {
+        cgu.unpack(tmp);
+        cgx.unpack(xr);   // (the normalised row is no longer needed)
+        drop.apply_pair(tmp, rbase, xr, rbase + off_x, lane);
+#pragma unroll
+        for (int k = 0; k < MAXV; ++k)
+#pragma unroll
+          for (int t = 0; t < EV; ++t) {
+            ur.v[k][t] += tmp.v[k][t];
+            gy.v[k][t] += xr.v[k][t];
+          }
+      }
+    }
+    if (!paired && p.concat_u) {
       if (loaded) {
         if constexpr (PF) cgu.unpack(tmp);
       } else {
         tmp.load(grow, D, lane, p.vec_ok);
       }
-      if (REGEN) drop.template apply<WHOLE, false>(tmp, rbase, D, lane);
+      if (REGEN) drop.template apply<WHOLE, false, JOINT>(tmp, rbase, D, lane);
       if constexpr (DROPOUT == 2) {
         if (PF && loaded) { if constexpr (PF) cmu.apply(tmp, p.drop_scale); }
         else apply_stored_mask(tmp, rbase, D, lane, p.mask, p.drop_scale);
@@ -954,13 +1049,13 @@ __global__ void __launch_bounds__(WARPS * 32) norm_mul_bwd_kernel(NormMulParams 
 #pragma unroll
         for (int t = 0; t < EV; ++t) ur.v[k][t] += tmp.v[k][t];
     }
-    if (p.concat_x) {
+    if (!paired && p.concat_x) {
       if (loaded) {
         if constexpr (PF) cgx.unpack(tmp);
       } else {
         tmp.load(grow + off_x, D, lane, p.vec_ok);
       }
-      if (REGEN) drop.template apply<WHOLE, false>(tmp, rbase + off_x, D, lane);
+      if (REGEN) drop.template apply<WHOLE, false, JOINT>(tmp, rbase + off_x, D, lane);
       if constexpr (DROPOUT == 2) {
         if (PF && loaded) { if constexpr (PF) cmx.apply(tmp, p.drop_scale); }
         else apply_stored_mask(tmp, rbase + off_x, D, lane, p.mask, p.drop_scale);
@@ -1294,7 +1389,7 @@ int ln_bwd_t(const void *dy, int64_t dy_rs, const void *x, int64_t x_rs, const v
     }
     count_launch();
     B200_CHECK_LAUNCH("layer_norm backward");
-    reduce_partial_kernel<E><<<(2 * D + 31) / 32, 256, 0, st>>>((const float *)partial, grid, D, (E *)dw, (E *)db);
+    reduce_partial_kernel<E><<<(2 * D + 31) / 32, REDUCE_WARPS * 32, 0, st>>>((const float *)partial, grid, D, (E *)dw, (E *)db);
     count_launch();
     B200_CHECK_LAUNCH("layer_norm backward (reduce)");
     return 0;
@@ -1307,7 +1402,7 @@ int ln_bwd_t(const void *dy, int64_t dy_rs, const void *x, int64_t x_rs, const v
   });
   count_launch();
   B200_CHECK_LAUNCH("layer_norm backward");
-  reduce_partial_kernel<E><<<(2 * D + 31) / 32, 256, 0, st>>>((const float *)partial, grid, D, (E *)dw, (E *)db);
+  reduce_partial_kernel<E><<<(2 * D + 31) / 32, REDUCE_WARPS * 32, 0, st>>>((const float *)partial, grid, D, (E *)dw, (E *)db);
   count_launch();
   B200_CHECK_LAUNCH("layer_norm backward (reduce)");
   return 0;
@@ -1416,7 +1511,7 @@ int norm_mul_t(const b200_hstu_norm_mul_args &a, bool bwd, cudaStream_t st) {
     group_norm_mul_kernel<E, true><<<grid, WARPS * 32, smem, st>>>(p);
     count_launch();
     B200_CHECK_LAUNCH("group_norm_mul backward");
-    reduce_partial_kernel<E><<<(2 * a.H + 31) / 32, 256, 0, st>>>(p.partial, grid, a.H, (E *)a.dweight,
+    reduce_partial_kernel<E><<<(2 * a.H + 31) / 32, REDUCE_WARPS * 32, 0, st>>>(p.partial, grid, a.H, (E *)a.dweight,
                                                                     (E *)a.dbias);
     count_launch();
     B200_CHECK_LAUNCH("group_norm_mul backward (reduce)");
@@ -1504,7 +1599,7 @@ int norm_mul_t(const b200_hstu_norm_mul_args &a, bool bwd, cudaStream_t st) {
   }
   count_launch();
   B200_CHECK_LAUNCH("norm_mul backward");
-  reduce_partial_kernel<E><<<(2 * D + 31) / 32, 256, 0, st>>>(p.partial, grid, D, (E *)a.dweight, (E *)a.dbias);
+  reduce_partial_kernel<E><<<(2 * D + 31) / 32, REDUCE_WARPS * 32, 0, st>>>(p.partial, grid, D, (E *)a.dweight, (E *)a.dbias);
   count_launch();
   B200_CHECK_LAUNCH("norm_mul backward (reduce)");
   return 0;
