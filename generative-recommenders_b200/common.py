@@ -3,6 +3,8 @@
 from enum import Enum, unique
 
 import torch
+from torch._C._profiler import _RecordFunctionFast
+from torch.autograd import forward_ad
 
 from . import _cabi
 
@@ -50,8 +52,55 @@ def require_cuda(*tensors) -> None:
             raise RuntimeError("tensors must live on a CUDA device; this library has no CPU path")
 
 
+# The calls of a layer on a small batch are bound by host time, so the helpers below do what the torch
+# functions beside them do without building Python objects on the way (per call: a stream object 6 us,
+# a device context 7 us, a profiler range 18 us, a no-op ``.to`` 1 us, an autograd node about 15 us).
 def stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    index = getattr(device, "index", None)
+    if type(index) is not int:
+        return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(index)
+
+
+class _Nothing:
+    __slots__ = ()
+
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_NOTHING = _Nothing()
+
+
+def on_device(device):
+    """``torch.cuda.device(device)`` around a launch; nothing where that is the thread's device already."""
+    return _NOTHING if device.index == torch._C._cuda_getDevice() else torch.cuda.device(device)
+
+
+def span(name: str):
+    """``record_function(name)`` while a profiler runs, else its light form (other observers see it too)."""
+    if torch.autograd._profiler_enabled():
+        return torch.autograd.profiler.record_function(name)
+    return _RecordFunctionFast(name)
+
+
+def as_dtype(t: torch.Tensor, dtype) -> torch.Tensor:
+    return t if t.dtype is dtype else t.to(dtype)
+
+
+def outside_autograd(*tensors) -> bool:
+    """True where an ``autograd.Function`` would do no more than run its forward: no input asks for a
+    gradient, and there is no forward-mode level, functorch transform, tracer or compiler that has to see
+    the node (or to refuse it)."""
+    if torch.is_grad_enabled():
+        for t in tensors:
+            if t is not None and t.requires_grad:
+                return False
+    return (forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
+            and torch._C._get_tracing_state() is None and not torch.compiler.is_compiling())
 
 
 def last_dim_contiguous(t: torch.Tensor) -> torch.Tensor:

@@ -12,7 +12,8 @@ from typing import Optional
 import torch
 
 from . import _cabi
-from .common import HammerKernel, _require_cuda_backend, dtype_code, last_dim_contiguous, require_cuda, stream_ptr
+from .common import (HammerKernel, _require_cuda_backend, as_dtype, dtype_code, last_dim_contiguous,
+                     on_device, outside_autograd, require_cuda, stream_ptr)
 
 _IMPL = {"auto": _cabi.IMPL_AUTO, "simt": _cabi.IMPL_SIMT, "tcgen05": _cabi.IMPL_TCGEN05}
 _forced_impl = "auto"
@@ -31,7 +32,7 @@ def _i32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     # int32 (flash_common.cpp:460-472).  The kernels read int32.
     if t is None:
         return None
-    return t.to(torch.int32).contiguous()
+    return as_dtype(t, torch.int32).contiguous()
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -86,7 +87,7 @@ def attention_status(a, which: int, device):
     """Status words ``[forward, backward dK/dV, backward dQ]`` of the launches that used the scratch
     in ``a`` (0 = ran to completion, otherwise the id of the wait that gave up); waits for the stream."""
     host = torch.zeros(3, dtype=torch.int32).pin_memory()
-    with torch.cuda.device(device):
+    with on_device(device):
         _cabi.check(_cabi.lib().b200_hstu_attn_status_async(
             a, which, ctypes.cast(host.data_ptr(), ctypes.POINTER(ctypes.c_int32)), stream_ptr(device)),
             "b200_hstu_attn_status_async")
@@ -132,7 +133,7 @@ def hstu_attention_fwd(max_seq_len, alpha, q, k, v, seq_offsets, num_targets, at
     ws = _workspace(a, 2 if plan_for_backward else 0, q.device)  # kept alive until the launch is queued
     if plan_for_backward and ws is not None:
         a.plan_mode = _PLAN_FOR_BACKWARD
-    with torch.cuda.device(q.device):
+    with on_device(q.device):
         _cabi.check(_cabi.lib().b200_hstu_attn_fwd(a, stream_ptr(q.device)), "b200_hstu_attn_fwd")
     if _CHECK_STATUS and ws is not None:
         _raise_on_status(a, 0, q.device, "b200_hstu_attn_fwd")
@@ -167,7 +168,7 @@ def hstu_attention_bwd(dout, max_seq_len, alpha, q, k, v, seq_offsets, num_targe
         a.workspace_bytes = planned_scratch.numel()
     else:
         ws = _workspace(a, 1, q.device)  # noqa: F841
-    with torch.cuda.device(q.device):
+    with on_device(q.device):
         _cabi.check(_cabi.lib().b200_hstu_attn_bwd(a, stream_ptr(q.device)), "b200_hstu_attn_bwd")
     if _CHECK_STATUS and a.workspace:
         _raise_on_status(a, 2 if reuse else 1, q.device, "b200_hstu_attn_bwd")
@@ -291,9 +292,14 @@ def hstu_mha(
             raise TypeError("dropout_seed must be a one-element int64 tensor")
     else:
         dropout_seed = None
-    out = _HstuMhaFunction.apply(q, k, v, seq_offsets, num_targets, attn_scale, bias_by_distance, int(max_seq_len),
-                                 float(alpha), int(max_attn_len), int(contextual_seq_len),
-                                 int(min_full_attn_seq_len), drop, dropout_seed)
+    if outside_autograd(q, k, v, attn_scale, bias_by_distance):
+        out = hstu_attention_fwd(int(max_seq_len), float(alpha), q, k, v, seq_offsets, num_targets, attn_scale,
+                                 int(max_attn_len), int(contextual_seq_len), int(min_full_attn_seq_len),
+                                 bias_by_distance, dropout_pr=drop, dropout_seed=dropout_seed)
+    else:
+        out = _HstuMhaFunction.apply(q, k, v, seq_offsets, num_targets, attn_scale, bias_by_distance,
+                                     int(max_seq_len), float(alpha), int(max_attn_len), int(contextual_seq_len),
+                                     int(min_full_attn_seq_len), drop, dropout_seed)
     return out * 0 if zero_all else out
 
 
@@ -347,6 +353,6 @@ def delta_hstu_mha(
     a.out = out.data_ptr()
     a.o_row_stride, a.o_head_stride = out.stride(0), out.stride(1)
     ws = _workspace(a, 0, q.device)  # noqa: F841  (kept alive until the launch is queued)
-    with torch.cuda.device(q.device):
+    with on_device(q.device):
         _cabi.check(_cabi.lib().b200_hstu_attn_fwd(a, stream_ptr(q.device)), "b200_hstu_attn_fwd (delta)")
     return out

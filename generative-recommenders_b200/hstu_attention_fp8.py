@@ -11,7 +11,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _cabi
-from .common import dtype_code, last_dim_contiguous, require_cuda, stream_ptr
+from .common import dtype_code, last_dim_contiguous, on_device, require_cuda, stream_ptr
 
 BLOCK = 128
 
@@ -39,7 +39,7 @@ def quantize_e4m3_block(x: torch.Tensor, seq_offsets: torch.Tensor,
     x8 = torch.empty((L, H, d), dtype=torch.float8_e4m3fn, device=x.device)
     scale = torch.ones((L // BLOCK + B, H), dtype=torch.float32, device=x.device)
     if L > 0:
-        with torch.cuda.device(x.device):
+        with on_device(x.device):
             _cabi.check(
                 _cabi.lib().b200_hstu_quantize_e4m3_block(
                     x.data_ptr(), dtype_code(x), x.stride(0), x.stride(1), x8.data_ptr(), scale.data_ptr(),
@@ -96,6 +96,6 @@ def hstu_mha_fp8(
     a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
     fa.q_scale, fa.k_scale, fa.v_scale = q_scale.data_ptr(), k_scale.data_ptr(), v_scale.data_ptr()
     fa.block_offsets = block_offsets.to(torch.int32).contiguous().data_ptr()
-    with torch.cuda.device(q8.device):
+    with on_device(q8.device):
         _cabi.check(_cabi.lib().b200_hstu_attn_fwd_fp8(fa, stream_ptr(q8.device)), "b200_hstu_attn_fwd_fp8")
     return out

@@ -7,7 +7,8 @@ from typing import Optional, Tuple
 import torch
 
 from . import _cabi
-from .common import HammerKernel, _require_cuda_backend, dtype_code, require_cuda, stream_ptr
+from .common import (HammerKernel, _require_cuda_backend, as_dtype, dtype_code, on_device, outside_autograd,
+                     require_cuda, stream_ptr)
 from .hstu_attention import hstu_mha
 from .layer_norm import layer_norm
 from .mm import addmm
@@ -23,7 +24,7 @@ class _SiluColumnsFunction(torch.autograd.Function):
         rows = x.shape[0]
         u = torch.empty((rows, width), dtype=x.dtype, device=x.device)
         if rows > 0:
-            with torch.cuda.device(x.device):
+            with on_device(x.device):
                 _cabi.check(
                     _cabi.lib().b200_hstu_silu_fwd(x.data_ptr(), x.stride(0), u.data_ptr(), u.stride(0), rows, width,
                                                    dtype_code(x), stream_ptr(x.device)),
@@ -40,7 +41,7 @@ class _SiluColumnsFunction(torch.autograd.Function):
             du = du.contiguous()
         dx = torch.zeros_like(x) if x.shape[1] != width else torch.empty_like(x)
         if rows > 0:
-            with torch.cuda.device(x.device):
+            with on_device(x.device):
                 _cabi.check(
                     _cabi.lib().b200_hstu_silu_bwd(du.data_ptr(), du.stride(0), x.data_ptr(), x.stride(0),
                                                    dx.data_ptr(), dx.stride(0), rows, width, dtype_code(x),
@@ -99,7 +100,7 @@ def _prepared_workspace(nw, nb, w, b, nbytes, device, allow_cache):
             or not all(isinstance(t, torch.nn.Parameter) for t in (w, nw, nb, b))):
         return torch.empty(nbytes, dtype=torch.uint8, device=device), False
     key = id(w)
-    stream = torch.cuda.current_stream(device).cuda_stream
+    stream = stream_ptr(device)
     sig = tuple((id(t), t.data_ptr(), t._version) for t in (w, nw, nb, b)) + (stream,)
     hit = _PREPARED.get(key)
     # the workspace was prepared on `stream`; a call on another stream is not ordered after that
@@ -113,14 +114,15 @@ def _prepared_workspace(nw, nb, w, b, nbytes, device, allow_cache):
     return ws, False
 
 
-def _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, allow_cache=False):
-    """One launch of the fused kernel: returns (uvqk [M, N], u [M, hv], mean [M], rstd [M])."""
+def _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, allow_cache=False, stats=True):
+    """One launch of the fused kernel: returns (uvqk [M, N], u [M, hv], mean [M], rstd [M]); without
+    ``stats`` the last two are None."""
     M, D = x.shape
     N = w.shape[1]
     uvqk = torch.empty((M, N), dtype=x.dtype, device=x.device)
     u = torch.empty((M, hv), dtype=x.dtype, device=x.device)
-    mean = torch.empty(M, dtype=torch.float32, device=x.device)
-    rstd = torch.empty(M, dtype=torch.float32, device=x.device)
+    mean = torch.empty(M, dtype=torch.float32, device=x.device) if stats else None
+    rstd = torch.empty(M, dtype=torch.float32, device=x.device) if stats else None
     nbytes = _cabi.lib().b200_hstu_ln_linear_workspace_bytes(D, N)
     ws, prepared = _prepared_workspace(nw, nb, w, b, nbytes, x.device, allow_cache)
     a = _cabi.LnLinearArgs()
@@ -128,12 +130,14 @@ def _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, allow_cache=False):
     a.skip_pre_activation = 1 if allow_cache else 0   # no gradient wanted: nobody reads the pre-activation u
     a.x, a.norm_weight, a.norm_bias, a.weight, a.bias = (x.data_ptr(), nw.data_ptr(), nb.data_ptr(),
                                                           w.data_ptr(), b.data_ptr())
-    a.out, a.u, a.mean, a.rstd = uvqk.data_ptr(), u.data_ptr(), mean.data_ptr(), rstd.data_ptr()
+    a.out, a.u = uvqk.data_ptr(), u.data_ptr()
+    if stats:
+        a.mean, a.rstd = mean.data_ptr(), rstd.data_ptr()
     a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
     a.x_row_stride, a.out_row_stride, a.u_row_stride = x.stride(0), uvqk.stride(0), u.stride(0)
     a.M, a.D, a.N, a.silu_cols = M, D, N, hv
     a.eps, a.dtype = eps, dtype_code(x)
-    with torch.cuda.device(x.device):
+    with on_device(x.device):
         _cabi.check(_cabi.lib().b200_hstu_ln_linear_silu_fwd(a, stream_ptr(x.device)),
                     "b200_hstu_ln_linear_silu_fwd")
     return uvqk, u, mean, rstd
@@ -149,7 +153,7 @@ def _fused_uqvk_backward(x, nw, nb, w, uvqk, mean, rstd, eps, hv, du, d_uvqk):
     lib = _cabi.lib()
     dt = dtype_code(x)
     st = stream_ptr(x.device)
-    with torch.cuda.device(x.device):
+    with on_device(x.device):
         if du is not None:
             if du.stride(-1) != 1:
                 du = du.contiguous()
@@ -179,6 +183,23 @@ def _fused_uqvk_backward(x, nw, nb, w, uvqk, mean, rstd, eps, hv, du, d_uvqk):
     return dx, dnw, dnb, dw, db
 
 
+def _uqvk_views(uvqk, num_heads, attn_dim, hidden_dim):
+    """(q, k, v) as ``[M, H, d]`` views of the uvqk buffer."""
+    hv, ha = hidden_dim * num_heads, attn_dim * num_heads
+    v, q, k = uvqk[:, hv:].split_with_sizes((hv, ha, ha), 1)
+    return (q.unflatten(1, (num_heads, attn_dim)), k.unflatten(1, (num_heads, attn_dim)),
+            v.unflatten(1, (num_heads, hidden_dim)))
+
+
+def _fused_uqvk_inference(x, norm_weight, norm_bias, eps, weight, bias, num_heads, attn_dim, hidden_dim):
+    """The fused stage where no gradient is wanted: ``(u, q, k, v)``."""
+    uvqk, u, _, _ = _fused_uqvk_launch(
+        x, as_dtype(norm_weight, x.dtype).contiguous(), as_dtype(norm_bias, x.dtype).contiguous(), eps,
+        _aligned16(as_dtype(weight, x.dtype).contiguous()), as_dtype(bias, x.dtype).contiguous(),
+        hidden_dim * num_heads, True, stats=False)
+    return (u,) + _uqvk_views(uvqk, num_heads, attn_dim, hidden_dim)
+
+
 class _FusedUqvkFunction(torch.autograd.Function):
     """``uvqk = LN(x) W + b`` and ``u = SiLU(uvqk[:, :hv])`` from one tensor-core kernel
     (csrc/ln_linear_sm100.cu)."""
@@ -187,10 +208,10 @@ class _FusedUqvkFunction(torch.autograd.Function):
     def forward(ctx, x, norm_weight, norm_bias, eps, weight, bias, num_heads, attn_dim, hidden_dim, grad_mode=True):
         M = x.shape[0]
         hv, ha = hidden_dim * num_heads, attn_dim * num_heads
-        nw = norm_weight.to(x.dtype).contiguous()
-        nb = norm_bias.to(x.dtype).contiguous()
-        w = _aligned16(weight.to(x.dtype).contiguous())
-        b = bias.to(x.dtype).contiguous()
+        nw = as_dtype(norm_weight, x.dtype).contiguous()
+        nb = as_dtype(norm_bias, x.dtype).contiguous()
+        w = _aligned16(as_dtype(weight, x.dtype).contiguous())
+        b = as_dtype(bias, x.dtype).contiguous()
         no_grad = not (grad_mode and any(ctx.needs_input_grad))
         uvqk, u, mean, rstd = _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, no_grad)
         ctx.set_materialize_grads(False)
@@ -215,7 +236,8 @@ class _FusedUqvkFunction(torch.autograd.Function):
             else:
                 d_uvqk[:, lo:lo + width].copy_(g.reshape(M, width))
         dx, dnw, dnb, dw, db = _fused_uqvk_backward(x, nw, nb, w, uvqk, mean, rstd, eps, hv, du, d_uvqk)
-        return dx, dnw.to(nw_dtype), dnb.to(nb_dtype), None, dw.to(w_dtype), db.to(b_dtype), None, None, None, None
+        return (dx, as_dtype(dnw, nw_dtype), as_dtype(dnb, nb_dtype), None, as_dtype(dw, w_dtype),
+                as_dtype(db, b_dtype), None, None, None, None)
 
 
 class _FusedPreprocessAttentionFunction(torch.autograd.Function):
@@ -231,10 +253,10 @@ class _FusedPreprocessAttentionFunction(torch.autograd.Function):
 
         M = x.shape[0]
         hv, ha = hidden_dim * num_heads, attn_dim * num_heads
-        nw = norm_weight.to(x.dtype).contiguous()
-        nb = norm_bias.to(x.dtype).contiguous()
-        w = _aligned16(weight.to(x.dtype).contiguous())
-        b = bias.to(x.dtype).contiguous()
+        nw = as_dtype(norm_weight, x.dtype).contiguous()
+        nb = as_dtype(norm_bias, x.dtype).contiguous()
+        w = _aligned16(as_dtype(weight, x.dtype).contiguous())
+        b = as_dtype(bias, x.dtype).contiguous()
         no_grad = not (grad_mode and any(ctx.needs_input_grad))
         uvqk, u, mean, rstd = _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, no_grad)
         v = uvqk[:, hv:2 * hv].view(M, num_heads, hidden_dim)
@@ -294,8 +316,8 @@ class _FusedPreprocessAttentionFunction(torch.autograd.Function):
         if dv_ext is not None:
             dv.add_(dv_ext)
         dx, dnw, dnb, dw, db = _fused_uqvk_backward(x, nw, nb, w, uvqk, mean, rstd, eps, hv, du, d_uvqk)
-        return (dx, dnw.to(nw_dtype), dnb.to(nb_dtype), None, dw.to(w_dtype), db.to(b_dtype), None, None, None,
-                None, None, d_bias, None, None, None, None, None, None)
+        return (dx, as_dtype(dnw, nw_dtype), as_dtype(dnb, nb_dtype), None, as_dtype(dw, w_dtype),
+                as_dtype(db, b_dtype), None, None, None, None, None, d_bias, None, None, None, None, None, None)
 
 
 _FUSED_UQVK = True
@@ -326,6 +348,9 @@ def hstu_compute_uqvk(
     require_cuda(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias)
     hv, ha = hidden_dim * num_heads, attn_dim * num_heads
     if _FUSED_UQVK and _fused_uqvk_supported(x, uvqk_weight, hv):
+        if outside_autograd(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias):
+            return _fused_uqvk_inference(x, norm_weight, norm_bias, float(norm_eps), uvqk_weight, uvqk_bias,
+                                         num_heads, attn_dim, hidden_dim)
         return _FusedUqvkFunction.apply(x, norm_weight, norm_bias, float(norm_eps), uvqk_weight, uvqk_bias,
                                         num_heads, attn_dim, hidden_dim, torch.is_grad_enabled())
     else:
@@ -339,9 +364,10 @@ def hstu_compute_uqvk(
 
 
 def _norm_mul_forward(attn, u, weight, bias, eps, num_heads, linear_dim, concat_u, concat_x, act, group_norm,
-                      dropout_ratio, dropout_seed, want_mask=False):
+                      dropout_ratio, dropout_seed, want_mask=False, stats=True):
     """One launch of the norm-mul kernel; returns ``(out, mean, rstd)`` (inputs already contiguous in
-    their last dimension, weight / bias already of the activation dtype)."""
+    their last dimension, weight / bias already of the activation dtype); without ``stats`` the last two
+    are None."""
     rows = attn.shape[0]
     D = num_heads * linear_dim
     if group_norm:
@@ -350,11 +376,13 @@ def _norm_mul_forward(attn, u, weight, bias, eps, num_heads, linear_dim, concat_
         mult = 1 + int(concat_u) + int(concat_x)
     out = torch.empty((rows, mult * D), dtype=attn.dtype, device=attn.device)
     groups = num_heads if group_norm else 1
-    mean = torch.empty(rows * groups, dtype=torch.float32, device=attn.device)
-    rstd = torch.empty(rows * groups, dtype=torch.float32, device=attn.device)
+    mean = torch.empty(rows * groups, dtype=torch.float32, device=attn.device) if stats else None
+    rstd = torch.empty(rows * groups, dtype=torch.float32, device=attn.device) if stats else None
     a = _cabi.NormMulArgs()
     a.attn, a.u, a.weight, a.bias = attn.data_ptr(), u.data_ptr(), weight.data_ptr(), bias.data_ptr()
-    a.out, a.mean, a.rstd = out.data_ptr(), mean.data_ptr(), rstd.data_ptr()
+    a.out = out.data_ptr()
+    if stats:
+        a.mean, a.rstd = mean.data_ptr(), rstd.data_ptr()
     a.attn_row_stride, a.u_row_stride, a.out_row_stride = attn.stride(0), u.stride(0), out.stride(0)
     a.rows, a.H, a.V = rows, num_heads, linear_dim
     a.concat_u, a.concat_x, a.act, a.group_norm = int(concat_u), int(concat_x), act, int(group_norm)
@@ -370,7 +398,7 @@ def _norm_mul_forward(attn, u, weight, bias, eps, num_heads, linear_dim, concat_
                 mask = torch.empty(nbytes, dtype=torch.uint8, device=attn.device)
                 a.dropout_mask = mask.data_ptr()
     if rows > 0:
-        with torch.cuda.device(attn.device):
+        with on_device(attn.device):
             _cabi.check(_cabi.lib().b200_hstu_norm_mul_fwd(a, stream_ptr(attn.device)), "b200_hstu_norm_mul_fwd")
     if want_mask:
         return out, mean, rstd, mask
@@ -405,7 +433,7 @@ def _norm_mul_backward(dout, attn, u, weight, bias, mean, rstd, eps, num_heads, 
         a.dropout_ratio, a.dropout_seed = dropout_ratio, dropout_seed.data_ptr()
         if dropout_mask is not None and dout.data_ptr() % 16 == 0 and dout.stride(0) % 8 == 0:
             a.dropout_mask = dropout_mask.data_ptr()
-    with torch.cuda.device(attn.device):
+    with on_device(attn.device):
         _cabi.check(_cabi.lib().b200_hstu_norm_mul_bwd(a, stream_ptr(attn.device)), "b200_hstu_norm_mul_bwd")
     return dattn, du, dw, db
 
@@ -431,8 +459,8 @@ class _NormMulFunction(torch.autograd.Function):
             attn = attn.contiguous()
         if u.stride(-1) != 1:
             u = u.contiguous()
-        weight = weight.to(attn.dtype).contiguous()
-        bias = bias.to(attn.dtype).contiguous()
+        weight = as_dtype(weight, attn.dtype).contiguous()
+        bias = as_dtype(bias, attn.dtype).contiguous()
         keep_mask = _STORE_DROPOUT_MASK and any(ctx.needs_input_grad)   # (grad mode is off inside forward())
         out, mean, rstd, mask = _norm_mul_forward(attn, u, weight, bias, eps, num_heads, linear_dim, concat_u, concat_x,
                                                   act, group_norm, dropout_ratio, dropout_seed, want_mask=True) \
@@ -464,9 +492,9 @@ class _OutputStageFunction(torch.autograd.Function):
             attn = attn.contiguous()
         if u.stride(-1) != 1:
             u = u.contiguous()
-        w = weight.to(attn.dtype).contiguous()
-        b = bias.to(attn.dtype).contiguous()
-        wo = output_weight.to(x.dtype)
+        w = as_dtype(weight, attn.dtype).contiguous()
+        b = as_dtype(bias, attn.dtype).contiguous()
+        wo = as_dtype(output_weight, x.dtype)
         cfg = (eps, num_heads, linear_dim, concat_u, concat_x, act, group_norm, dropout_ratio)
         y, mean, rstd = _norm_mul_forward(attn, u, w, b, *cfg, dropout_seed)
         out = torch.addmm(x, y, wo)
@@ -486,8 +514,8 @@ class _OutputStageFunction(torch.autograd.Function):
         dy = dout @ wo.t()
         dattn, du, dw, db = _norm_mul_backward(dy, attn, u, w, b, mean, rstd, *ctx.cfg, dropout_seed)
         wdt, bdt, odt = ctx.dtypes
-        return (dattn, du, dout, dw.to(wdt), db.to(bdt), d_wo.to(odt), None, None, None, None, None, None, None, None,
-                None)
+        return (dattn, du, dout, as_dtype(dw, wdt), as_dtype(db, bdt), as_dtype(d_wo, odt), None, None, None, None,
+                None, None, None, None, None)
 
 
 def _draw_dropout_seed(device) -> torch.Tensor:
@@ -532,9 +560,15 @@ def hstu_norm_mul_dropout(
     fused_drop = drop and not group_norm and dropout_ratio < 1.0
     if fused_drop and dropout_seed is None:
         dropout_seed = _draw_dropout_seed(attn.device)
-    y = _NormMulFunction.apply(attn, u, norm_weight, norm_bias, float(norm_eps), int(num_heads), int(linear_dim),
-                               bool(concat_u), bool(concat_x), act, bool(group_norm),
-                               float(dropout_ratio) if fused_drop else 0.0, dropout_seed if fused_drop else None)
+    cfg = (float(norm_eps), int(num_heads), int(linear_dim), bool(concat_u), bool(concat_x), act, bool(group_norm),
+           float(dropout_ratio) if fused_drop else 0.0, dropout_seed if fused_drop else None)
+    if not group_norm and outside_autograd(attn, u, norm_weight, norm_bias):
+        y, _, _ = _norm_mul_forward(
+            attn if attn.stride(-1) == 1 else attn.contiguous(), u if u.stride(-1) == 1 else u.contiguous(),
+            as_dtype(norm_weight, attn.dtype).contiguous(), as_dtype(norm_bias, attn.dtype).contiguous(), *cfg,
+            stats=False)
+    else:
+        y = _NormMulFunction.apply(attn, u, norm_weight, norm_bias, *cfg)
     if drop and not fused_drop:
         y = torch.nn.functional.dropout(y, p=dropout_ratio, training=True)
     return y
@@ -580,7 +614,7 @@ def hstu_compute_output(
                                               g_, float(dropout_ratio) if seed is not None else 0.0, seed)
     y = hstu_norm_mul_dropout(attn, u, norm_weight, norm_bias, norm_eps, dropout_ratio, training, concat_u, concat_x,
                               mul_u_activation_type, group_norm, num_heads, linear_dim)
-    return addmm(x, y, output_weight.to(x.dtype), kernel)
+    return addmm(x, y, as_dtype(output_weight, x.dtype), kernel)
 
 
 def hstu_preprocess_and_attention(
@@ -631,6 +665,13 @@ def hstu_preprocess_and_attention(
         if nt is not None and nt.numel() != offs.numel() - 1:
             raise RuntimeError("num_targets must have one entry per sequence")
         rab = None if bias_by_distance is None else bias_by_distance.to(torch.float32).reshape(-1).contiguous()
+        if outside_autograd(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias, rab):
+            from .hstu_attention import hstu_attention_fwd
+            u, q, k, v = _fused_uqvk_inference(x, norm_weight, norm_bias, float(norm_eps), uvqk_weight, uvqk_bias,
+                                               num_heads, attn_dim, hidden_dim)
+            attn = hstu_attention_fwd(int(max_seq_len), float(attn_alpha), q, k, v, offs, nt, None,
+                                      int(max_attn_len), int(contextual_seq_len), 0, rab)
+            return u, attn.view(-1, hv), k, v
         u, attn, k, v = _FusedPreprocessAttentionFunction.apply(
             x, norm_weight, norm_bias, float(norm_eps), uvqk_weight, uvqk_bias, num_heads, attn_dim, hidden_dim,
             offs, nt, rab, int(max_seq_len), float(attn_alpha), int(max_attn_len), int(contextual_seq_len),

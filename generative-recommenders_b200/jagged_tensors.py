@@ -13,7 +13,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _cabi
-from .common import HammerKernel, _require_cuda_backend, require_cuda, stream_ptr
+from .common import HammerKernel, _require_cuda_backend, on_device, outside_autograd, require_cuda, stream_ptr
 
 
 def _offsets_arg(off: Optional[torch.Tensor], device) -> Optional[torch.Tensor]:
@@ -41,18 +41,23 @@ def _run(split: bool, left, right, combined, off_l, off_r, dense_l, dense_r, B, 
         return
     a = _args(left, right, combined, off_l, off_r, dense_l, dense_r, B, shift)
     fn = _cabi.lib().b200_hstu_split_2d_jagged if split else _cabi.lib().b200_hstu_concat_2d_jagged
-    with torch.cuda.device(combined.device):
+    with on_device(combined.device):
         _cabi.check(fn(a, stream_ptr(combined.device)),
                     "b200_hstu_split_2d_jagged" if split else "b200_hstu_concat_2d_jagged")
+
+
+def _concat(left, right, off_l, off_r, dense_l, dense_r, B, shift=0):
+    left = left.contiguous()
+    right = right.contiguous()
+    out = torch.empty((left.shape[0] + right.shape[0], left.shape[1]), dtype=left.dtype, device=left.device)
+    _run(False, left, right, out, off_l, off_r, dense_l, dense_r, B, shift)
+    return out
 
 
 class _Concat2DJagged(torch.autograd.Function):
     @staticmethod
     def forward(ctx, left, right, off_l, off_r, dense_l, dense_r, B, shift=0):
-        left = left.contiguous()
-        right = right.contiguous()
-        out = torch.empty((left.shape[0] + right.shape[0], left.shape[1]), dtype=left.dtype, device=left.device)
-        _run(False, left, right, out, off_l, off_r, dense_l, dense_r, B, shift)
+        out = _concat(left, right, off_l, off_r, dense_l, dense_r, B, shift)
         ctx.meta = (off_l, off_r, dense_l, dense_r, B, left.shape[0], right.shape[0], shift)
         return out
 
@@ -126,9 +131,9 @@ def concat_2D_jagged(
             B = values_right.shape[0] // max_len_right
     else:
         torch._assert(off_r.numel() - 1 == B, "offsets_left and offsets_right must describe the same batch")
-    return _Concat2DJagged.apply(values_left, values_right, off_l, off_r,
-                                 max_len_left if off_l is None else 0,
-                                 max_len_right if off_r is None else 0, B)
+    run = _concat if outside_autograd(values_left, values_right) else _Concat2DJagged.apply
+    return run(values_left, values_right, off_l, off_r, max_len_left if off_l is None else 0,
+               max_len_right if off_r is None else 0, B)
 
 
 def split_2D_jagged(

@@ -5,7 +5,7 @@ generative_recommenders/ops/pytorch/pt_layer_norm.py:24-38 does)."""
 import torch
 
 from . import _cabi
-from .common import HammerKernel, _require_cuda_backend, dtype_code, require_cuda, stream_ptr
+from .common import HammerKernel, _require_cuda_backend, dtype_code, on_device, require_cuda, stream_ptr
 
 
 def _rows2d(x: torch.Tensor) -> torch.Tensor:
@@ -26,7 +26,7 @@ class _LayerNormFunction(torch.autograd.Function):
         mean = torch.empty(rows, dtype=torch.float32, device=x.device)
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
         if rows > 0:
-            with torch.cuda.device(x.device):
+            with on_device(x.device):
                 _cabi.check(
                     _cabi.lib().b200_hstu_layer_norm_fwd(
                         x2.data_ptr(), x2.stride(0), weight.data_ptr(), bias.data_ptr(), y.data_ptr(), y.stride(0),
@@ -46,7 +46,7 @@ class _LayerNormFunction(torch.autograd.Function):
         db = torch.empty(D, dtype=x2.dtype, device=x2.device)
         nbytes = _cabi.lib().b200_hstu_layer_norm_bwd_workspace_bytes(D)
         partial = torch.empty(nbytes, dtype=torch.uint8, device=x2.device)
-        with torch.cuda.device(x2.device):
+        with on_device(x2.device):
             _cabi.check(
                 _cabi.lib().b200_hstu_layer_norm_bwd(
                     dy2.data_ptr(), dy2.stride(0), x2.data_ptr(), x2.stride(0), weight.data_ptr(), mean.data_ptr(),

@@ -13,7 +13,7 @@ from typing import Optional
 import torch
 
 from . import _cabi
-from .common import HammerKernel, _require_cuda_backend, dtype_code, require_cuda, stream_ptr
+from .common import HammerKernel, _require_cuda_backend, dtype_code, on_device, require_cuda, stream_ptr
 
 
 def _fill(a, seq_offsets, seq_lengths, num_targets, timestamps, total, D, pos_w, ts_w, max_contextual_seq_len,
@@ -51,7 +51,7 @@ class _AddTimestampPositionalEmbeddings(torch.autograd.Function):
               _cabi.F32 if table_dtype == torch.float32 else dtype_code(x))
         a.seq_embeddings, a.pos_weight, a.ts_weight, a.out = x.data_ptr(), pw.data_ptr(), tw.data_ptr(), out.data_ptr()
         if x.shape[0] > 0:
-            with torch.cuda.device(x.device):
+            with on_device(x.device):
                 _cabi.check(_cabi.lib().b200_hstu_add_timestamp_positional_embeddings_fwd(a, stream_ptr(x.device)),
                             "b200_hstu_add_timestamp_positional_embeddings_fwd")
         ctx.save_for_backward(seq_offsets, seq_lengths, num_targets, timestamps)
@@ -73,7 +73,7 @@ class _AddTimestampPositionalEmbeddings(torch.autograd.Function):
         a.d_out, a.d_seq_embeddings = d_out.data_ptr(), dx.data_ptr()
         a.d_pos_weight, a.d_ts_weight = d_pos.data_ptr(), d_ts.data_ptr()
         if d_out.shape[0] > 0:
-            with torch.cuda.device(d_out.device):
+            with on_device(d_out.device):
                 _cabi.check(_cabi.lib().b200_hstu_add_timestamp_positional_embeddings_bwd(a, stream_ptr(d_out.device)),
                             "b200_hstu_add_timestamp_positional_embeddings_bwd")
         return (dx, d_pos.to(pos_dtype), d_ts.to(ts_dtype), None, None, None, None, None, None, None, None)

@@ -22,7 +22,7 @@ from typing import List, Optional
 
 import torch
 
-from .common import HammerKernel
+from .common import HammerKernel, as_dtype, span
 from .hstu_attention import delta_hstu_mha
 from .hstu_compute import hstu_compute_output, hstu_compute_uqvk, hstu_preprocess_and_attention
 from .jagged_tensors import concat_2D_jagged, split_2D_jagged
@@ -168,7 +168,9 @@ class STULayer(torch.nn.Module):
                                          values_right=delta, max_len_left=self.max_kv_caching_len,
                                          max_len_right=delta_size, offsets_left=self.kv_caching_offsets,
                                          offsets_right=None, kernel=self._hammer_kernel))
-        offsets = self.kv_caching_offsets + delta_size * torch.arange(B + 1, device=delta_k.device)
+        offsets = self.kv_caching_offsets
+        if delta_size > 0:
+            offsets = offsets + torch.arange(0, delta_size * (B + 1), delta_size, device=delta_k.device)
         return full[0], full[1], self.max_kv_caching_len + delta_size, offsets
 
     def cached_forward(
@@ -182,17 +184,17 @@ class STULayer(torch.nn.Module):
         (reference stu.py:358-424); ``delta_x`` is ``[B * delta_size, D]``."""
         if self._rel_bias_table is not None:
             raise NotImplementedError("cached_forward with a relative bias table")
-        with torch.autograd.profiler.record_function("## stu_compute_uqvk ##"):
+        with span("## stu_compute_uqvk ##"):
             delta_u, delta_q, delta_k, delta_v = hstu_compute_uqvk(
                 x=delta_x,
-                norm_weight=self._input_norm_weight.to(delta_x.dtype),
-                norm_bias=self._input_norm_bias.to(delta_x.dtype),
+                norm_weight=as_dtype(self._input_norm_weight, delta_x.dtype),
+                norm_bias=as_dtype(self._input_norm_bias, delta_x.dtype),
                 norm_eps=1e-6,
                 num_heads=self._num_heads,
                 attn_dim=self._attention_dim,
                 hidden_dim=self._hidden_dim,
-                uvqk_weight=self._uvqk_weight.to(delta_x.dtype),
-                uvqk_bias=self._uvqk_beta.to(delta_x.dtype),
+                uvqk_weight=as_dtype(self._uvqk_weight, delta_x.dtype),
+                uvqk_bias=as_dtype(self._uvqk_beta, delta_x.dtype),
                 kernel=self._hammer_kernel,
             )
         k, v, max_seq_len, seq_offsets = self.construct_full_kv(
@@ -201,7 +203,7 @@ class STULayer(torch.nn.Module):
         v = v.view(-1, self._num_heads, self._hidden_dim)
         self.update_kv_cache(max_seq_len=max_seq_len, seq_offsets=seq_offsets, k=k, v=v,
                              max_kv_caching_len=max_kv_caching_len, kv_caching_lengths=kv_caching_lengths)
-        with torch.autograd.profiler.record_function("## delta_hstu_mha ##"):
+        with span("## delta_hstu_mha ##"):
             delta_attn_output = delta_hstu_mha(
                 max_seq_len=max_seq_len,
                 alpha=self._attn_alpha,
@@ -214,16 +216,16 @@ class STULayer(torch.nn.Module):
                 contextual_seq_len=self._contextual_seq_len,
                 kernel=self._hammer_kernel,
             ).view(-1, self._hidden_dim * self._num_heads)
-        with torch.autograd.profiler.record_function("## stu_compute_output ##"):
+        with span("## stu_compute_output ##"):
             return hstu_compute_output(
                 attn=delta_attn_output,
                 u=delta_u,
                 x=delta_x,
-                norm_weight=self._output_norm_weight.to(delta_x.dtype),
-                norm_bias=self._output_norm_bias.to(delta_x.dtype),
+                norm_weight=as_dtype(self._output_norm_weight, delta_x.dtype),
+                norm_bias=as_dtype(self._output_norm_bias, delta_x.dtype),
                 norm_eps=1e-6,
                 dropout_ratio=self._output_dropout_ratio,
-                output_weight=self._output_weight.to(delta_x.dtype),
+                output_weight=as_dtype(self._output_weight, delta_x.dtype),
                 group_norm=self._use_group_norm,
                 num_heads=self._num_heads,
                 linear_dim=self._hidden_dim,
@@ -248,17 +250,17 @@ class STULayer(torch.nn.Module):
         bias = None
         if self._rel_bias_table is not None:
             bias = position_bias_by_distance(self._rel_bias_table, max_seq_len)
-        with torch.autograd.profiler.record_function("## stu_preprocess_and_attention ##"):
+        with span("## stu_preprocess_and_attention ##"):
             u, attn_output, k, v = hstu_preprocess_and_attention(
                 x=x,
-                norm_weight=self._input_norm_weight.to(x.dtype),
-                norm_bias=self._input_norm_bias.to(x.dtype),
+                norm_weight=as_dtype(self._input_norm_weight, x.dtype),
+                norm_bias=as_dtype(self._input_norm_bias, x.dtype),
                 norm_eps=1e-6,
                 num_heads=self._num_heads,
                 attn_dim=self._attention_dim,
                 hidden_dim=self._hidden_dim,
-                uvqk_weight=self._uvqk_weight.to(x.dtype),
-                uvqk_bias=self._uvqk_beta.to(x.dtype),
+                uvqk_weight=as_dtype(self._uvqk_weight, x.dtype),
+                uvqk_bias=as_dtype(self._uvqk_beta, x.dtype),
                 max_seq_len=max_seq_len,
                 seq_offsets=x_offsets,
                 attn_alpha=self._attn_alpha,
@@ -274,16 +276,16 @@ class STULayer(torch.nn.Module):
             )
         self.update_kv_cache(max_seq_len=max_seq_len, seq_offsets=x_offsets, k=k, v=v,
                              max_kv_caching_len=max_kv_caching_len, kv_caching_lengths=kv_caching_lengths)
-        with torch.autograd.profiler.record_function("## stu_compute_output ##"):
+        with span("## stu_compute_output ##"):
             return hstu_compute_output(
                 attn=attn_output,
                 u=u,
                 x=x,
-                norm_weight=self._output_norm_weight.to(x.dtype),
-                norm_bias=self._output_norm_bias.to(x.dtype),
+                norm_weight=as_dtype(self._output_norm_weight, x.dtype),
+                norm_bias=as_dtype(self._output_norm_bias, x.dtype),
                 norm_eps=1e-6,
                 dropout_ratio=self._output_dropout_ratio,
-                output_weight=self._output_weight.to(x.dtype),
+                output_weight=as_dtype(self._output_weight, x.dtype),
                 group_norm=self._use_group_norm,
                 num_heads=self._num_heads,
                 linear_dim=self._hidden_dim,

@@ -237,3 +237,27 @@ def test_recompute_flags_change_memory_not_results():
     assert float((res[True][0] == res[False][0]).float().mean()) == 1.0
     # per layer the projection (2048 columns) and the concat (1536) go, of ~7 D columns kept otherwise
     assert held[True] < 0.7 * held[False], held
+
+
+def test_calls_without_gradients_equal_the_autograd_path():
+    # where no gradient is asked for the ops run without an autograd node: same numbers as the nodes'
+    # forward, and an input with a forward-mode tangent is refused as by the node, not passed through
+    import torch.autograd.forward_ad as fwad
+
+    g = torch.Generator().manual_seed(3)
+    lengths = torch.tensor([130, 1, 64, 257]).cuda()
+    offs = torch.cat([lengths.new_zeros(1), torch.cumsum(lengths, 0)])
+    nt = torch.tensor([5, 0, 1, 20]).cuda()
+    x = torch.randn(int(lengths.sum()), 256, generator=g).bfloat16().cuda()
+    torch.manual_seed(0)
+    layer = G.STULayer(G.STULayerConfig(embedding_dim=256, num_heads=2, hidden_dim=64, attention_dim=64,
+                                        contextual_seq_len=1)).cuda().bfloat16().eval()
+    with torch.no_grad():
+        plain = layer(x, lengths, offs, 300, nt)
+    node = layer(x.requires_grad_(), lengths, offs, 300, nt)
+    assert torch.equal(plain, node.detach())
+    q, k, v = (torch.randn(x.shape[0], 2, 64, generator=g).bfloat16().cuda() for _ in range(3))
+    with fwad.dual_level():
+        dual = fwad.make_dual(q, torch.ones_like(q))
+        with pytest.raises(Exception):
+            G.hstu_mha(300, 0.1, dual, k, v, offs, num_targets=nt)
