@@ -13,6 +13,7 @@ LIB_PATH = os.path.join(_HERE, "libb200_hstu.so")
 
 F32, BF16, F16, E4M3 = 0, 1, 2, 3
 IMPL_AUTO, IMPL_SIMT, IMPL_TCGEN05 = 0, 1, 2
+OFFSETS_I64, TARGETS_I64 = 0x100, 0x200   # or-ed into impl
 
 EXPORTS = [
     "b200_hstu_attn_fwd",

@@ -137,9 +137,9 @@ int b200_hstu_attn_fwd(const b200_hstu_attn_args *a, b200_hstu_stream_t stream) 
   if (a->B == 0 || a->total_L == 0) return 0;
   const char *why = "";
   bool tc = attn_tc_applicable(*a, false, &why);
-  if (a->impl == B200_HSTU_IMPL_TCGEN05 && !tc)
+  if (impl_of(*a) == B200_HSTU_IMPL_TCGEN05 && !tc)
     return fail(B200_HSTU_EUNSUPPORTED, "tcgen05 forward not applicable: %s", why);
-  if (tc && a->impl != B200_HSTU_IMPL_SIMT) return attn_tc_fwd(*a, (cudaStream_t)stream);
+  if (tc && impl_of(*a) != B200_HSTU_IMPL_SIMT) return attn_tc_fwd(*a, (cudaStream_t)stream);
   return attn_simt(*a, (cudaStream_t)stream, false);
 }
 
@@ -149,16 +149,16 @@ int b200_hstu_attn_bwd(const b200_hstu_attn_args *a, b200_hstu_stream_t stream) 
   if (a->B == 0 || a->total_L == 0) return 0;
   const char *why = "";
   bool tc = attn_tc_applicable(*a, true, &why);
-  if (a->impl == B200_HSTU_IMPL_TCGEN05 && !tc)
+  if (impl_of(*a) == B200_HSTU_IMPL_TCGEN05 && !tc)
     return fail(B200_HSTU_EUNSUPPORTED, "tcgen05 backward not applicable: %s", why);
-  if (tc && a->impl != B200_HSTU_IMPL_SIMT) return attn_tc_bwd(*a, (cudaStream_t)stream);
+  if (tc && impl_of(*a) != B200_HSTU_IMPL_SIMT) return attn_tc_bwd(*a, (cudaStream_t)stream);
   return attn_simt(*a, (cudaStream_t)stream, true);
 }
 
 int64_t b200_hstu_attn_workspace_bytes(const b200_hstu_attn_args *a, int backward) {
   if (a == nullptr) return 0;
   const char *why = "";
-  if (a->impl == B200_HSTU_IMPL_SIMT || !attn_tc_applicable(*a, backward == 1, &why)) return 0;
+  if (impl_of(*a) == B200_HSTU_IMPL_SIMT || !attn_tc_applicable(*a, backward == 1, &why)) return 0;
   return attn_tc_workspace_bytes(*a, backward);
 }
 
@@ -339,8 +339,8 @@ void b200_hstu_host_bwd_q_tiles(int32_t len, int32_t num_targets, int32_t max_se
                                 int32_t max_attn_len, int32_t min_full_attn_seq_len, int32_t kt, int32_t *t_lo,
                                 int32_t *n_main, int32_t *extra_tile) {
   AttnGeomParams g;
-  g.seq_offsets = nullptr;
-  g.num_targets = nullptr;
+  g.seq_offsets = {nullptr, 1};
+  g.num_targets = {nullptr, 1};
   g.B = 1;
   g.H = 1;
   g.max_seq_len = max_seq_len;
@@ -363,8 +363,8 @@ int b200_hstu_host_interval_mask(int32_t len, int32_t num_targets, int32_t max_s
                                  int32_t max_attn_len, int32_t min_full_attn_seq_len, int32_t i, int32_t j,
                                  int32_t transposed) {
   AttnGeomParams g;
-  g.seq_offsets = nullptr;
-  g.num_targets = nullptr;
+  g.seq_offsets = {nullptr, 1};
+  g.num_targets = {nullptr, 1};
   g.B = 1;
   g.H = 1;
   g.max_seq_len = max_seq_len;

@@ -990,8 +990,8 @@ int launch_bwd_tc(const b200_hstu_attn_args &a, cudaStream_t st) {
   if ((rc = make_tile_map_rows(&mv, a.v, a.total_L, cols, a.v_row_stride, 2, IS_BF16, TILE)) != 0) return rc;
   if ((rc = make_tile_map_rows(&mdo, a.dout, a.total_L, cols, a.do_row_stride, 2, IS_BF16, TILE)) != 0) return rc;
   BwdParams p;
-  p.g.seq_offsets = a.seq_offsets;
-  p.g.num_targets = a.num_targets;
+  p.g.seq_offsets = seq_offsets_of(a);
+  p.g.num_targets = num_targets_of(a);
   p.g.B = a.B;
   p.g.H = a.H;
   p.g.max_seq_len = a.max_seq_len;

@@ -815,8 +815,8 @@ int attn_tc_fwd_fp8(const b200_hstu_attn_fp8_args &fa, cudaStream_t st) {
   if ((rc = make_tile_map(&mk, a.k, a.total_L, (int64_t)a.H * D, a.k_row_stride, 1, false)) != 0) return rc;
   if ((rc = make_tile_map(&mv, a.v, a.total_L, (int64_t)a.H * D, a.v_row_stride, 1, false)) != 0) return rc;
   Fp8Params p;
-  p.g.seq_offsets = a.seq_offsets;
-  p.g.num_targets = a.num_targets;
+  p.g.seq_offsets = seq_offsets_of(a);
+  p.g.num_targets = num_targets_of(a);
   p.g.B = a.B;
   p.g.H = a.H;
   p.g.max_seq_len = a.max_seq_len;

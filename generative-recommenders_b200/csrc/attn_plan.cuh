@@ -38,7 +38,7 @@ struct __align__(16) ItemDesc {
 };
 
 struct AttnGeomParams {
-  const int32_t *seq_offsets, *num_targets;
+  IndexTensor seq_offsets, num_targets;
   int B, H, max_seq_len, W, c, F;
   int delta;   // > 0: the query rows are the last `delta` positions of each sequence (cached inference)
 };

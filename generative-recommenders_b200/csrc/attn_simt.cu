@@ -30,7 +30,7 @@ constexpr int NTHREADS = 128;  // 4 warps; thread t owns row t/4 and the 8 colum
 struct SimtParams {
   const void *q, *k, *v, *dout;
   void *out, *dq, *dk, *dv;
-  const int32_t *seq_offsets, *num_targets;
+  IndexTensor seq_offsets, num_targets;
   const float *attn_scale;
   int64_t attn_scale_numel;
   const float *bias;
@@ -713,7 +713,7 @@ SimtParams make_params(const b200_hstu_attn_args &a) {
   SimtParams p;
   p.q = a.q; p.k = a.k; p.v = a.v; p.dout = a.dout;
   p.out = a.out; p.dq = a.dq; p.dk = a.dk; p.dv = a.dv_;
-  p.seq_offsets = a.seq_offsets; p.num_targets = a.num_targets;
+  p.seq_offsets = seq_offsets_of(a); p.num_targets = num_targets_of(a);
   p.attn_scale = a.attn_scale; p.attn_scale_numel = a.attn_scale_numel;
   p.bias = a.bias_by_distance; p.bias_numel = a.bias_numel;
   p.dbias = a.bias_by_distance != nullptr ? a.d_bias_by_distance : nullptr;

@@ -45,6 +45,24 @@ struct ProfileScope {
     if (_st != 0) return _st;                                     \
   } while (0)
 
+// Offsets and target counts as the caller has them: int32, or int64 whose low words count (sizes fit 32
+// bits; what a conversion to int32 gives).  `step` is the number of 32-bit words per value.
+struct IndexTensor {
+  const int32_t *p;
+  int step;
+  __host__ __device__ __forceinline__ int operator[](int i) const { return p[(int64_t)i * step]; }
+  __host__ __device__ __forceinline__ explicit operator bool() const { return p != nullptr; }
+};
+inline IndexTensor seq_offsets_of(const b200_hstu_attn_args &a) {
+  return {a.seq_offsets, (a.impl & B200_HSTU_OFFSETS_I64) ? 2 : 1};
+}
+inline IndexTensor num_targets_of(const b200_hstu_attn_args &a) {
+  return {a.num_targets, (a.impl & B200_HSTU_TARGETS_I64) ? 2 : 1};
+}
+inline int impl_of(const b200_hstu_attn_args &a) {
+  return a.impl & ~(B200_HSTU_OFFSETS_I64 | B200_HSTU_TARGETS_I64);
+}
+
 // ---------------------------------------------------------------------------------------
 // element conversion
 // ---------------------------------------------------------------------------------------

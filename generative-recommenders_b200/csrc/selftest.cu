@@ -54,7 +54,7 @@ int b200_hstu_attn_status_async(const b200_hstu_attn_args *a, int which, int32_t
   if (which < 0 || which > 2) return fail(B200_HSTU_EINVAL, "which must be 0 (forward), 1 (backward) or 2 (forward that planned the backward)");
   host_status[0] = host_status[1] = host_status[2] = 0;
   const char *why = "";
-  if (a->workspace == nullptr || a->impl == B200_HSTU_IMPL_SIMT || !attn_tc_applicable(*a, which == 1, &why))
+  if (a->workspace == nullptr || impl_of(*a) == B200_HSTU_IMPL_SIMT || !attn_tc_applicable(*a, which == 1, &why))
     return 0;   // the CUDA-core kernels have no waits and no status
   if (a->workspace_bytes < attn_tc_workspace_bytes(*a, which))
     return fail(B200_HSTU_EWORKSPACE, "workspace is smaller than this call's scratch");

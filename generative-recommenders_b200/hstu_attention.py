@@ -27,6 +27,14 @@ def set_attention_impl(name: str) -> None:
     _forced_impl = name
 
 
+def _index(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    # a call without a backward hands int64 offsets to the kernels as they are (no conversion launch);
+    # one with a backward keeps an int32 copy of its own, which a caller may overwrite the original of
+    if t is None or t.dtype is torch.int64:
+        return t if t is None else t.contiguous()
+    return _i32(t)
+
+
 def _i32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     # tests of the reference pass int64 offsets (hstu_attention_test.py:81-84); its CUDA op wants
     # int32 (flash_common.cpp:460-472).  The kernels read int32.
@@ -60,7 +68,12 @@ def _fill_common(a, q, k, v, seq_offsets, num_targets, attn_scale, max_seq_len, 
     a.contextual_seq_len = contextual_seq_len
     a.min_full_attn_seq_len = min_full_attn_seq_len
     a.dtype = dtype_code(q)
-    a.impl = _IMPL[_forced_impl]
+    impl = _IMPL[_forced_impl]
+    if seq_offsets.dtype is torch.int64:
+        impl |= _cabi.OFFSETS_I64
+    if num_targets is not None and num_targets.dtype is torch.int64:
+        impl |= _cabi.TARGETS_I64
+    a.impl = impl
     if bias_by_distance is not None:
         a.bias_by_distance = bias_by_distance.data_ptr()
         a.bias_numel = bias_by_distance.numel()
@@ -116,7 +129,7 @@ def _workspace(a, which: int, device) -> Optional[torch.Tensor]:
 def hstu_attention_fwd(max_seq_len, alpha, q, k, v, seq_offsets, num_targets, attn_scale, max_attn_len,
                        contextual_seq_len, min_full_attn_seq_len, bias_by_distance=None, plan_for_backward=False,
                        dropout_pr=0.0, dropout_seed=None):
-    """One forward launch; all tensors already validated / int32 / on the device.
+    """One forward launch; all tensors already validated / on the device, index tensors int32 or int64.
 
     With ``plan_for_backward`` the planning kernel also builds the backward's work lists and the
     scratch tensor holding them is returned next to the output (``(out, scratch)``), to be passed
@@ -268,8 +281,9 @@ def hstu_mha(
     q = last_dim_contiguous(q)
     k = last_dim_contiguous(k)
     v = last_dim_contiguous(v)
-    seq_offsets = _i32(seq_offsets)
-    num_targets = _i32(num_targets)
+    inference = outside_autograd(q, k, v, attn_scale, bias_by_distance)
+    seq_offsets = _index(seq_offsets) if inference else _i32(seq_offsets)
+    num_targets = _index(num_targets) if inference else _i32(num_targets)
     if num_targets is not None and num_targets.numel() != seq_offsets.numel() - 1:
         raise RuntimeError("num_targets must have one entry per sequence")
     if attn_scale is not None:
@@ -292,7 +306,7 @@ def hstu_mha(
             raise TypeError("dropout_seed must be a one-element int64 tensor")
     else:
         dropout_seed = None
-    if outside_autograd(q, k, v, attn_scale, bias_by_distance):
+    if inference:
         out = hstu_attention_fwd(int(max_seq_len), float(alpha), q, k, v, seq_offsets, num_targets, attn_scale,
                                  int(max_attn_len), int(contextual_seq_len), int(min_full_attn_seq_len),
                                  bias_by_distance, dropout_pr=drop, dropout_seed=dropout_seed)
@@ -344,8 +358,8 @@ def delta_hstu_mha(
     q = last_dim_contiguous(delta_q.detach())
     k = last_dim_contiguous(k.detach())
     v = last_dim_contiguous(v.detach())
-    seq_offsets = _i32(seq_offsets)
-    num_targets = _i32(num_targets)
+    seq_offsets = _index(seq_offsets)
+    num_targets = _index(num_targets)
     a = _cabi.AttnArgs()
     _fill_common(a, q, k, v, seq_offsets, num_targets, None, int(max_seq_len), float(alpha), int(max_attn_len),
                  int(contextual_seq_len), 0, None)

@@ -12,6 +12,7 @@ import torch
 
 from . import _cabi
 from .common import dtype_code, last_dim_contiguous, on_device, require_cuda, stream_ptr
+from .hstu_attention import _index
 
 BLOCK = 128
 
@@ -73,8 +74,7 @@ def hstu_mha_fp8(
     out = torch.empty((L, H, d), dtype=torch.bfloat16, device=q8.device)
     if L == 0:
         return out
-    seq_offsets = seq_offsets.to(torch.int32).contiguous()
-    nt = None if num_targets is None else num_targets.to(torch.int32).contiguous()
+    seq_offsets, nt = _index(seq_offsets), _index(num_targets)
     fa = _cabi.AttnFp8Args()
     a = fa.base
     a.q, a.k, a.v, a.out = q8.data_ptr(), k8.data_ptr(), v8.data_ptr(), out.data_ptr()
@@ -89,6 +89,10 @@ def hstu_mha_fp8(
     a.min_full_attn_seq_len = int(min_full_attn_seq_len)
     a.dtype = _cabi.BF16
     a.impl = _cabi.IMPL_TCGEN05
+    if seq_offsets.dtype is torch.int64:
+        a.impl |= _cabi.OFFSETS_I64
+    if nt is not None and nt.dtype is torch.int64:
+        a.impl |= _cabi.TARGETS_I64
     nbytes = _cabi.lib().b200_hstu_attn_workspace_bytes(a, 0)
     # the fp8 forward uses the same work list as the bf16 forward; size it from the same query
     # (q8 is not 2-byte data, so ask with the bf16 layout the list size depends on: B and total_L)

@@ -658,15 +658,15 @@ def hstu_preprocess_and_attention(
     if (_FUSED_UQVK and x.is_cuda and _fused_uqvk_supported(x, uvqk_weight, hv)
             and attn_dim == hidden_dim and attn_dim in (64, 128)):
         # one autograd node for the stage and the attention (see _FusedPreprocessAttentionFunction)
-        from .hstu_attention import _i32
+        from .hstu_attention import _i32, _index, hstu_attention_fwd
         require_cuda(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias, seq_offsets, num_targets, bias_by_distance)
-        offs = _i32(seq_offsets)
-        nt = _i32(num_targets)
+        inference = outside_autograd(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias, bias_by_distance)
+        offs = _index(seq_offsets) if inference else _i32(seq_offsets)
+        nt = _index(num_targets) if inference else _i32(num_targets)
         if nt is not None and nt.numel() != offs.numel() - 1:
             raise RuntimeError("num_targets must have one entry per sequence")
         rab = None if bias_by_distance is None else bias_by_distance.to(torch.float32).reshape(-1).contiguous()
-        if outside_autograd(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias, rab):
-            from .hstu_attention import hstu_attention_fwd
+        if inference:
             u, q, k, v = _fused_uqvk_inference(x, norm_weight, norm_bias, float(norm_eps), uvqk_weight, uvqk_bias,
                                                num_heads, attn_dim, hidden_dim)
             attn = hstu_attention_fwd(int(max_seq_len), float(attn_alpha), q, k, v, offs, nt, None,

@@ -49,6 +49,10 @@ extern "C" {
 #define B200_HSTU_IMPL_AUTO 0    /* tcgen05 when dtype/head-dim allow, else SIMT */
 #define B200_HSTU_IMPL_SIMT 1    /* fp32-accumulating CUDA-core kernels          */
 #define B200_HSTU_IMPL_TCGEN05 2 /* tensor-core kernels; error if not applicable */
+/* or-ed into `impl`: that index tensor holds int64 values (the kernels take their low 32 bits), so that
+ * a caller with int64 offsets needs no conversion launches of its own */
+#define B200_HSTU_OFFSETS_I64 0x100 /* seq_offsets */
+#define B200_HSTU_TARGETS_I64 0x200 /* num_targets */
 
 typedef void *b200_hstu_stream_t; /* a cudaStream_t */
 
@@ -89,7 +93,7 @@ typedef struct b200_hstu_attn_args {
   int32_t contextual_seq_len;    /* 0 = none */
   int32_t min_full_attn_seq_len; /* 0 = none */
   int32_t dtype;                 /* B200_HSTU_F32 / BF16 / F16 (q, k, v, out, dout, dq, dk, dv) */
-  int32_t impl;                  /* B200_HSTU_IMPL_* */
+  int32_t impl;                  /* B200_HSTU_IMPL_*, with the index flags */
   /* optional relative position bias added to alpha*<q,k> before SiLU, shared by all heads:
      bias_by_distance[|i - j|] when |i - j| < bias_numel, else 0 (fp32); NULL = none */
   const float *bias_by_distance;

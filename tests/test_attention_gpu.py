@@ -646,3 +646,27 @@ def test_cuda_core_vector_form_equals_element_wise(dtype, d, kw):
         else:
             eps = 2.0 ** -22 if dtype == torch.float32 else 2.0 ** -8   # (16 bits: one rounding may flip)
             torch.testing.assert_close(x, y, rtol=eps, atol=eps * float(y.abs().max()))
+
+
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 128), (torch.float16, 64), (torch.float32, 32),
+                                     (torch.float32, 40)])
+def test_int64_and_int32_offsets_are_the_same_call(dtype, d):
+    # inference hands int64 index tensors to the kernels as they are: every mix of the two types, and a
+    # strided view, gives the same bits (tensor-core, vector and element-wise kernels, and the cached form)
+    g = torch.Generator().manual_seed(1)
+    lengths = torch.tensor([130, 0, 1, 64, 257])
+    nt = torch.tensor([5, 0, 0, 1, 20])
+    offs = torch.cat([torch.zeros(1, dtype=torch.int64), torch.cumsum(lengths, 0)])
+    L = int(offs[-1])
+    q, k, v = (torch.randn(L, 2, d, generator=g).to(dtype).cuda() for _ in range(3))
+    ref = G.hstu_mha(300, 0.1, q, k, v, offs.int().cuda(), num_targets=nt.int().cuda())
+    strided = torch.stack([offs, offs + 7], 1).cuda()[:, 0]
+    for o, n in ((offs.cuda(), nt.cuda()), (offs.cuda(), nt.int().cuda()), (offs.int().cuda(), nt.cuda()),
+                 (strided, nt.cuda())):
+        assert torch.equal(G.hstu_mha(300, 0.1, q, k, v, o, num_targets=n), ref)
+    full = offs + 20 * torch.arange(6)           # every sequence at least as long as its 20 new rows
+    kf, vf = (torch.randn(int(full[-1]), 2, d, generator=g).to(dtype).cuda() for _ in range(2))
+    dq = torch.randn(5 * 20, 2, d, generator=g).to(dtype).cuda()
+    n20 = torch.full((5,), 20)
+    a = G.delta_hstu_mha(300, 0.1, dq, kf, vf, full.int().cuda(), n20.int().cuda())
+    assert torch.equal(a, G.delta_hstu_mha(300, 0.1, dq, kf, vf, full.cuda(), n20.cuda()))
