@@ -141,9 +141,12 @@ __global__ void __launch_bounds__(QTHREADS, 4) quantize_e4m3_vec_kernel(const E 
   if (threadIdx.x == 0) scale[(int64_t)blk * H + h] = sc;
   // The result is defined by the true quotient f / sc, rounded to fp32 and then to e4m3.  With the
   // reciprocal rounded to nearest, one residual step gives the same fp32 value as the division
-  // (Markstein, IBM J. Res. Dev. 34, 1990) in three instructions: q = f y, q' = q + (f - q sc) y.  Only
-  // results far below e4m3's smallest step can see an underflow in it, and those round to zero either
-  // way.  A block with an infinity has sc = inf and takes the division.
+  // (Markstein, IBM J. Res. Dev. 34, 1990) in three instructions: q = f y, q' = q + (q sc - f)(-y).  The
+  // residual is taken with that sign so that -0 stays -0: where it vanishes it is +0, its product with -y
+  // is -0, and q - 0 = q (with f - q sc the sum -0 + 0 gave +0).  Only results far below e4m3's smallest
+  // step can see an underflow in it, and those round to zero either way: the bytes are the division's for
+  // every pair of a 16-bit f and a 16-bit maximum.  A block with an infinity has sc = inf and takes the
+  // division.
   const float inv = 1.f / sc;
   uint8_t *dst = x8 + (row0 * H + h) * D + c * 8;
   if (!(sc < INFINITY)) {   // (its own loop over memory: inside the one below the compiler divides always)
@@ -163,7 +166,7 @@ __global__ void __launch_bounds__(QTHREADS, 4) quantize_e4m3_vec_kernel(const E 
     for (int j = 0; j < 8; ++j) {
       const float f = to_f32(j & 1 ? e[j / 2].y : e[j / 2].x);
       const float t = f * inv;
-      q[j] = fmaf(fmaf(-t, sc, f), inv, t);
+      q[j] = fmaf(fmaf(t, sc, -f), -inv, t);
     }
     uint2 o;
     o.x = pack_e4m3(q[0], q[1]) | pack_e4m3(q[2], q[3]) << 16;

@@ -167,3 +167,22 @@ def test_quantizer_is_the_quotient_bit_by_bit(dtype, d):
             got = x8[offs[b] + r:offs[b] + min(n, r + 128)]
             nan = (want & 127) == 127          # (the sign of a NaN is nobody's)
             assert torch.equal(got & 127 == 127, nan) and torch.equal(got[~nan], want[~nan])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("d", [64, 128])
+def test_quantizer_keeps_the_sign_of_zero(dtype, d):
+    # as the division: -0 gives the byte 0x80 - in a block of numbers, in a block of zeros only, and for
+    # negative values that round to zero
+    x = torch.ones(260, 2, d)
+    x[::2, :, ::3] = -0.0
+    x[1::2, :, ::5] = 0.0
+    x[3::4, :, 1::2] = -2.0 ** -20
+    x[128:256] = torch.where(torch.arange(d) % 2 == 0, -0.0, 0.0)
+    x = x.to(dtype)
+    offs = torch.tensor([0, 128, 260])
+    x8, scale, _ = G.quantize_e4m3_block(x.to(DEV), offs.to(DEV))
+    rows = torch.tensor([0] * 128 + [1] * 128 + [2] * 4)
+    want = (x.float() / scale.cpu()[rows][:, :, None]).to(torch.float8_e4m3fn)
+    assert int((want.view(torch.uint8) == 0x80).sum()) > 0
+    assert torch.equal(x8.cpu().view(torch.uint8), want.view(torch.uint8))
