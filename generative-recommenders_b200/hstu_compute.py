@@ -80,7 +80,8 @@ _PREPARED_ON = True
 
 def clear_prepared_weights() -> None:
     """Forget every cached preparation of the fused uvqk stage (see the comment above)."""
-    _PREPARED.clear()
+    global _PREPARED
+    _PREPARED = {}   # (a call under way adds to the old one)
 
 
 def set_prepared_weights_cache(on: bool) -> None:
@@ -89,29 +90,36 @@ def set_prepared_weights_cache(on: bool) -> None:
     global _PREPARED_ON
     _PREPARED_ON = bool(on)
     if not on:
-        _PREPARED.clear()
+        clear_prepared_weights()
 
 
 def _prepared_workspace(nw, nb, w, b, nbytes, device, allow_cache):
+    """``(workspace, prepared, remember)``: ``remember()``, if there is one, keeps the workspace for later
+    calls.  It is called when the preparation is in the stream and not before: a call of another thread
+    that found the workspace earlier could be queued ahead of it, and after a launch that returned an
+    error there is nothing to find."""
     # Only module parameters are worth remembering, and only when all four tensors are the
     # parameters themselves: a cast copy made for one call never comes back, and its id / address /
     # version can recur on a later, different copy.
     if (not allow_cache or not _PREPARED_ON or torch.cuda.is_current_stream_capturing()
             or not all(isinstance(t, torch.nn.Parameter) for t in (w, nw, nb, b))):
-        return torch.empty(nbytes, dtype=torch.uint8, device=device), False
-    key = id(w)
+        return torch.empty(nbytes, dtype=torch.uint8, device=device), False, None
+    known, key = _PREPARED, id(w)
     stream = stream_ptr(device)
     sig = tuple((id(t), t.data_ptr(), t._version) for t in (w, nw, nb, b)) + (stream,)
-    hit = _PREPARED.get(key)
+    hit = known.get(key)
     # the workspace was prepared on `stream`; a call on another stream is not ordered after that
     # preparation, so it prepares (and then owns) a new one
     if hit is not None and hit[0]() is w and hit[1] == sig and hit[2].numel() == nbytes:
-        return hit[2], True
+        return hit[2], True, None
     ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
-    if len(_PREPARED) > 256:
-        _PREPARED.clear()
-    _PREPARED[key] = (weakref.ref(w), sig, ws)
-    return ws, False
+
+    def remember():
+        if len(known) > 256:
+            known.clear()
+        known[key] = (weakref.ref(w), sig, ws)
+
+    return ws, False, remember
 
 
 def _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, allow_cache=False, stats=True):
@@ -124,7 +132,7 @@ def _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, allow_cache=False, stats=True):
     mean = torch.empty(M, dtype=torch.float32, device=x.device) if stats else None
     rstd = torch.empty(M, dtype=torch.float32, device=x.device) if stats else None
     nbytes = _cabi.lib().b200_hstu_ln_linear_workspace_bytes(D, N)
-    ws, prepared = _prepared_workspace(nw, nb, w, b, nbytes, x.device, allow_cache)
+    ws, prepared, remember = _prepared_workspace(nw, nb, w, b, nbytes, x.device, allow_cache)
     a = _cabi.LnLinearArgs()
     a.weights_prepared = 1 if prepared else 0
     a.skip_pre_activation = 1 if allow_cache else 0   # no gradient wanted: nobody reads the pre-activation u
@@ -140,6 +148,8 @@ def _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, allow_cache=False, stats=True):
     with on_device(x.device):
         _cabi.check(_cabi.lib().b200_hstu_ln_linear_silu_fwd(a, stream_ptr(x.device)),
                     "b200_hstu_ln_linear_silu_fwd")
+    if remember is not None:
+        remember()
     return uvqk, u, mean, rstd
 
 

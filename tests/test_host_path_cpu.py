@@ -1,0 +1,95 @@
+"""Host side of the ops, without a device: the launches are answered by a stand-in for the library."""
+
+import importlib
+
+import pytest
+import torch
+
+import generative_recommenders_b200 as G
+
+HC = importlib.import_module("generative-recommenders_b200.hstu_compute")
+
+
+class _Library:
+    """Answers the fused uvqk launch; ``rc`` is its return code, ``during`` runs inside the call."""
+
+    def __init__(self):
+        self.rc, self.during, self.prepared = 0, None, []
+
+    def b200_hstu_ln_linear_workspace_bytes(self, D, N):
+        return 4096
+
+    def b200_hstu_ln_linear_silu_fwd(self, a, stream):
+        self.prepared.append(a.weights_prepared)
+        if self.during is not None:
+            run, self.during = self.during, None
+            run()
+        return self.rc
+
+
+@pytest.fixture
+def uvqk(monkeypatch):
+    """(library, parameters, call): ``call()`` queues the fused stage on the parameters in the list."""
+    lib = _Library()
+
+    def check(rc, what):
+        if rc != 0:
+            raise RuntimeError(what)
+
+    class _Device:
+        def __enter__(self):
+            return None
+
+        def __exit__(self, *exc):
+            return False
+
+    monkeypatch.setattr(HC._cabi, "lib", lambda: lib)
+    monkeypatch.setattr(HC._cabi, "check", check)
+    monkeypatch.setattr(HC, "stream_ptr", lambda device: 0)
+    monkeypatch.setattr(HC, "on_device", lambda device: _Device())
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    HC.clear_prepared_weights()
+    D, N, hv = 16, 32, 8
+    params = [torch.nn.Parameter(torch.ones(n, dtype=torch.bfloat16), requires_grad=False) for n in (D, D)]
+    params += [torch.nn.Parameter(torch.ones(s, dtype=torch.bfloat16), requires_grad=False) for s in ((D, N), (N,))]
+    x = torch.ones(4, D, dtype=torch.bfloat16)
+    yield lib, params, lambda: HC._fused_uqvk_launch(x, params[0], params[1], 1e-6, params[2], params[3], hv, True)
+    HC.clear_prepared_weights()
+
+
+def test_prepared_weights_are_kept_while_the_parameters_are_unchanged(uvqk):
+    lib, params, call = uvqk
+    call(), call()
+    with torch.no_grad():
+        params[2].mul_(2)
+    call(), call()
+    assert lib.prepared == [0, 1, 0, 1]
+
+
+def test_failed_launch_leaves_no_prepared_weights(uvqk):
+    # the workspace of a call that returned an error holds nothing
+    lib, params, call = uvqk
+    lib.rc = 1
+    with pytest.raises(RuntimeError, match="ln_linear"):
+        call()
+    lib.rc = 0
+    call(), call()
+    assert lib.prepared == [0, 0, 1]
+
+
+def test_prepared_weights_are_shared_after_their_preparation_is_queued(uvqk):
+    # another thread's call may come between the lookup of this one and its launch: it must not take a
+    # workspace whose preparation is not in the stream yet
+    lib, params, call = uvqk
+    lib.during = call
+    call()
+    assert lib.prepared == [0, 0]
+    call()
+    assert lib.prepared == [0, 0, 1]
+
+
+def test_weights_forgotten_during_a_call_stay_forgotten(uvqk):
+    lib, params, call = uvqk
+    lib.during = HC.clear_prepared_weights
+    call(), call()
+    assert lib.prepared == [0, 0]
