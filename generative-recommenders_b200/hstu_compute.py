@@ -104,20 +104,21 @@ def _prepared_workspace(nw, nb, w, b, nbytes, device, allow_cache):
     if (not allow_cache or not _PREPARED_ON or torch.cuda.is_current_stream_capturing()
             or not all(isinstance(t, torch.nn.Parameter) for t in (w, nw, nb, b))):
         return torch.empty(nbytes, dtype=torch.uint8, device=device), False, None
-    known, key = _PREPARED, id(w)
+    known, key = _PREPARED, id(w)   # (an id can recur as well: the entry holds weak references to compare)
     stream = stream_ptr(device)
     sig = tuple((id(t), t.data_ptr(), t._version) for t in (w, nw, nb, b)) + (stream,)
     hit = known.get(key)
     # the workspace was prepared on `stream`; a call on another stream is not ordered after that
     # preparation, so it prepares (and then owns) a new one
-    if hit is not None and hit[0]() is w and hit[1] == sig and hit[2].numel() == nbytes:
+    if (hit is not None and hit[1] == sig and hit[2].numel() == nbytes
+            and all(r() is t for r, t in zip(hit[0], (w, nw, nb, b)))):
         return hit[2], True, None
     ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
 
     def remember():
         if len(known) > 256:
             known.clear()
-        known[key] = (weakref.ref(w), sig, ws)
+        known[key] = (tuple(weakref.ref(t) for t in (w, nw, nb, b)), sig, ws)
 
     return ws, False, remember
 

@@ -93,3 +93,16 @@ def test_weights_forgotten_during_a_call_stay_forgotten(uvqk):
     lib.during = HC.clear_prepared_weights
     call(), call()
     assert lib.prepared == [0, 0]
+
+
+@pytest.mark.parametrize("which", range(4))
+def test_replaced_parameter_is_not_the_prepared_one(uvqk, monkeypatch, which):
+    # an id, an address and a version can all come back with a new parameter once the old one is gone
+    lib, params, call = uvqk
+    monkeypatch.setattr(HC, "id", lambda t: 7, raising=False)
+    call()
+    storage = params[which].detach()
+    params[which] = None
+    params[which] = torch.nn.Parameter(storage, requires_grad=False)
+    call()
+    assert lib.prepared == [0, 0]
