@@ -100,9 +100,9 @@ def _prepared_workspace(nw, nb, w, b, nbytes, device, allow_cache):
     error there is nothing to find."""
     # Only module parameters are worth remembering, and only when all four tensors are the
     # parameters themselves: a cast copy made for one call never comes back, and its id / address /
-    # version can recur on a later, different copy.
+    # version can recur on a later, different copy.  Parameters made in inference mode have no version.
     if (not allow_cache or not _PREPARED_ON or torch.cuda.is_current_stream_capturing()
-            or not all(isinstance(t, torch.nn.Parameter) for t in (w, nw, nb, b))):
+            or not all(isinstance(t, torch.nn.Parameter) and not t.is_inference() for t in (w, nw, nb, b))):
         return torch.empty(nbytes, dtype=torch.uint8, device=device), False, None
     known, key = _PREPARED, id(w)   # (an id can recur as well: the entry holds weak references to compare)
     stream = stream_ptr(device)

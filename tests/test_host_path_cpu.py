@@ -106,3 +106,12 @@ def test_replaced_parameter_is_not_the_prepared_one(uvqk, monkeypatch, which):
     params[which] = torch.nn.Parameter(storage, requires_grad=False)
     call()
     assert lib.prepared == [0, 0]
+
+
+def test_parameters_made_in_inference_mode_are_not_remembered(uvqk):
+    # they carry no version counter, so nothing would tell a changed one
+    lib, params, call = uvqk
+    with torch.inference_mode():
+        params[:] = [torch.nn.Parameter(p.detach().clone(), requires_grad=False) for p in params]
+        call(), call()
+    assert lib.prepared == [0, 0]
