@@ -81,8 +81,9 @@ def on_device(device):
 
 
 def span(name: str):
-    """``record_function(name)`` while a profiler runs, else its light form (other observers see it too)."""
-    if torch.autograd._profiler_enabled():
+    """``record_function(name)`` while a profiler runs, else its light form (other observers see it too).
+    The compiler knows the former only."""
+    if torch.compiler.is_compiling() or torch.autograd._profiler_enabled():
         return torch.autograd.profiler.record_function(name)
     return _RecordFunctionFast(name)
 
@@ -95,12 +96,14 @@ def outside_autograd(*tensors) -> bool:
     """True where an ``autograd.Function`` would do no more than run its forward: no input asks for a
     gradient, and there is no forward-mode level, functorch transform, tracer or compiler that has to see
     the node (or to refuse it)."""
+    if torch.compiler.is_compiling():   # (first: the compiler need not see the rest)
+        return False
     if torch.is_grad_enabled():
         for t in tensors:
             if t is not None and t.requires_grad:
                 return False
     return (forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
-            and torch._C._get_tracing_state() is None and not torch.compiler.is_compiling())
+            and torch._C._get_tracing_state() is None)
 
 
 def last_dim_contiguous(t: torch.Tensor) -> torch.Tensor:

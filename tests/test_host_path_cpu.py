@@ -115,3 +115,17 @@ def test_parameters_made_in_inference_mode_are_not_remembered(uvqk):
         params[:] = [torch.nn.Parameter(p.detach().clone(), requires_grad=False) for p in params]
         call(), call()
     assert lib.prepared == [0, 0]
+
+
+def test_span_and_the_autograd_rule_are_seen_through_by_the_compiler():
+    common = importlib.import_module("generative-recommenders_b200.common")
+
+    def step(x):
+        with common.span("## step ##"):
+            y = x + 1
+        return y * 2 if common.outside_autograd(y) else y * 3
+
+    x = torch.ones(3)
+    # (under the compiler a call keeps its autograd node)
+    assert torch.equal(torch.compile(step, fullgraph=True, backend="eager")(x), torch.full((3,), 6.0))
+    assert torch.equal(step(x), torch.full((3,), 4.0))
