@@ -77,7 +77,8 @@ _NOTHING = _Nothing()
 
 def on_device(device):
     """``torch.cuda.device(device)`` around a launch; nothing where that is the thread's device already."""
-    return _NOTHING if device.index == torch._C._cuda_getDevice() else torch.cuda.device(device)
+    index = getattr(device, "index", None)   # (an int or None has none, a str a method)
+    return _NOTHING if index == torch._C._cuda_getDevice() else torch.cuda.device(device)
 
 
 def span(name: str):

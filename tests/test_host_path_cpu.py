@@ -129,3 +129,16 @@ def test_span_and_the_autograd_rule_are_seen_through_by_the_compiler():
     # (under the compiler a call keeps its autograd node)
     assert torch.equal(torch.compile(step, fullgraph=True, backend="eager")(x), torch.full((3,), 6.0))
     assert torch.equal(step(x), torch.full((3,), 4.0))
+
+
+@pytest.mark.parametrize("device", [1, None, "cuda:1", torch.device("cuda", 1), torch.device("cuda")])
+def test_on_device_takes_what_the_device_context_takes(device, monkeypatch):
+    common = importlib.import_module("generative-recommenders_b200.common")
+    entered = []
+    monkeypatch.setattr(torch.cuda, "device", entered.append)
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 0, raising=False)
+    common.on_device(device)
+    assert entered == [device]
+    with common.on_device(torch.device("cuda", 0)):
+        pass
+    assert entered == [device]
