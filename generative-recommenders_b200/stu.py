@@ -168,10 +168,9 @@ class STULayer(torch.nn.Module):
                                          values_right=delta, max_len_left=self.max_kv_caching_len,
                                          max_len_right=delta_size, offsets_left=self.kv_caching_offsets,
                                          offsets_right=None, kernel=self._hammer_kernel))
-        offsets = self.kv_caching_offsets
-        if delta_size > 0:
-            offsets = offsets + torch.arange(0, delta_size * (B + 1), delta_size, device=delta_k.device)
-        return full[0], full[1], self.max_kv_caching_len + delta_size, offsets
+        steps = (torch.arange(0, delta_size * (B + 1), delta_size, device=delta_k.device) if delta_size > 0
+                 else torch.zeros(B + 1, dtype=torch.int64, device=delta_k.device))
+        return full[0], full[1], self.max_kv_caching_len + delta_size, self.kv_caching_offsets + steps
 
     def cached_forward(
         self,

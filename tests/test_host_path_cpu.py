@@ -142,3 +142,19 @@ def test_on_device_takes_what_the_device_context_takes(device, monkeypatch):
     with common.on_device(torch.device("cuda", 0)):
         pass
     assert entered == [device]
+
+
+@pytest.mark.parametrize("rows", [0, 6])
+def test_full_kv_offsets_are_the_callers_own(rows, monkeypatch):
+    # what the caller does to the offsets it got must not change those of the cache, new rows or none
+    stu = importlib.import_module("generative-recommenders_b200.stu")
+    monkeypatch.setattr(stu, "concat_2D_jagged", lambda values_left, **kw: values_left)
+    layer = G.STULayer(G.STULayerConfig(embedding_dim=16, num_heads=1, hidden_dim=16, attention_dim=16))
+    layer.k_cache = layer.v_cache = torch.zeros(9, 16)
+    layer.kv_caching_offsets, layer.max_kv_caching_len = torch.tensor([0, 4, 9], dtype=torch.int32), 5
+    delta = torch.zeros(rows, 16)
+    _, _, longest, offsets = layer.construct_full_kv(delta, delta)
+    n = rows // 2
+    assert longest == 5 + n and offsets.dtype == torch.int64 and offsets.tolist() == [0, 4 + n, 9 + 2 * n]
+    offsets.zero_()
+    assert layer.kv_caching_offsets.tolist() == [0, 4, 9]
