@@ -18,6 +18,14 @@ DEV = "cuda:0"
     (torch.float16, 2, 96, (True, False)),
     (torch.float32, 2, 64, (True, True)),       # 4 elements per 16-byte vector: half a generator call each
     (torch.bfloat16, 2, 34, (True, True)),      # H*V = 68: rows not made of whole vectors (element-wise path)
+    # rows of one vector per lane: the backward masks du and dattn in one step where both are concatenated
+    (torch.bfloat16, 4, 64, (True, True)),
+    (torch.float16, 2, 96, (True, True)),
+    (torch.bfloat16, 1, 8, (True, True)),       # a single vector
+    # two vectors per lane: one-sided concats, and a second vector that only some lanes have
+    (torch.bfloat16, 4, 128, (True, False)),
+    (torch.bfloat16, 4, 128, (False, True)),
+    (torch.bfloat16, 3, 104, (True, True)),
 ])
 def test_dropout_mask_replay_forward_backward(dtype, H, V, concat):
     g = torch.Generator().manual_seed(11)
@@ -102,6 +110,14 @@ def test_group_norm_variant_keeps_torch_dropout():
     (torch.bfloat16, 2, 64, (False, False)),
     (torch.bfloat16, 2, 34, (True, True)),      # rows not made of whole vectors: no mask is stored
     (torch.float32, 2, 64, (True, True)),       # 32-bit elements: no mask is stored
+    # rows of one vector per lane: the backward masks du and dattn in one step where both are concatenated
+    (torch.bfloat16, 4, 64, (True, True)),
+    (torch.float16, 2, 96, (True, True)),
+    (torch.bfloat16, 1, 8, (True, True)),       # a single vector
+    # two vectors per lane: one-sided concats, and a second vector that only some lanes have
+    (torch.bfloat16, 4, 128, (True, False)),
+    (torch.bfloat16, 4, 128, (False, True)),
+    (torch.bfloat16, 3, 104, (True, True)),
 ])
 def test_stored_mask_and_regenerated_mask_give_the_same_backward(dtype, H, V, concat):
     """The forward keeps its dropout mask as bits for the backward where it can; a backward that
