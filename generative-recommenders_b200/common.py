@@ -5,6 +5,7 @@ from enum import Enum, unique
 import torch
 from torch._C._profiler import _RecordFunctionFast
 from torch.autograd import forward_ad
+from torch.compiler import is_compiling
 
 from . import _cabi
 
@@ -84,7 +85,7 @@ def on_device(device):
 def span(name: str):
     """``record_function(name)`` while a profiler runs, else its light form (other observers see it too).
     The compiler knows the former only."""
-    if torch.compiler.is_compiling() or torch.autograd._profiler_enabled():
+    if is_compiling() or torch.autograd._profiler_enabled():
         return torch.autograd.profiler.record_function(name)
     return _RecordFunctionFast(name)
 
@@ -97,7 +98,7 @@ def outside_autograd(*tensors) -> bool:
     """True where an ``autograd.Function`` would do no more than run its forward: no input asks for a
     gradient, and there is no forward-mode level, functorch transform, tracer or compiler that has to see
     the node (or to refuse it)."""
-    if torch.compiler.is_compiling():   # (first: the compiler need not see the rest)
+    if is_compiling():   # (first: the compiler need not see the rest)
         return False
     if torch.is_grad_enabled():
         for t in tensors:

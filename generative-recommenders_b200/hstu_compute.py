@@ -93,32 +93,40 @@ def set_prepared_weights_cache(on: bool) -> None:
         clear_prepared_weights()
 
 
+def _prepared_state(w, nw, nb, b, stream):
+    return (w.data_ptr(), w._version, nw.data_ptr(), nw._version, nb.data_ptr(), nb._version, b.data_ptr(),
+            b._version, stream)
+
+
 def _prepared_workspace(nw, nb, w, b, nbytes, device, allow_cache):
     """``(workspace, prepared, remember)``: ``remember()``, if there is one, keeps the workspace for later
     calls.  It is called when the preparation is in the stream and not before: a call of another thread
     that found the workspace earlier could be queued ahead of it, and after a launch that returned an
     error there is nothing to find."""
-    # Only module parameters are worth remembering, and only when all four tensors are the
-    # parameters themselves: a cast copy made for one call never comes back, and its id / address /
-    # version can recur on a later, different copy.  Parameters made in inference mode have no version.
-    if (not allow_cache or not _PREPARED_ON or torch.cuda.is_current_stream_capturing()
-            or not all(isinstance(t, torch.nn.Parameter) and not t.is_inference() for t in (w, nw, nb, b))):
+    if not allow_cache or not _PREPARED_ON or torch.cuda.is_current_stream_capturing():
         return torch.empty(nbytes, dtype=torch.uint8, device=device), False, None
-    known, key = _PREPARED, id(w)   # (an id can recur as well: the entry holds weak references to compare)
-    stream = stream_ptr(device)
-    sig = tuple((id(t), t.data_ptr(), t._version) for t in (w, nw, nb, b)) + (stream,)
-    hit = known.get(key)
-    # the workspace was prepared on `stream`; a call on another stream is not ordered after that
+    known, key = _PREPARED, id(w)
+    # the workspace was prepared on this stream; a call on another stream is not ordered after that
     # preparation, so it prepares (and then owns) a new one
-    if (hit is not None and hit[1] == sig and hit[2].numel() == nbytes
-            and all(r() is t for r, t in zip(hit[0], (w, nw, nb, b)))):
-        return hit[2], True, None
+    stream = stream_ptr(device)
+    hit = known.get(key)   # (an id can recur: the entry holds weak references to compare)
+    if hit is not None:
+        rw, rnw, rnb, rb, sig, ws = hit
+        if (rw() is w and rnw() is nw and rnb() is nb and rb() is b and ws.numel() == nbytes
+                and sig == _prepared_state(w, nw, nb, b, stream)):
+            return ws, True, None
     ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    # Only module parameters are worth remembering, and only when all four tensors are the
+    # parameters themselves: a cast copy made for one call never comes back.  Parameters made in
+    # inference mode have no version.
+    if not all(isinstance(t, torch.nn.Parameter) and not t.is_inference() for t in (w, nw, nb, b)):
+        return ws, False, None
+    sig = _prepared_state(w, nw, nb, b, stream)
 
     def remember():
         if len(known) > 256:
             known.clear()
-        known[key] = (tuple(weakref.ref(t) for t in (w, nw, nb, b)), sig, ws)
+        known[key] = (weakref.ref(w), weakref.ref(nw), weakref.ref(nb), weakref.ref(b), sig, ws)
 
     return ws, False, remember
 
