@@ -98,12 +98,12 @@ def _prepared_state(w, nw, nb, b, stream):
             b._version, stream)
 
 
-def _prepared_workspace(nw, nb, w, b, nbytes, device, allow_cache):
+def _prepared_workspace(nw, nb, w, b, nbytes, device, keep):
     """``(workspace, prepared, remember)``: ``remember()``, if there is one, keeps the workspace for later
     calls.  It is called when the preparation is in the stream and not before: a call of another thread
     that found the workspace earlier could be queued ahead of it, and after a launch that returned an
     error there is nothing to find."""
-    if not allow_cache or not _PREPARED_ON or torch.cuda.is_current_stream_capturing():
+    if not keep or not _PREPARED_ON or torch.cuda.is_current_stream_capturing():
         return torch.empty(nbytes, dtype=torch.uint8, device=device), False, None
     known, key = _PREPARED, id(w)
     # the workspace was prepared on this stream; a call on another stream is not ordered after that
@@ -131,24 +131,25 @@ def _prepared_workspace(nw, nb, w, b, nbytes, device, allow_cache):
     return ws, False, remember
 
 
-def _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, allow_cache=False, stats=True):
-    """One launch of the fused kernel: returns (uvqk [M, N], u [M, hv], mean [M], rstd [M]); without
-    ``stats`` the last two are None."""
+def _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, inference=False):
+    """One launch of the fused kernel: returns (uvqk [M, N], u [M, hv], mean [M], rstd [M]).  For
+    ``inference`` the derived weights may be kept, the pre-activation u columns of uvqk stay unwritten
+    and mean and rstd are None."""
     M, D = x.shape
     N = w.shape[1]
     uvqk = torch.empty((M, N), dtype=x.dtype, device=x.device)
     u = torch.empty((M, hv), dtype=x.dtype, device=x.device)
-    mean = torch.empty(M, dtype=torch.float32, device=x.device) if stats else None
-    rstd = torch.empty(M, dtype=torch.float32, device=x.device) if stats else None
+    mean = torch.empty(M, dtype=torch.float32, device=x.device) if not inference else None
+    rstd = torch.empty(M, dtype=torch.float32, device=x.device) if not inference else None
     nbytes = _cabi.lib().b200_hstu_ln_linear_workspace_bytes(D, N)
-    ws, prepared, remember = _prepared_workspace(nw, nb, w, b, nbytes, x.device, allow_cache)
+    ws, prepared, remember = _prepared_workspace(nw, nb, w, b, nbytes, x.device, inference)
     a = _cabi.LnLinearArgs()
     a.weights_prepared = 1 if prepared else 0
-    a.skip_pre_activation = 1 if allow_cache else 0   # no gradient wanted: nobody reads the pre-activation u
+    a.skip_pre_activation = 1 if inference else 0   # only the backward reads it
     a.x, a.norm_weight, a.norm_bias, a.weight, a.bias = (x.data_ptr(), nw.data_ptr(), nb.data_ptr(),
                                                           w.data_ptr(), b.data_ptr())
     a.out, a.u = uvqk.data_ptr(), u.data_ptr()
-    if stats:
+    if not inference:
         a.mean, a.rstd = mean.data_ptr(), rstd.data_ptr()
     a.workspace, a.workspace_bytes = ws.data_ptr(), nbytes
     a.x_row_stride, a.out_row_stride, a.u_row_stride = x.stride(0), uvqk.stride(0), u.stride(0)
@@ -202,6 +203,12 @@ def _fused_uqvk_backward(x, nw, nb, w, uvqk, mean, rstd, eps, hv, du, d_uvqk):
     return dx, dnw, dnb, dw, db
 
 
+def _stage_parameters(x, norm_weight, norm_bias, weight, bias):
+    """The parameters as the fused kernel reads them (a parameter that is so already: itself)."""
+    return (as_dtype(norm_weight, x.dtype).contiguous(), as_dtype(norm_bias, x.dtype).contiguous(),
+            _aligned16(as_dtype(weight, x.dtype).contiguous()), as_dtype(bias, x.dtype).contiguous())
+
+
 def _uqvk_views(uvqk, num_heads, attn_dim, hidden_dim):
     """(q, k, v) as ``[M, H, d]`` views of the uvqk buffer."""
     hv, ha = hidden_dim * num_heads, attn_dim * num_heads
@@ -212,10 +219,8 @@ def _uqvk_views(uvqk, num_heads, attn_dim, hidden_dim):
 
 def _fused_uqvk_inference(x, norm_weight, norm_bias, eps, weight, bias, num_heads, attn_dim, hidden_dim):
     """The fused stage where no gradient is wanted: ``(u, q, k, v)``."""
-    uvqk, u, _, _ = _fused_uqvk_launch(
-        x, as_dtype(norm_weight, x.dtype).contiguous(), as_dtype(norm_bias, x.dtype).contiguous(), eps,
-        _aligned16(as_dtype(weight, x.dtype).contiguous()), as_dtype(bias, x.dtype).contiguous(),
-        hidden_dim * num_heads, True, stats=False)
+    nw, nb, w, b = _stage_parameters(x, norm_weight, norm_bias, weight, bias)
+    uvqk, u, _, _ = _fused_uqvk_launch(x, nw, nb, eps, w, b, hidden_dim * num_heads, inference=True)
     return (u,) + _uqvk_views(uvqk, num_heads, attn_dim, hidden_dim)
 
 
@@ -224,24 +229,16 @@ class _FusedUqvkFunction(torch.autograd.Function):
     (csrc/ln_linear_sm100.cu)."""
 
     @staticmethod
-    def forward(ctx, x, norm_weight, norm_bias, eps, weight, bias, num_heads, attn_dim, hidden_dim, grad_mode=True):
-        M = x.shape[0]
+    def forward(ctx, x, norm_weight, norm_bias, eps, weight, bias, num_heads, attn_dim, hidden_dim):
         hv, ha = hidden_dim * num_heads, attn_dim * num_heads
-        nw = as_dtype(norm_weight, x.dtype).contiguous()
-        nb = as_dtype(norm_bias, x.dtype).contiguous()
-        w = _aligned16(as_dtype(weight, x.dtype).contiguous())
-        b = as_dtype(bias, x.dtype).contiguous()
-        no_grad = not (grad_mode and any(ctx.needs_input_grad))
-        uvqk, u, mean, rstd = _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, no_grad)
+        nw, nb, w, b = _stage_parameters(x, norm_weight, norm_bias, weight, bias)
+        uvqk, u, mean, rstd = _fused_uqvk_launch(x, nw, nb, eps, w, b, hv)
         ctx.set_materialize_grads(False)
         ctx.save_for_backward(x, nw, nb, w, uvqk, mean, rstd)
         ctx.cfg = (eps, hv, ha, norm_weight.dtype, norm_bias.dtype, weight.dtype, bias.dtype)
         # q, k, v are views of the uvqk buffer, handed out as separate results so that the backward
         # receives their gradients one by one instead of three zero-padded [M, N] sums
-        v = uvqk[:, hv:2 * hv].view(M, num_heads, hidden_dim)
-        q = uvqk[:, 2 * hv:2 * hv + ha].view(M, num_heads, attn_dim)
-        k = uvqk[:, 2 * hv + ha:].view(M, num_heads, attn_dim)
-        return u, q, k, v
+        return (u,) + _uqvk_views(uvqk, num_heads, attn_dim, hidden_dim)
 
     @staticmethod
     def backward(ctx, du, dq, dk, dv):
@@ -256,7 +253,7 @@ class _FusedUqvkFunction(torch.autograd.Function):
                 d_uvqk[:, lo:lo + width].copy_(g.reshape(M, width))
         dx, dnw, dnb, dw, db = _fused_uqvk_backward(x, nw, nb, w, uvqk, mean, rstd, eps, hv, du, d_uvqk)
         return (dx, as_dtype(dnw, nw_dtype), as_dtype(dnb, nb_dtype), None, as_dtype(dw, w_dtype),
-                as_dtype(db, b_dtype), None, None, None, None)
+                as_dtype(db, b_dtype), None, None, None)
 
 
 class _FusedPreprocessAttentionFunction(torch.autograd.Function):
@@ -266,22 +263,15 @@ class _FusedPreprocessAttentionFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, norm_weight, norm_bias, eps, weight, bias, num_heads, attn_dim, hidden_dim, seq_offsets,
-                num_targets, bias_by_distance, max_seq_len, alpha, max_attn_len, contextual_seq_len, grad_mode=True,
+                num_targets, bias_by_distance, max_seq_len, alpha, max_attn_len, contextual_seq_len,
                 recompute_uvqk=False):
         from .hstu_attention import hstu_attention_fwd
 
-        M = x.shape[0]
-        hv, ha = hidden_dim * num_heads, attn_dim * num_heads
-        nw = as_dtype(norm_weight, x.dtype).contiguous()
-        nb = as_dtype(norm_bias, x.dtype).contiguous()
-        w = _aligned16(as_dtype(weight, x.dtype).contiguous())
-        b = as_dtype(bias, x.dtype).contiguous()
-        no_grad = not (grad_mode and any(ctx.needs_input_grad))
-        uvqk, u, mean, rstd = _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, no_grad)
-        v = uvqk[:, hv:2 * hv].view(M, num_heads, hidden_dim)
-        q = uvqk[:, 2 * hv:2 * hv + ha].view(M, num_heads, attn_dim)
-        k = uvqk[:, 2 * hv + ha:].view(M, num_heads, attn_dim)
-        plan = not no_grad and (any(ctx.needs_input_grad[:6]) or ctx.needs_input_grad[11])
+        hv = hidden_dim * num_heads
+        nw, nb, w, b = _stage_parameters(x, norm_weight, norm_bias, weight, bias)
+        uvqk, u, mean, rstd = _fused_uqvk_launch(x, nw, nb, eps, w, b, hv)
+        q, k, v = _uqvk_views(uvqk, num_heads, attn_dim, hidden_dim)
+        plan = any(ctx.needs_input_grad[:6]) or ctx.needs_input_grad[11]
         ctx.set_materialize_grads(False)  # k / v usually get no gradient: do not add zeros for them
         out = hstu_attention_fwd(max_seq_len, alpha, q, k, v, seq_offsets, num_targets, None, max_attn_len,
                                  contextual_seq_len, 0, bias_by_distance, plan_for_backward=plan)
@@ -293,7 +283,7 @@ class _FusedPreprocessAttentionFunction(torch.autograd.Function):
         # generative_recommenders/ops/triton/triton_hstu_preprocess_and_attention.py:122-127, 185-203).
         # k and v go out as views of that buffer either way: it lives on only while the caller keeps them
         # (the layer does so for its KV cache, otherwise it drops them at once).
-        keep = None if (recompute_uvqk and not no_grad) else uvqk
+        keep = None if recompute_uvqk else uvqk
         ctx.save_for_backward(x, nw, nb, w, b, keep, mean, rstd, seq_offsets, num_targets, bias_by_distance)
         ctx.cfg = (eps, num_heads, attn_dim, hidden_dim, max_seq_len, alpha, max_attn_len, contextual_seq_len,
                    norm_weight.dtype, norm_bias.dtype, weight.dtype, bias.dtype)
@@ -308,7 +298,7 @@ class _FusedPreprocessAttentionFunction(torch.autograd.Function):
          nw_dtype, nb_dtype, w_dtype, b_dtype) = ctx.cfg
         hv, ha = V * H, A * H
         if uvqk is None:   # not kept: one more launch of the fused kernel
-            uvqk, _, mean, rstd = _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, False)
+            uvqk, _, mean, rstd = _fused_uqvk_launch(x, nw, nb, eps, w, b, hv)
         M, N = uvqk.shape
         d_uvqk = torch.empty((M, N), dtype=x.dtype, device=x.device)
         dv = d_uvqk[:, hv:2 * hv].view(M, H, V)
@@ -321,9 +311,7 @@ class _FusedPreprocessAttentionFunction(torch.autograd.Function):
             if (dattn.stride(-1) != 1 or dattn.stride(1) != dattn.shape[2]
                     or dattn.stride(0) < dattn.shape[1] * dattn.shape[2]):
                 dattn = dattn.contiguous()
-            v_ = uvqk[:, hv:2 * hv].view(M, H, V)
-            q_ = uvqk[:, 2 * hv:2 * hv + ha].view(M, H, A)
-            k_ = uvqk[:, 2 * hv + ha:].view(M, H, A)
+            q_, k_, v_ = _uqvk_views(uvqk, H, A, V)
             planned, ctx.planned_scratch = ctx.planned_scratch, None
             if bias_by_distance is not None and ctx.needs_input_grad[11]:
                 d_bias = torch.zeros_like(bias_by_distance)
@@ -336,7 +324,7 @@ class _FusedPreprocessAttentionFunction(torch.autograd.Function):
             dv.add_(dv_ext)
         dx, dnw, dnb, dw, db = _fused_uqvk_backward(x, nw, nb, w, uvqk, mean, rstd, eps, hv, du, d_uvqk)
         return (dx, as_dtype(dnw, nw_dtype), as_dtype(dnb, nb_dtype), None, as_dtype(dw, w_dtype),
-                as_dtype(db, b_dtype), None, None, None, None, None, d_bias, None, None, None, None, None, None)
+                as_dtype(db, b_dtype), None, None, None, None, None, d_bias, None, None, None, None, None)
 
 
 _FUSED_UQVK = True
@@ -371,7 +359,7 @@ def hstu_compute_uqvk(
             return _fused_uqvk_inference(x, norm_weight, norm_bias, float(norm_eps), uvqk_weight, uvqk_bias,
                                          num_heads, attn_dim, hidden_dim)
         return _FusedUqvkFunction.apply(x, norm_weight, norm_bias, float(norm_eps), uvqk_weight, uvqk_bias,
-                                        num_heads, attn_dim, hidden_dim, torch.is_grad_enabled())
+                                        num_heads, attn_dim, hidden_dim)
     else:
         normed_x = layer_norm(x, weight=norm_weight, bias=norm_bias, eps=norm_eps, kernel=kernel)
         uvqk = addmm(uvqk_bias, normed_x, uvqk_weight, kernel)
@@ -694,7 +682,7 @@ def hstu_preprocess_and_attention(
         u, attn, k, v = _FusedPreprocessAttentionFunction.apply(
             x, norm_weight, norm_bias, float(norm_eps), uvqk_weight, uvqk_bias, num_heads, attn_dim, hidden_dim,
             offs, nt, rab, int(max_seq_len), float(attn_alpha), int(max_attn_len), int(contextual_seq_len),
-            torch.is_grad_enabled(), bool(recompute_uvqk_in_backward))
+            bool(recompute_uvqk_in_backward))
         return u, attn.view(-1, hidden_dim * num_heads), k, v
     u, q, k, v = hstu_compute_uqvk(
         x=x, norm_weight=norm_weight, norm_bias=norm_bias, norm_eps=norm_eps, num_heads=num_heads,
