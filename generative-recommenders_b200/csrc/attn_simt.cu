@@ -6,7 +6,8 @@
 // The backward uses two kernels so that every gradient element has a single owner: no atomics, no
 // scratch, bit-reproducible.
 //
-// Two forms with the same sums in the same order.  Head dimensions 32 / 64 / 128 (d_qk = d_v) on the
+// Two forms with the same sums in the same order (they may differ where the compiler contracts a product
+// into a sum in one of them only: 2 ulp of fp32).  Head dimensions 32 / 64 / 128 (d_qk = d_v) on the
 // grid of four elements run the vector kernels below; any other shape runs the element-wise kernels
 // that come first.
 //
@@ -344,8 +345,14 @@ __global__ void __launch_bounds__(NTHREADS) attn_kv_stationary_bwd_kernel(SimtPa
 // other, each a chain of scalar loads with an index division between them and of dot products with
 // nine shared-memory loads for eight products.  Here 256 threads fetch the next tile into registers
 // (16-byte loads) while the present one is computed, the tile of S is 2 x 2 per thread and its second
-// product 4 columns per thread, both on 16-byte shared loads.  Measured in fp32 on 16 sequences of up
-// to 256 rows, 2 heads x 32: forward 65 -> 21 us, dQ 52 -> 26, dK / dV 74 -> 36.
+// product 4 columns per thread, both on 16-byte shared loads.  Measured on 2 heads, sequences of up to 256
+// rows, element-wise -> vector form in us, forward / dQ / dK and dV:
+//              16 sequences                               384 sequences
+//   fp32  32    52 ->  21 /  65 ->  26 /  69 ->  30        182 -> 131 /  247 -> 165 /  331 -> 229
+//   fp32  64    87 ->  28 / 115 ->  38 / 113 ->  42        351 -> 180 /  509 -> 251 /  592 -> 323
+//   fp32 128   288 ->  33 / 202 ->  46 / 220 ->  57       1139 -> 364 / 1102 -> 499 / 1574 -> 616
+// and bf16 within 9 % of these.  On the small fp32 calls at 32 a scheduler issues in 30 % of the cycles and its
+// two to three warps wait for shared memory most of the time.
 // ---------------------------------------------------------------------------------------
 constexpr int VTHREADS = 256;
 constexpr int PLD = T + 4;   // leading dimension of the P / dS tiles
@@ -659,7 +666,8 @@ __device__ __forceinline__ void kv_tile_vec(const SimtParams &p, float *smem) {
   }
 }
 
-// PART 0: forward, 1: dQ, 2: dK and dV
+// PART 0: forward, 1: dQ, 2: dK and dV.  At D = 32 and 64 two CTAs fit an SM (128 registers; dQ and dK / dV in
+// fp32 at D = 64 spill one of them); at D = 128 a thread holds 166 to 200, which leaves room for one.
 template <typename E, int D, int PART>
 __global__ void __launch_bounds__(VTHREADS, D == 128 ? 1 : 2) attn_vec_kernel(SimtParams p) {
   extern __shared__ __align__(16) float smem[];

@@ -28,8 +28,9 @@ def set_attention_impl(name: str) -> None:
 
 
 def _index(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
-    # a call without a backward hands int64 offsets to the kernels as they are (no conversion launch);
-    # one with a backward keeps an int32 copy of its own, which a caller may overwrite the original of
+    # a call without a backward hands int64 offsets to the kernels as they are (no conversion launch); one
+    # with a backward converts them (_i32), so that its copy outlives what a caller does to the original.
+    # int32 tensors are read in place either way.
     if t is None or t.dtype is torch.int64:
         return t if t is None else t.contiguous()
     return _i32(t)
@@ -37,7 +38,7 @@ def _index(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
 
 def _i32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     # tests of the reference pass int64 offsets (hstu_attention_test.py:81-84); its CUDA op wants
-    # int32 (flash_common.cpp:460-472).  The kernels read int32.
+    # int32 (flash_common.cpp:460-472).
     if t is None:
         return None
     return as_dtype(t, torch.int32).contiguous()

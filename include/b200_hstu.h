@@ -74,8 +74,8 @@ typedef struct b200_hstu_attn_args {
   void *out;              /* fwd: written.  [total_L, H, dv]; bwd: unused (may be NULL) */
   const void *dout;       /* bwd only: [total_L, H, dv] */
   void *dq, *dk, *dv_;    /* bwd only: written, same shapes as q, k, v */
-  const int32_t *seq_offsets; /* [B + 1] */
-  const int32_t *num_targets; /* [B] or NULL */
+  const int32_t *seq_offsets; /* [B + 1]; int64 values where impl has B200_HSTU_OFFSETS_I64 */
+  const int32_t *num_targets; /* [B] or NULL; int64 values where impl has B200_HSTU_TARGETS_I64 */
   const float *attn_scale;    /* NULL, or fp32 [1] (scalar) or [total_L] (per query token) */
   int64_t attn_scale_numel;   /* 0, 1 or total_L */
   /* strides, in elements */
