@@ -99,7 +99,8 @@ def hstu_mha_fp8(
     ws = torch.empty(max(int(nbytes), 64 + 32 * (L // BLOCK + a.B + 1) + 256), dtype=torch.uint8, device=q8.device)
     a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
     fa.q_scale, fa.k_scale, fa.v_scale = q_scale.data_ptr(), k_scale.data_ptr(), v_scale.data_ptr()
-    fa.block_offsets = block_offsets.to(torch.int32).contiguous().data_ptr()
+    block_offsets = block_offsets.to(torch.int32).contiguous()   # (kept alive until the launch is queued)
+    fa.block_offsets = block_offsets.data_ptr()
     with on_device(q8.device):
         _cabi.check(_cabi.lib().b200_hstu_attn_fwd_fp8(fa, stream_ptr(q8.device)), "b200_hstu_attn_fwd_fp8")
     return out

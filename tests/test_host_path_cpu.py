@@ -158,3 +158,48 @@ def test_full_kv_offsets_are_the_callers_own(rows, monkeypatch):
     assert longest == 5 + n and offsets.dtype == torch.int64 and offsets.tolist() == [0, 4 + n, 9 + 2 * n]
     offsets.zero_()
     assert layer.kv_caching_offsets.tolist() == [0, 4, 9]
+
+
+@pytest.fixture
+def fp8(monkeypatch):
+    """(module, seen): ``seen`` collects the block offsets, as int32, that the launches are given; before they
+    are read, the memory that a dropped tensor would have left is written over."""
+    import ctypes
+
+    module = importlib.import_module("generative-recommenders_b200.hstu_attention_fp8")
+    seen = []
+
+    def read(address, n):
+        keep = [torch.full((n,), -1, dtype=torch.int32) for _ in range(64)]
+        seen.append(list((ctypes.c_int32 * n).from_address(address)))
+        del keep
+        return 0
+
+    class Library:
+        def b200_hstu_attn_workspace_bytes(self, a, which):
+            return 0
+
+        def b200_hstu_attn_fwd_fp8(self, fa, stream):
+            return read(fa.block_offsets, fa.base.B + 1)
+
+        def b200_hstu_quantize_e4m3_block(self, *args):
+            return read(args[7], args[8] + 1)
+
+    monkeypatch.setattr(module._cabi, "lib", Library)
+    monkeypatch.setattr(module, "require_cuda", lambda *tensors: None)
+    monkeypatch.setattr(module, "stream_ptr", lambda device: 0)
+    monkeypatch.setattr(module, "on_device", lambda device: importlib.import_module("contextlib").nullcontext())
+    return module, seen
+
+
+# a caller may hold them in any integer type and layout
+_BLOCKS = [torch.tensor([0, 1, 3], dtype=torch.int32), torch.tensor([0, 1, 3]),
+           torch.tensor([[0, 1, 3], [9, 9, 9]], dtype=torch.int32).t().contiguous()[:, 0]]
+
+
+@pytest.mark.parametrize("blocks", _BLOCKS)
+def test_block_offsets_reach_the_fp8_forward(fp8, blocks):
+    module, seen = fp8
+    x8, scale = torch.zeros(300, 1, 64).to(torch.float8_e4m3fn), torch.ones(4, 1)
+    module.hstu_mha_fp8(256, 1.0, x8, x8, x8, scale, scale, scale, blocks, torch.tensor([0, 100, 300]))
+    assert seen == [[0, 1, 3]]
