@@ -11,7 +11,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _cabi
-from .common import dtype_code, last_dim_contiguous, on_device, require_cuda, stream_ptr
+from .common import as_dtype, dtype_code, last_dim_contiguous, on_device, require_cuda, stream_ptr
 from .hstu_attention import _index
 
 BLOCK = 128
@@ -37,6 +37,7 @@ def quantize_e4m3_block(x: torch.Tensor, seq_offsets: torch.Tensor,
     B = seq_offsets.numel() - 1
     if block_offsets is None:
         block_offsets = block_offsets_for(seq_offsets)
+    blocks = as_dtype(block_offsets, torch.int32).contiguous()
     x8 = torch.empty((L, H, d), dtype=torch.float8_e4m3fn, device=x.device)
     scale = torch.ones((L // BLOCK + B, H), dtype=torch.float32, device=x.device)
     if L > 0:
@@ -44,7 +45,7 @@ def quantize_e4m3_block(x: torch.Tensor, seq_offsets: torch.Tensor,
             _cabi.check(
                 _cabi.lib().b200_hstu_quantize_e4m3_block(
                     x.data_ptr(), dtype_code(x), x.stride(0), x.stride(1), x8.data_ptr(), scale.data_ptr(),
-                    seq_offsets.data_ptr(), block_offsets.data_ptr(), B, H, d, L, 1 << 30, stream_ptr(x.device)),
+                    seq_offsets.data_ptr(), blocks.data_ptr(), B, H, d, L, 1 << 30, stream_ptr(x.device)),
                 "b200_hstu_quantize_e4m3_block")
     return x8, scale, block_offsets
 
@@ -99,7 +100,7 @@ def hstu_mha_fp8(
     ws = torch.empty(max(int(nbytes), 64 + 32 * (L // BLOCK + a.B + 1) + 256), dtype=torch.uint8, device=q8.device)
     a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
     fa.q_scale, fa.k_scale, fa.v_scale = q_scale.data_ptr(), k_scale.data_ptr(), v_scale.data_ptr()
-    block_offsets = block_offsets.to(torch.int32).contiguous()   # (kept alive until the launch is queued)
+    block_offsets = as_dtype(block_offsets, torch.int32).contiguous()   # (kept alive until the launch is queued)
     fa.block_offsets = block_offsets.data_ptr()
     with on_device(q8.device):
         _cabi.check(_cabi.lib().b200_hstu_attn_fwd_fp8(fa, stream_ptr(q8.device)), "b200_hstu_attn_fwd_fp8")

@@ -203,3 +203,11 @@ def test_block_offsets_reach_the_fp8_forward(fp8, blocks):
     x8, scale = torch.zeros(300, 1, 64).to(torch.float8_e4m3fn), torch.ones(4, 1)
     module.hstu_mha_fp8(256, 1.0, x8, x8, x8, scale, scale, scale, blocks, torch.tensor([0, 100, 300]))
     assert seen == [[0, 1, 3]]
+
+
+@pytest.mark.parametrize("blocks", _BLOCKS)
+def test_block_offsets_reach_the_quantiser(fp8, blocks):
+    module, seen = fp8
+    _, _, out = module.quantize_e4m3_block(torch.zeros(300, 1, 64), torch.tensor([0, 100, 300]), blocks)
+    assert seen == [[0, 1, 3]]
+    assert out is blocks
