@@ -385,8 +385,8 @@ __global__ void __launch_bounds__(WARPS * 32, MAXV <= 2 ? 3 : (MAXV <= 4 ? 2 : 1
 // result does not depend on timing.  There are as many rows as the backward has CTAs: three per SM = 444 for
 // norm-mul and for LayerNorm of up to two vectors per lane, 296 and 148 for LayerNorm of four and eight; a
 // lane makes 14, 10 or 5 loads, five of them in flight.  Against eight warps with four in flight, LayerNorm
-// backward in 16 bits: 444 rows of 1024 columns 6.6 -> 3.5 us on 8 k rows, 8 -> 4 on
-// 200 k; 296 rows of 2048 4.9 -> 3.1, 148 of 4096 3.9 -> 2.4.
+// backward in 16 bits: 444 rows of 1024 columns 6.6 -> 3.5 us after 8 k tokens (8 -> 4 after 200 k), 296 of 2048
+// 4.9 -> 3.1, 148 of 4096 3.9 -> 2.4.
 constexpr int REDUCE_WARPS = 32;
 template <typename E>
 __global__ void __launch_bounds__(REDUCE_WARPS * 32)
