@@ -47,6 +47,7 @@ EXPORTS = [
     "b200_hstu_host_kv_range",
     "b200_hstu_host_mask",
     "b200_hstu_host_bwd_q_tiles",
+    "b200_hstu_host_bwd_q_visits",
     "b200_hstu_host_interval_mask",
     "b200_hstu_profile_enable",
     "b200_hstu_profile_collect",
@@ -229,6 +230,8 @@ def lib():
     L.b200_hstu_host_kv_range.restype = None
     L.b200_hstu_host_bwd_q_tiles.argtypes = [c_int32] * 7 + [POINTER(c_int32)] * 3
     L.b200_hstu_host_bwd_q_tiles.restype = None
+    L.b200_hstu_host_bwd_q_visits.argtypes = [c_int32] * 8
+    L.b200_hstu_host_bwd_q_visits.restype = ctypes.c_int
     L.b200_hstu_profile_enable.argtypes = [ctypes.c_int]
     L.b200_hstu_profile_enable.restype = None
     L.b200_hstu_profile_collect.argtypes = [ctypes.c_int, POINTER(c_float), ctypes.c_int]

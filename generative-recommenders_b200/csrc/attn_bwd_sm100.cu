@@ -423,9 +423,17 @@ struct __align__(16) ItemGeom {
   int start, len, nt;        // first token row, untruncated length, number of targets
   int m0, n_tiles, t_lo, n_main;
   int extra_tile, L, u, regular;
-  int max_id, pad0, pad1, pad2;
-  __device__ __forceinline__ int tile_at(int j) const { return j < n_main ? t_lo + j : extra_tile; }
+  int max_id;
+  uint32_t gap;              // of the main range: where it is (upper 16 bits) and how many tiles it leaves out
+  int pad[2];
+  // Only items of the kv-stationary launch have a gap, and their extra tile is tile 0.
+  template <bool DKDV>
+  __device__ __forceinline__ int tile_at(int j, uint32_t gap_) const {
+    if (DKDV) return j < n_main ? t_lo + j + (j >= (int)(gap_ >> 16) ? (int)(gap_ & 0xffffu) : 0) : 0;
+    return j < n_main ? t_lo + j : extra_tile;
+  }
 };
+constexpr int GEOM_INTS = 14;
 constexpr int GEOM_SLOTS = 4;
 constexpr int GEOM_SLOT_BYTES = 64;
 
@@ -434,7 +442,7 @@ __device__ __forceinline__ void geom_from_item(ItemGeom &g, const TileItem &it, 
   g.start = it.start; g.len = it.len; g.nt = it.nt;
   g.m0 = it.m0; g.n_tiles = it.n_tiles; g.t_lo = it.t_lo; g.n_main = it.n_main;
   g.extra_tile = it.extra_tile; g.L = it.m.L; g.u = it.u; g.regular = it.regular ? 1 : 0;
-  g.max_id = it.m.max_id; g.pad0 = g.pad1 = g.pad2 = 0;
+  g.max_id = it.m.max_id; g.gap = (uint32_t)it.gap_at << 16 | (uint32_t)it.gap; g.pad[0] = g.pad[1] = 0;
 }
 // the fields the activation and epilogue code reads (no tile ranges are recomputed)
 __device__ __forceinline__ void item_from_geom(TileItem &it, const ItemGeom &g, const AttnGeomParams &gp) {
@@ -464,7 +472,7 @@ __device__ __forceinline__ bool geom_fetch(const WaitCtx &wc, const uint8_t *rin
   const volatile int *src = reinterpret_cast<const volatile int *>(ring + slot * GEOM_SLOT_BYTES);
   int *dst = reinterpret_cast<int *>(&g);
 #pragma unroll
-  for (int i = 0; i < 13; ++i) dst[i] = src[i];
+  for (int i = 0; i < GEOM_INTS; ++i) dst[i] = src[i];
   __syncwarp();
   if (arrive) mbar_arrive(empty0 + 8 * slot);
   return true;
@@ -625,7 +633,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
         // order of requests = order of first use: X0, Y0(0) feed G1; X1, Y1(0) feed G2
         for (int j = 0; j < g.n_tiles; ++j, ++cnt) {
           const int s0 = cnt % Y0_STAGES, s1 = cnt % Y1_STAGES;
-          const int row = g.start + g.tile_at(j) * TILE;
+          const int row = g.start + g.template tile_at<DKDV>(j, g.gap) * TILE;
           if (j == 0) {
             ok = mbar_wait(wc, x_empty, (it_cnt & 1) ^ 1, 401);
             if (!ok) break;
@@ -826,7 +834,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
     tr.init(p.trace, 2, warp == 2 && lane == 0);
     if ((int)blockIdx.x < num_items) {
       ItemGeom g;
-      ok = geom_fetch(wc, sched_ring, sched_full, sched_empty, 0, g, lane == 0);
+      // (these warps hand an item's slot back when they are through with the item)
+      ok = geom_fetch(wc, sched_ring, sched_full, sched_empty, 0, g, false);
       while (ok && g.idx < num_items) {
         TileItem it;
         item_from_geom(it, g, p.g);
@@ -842,7 +851,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
           ColInterval ci;
           RowInterval ri;
           if (DKDV) ci = col_interval(it, own_j); else ri = row_interval(it, own_j);
-          const int o0 = it.tile_at(j) * TILE;  // first position of the streamed tile
+          // (the gap is read from the item's slot each time: this loop has no register to keep it in)
+          const uint32_t gap =
+              DKDV ? reinterpret_cast<const volatile ItemGeom *>(sched_ring + (item_no % GEOM_SLOTS) * GEOM_SLOT_BYTES)->gap
+                   : 0u;
+          const int o0 = g.template tile_at<DKDV>(j, gap) * TILE;  // first position of the streamed tile
           const int c0 = o0 + wg * 64;  // first streamed position of this thread's 64 columns
           ActTile at;
           at.tS = tS;
@@ -881,8 +894,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
           }
         }
         if (!ok) break;
+        if (lane == 0) mbar_arrive(sched_empty + 8 * (item_no % GEOM_SLOTS));
         ++item_no;
-        ok = geom_fetch(wc, sched_ring, sched_full, sched_empty, item_no, g, lane == 0);
+        ok = geom_fetch(wc, sched_ring, sched_full, sched_empty, item_no, g, false);
       }
     }
   } else {

@@ -55,12 +55,12 @@ struct TileItem {
   SeqMask m;
   int t_lo, n_main;       // opposite-side tiles [t_lo, t_lo + n_main)
   int extra_tile;         // >= 0: one more tile outside the main range
+  int gap_at, gap;        // the main range leaves out `gap` tiles after its first `gap_at` (kv items only; 16 bits)
   int n_tiles;
   int u;                  // first target position
   bool regular;           // closed-form row intervals / tile classification are valid
-  __host__ __device__ __forceinline__ int tile_at(int j) const { return j < n_main ? t_lo + j : extra_tile; }
-  __host__ __device__ __forceinline__ bool visits(int t) const {
-    return (t >= t_lo && t < t_lo + n_main) || t == extra_tile;
+  __host__ __device__ __forceinline__ int tile_at(int j) const {
+    return j < n_main ? t_lo + j + (j >= gap_at ? gap : 0) : extra_tile;
   }
 };
 
@@ -75,6 +75,16 @@ __host__ __device__ __forceinline__ void fill_common(TileItem &it, const AttnGeo
   it.m0 = t * TILE + (g.delta > 0 ? it.m.L - g.delta : 0);
   it.u = len - nt;
   it.regular = (it.u >= g.c + 1) && (nt >= 0) && (len <= it.m.L);
+  it.gap_at = it.gap = 0;
+}
+
+// The last row of a query tile (rows [m0, rows_end)) that sees a window instead of everything before it, as
+// a position (a target stands where the history ends); below m0 when the tile has none.
+__host__ __device__ __forceinline__ int last_windowed_row(const TileItem &it, int rows_end) {
+  const SeqMask &m = it.m;
+  const int last = rows_end - 1;
+  if (m.F > 0) return last < it.u - m.F - 1 ? last : it.u - m.F - 1;
+  return last < it.u ? last : it.u;
 }
 
 // kv tiles that the query tile `mt` of a sequence visits
@@ -113,10 +123,8 @@ __host__ __device__ __forceinline__ bool tile_pair_is_full(const TileItem &it, i
   int lim = it.m0 < it.u ? it.m0 : it.u;
   if (n0 + TILE > lim) return false;
   if (m.W > 0) {
-    if (m.F > 0) return false;
-    int rows_end = it.m0 + TILE < m.L ? it.m0 + TILE : m.L;
-    int eff_last = rows_end - 1 < it.u ? rows_end - 1 : it.u;
-    if (eff_last - n0 > m.W) return false;
+    const int last = last_windowed_row(it, it.m0 + TILE < m.L ? it.m0 + TILE : m.L);
+    if ((m.F == 0 || last >= it.m0) && last - n0 > m.W) return false;
   }
   return true;
 }
@@ -134,11 +142,9 @@ __host__ __device__ __forceinline__ FullRange full_tile_range(const TileItem &it
   const int lim = it.m0 < it.u ? it.m0 : it.u;
   int lo = m.c > 0 ? (m.c + TILE - 1) / TILE : 0;
   if (m.W > 0) {
-    if (m.F > 0) return r;
-    const int rows_end = it.m0 + TILE < m.L ? it.m0 + TILE : m.L;
-    const int eff_last = rows_end - 1 < it.u ? rows_end - 1 : it.u;
-    const int first = eff_last - m.W;   // n0 >= first
-    if (first > 0) {
+    const int last = last_windowed_row(it, it.m0 + TILE < m.L ? it.m0 + TILE : m.L);
+    const int first = last - m.W;   // n0 >= first
+    if (first > 0 && (m.F == 0 || last >= it.m0)) {
       const int t = (first + TILE - 1) / TILE;
       lo = t > lo ? t : lo;
     }
@@ -150,8 +156,11 @@ __host__ __device__ __forceinline__ FullRange full_tile_range(const TileItem &it
 }
 
 // q tiles that the kv tile `kt` of a sequence has to visit (backward, kv-stationary): a
-// conservative contiguous range [t_lo, t_hi) plus, when contextual rows exist and fit one tile,
-// tile 0.
+// conservative range [t_lo, t_hi) plus, when contextual rows exist and fit one tile, tile 0.  With a
+// window and a full-attention tail the range has a gap: the rows whose window reaches the tile,
+// then the tail and the targets.  (23 sequences of 37 - 3001 rows, window 517, tail 100, 6 heads of 64: with
+// every tile from the diagonal on visited and masked 183 us, now 139; forward and dQ launch, whose query
+// tiles outside the tail now start at their window: 151 -> 109 and 157 -> 114.)
 __host__ __device__ __forceinline__ void fill_kv_item(TileItem &it, const AttnGeomParams &g, int b, int kt, int start,
                                                       int len, int nt) {
   fill_common(it, g, b, kt, start, len, nt);
@@ -166,7 +175,7 @@ __host__ __device__ __forceinline__ void fill_kv_item(TileItem &it, const AttnGe
     if (n0 >= it.u) {
       // only target columns: each is seen by its own row alone
       t_hi = kt + 1;
-    } else if (g.W > 0 && g.F == 0) {
+    } else if (g.W > 0) {
       // history rows i see j >= i - W; target rows see j >= u - W.  Last history row that can
       // still see a column of this tile: n1 - 1 + W.
       int last_row = n1 - 1 + g.W;
@@ -183,6 +192,15 @@ __host__ __device__ __forceinline__ void fill_kv_item(TileItem &it, const AttnGe
         int hist_end = L - 1 < last_row ? L - 1 : last_row;
         t_hi = hist_end / TILE + 1;
       }
+      if (g.F > 0) {
+        const int w_end = (it.u - 1 < last_row ? it.u - 1 : last_row) / TILE + 1;   // behind the windowed rows
+        const int tail = it.u - g.F > n0 ? (it.u - g.F) / TILE : kt;
+        t_hi = ntiles;
+        if (tail > w_end && tail <= 0xffff) {
+          it.gap_at = w_end;   // (made relative to t_lo below)
+          it.gap = tail - w_end;
+        }
+      }
       if (t_hi < kt + 1) t_hi = kt + 1;
       if (t_hi > ntiles) t_hi = ntiles;
     }
@@ -198,7 +216,8 @@ __host__ __device__ __forceinline__ void fill_kv_item(TileItem &it, const AttnGe
     }
   }
   it.t_lo = t_lo;
-  it.n_main = t_hi - t_lo;
+  it.n_main = t_hi - t_lo - it.gap;
+  if (it.gap > 0) it.gap_at -= t_lo;
   if (it.n_main < 0) it.n_main = 0;
   it.n_tiles = it.n_main + (it.extra_tile >= 0 ? 1 : 0);
 }

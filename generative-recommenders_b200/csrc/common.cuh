@@ -167,7 +167,9 @@ __host__ __device__ __forceinline__ KvRange kv_range_for_q_tile(const SeqMask &m
   }
   int first = m0 < u ? m0 : u;  // smallest effective row position in the tile
   int lo = 0;
-  if (m.W > 0 && m.F == 0) {
+  // a tile that reaches into the full-attention tail (its last `F` history rows, and then the targets) has
+  // rows that see everything before them
+  if (m.W > 0 && !(m.F > 0 && m1 > u - m.F)) {
     lo = first - m.W;
     if (lo < m.c) lo = 0;  // first - W <= c - 1: the row also sees the contextual prefix
   }

@@ -399,10 +399,13 @@ void b200_hstu_host_kv_range(int32_t len, int32_t num_targets, int32_t max_seq_l
                              int32_t max_attn_len, int32_t min_full_attn_seq_len, int32_t m0, int32_t tile,
                              int32_t *lo, int32_t *hi, int32_t *diag_lo);
 /* Query tiles (128 rows each) the backward's K/V-stationary kernel visits for kv tile kt:
-   [t_lo, t_lo + n_main) plus extra_tile when it is >= 0. */
+   [t_lo, t_lo + n_main) plus extra_tile when it is >= 0 (a superset where a window and a full-attention
+   tail come together; b200_hstu_host_bwd_q_visits() says of one query tile whether it is visited). */
 void b200_hstu_host_bwd_q_tiles(int32_t len, int32_t num_targets, int32_t max_seq_len, int32_t contextual_seq_len,
                                 int32_t max_attn_len, int32_t min_full_attn_seq_len, int32_t kt, int32_t *t_lo,
                                 int32_t *n_main, int32_t *extra_tile);
+int b200_hstu_host_bwd_q_visits(int32_t len, int32_t num_targets, int32_t max_seq_len, int32_t contextual_seq_len,
+                                int32_t max_attn_len, int32_t min_full_attn_seq_len, int32_t kt, int32_t qt);
 /* mask(i, j) from the closed-form row (transposed = 0) / column (transposed = 1) intervals used on
    partially visible tiles; -1 when the closed form does not apply to this sequence. */
 int b200_hstu_host_interval_mask(int32_t len, int32_t num_targets, int32_t max_seq_len, int32_t contextual_seq_len,

@@ -670,3 +670,20 @@ def test_int64_and_int32_offsets_are_the_same_call(dtype, d):
     n20 = torch.full((5,), 20)
     a = G.delta_hstu_mha(300, 0.1, dq, kf, vf, full.int().cuda(), n20.int().cuda())
     assert torch.equal(a, G.delta_hstu_mha(300, 0.1, dq, kf, vf, full.cuda(), n20.cuda()))
+
+
+@pytest.mark.parametrize("impl", ["tcgen05", "simt"])
+@pytest.mark.parametrize("case", [
+    # several tiles between the window and the tail; tail and targets longer than a tile; a prefix over
+    # two tiles; a tail of one row
+    (3, 700, 1400, 1400, 1, 128, 20, 5, 100, 128),
+    (3, 700, 1400, 1400, 2, 64, 150, 0, 129, 200),
+    (2, 1000, 1400, 1400, 1, 64, 0, 130, 128, 1),
+])
+def test_window_with_full_tail_over_many_tiles(impl, case):
+    B, lo, hi, N, H, d, targets, ctx, Wn, F = case
+    G.set_attention_impl(impl)
+    q, k, v, offs, nt, dout = _random_case(31 + B * d + F, B, lo, hi, N, H, d, torch.bfloat16, targets, ctx, std=0.7)
+    out, grads = _run(q, k, v, offs, N, 1.0 / d ** 0.5, nt, Wn, ctx, F, dout)
+    ref, rgrads = _oracle(q, k, v, offs, N, 1.0 / d ** 0.5, nt, Wn, ctx, F, dout)
+    _check_all(("gap", impl, case), out, grads, ref, rgrads, offs)

@@ -172,3 +172,37 @@ def test_closed_form_row_and_column_masks_equal_the_exact_mask():
             assert torch.equal(torch.tensor(got, dtype=torch.bool), mask), (L, t, c, W, F, tr)
             checked += 1
     assert checked > 300
+
+
+def test_backward_tile_rule_leaves_out_what_lies_between_window_and_tail():
+    """With a window and a full-attention tail the visited set of a kv tile has a gap: every query tile
+    that holds a row that sees it is visited, none twice, and nothing between the two is."""
+    lib = _cabi.lib()
+    rng = random.Random(77)
+    T = 128
+    gaps = 0
+    for _ in range(150):
+        N = 1500
+        L = rng.randint(1, N)
+        c = rng.choice([0, 0, 5, 127, 128, 300])
+        t = rng.randint(0, max(0, min(L - 1, rng.choice([1, 60, 300]))))
+        W = rng.choice([1, 127, 128, 129, 400])
+        F = rng.choice([1, 100, 128, 129, 700])
+        mask = O.valid_attn_mask(L, t, True, W, c, F)
+        ntiles = (L + T - 1) // T
+        for kt in range(ntiles):
+            visits = [lib.b200_hstu_host_bwd_q_visits(L, t, N, c, W, F, kt, qt) for qt in range(ntiles)]
+            sees = [bool(mask[qt * T:(qt + 1) * T, kt * T:(kt + 1) * T].any()) for qt in range(ntiles)]
+            assert max(visits) == 1
+            assert all(v or not s for v, s in zip(visits, sees)), (L, t, c, W, F, kt, visits, sees)
+            if L - t >= c + 1 and c <= T:   # tight: only the tile of the prefix may come for nothing
+                assert visits[1:] == [int(s) for s in sees[1:]], (L, t, c, W, F, kt, visits, sees)
+            held = [qt for qt in range(1, ntiles) if visits[qt]]
+            gaps += bool(held) and len(held) < held[-1] - held[0] + 1
+        for qt in range(ntiles):
+            # forward and dQ launch: a query tile without rows of the tail starts at its window
+            lo, hi, dg = _range(lib, L, t, N, c, W, F, qt * T, T)
+            cols = torch.nonzero(mask[qt * T:(qt + 1) * T].any(dim=0)).flatten()
+            if L - t >= c + 1 and qt * T >= c and c == 0:
+                assert lo // T == int(cols[0]) // T
+    assert gaps > 100
