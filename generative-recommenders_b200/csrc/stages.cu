@@ -96,6 +96,21 @@ struct RawRow {
   }
 };
 
+template <typename E>
+__device__ __forceinline__ void unpack_vec(const uint4 &raw, float (&v)[VecInfo<E>::EV]) {
+  const E *pe = reinterpret_cast<const E *>(&raw);
+#pragma unroll
+  for (int t = 0; t < VecInfo<E>::EV; ++t) v[t] = to_f32(pe[t]);
+}
+template <typename E>
+__device__ __forceinline__ void store_vec(E *dst, const float (&v)[VecInfo<E>::EV]) {
+  uint4 raw;
+  E *pe = reinterpret_cast<E *>(&raw);
+#pragma unroll
+  for (int t = 0; t < VecInfo<E>::EV; ++t) pe[t] = from_f32<E>(v[t]);
+  *reinterpret_cast<uint4 *>(dst) = raw;
+}
+
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // mean / rstd of a row held in registers (two-pass: mean first, then centred second moment)
@@ -911,6 +926,133 @@ __global__ void __launch_bounds__(WARPS * 32, MAXV <= 4 ? 2 : 1) norm_mul_fwd_pa
   }
 }
 
+__device__ __forceinline__ void copy_async16(uint4 *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+// Forward with dropout for rows of up to two vectors per lane: bound by HBM and by the issue of the generator's
+// and the row's arithmetic together.  The rows come through shared memory by asynchronous copies (every lane
+// reads what it has copied itself: no barrier), three CTAs of eight warps fit an SM, and the generator
+// runs beside the sums of the statistics.  For few rows (see where it is chosen); on many the register-resident
+// kernel is 8 % faster.
+// Vector path only (aligned pointers and strides, D a multiple of the vector width, 16-bit elements).
+// Shared memory: [WARPS][STAGES][2][MAXV][32] vectors: attn, u.
+template <typename E, int MAXV, int STAGES>
+__global__ void __launch_bounds__(WARPS * 32, 3) norm_mul_fwd_staged_kernel(NormMulParams p) {
+  static_assert(VecInfo<E>::EV == 8, "one generator call for a vector");
+  extern __shared__ uint4 ring[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int D = p.H * p.V;
+  Dropout drop;
+  drop.init(p);
+  const int off_x = p.concat_u ? D : 0;
+  const int off_y = off_x + (p.concat_x ? D : 0);
+  const int width = off_y + D;
+  uint4 *mine = ring + warp * (STAGES * 2 * MAXV * 32) + lane;
+  auto request = [&](int64_t r, int stage) {
+    if (r < p.rows) {
+      const E *xr = (const E *)p.attn + r * p.attn_rs, *ur = (const E *)p.u + r * p.u_rs;
+      uint4 *dst = mine + stage * (2 * MAXV * 32);
+#pragma unroll
+      for (int k = 0; k < MAXV; ++k) {
+        const int e0 = (k * 32 + lane) * 8;
+        if (e0 >= D) continue;
+        copy_async16(dst + k * 32, xr + e0);
+        copy_async16(dst + (MAXV + k) * 32, ur + e0);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");   // (a group for every row, so that they can be counted)
+  };
+  const int64_t step = (int64_t)gridDim.x * WARPS;
+  int64_t row = (int64_t)blockIdx.x * WARPS + warp;
+#pragma unroll
+  for (int s = 0; s + 1 < STAGES; ++s) request(row + s * step, s);
+  int stage = 0;
+  for (; row < p.rows; row += step) {
+    request(row + (STAGES - 1) * step, stage == 0 ? STAGES - 1 : stage - 1);   // the slot of the row before
+    const uint64_t base = ((uint64_t)row * (uint64_t)width >> 3) + (uint64_t)lane;   // generator call of the row's first vector
+    auto words = [&](int off, uint32_t (&o)[MAXV][4]) {
+      uint64_t g[MAXV];
+#pragma unroll
+      for (int k = 0; k < MAXV; ++k) g[k] = base + (uint64_t)((off >> 3) + k * 32);
+      philox_many<MAXV>(drop.k0, drop.k1, g, o);
+    };
+    E *orow = (E *)p.out + row * p.out_rs;
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+    const uint4 *in = mine + stage * (2 * MAXV * 32);
+    // statistics as in row_stats()
+    float mean = 0.f;
+#pragma unroll
+    for (int k = 0; k < MAXV; ++k) {
+      float x[8];
+      if ((k * 32 + lane) * 8 >= D) continue;
+      unpack_vec<E>(in[k * 32], x);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) mean += x[t];
+    }
+    uint32_t o[MAXV][4];
+    if (p.concat_u) words(0, o);
+    mean = warp_sum(mean) / (float)D;
+    float rstd = 0.f;
+#pragma unroll
+    for (int k = 0; k < MAXV; ++k) {
+      float x[8];
+      if ((k * 32 + lane) * 8 >= D) continue;
+      unpack_vec<E>(in[k * 32], x);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        const float d = x[t] - mean;
+        rstd += d * d;
+      }
+    }
+    if (p.concat_u) {
+#pragma unroll
+      for (int k = 0; k < MAXV; ++k) {
+        const int e0 = (k * 32 + lane) * 8;
+        if (e0 >= D) continue;
+        float u[8];
+        unpack_vec<E>(in[(MAXV + k) * 32], u);
+        drop.mask8(u, o[k]);
+        store_vec<E>(orow + e0, u);
+      }
+    }
+    if (p.concat_x) words(off_x, o);
+    rstd = rsqrtf(warp_sum(rstd) / (float)D + p.eps);
+    if (p.concat_x) {
+#pragma unroll
+      for (int k = 0; k < MAXV; ++k) {
+        const int e0 = (k * 32 + lane) * 8;
+        if (e0 >= D) continue;
+        float x[8];
+        unpack_vec<E>(in[k * 32], x);
+        drop.mask8(x, o[k]);
+        store_vec<E>(orow + off_x + e0, x);
+      }
+    }
+    words(off_y, o);
+#pragma unroll
+    for (int k = 0; k < MAXV; ++k) {
+      const int e0 = (k * 32 + lane) * 8;
+      if (e0 >= D) continue;
+      float x[8], u[8], w[8], b[8];
+      unpack_vec<E>(in[k * 32], x);
+      unpack_vec<E>(in[(MAXV + k) * 32], u);
+      unpack_vec<E>(__ldg(reinterpret_cast<const uint4 *>((const E *)p.w + e0)), w);   // (L1)
+      unpack_vec<E>(__ldg(reinterpret_cast<const uint4 *>((const E *)p.b + e0)), b);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) x[t] = act_f(u[t], p.act) * ((x[t] - mean) * rstd * w[t] + b[t]);
+      drop.mask8(x, o[k]);
+      store_vec<E>(orow + off_y + e0, x);
+    }
+    if (lane == 0) {
+      if (p.mean) p.mean[row] = mean;
+      if (p.rstd) p.rstd[row] = rstd;
+    }
+    stage = stage + 1 == STAGES ? 0 : stage + 1;
+  }
+}
+
 // DROPOUT: 0 = none, 1 = the forward's mask regenerated from the seed, 2 = read from p.mask,
 // 3 = regenerated, rows of whole vectors
 template <typename E, int MAXV, int DROPOUT>
@@ -1071,6 +1213,139 @@ __global__ void __launch_bounds__(WARPS * 32) norm_mul_bwd_kernel(NormMulParams 
     ur.store((E *)p.du + row * p.du_rs, D, lane, p.vec_ok);
     gy.store((E *)p.dattn + row * p.dattn_rs, D, lane, p.vec_ok);
   }
+  float *prow = p.partial + (int64_t)blockIdx.x * 2 * D;
+  reduce_columns_to_partial(dw, smem, prow, D, lane, warp);
+  reduce_columns_to_partial(db, smem, prow + D, D, lane, warp);
+}
+
+// The backward with the forward's mask regenerated, for rows of up to two vectors per lane: bound by HBM and
+// by the issue of the generator's and the row's arithmetic together, so it has to keep both busy.  The rows come
+// through shared memory by asynchronous copies (every lane reads what it has copied itself: no barrier), so
+// that the registers hold the row being worked on only and two CTAs fit an SM - the kernel above, whose
+// next row waits in registers, takes 255 of them and runs with eight warps: 415 -> 372 us on 200 k rows of 512
+// (figures at other sizes where the kernel is chosen).
+// Vector path only (aligned pointers and strides, D a multiple of the vector width, 16-bit elements).
+// Shared memory: [WARPS][STAGES][5][MAXV][32] vectors: attn, u, dout's y, u and x part.
+template <typename E, int MAXV, int STAGES>
+__global__ void __launch_bounds__(WARPS * 32, 2) norm_mul_bwd_staged_kernel(NormMulParams p) {
+  static_assert(VecInfo<E>::EV == 8, "one generator call for a vector");
+  extern __shared__ uint4 ring[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int D = p.H * p.V;
+  Dropout drop;
+  drop.init(p);
+  const int off_x = p.concat_u ? D : 0;
+  const int off_y = off_x + (p.concat_x ? D : 0);
+  const int width = off_y + D;
+  const float invD = 1.f / (float)D;
+  Row<E, MAXV> dw, db;
+  dw.zero();
+  db.zero();
+  uint4 *mine = ring + warp * (STAGES * 5 * MAXV * 32) + lane;
+  auto request = [&](int64_t r, int stage) {
+    if (r < p.rows) {
+      const E *xr = (const E *)p.attn + r * p.attn_rs, *ur = (const E *)p.u + r * p.u_rs;
+      const E *gr = (const E *)p.dout + r * p.dout_rs;
+      uint4 *dst = mine + stage * (5 * MAXV * 32);
+#pragma unroll
+      for (int k = 0; k < MAXV; ++k) {
+        const int e0 = (k * 32 + lane) * 8;
+        if (e0 >= D) continue;
+        copy_async16(dst + (0 * MAXV + k) * 32, xr + e0);
+        copy_async16(dst + (1 * MAXV + k) * 32, ur + e0);
+        copy_async16(dst + (2 * MAXV + k) * 32, gr + off_y + e0);
+        if (p.concat_u) copy_async16(dst + (3 * MAXV + k) * 32, gr + e0);
+        if (p.concat_x) copy_async16(dst + (4 * MAXV + k) * 32, gr + off_x + e0);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");   // (a group for every row, so that they can be counted)
+  };
+  const int64_t step = (int64_t)gridDim.x * WARPS;
+  int64_t row = (int64_t)blockIdx.x * WARPS + warp;
+#pragma unroll
+  for (int s = 0; s + 1 < STAGES; ++s) request(row + s * step, s);
+  int stage = 0;
+  for (; row < p.rows; row += step) {
+    request(row + (STAGES - 1) * step, stage == 0 ? STAGES - 1 : stage - 1);   // the slot of the row before
+    const float mean = p.mean[row], rstd = p.rstd[row];
+    const uint64_t base = ((uint64_t)row * (uint64_t)width >> 3) + (uint64_t)lane;   // generator call of the row's first vector
+    uint32_t oy[MAXV][4], ou[MAXV][4], ox[MAXV][4];
+    auto words = [&](int off, uint32_t (&o)[MAXV][4]) {
+      uint64_t g[MAXV];
+#pragma unroll
+      for (int k = 0; k < MAXV; ++k) g[k] = base + (uint64_t)((off >> 3) + k * 32);
+      philox_many<MAXV>(drop.k0, drop.k1, g, o);
+    };
+    words(off_y, oy);
+    if (p.concat_u) words(0, ou);
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+    uint4 *in = mine + stage * (5 * MAXV * 32);
+    E *du_row = (E *)p.du + row * p.du_rs, *dx_row = (E *)p.dattn + row * p.dattn_rs;
+    float c1 = 0.f, c2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < MAXV; ++k) {
+      const int e0 = (k * 32 + lane) * 8;
+      if (e0 >= D) continue;
+      float x[8], u[8], g[8];
+      unpack_vec<E>(in[(0 * MAXV + k) * 32], x);
+      unpack_vec<E>(in[(1 * MAXV + k) * 32], u);
+      unpack_vec<E>(in[(2 * MAXV + k) * 32], g);
+      drop.mask8(g, oy[k]);
+      // (weight and bias come from L1 each time)
+      const uint4 wv = __ldg(reinterpret_cast<const uint4 *>((const E *)p.w + e0));
+      const uint4 bv = __ldg(reinterpret_cast<const uint4 *>((const E *)p.b + e0));
+      const E *pw = reinterpret_cast<const E *>(&wv), *pb = reinterpret_cast<const E *>(&bv);
+      alignas(16) float du[8], gw[8];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        const float w = to_f32(pw[t]);
+        const float xhat = (x[t] - mean) * rstd;
+        const float ga = g[t] * act_f(u[t], p.act);   // gradient w.r.t. the normalised value
+        du[t] = g[t] * (xhat * w + to_f32(pb[t])) * dact_f(u[t], p.act);
+        dw.v[k][t] += ga * xhat;
+        db.v[k][t] += ga;
+        gw[t] = ga * w;
+        c1 += gw[t] * xhat;
+        c2 += gw[t];
+      }
+      // (over what has been read, until the row's sums are there)
+      in[(1 * MAXV + k) * 32] = *reinterpret_cast<const uint4 *>(&gw[0]);
+      in[(2 * MAXV + k) * 32] = *reinterpret_cast<const uint4 *>(&gw[4]);
+      if (p.concat_u) {
+        float more[8];
+        unpack_vec<E>(in[(3 * MAXV + k) * 32], more);
+        drop.mask8(more, ou[k]);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) du[t] += more[t];
+      }
+      store_vec<E>(du_row + e0, du);
+    }
+    if (p.concat_x) words(off_x, ox);
+    c1 = warp_sum(c1) * invD;
+    c2 = warp_sum(c2) * invD;
+#pragma unroll
+    for (int k = 0; k < MAXV; ++k) {
+      const int e0 = (k * 32 + lane) * 8;
+      if (e0 >= D) continue;
+      alignas(16) float x[8], dx[8];
+      unpack_vec<E>(in[(0 * MAXV + k) * 32], x);
+      *reinterpret_cast<uint4 *>(&dx[0]) = in[(1 * MAXV + k) * 32];
+      *reinterpret_cast<uint4 *>(&dx[4]) = in[(2 * MAXV + k) * 32];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) dx[t] = (dx[t] - c2 - (x[t] - mean) * rstd * c1) * rstd;
+      if (p.concat_x) {
+        float more[8];
+        unpack_vec<E>(in[(4 * MAXV + k) * 32], more);
+        drop.mask8(more, ox[k]);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) dx[t] += more[t];
+      }
+      store_vec<E>(dx_row + e0, dx);
+    }
+    stage = stage + 1 == STAGES ? 0 : stage + 1;
+  }
+  __syncthreads();   // the column sums go over the ring
+  float *smem = reinterpret_cast<float *>(ring);
   float *prow = p.partial + (int64_t)blockIdx.x * 2 * D;
   reduce_columns_to_partial(dw, smem, prow, D, lane, warp);
   reduce_columns_to_partial(db, smem, prow + D, D, lane, warp);
@@ -1466,6 +1741,15 @@ int64_t norm_mul_mask_bytes(const b200_hstu_norm_mul_args &a) {
   return a.rows * width / 8;
 }
 
+// Which dropout kernel: device time in us, dropout 0.3, [u | attn | y], bf16, register-resident / staged rows.
+//   forward    D = 512: 300 rows 4.5 / 3.9, 2000 5.7 / 5.1, 15000 24.9 / 24.1, 30000 46.5 / 47.3, 200003 268 / 291
+//              D = 256: 8000 10.1 / 9.3, 15000 15.5 / 15.1, 30000 27.5 / 28.0, 200003 154 / 175
+//   backward   D = 512: 300 rows 12.5 / 9.8, 15000 45.8 / 38.4, 60000 134 / 120, 200003 415 / 372
+//              D = 256: 300 8.6 / 6.7, 15000 24.5 / 21.2, 60000 69.3 / 68.7, 120000 127 / 129, 200003 204 / 208
+// Few rows are few per warp: what a kernel does before its first row counts, and the staged kernels do little.
+constexpr int64_t STAGED_FWD_ROWS = 20000;
+constexpr int64_t STAGED_BWD_ROWS_ONE_VECTOR = 65536;
+
 template <typename E>
 int norm_mul_t(const b200_hstu_norm_mul_args &a, bool bwd, cudaStream_t st) {
   constexpr int EV = VecInfo<E>::EV;
@@ -1545,6 +1829,16 @@ int norm_mul_t(const b200_hstu_norm_mul_args &a, bool bwd, cudaStream_t st) {
       norm_mul_fwd_packed_kernel<E, 4, 2><<<grid, WARPS * 32, 0, st>>>(p);
     } else if (dropout && p.mask != nullptr) {
       DISPATCH_MAXV(pick_maxv<E>(D), (norm_mul_fwd_kernel<E, MV, 3><<<grid, WARPS * 32, 0, st>>>(p)));
+    } else if (EV == 8 && dropout && vec_ok && pick_maxv<E>(D) <= 2 && a.rows <= STAGED_FWD_ROWS) {
+      if constexpr (EV == 8) {
+        const bool one = pick_maxv<E>(D) == 1;
+        const size_t ring = (size_t)WARPS * 4 * 2 * (one ? 1 : 2) * 32 * sizeof(uint4);   // 64 KB, three CTAs an SM
+        auto kern = one ? norm_mul_fwd_staged_kernel<E, 1, 4> : norm_mul_fwd_staged_kernel<E, 2, 4>;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
+        if (e != cudaSuccess) return check_cuda(e, "norm_mul forward smem attribute");
+        if (grid > 3 * num_sms()) grid = 3 * num_sms();
+        kern<<<grid, WARPS * 32, ring, st>>>(p);
+      }
     } else if (dropout && D % EV == 0) {
       DISPATCH_MAXV(pick_maxv<E>(D), (norm_mul_fwd_kernel<E, MV, 2><<<grid, WARPS * 32, 0, st>>>(p)));
     } else if (dropout) {
@@ -1583,6 +1877,18 @@ int norm_mul_t(const b200_hstu_norm_mul_args &a, bool bwd, cudaStream_t st) {
       if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       kern<<<grid, WARPS * 32, smem, st>>>(p);
     });
+  } else if (EV == 8 && dropout && vec_ok && pick_maxv<E>(D) <= 2 &&
+             (pick_maxv<E>(D) == 2 || a.rows <= STAGED_BWD_ROWS_ONE_VECTOR)) {
+    if constexpr (EV == 8) {
+      const bool one = pick_maxv<E>(D) == 1;
+      const int stages = one ? 4 : 2;
+      const size_t ring = (size_t)WARPS * stages * 5 * (one ? 1 : 2) * 32 * sizeof(uint4);   // 80 KB, two CTAs an SM
+      auto kern = one ? norm_mul_bwd_staged_kernel<E, 1, 4> : norm_mul_bwd_staged_kernel<E, 2, 2>;
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
+      if (e != cudaSuccess) return check_cuda(e, "norm_mul backward smem attribute");
+      if (grid > 2 * num_sms()) grid = 2 * num_sms();
+      kern<<<grid, WARPS * 32, ring, st>>>(p);
+    }
   } else if (dropout && D % EV == 0) {
     DISPATCH_MAXV(pick_maxv<E>(D), {
       auto kern = norm_mul_bwd_kernel<E, MV, 3>;

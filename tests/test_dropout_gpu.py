@@ -261,3 +261,23 @@ def test_attention_dropout_modes():
     ref.backward(dout.float())
     P.check(("attention dropout", "bias", "out"), out, ref.detach(), offs)
     assert O.rel_l2(bd.grad, br.grad) < 2.5e-2
+
+
+@pytest.mark.parametrize("H,V,rows", [(4, 128, 20001), (4, 64, 65537), (3, 104, 20001)])
+def test_dropout_kernels_for_few_and_many_rows_agree(H, V, rows):
+    """The mask of a row depends on its number, not on the batch: a call on the first rows alone, which another
+    kernel serves, gives the same bits."""
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    D = H * V
+    attn, u = (torch.randn(rows, D, generator=g, device=DEV).bfloat16() for _ in range(2))
+    w, b = (torch.randn(D, generator=g, device=DEV).bfloat16() for _ in range(2))
+    dy = torch.randn(rows, 3 * D, generator=g, device=DEV).bfloat16()
+    seed = torch.tensor([77], dtype=torch.int64, device=DEV)
+    results = []
+    for n in (rows, 70):
+        leaves = [attn[:n].clone().requires_grad_(True), u[:n].clone().requires_grad_(True)]
+        y = G.hstu_norm_mul_dropout(leaves[0], leaves[1], w, b, 1e-6, 0.3, True, True, True, "silu", False, H, V,
+                                    dropout_seed=seed)
+        results.append((y,) + torch.autograd.grad(y, leaves, dy[:n]))
+    for many, few in zip(*results):
+        assert torch.equal(many[:70], few)
