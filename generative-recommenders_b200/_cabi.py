@@ -10,6 +10,7 @@ from ctypes import POINTER, Structure, c_char_p, c_float, c_int32, c_int64, c_vo
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libb200_hstu.so")
+HOST_PATH = os.path.join(_HERE, "_host.so")
 
 F32, BF16, F16, E4M3 = 0, 1, 2, 3
 IMPL_AUTO, IMPL_SIMT, IMPL_TCGEN05 = 0, 1, 2
@@ -242,6 +243,24 @@ def lib():
     L.b200_hstu_host_mask.restype = ctypes.c_int
     _lib = L
     return L
+
+
+_host = None
+
+
+def host():
+    """The extension module over the library that queues whole stages (csrc/host.cpp)."""
+    global _host
+    if _host is None:
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(
+                "_host.so is missing (%s). Build it with "
+                "`python generative-recommenders_b200/build.py`; there is no fallback path." % HOST_PATH
+            )
+        from . import _host as module
+        _host = module
+    return _host
 
 
 def check(status, what):

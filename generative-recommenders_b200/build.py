@@ -2,6 +2,7 @@
 
     python generative-recommenders_b200/build.py [--force] [--verbose]
 
+csrc/host.cpp becomes _host.so, the extension module through which the ops queue whole stages.
 Each csrc/*.cu becomes build/<name>.o; the objects are linked into
 generative-recommenders_b200/libb200_hstu.so.  Files are rebuilt when they or any header
 in csrc/ or include/ are newer than their object.
@@ -19,6 +20,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libb200_hstu.so")
+HOST = os.path.join(HERE, "_host.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -50,6 +52,30 @@ def _compile(src, obj, verbose):
     return src, r.returncode, r.stdout + r.stderr
 
 
+def _build_host(force, verbose):
+    """csrc/host.cpp -> _host.so, an extension module linked against the library beside it."""
+    src, hdr = os.path.join(CSRC, "host.cpp"), os.path.join(ROOT, "include", "b200_hstu.h")
+    if not force and os.path.exists(HOST) and os.path.getmtime(HOST) >= max(os.path.getmtime(src), os.path.getmtime(hdr)):
+        return
+    import sysconfig
+
+    import torch
+
+    t = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    includes = [os.path.join(t, "include"), os.path.join(t, "include", "torch", "csrc", "api", "include"),
+                sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI]
+           + [a for i in includes for a in ("-isystem", i)] + ["-I" + os.path.dirname(hdr), src, "-o", HOST]
+           + ["-L" + HERE, "-lb200_hstu", "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
+              "-ltorch", "-ltorch_python", "-L" + os.path.join(cuda, "lib64"), "-lcudart", "-Wl,-rpath,$ORIGIN"])
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0 or verbose:
+        sys.stderr.write("== host.cpp (exit %d)\n%s\n" % (r.returncode, r.stdout + r.stderr))
+    if r.returncode != 0:
+        raise RuntimeError("building _host.so failed")
+
+
 def build(force=False, verbose=False):
     os.makedirs(BUILD, exist_ok=True)
     srcs = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
@@ -74,6 +100,7 @@ def build(force=False, verbose=False):
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("link failed:\n" + r.stdout + r.stderr)
+    _build_host(force, verbose)
     return LIB
 
 

@@ -136,21 +136,13 @@ def hstu_attention_fwd(max_seq_len, alpha, q, k, v, seq_offsets, num_targets, at
     scratch tensor holding them is returned next to the output (``(out, scratch)``), to be passed
     to one ``hstu_attention_bwd`` call: one planning launch per training step instead of two."""
     L, H, _ = q.shape
-    out = torch.empty((L, H, v.shape[2]), dtype=q.dtype, device=q.device)
     if L == 0:
+        out = torch.empty((L, H, v.shape[2]), dtype=q.dtype, device=q.device)
         return (out, None) if plan_for_backward else out
-    a = _cabi.AttnArgs()
-    _fill_common(a, q, k, v, seq_offsets, num_targets, attn_scale, max_seq_len, alpha, max_attn_len,
-                 contextual_seq_len, min_full_attn_seq_len, bias_by_distance, dropout_pr, dropout_seed)
-    a.out = out.data_ptr()
-    a.o_row_stride, a.o_head_stride = out.stride(0), out.stride(1)
-    ws = _workspace(a, 2 if plan_for_backward else 0, q.device)  # kept alive until the launch is queued
-    if plan_for_backward and ws is not None:
-        a.plan_mode = _PLAN_FOR_BACKWARD
-    with on_device(q.device):
-        _cabi.check(_cabi.lib().b200_hstu_attn_fwd(a, stream_ptr(q.device)), "b200_hstu_attn_fwd")
-    if _CHECK_STATUS and ws is not None:
-        _raise_on_status(a, 0, q.device, "b200_hstu_attn_fwd")
+    out, ws = _cabi.host().attention_forward(
+        q, k, v, seq_offsets, num_targets, attn_scale, bias_by_distance, max_seq_len, alpha, max_attn_len,
+        contextual_seq_len, min_full_attn_seq_len, _IMPL[_forced_impl], dtype_code(q), plan_for_backward, dropout_pr,
+        dropout_seed, 0, _CHECK_STATUS)
     return (out, ws) if plan_for_backward else out
 
 
@@ -164,28 +156,10 @@ def hstu_attention_bwd(dout, max_seq_len, alpha, q, k, v, seq_offsets, num_targe
     bias is added into it."""
     if q.shape[0] == 0:
         return
-    a = _cabi.AttnArgs()
-    _fill_common(a, q, k, v, seq_offsets, num_targets, attn_scale, max_seq_len, alpha, max_attn_len,
-                 contextual_seq_len, min_full_attn_seq_len, bias_by_distance, dropout_pr, dropout_seed)
-    a.dout = dout.data_ptr()
-    a.dq, a.dk, a.dv_ = dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
-    a.do_row_stride, a.do_head_stride = dout.stride(0), dout.stride(1)
-    a.dq_row_stride, a.dq_head_stride = dq.stride(0), dq.stride(1)
-    a.dk_row_stride, a.dk_head_stride = dk.stride(0), dk.stride(1)
-    a.dv_row_stride, a.dv_head_stride = dv.stride(0), dv.stride(1)
-    if d_bias is not None and bias_by_distance is not None:
-        a.d_bias_by_distance = d_bias.data_ptr()
-    reuse = planned_scratch is not None and _cabi.lib().b200_hstu_attn_workspace_bytes(a, 1) > 0
-    if reuse:
-        a.plan_mode = _PLAN_REUSE
-        a.workspace = planned_scratch.data_ptr()
-        a.workspace_bytes = planned_scratch.numel()
-    else:
-        ws = _workspace(a, 1, q.device)  # noqa: F841
-    with on_device(q.device):
-        _cabi.check(_cabi.lib().b200_hstu_attn_bwd(a, stream_ptr(q.device)), "b200_hstu_attn_bwd")
-    if _CHECK_STATUS and a.workspace:
-        _raise_on_status(a, 2 if reuse else 1, q.device, "b200_hstu_attn_bwd")
+    _cabi.host().attention_backward(
+        dout, q, k, v, seq_offsets, num_targets, attn_scale, bias_by_distance, max_seq_len, alpha, max_attn_len,
+        contextual_seq_len, min_full_attn_seq_len, _IMPL[_forced_impl], dtype_code(q), dq, dk, dv, planned_scratch,
+        d_bias, dropout_pr, dropout_seed, _CHECK_STATUS)
 
 
 class _HstuMhaFunction(torch.autograd.Function):
@@ -353,21 +327,12 @@ def delta_hstu_mha(
     if k.dtype != delta_q.dtype or v.dtype != delta_q.dtype:
         raise TypeError("delta_q, k, v must share a dtype")
     delta = L // B
-    out = torch.zeros((L, H, v.shape[2]), dtype=delta_q.dtype, device=delta_q.device)
     if L == 0 or k.shape[0] == 0:
-        return out
+        return torch.zeros((L, H, v.shape[2]), dtype=delta_q.dtype, device=delta_q.device)
     q = last_dim_contiguous(delta_q.detach())
     k = last_dim_contiguous(k.detach())
     v = last_dim_contiguous(v.detach())
-    seq_offsets = _index(seq_offsets)
-    num_targets = _index(num_targets)
-    a = _cabi.AttnArgs()
-    _fill_common(a, q, k, v, seq_offsets, num_targets, None, int(max_seq_len), float(alpha), int(max_attn_len),
-                 int(contextual_seq_len), 0, None)
-    a.delta_size = delta
-    a.out = out.data_ptr()
-    a.o_row_stride, a.o_head_stride = out.stride(0), out.stride(1)
-    ws = _workspace(a, 0, q.device)  # noqa: F841  (kept alive until the launch is queued)
-    with on_device(q.device):
-        _cabi.check(_cabi.lib().b200_hstu_attn_fwd(a, stream_ptr(q.device)), "b200_hstu_attn_fwd (delta)")
+    out, _ = _cabi.host().attention_forward(
+        q, k, v, _index(seq_offsets), _index(num_targets), None, None, int(max_seq_len), float(alpha), int(max_attn_len),
+        int(contextual_seq_len), 0, _IMPL[_forced_impl], dtype_code(q), False, 0.0, None, delta, False)
     return out

@@ -9,7 +9,8 @@ import torch
 from . import _cabi
 from .common import (HammerKernel, _require_cuda_backend, as_dtype, dtype_code, on_device, outside_autograd,
                      require_cuda, stream_ptr)
-from .hstu_attention import hstu_mha
+from . import hstu_attention as _attention
+from .hstu_attention import _i32, _index, hstu_mha
 from .layer_norm import layer_norm
 from .mm import addmm
 
@@ -60,10 +61,7 @@ def _aligned16(t: torch.Tensor) -> torch.Tensor:
 def _fused_uqvk_supported(x, uvqk_weight, hv) -> bool:
     if x.dtype not in (torch.bfloat16, torch.float16) or x.dim() != 2 or x.shape[0] == 0:
         return False
-    if x.stride(-1) != 1 or x.stride(0) % 8 or x.stride(0) < x.shape[1] or x.data_ptr() % 16:
-        return False
-    D, N = uvqk_weight.shape
-    return bool(_cabi.lib().b200_hstu_ln_linear_supported(D, N, hv, dtype_code(x)))
+    return _cabi.host().uvqk_supported(x, uvqk_weight, hv, dtype_code(x))
 
 
 # Inference only: the workspace of the fused kernel holds what the preparation launches derive from
@@ -169,38 +167,7 @@ def _fused_uqvk_backward(x, nw, nb, w, uvqk, mean, rstd, eps, hv, du, d_uvqk):
     statistics (the reference's ``recompute_normed_x_in_backward``,
     generative_recommenders/ops/triton/triton_hstu_preprocess_and_attention.py:122-127, 185-203)
     and uses library GEMMs.  Returns (dx, d_norm_weight, d_norm_bias, d_weight, d_bias)."""
-    M, D = x.shape
-    lib = _cabi.lib()
-    dt = dtype_code(x)
-    st = stream_ptr(x.device)
-    with on_device(x.device):
-        if du is not None:
-            if du.stride(-1) != 1:
-                du = du.contiguous()
-            _cabi.check(lib.b200_hstu_silu_bwd(du.data_ptr(), du.stride(0), uvqk.data_ptr(), uvqk.stride(0),
-                                               d_uvqk.data_ptr(), d_uvqk.stride(0), M, hv, dt, st),
-                        "b200_hstu_silu_bwd")
-        else:
-            d_uvqk[:, :hv].zero_()
-        normed = torch.empty_like(x)
-        _cabi.check(lib.b200_hstu_layer_norm_fwd(x.data_ptr(), x.stride(0), nw.data_ptr(), nb.data_ptr(),
-                                                 normed.data_ptr(), normed.stride(0), None, None, M, D, eps, dt, st),
-                    "b200_hstu_layer_norm_fwd")
-        dw = normed.t() @ d_uvqk
-        # column sums on the tensor cores: cheaper than a strided reduction over [M, N]
-        db = (torch.ones((1, M), dtype=x.dtype, device=x.device) @ d_uvqk).view(-1)
-        dnormed = d_uvqk @ w.t()
-        dx = torch.empty_like(x)
-        dnw = torch.empty(D, dtype=x.dtype, device=x.device)
-        dnb = torch.empty(D, dtype=x.dtype, device=x.device)
-        nbytes = lib.b200_hstu_layer_norm_bwd_workspace_bytes(D)
-        partial = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
-        _cabi.check(lib.b200_hstu_layer_norm_bwd(dnormed.data_ptr(), dnormed.stride(0), x.data_ptr(), x.stride(0),
-                                                 nw.data_ptr(), mean.data_ptr(), rstd.data_ptr(), dx.data_ptr(),
-                                                 dx.stride(0), dnw.data_ptr(), dnb.data_ptr(), partial.data_ptr(),
-                                                 nbytes, M, D, dt, st),
-                    "b200_hstu_layer_norm_bwd")
-    return dx, dnw, dnb, dw, db
+    return _cabi.host().uvqk_backward(x, nw, nb, w, uvqk, mean, rstd, eps, hv, du, d_uvqk, dtype_code(x))
 
 
 def _stage_parameters(x, norm_weight, norm_bias, weight, bias):
@@ -256,6 +223,10 @@ class _FusedUqvkFunction(torch.autograd.Function):
                 as_dtype(db, b_dtype), None, None, None)
 
 
+def _attention_switches(x):
+    return _attention._IMPL[_attention._forced_impl], dtype_code(x)
+
+
 class _FusedPreprocessAttentionFunction(torch.autograd.Function):
     """The fused uvqk stage and the attention as one autograd node: the attention backward writes
     dq / dk / dv straight into the column blocks of ``d_uvqk``, which then feeds the stage's
@@ -265,19 +236,14 @@ class _FusedPreprocessAttentionFunction(torch.autograd.Function):
     def forward(ctx, x, norm_weight, norm_bias, eps, weight, bias, num_heads, attn_dim, hidden_dim, seq_offsets,
                 num_targets, bias_by_distance, max_seq_len, alpha, max_attn_len, contextual_seq_len,
                 recompute_uvqk=False):
-        from .hstu_attention import hstu_attention_fwd
-
-        hv = hidden_dim * num_heads
         nw, nb, w, b = _stage_parameters(x, norm_weight, norm_bias, weight, bias)
-        uvqk, u, mean, rstd = _fused_uqvk_launch(x, nw, nb, eps, w, b, hv)
-        q, k, v = _uqvk_views(uvqk, num_heads, attn_dim, hidden_dim)
         plan = any(ctx.needs_input_grad[:6]) or ctx.needs_input_grad[11]
         ctx.set_materialize_grads(False)  # k / v usually get no gradient: do not add zeros for them
-        out = hstu_attention_fwd(max_seq_len, alpha, q, k, v, seq_offsets, num_targets, None, max_attn_len,
-                                 contextual_seq_len, 0, bias_by_distance, plan_for_backward=plan)
-        ctx.planned_scratch = None
-        if plan:
-            out, ctx.planned_scratch = out
+        u, out, k, v, uvqk, mean, rstd, ctx.planned_scratch = _cabi.host().uvqk_attention_forward(
+            x, nw, nb, w, b, eps, num_heads, attn_dim, hidden_dim, seq_offsets, num_targets, bias_by_distance,
+            max_seq_len, alpha, max_attn_len, contextual_seq_len, *_attention_switches(x), plan, _attention._CHECK_STATUS)
+        if not plan:
+            ctx.planned_scratch = None
         # recompute_uvqk: the [M, 4 H d] projection - the largest activation of the layer - is not kept;
         # the backward runs the fused kernel once more (the reference's recompute_uvqk_in_backward,
         # generative_recommenders/ops/triton/triton_hstu_preprocess_and_attention.py:122-127, 185-203).
@@ -291,38 +257,16 @@ class _FusedPreprocessAttentionFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, du, dattn, dk_ext, dv_ext):
-        from .hstu_attention import hstu_attention_bwd
-
         x, nw, nb, w, b, uvqk, mean, rstd, seq_offsets, num_targets, bias_by_distance = ctx.saved_tensors
         (eps, H, A, V, max_seq_len, alpha, max_attn_len, contextual_seq_len,
          nw_dtype, nb_dtype, w_dtype, b_dtype) = ctx.cfg
-        hv, ha = V * H, A * H
-        if uvqk is None:   # not kept: one more launch of the fused kernel
-            uvqk, _, mean, rstd = _fused_uqvk_launch(x, nw, nb, eps, w, b, hv)
-        M, N = uvqk.shape
-        d_uvqk = torch.empty((M, N), dtype=x.dtype, device=x.device)
-        dv = d_uvqk[:, hv:2 * hv].view(M, H, V)
-        dq = d_uvqk[:, 2 * hv:2 * hv + ha].view(M, H, A)
-        dk = d_uvqk[:, 2 * hv + ha:].view(M, H, A)
-        d_bias = None
-        if dattn is None:
-            d_uvqk[:, hv:].zero_()
-        else:
-            if (dattn.stride(-1) != 1 or dattn.stride(1) != dattn.shape[2]
-                    or dattn.stride(0) < dattn.shape[1] * dattn.shape[2]):
-                dattn = dattn.contiguous()
-            q_, k_, v_ = _uqvk_views(uvqk, H, A, V)
+        planned = None
+        if dattn is not None:
             planned, ctx.planned_scratch = ctx.planned_scratch, None
-            if bias_by_distance is not None and ctx.needs_input_grad[11]:
-                d_bias = torch.zeros_like(bias_by_distance)
-            hstu_attention_bwd(dattn, max_seq_len, alpha, q_, k_, v_, seq_offsets, num_targets, None, max_attn_len,
-                               contextual_seq_len, 0, dq, dk, dv, bias_by_distance, planned_scratch=planned,
-                               d_bias=d_bias)
-        if dk_ext is not None:
-            dk.add_(dk_ext)
-        if dv_ext is not None:
-            dv.add_(dv_ext)
-        dx, dnw, dnb, dw, db = _fused_uqvk_backward(x, nw, nb, w, uvqk, mean, rstd, eps, hv, du, d_uvqk)
+        dx, dnw, dnb, dw, db, d_bias = _cabi.host().uvqk_attention_backward(
+            x, nw, nb, w, b, uvqk, mean, rstd, eps, H, A, V, seq_offsets, num_targets, bias_by_distance, max_seq_len,
+            alpha, max_attn_len, contextual_seq_len, *_attention_switches(x), du, dattn, dk_ext, dv_ext, planned,
+            bias_by_distance is not None and ctx.needs_input_grad[11], _attention._CHECK_STATUS)
         return (dx, as_dtype(dnw, nw_dtype), as_dtype(dnb, nb_dtype), None, as_dtype(dw, w_dtype),
                 as_dtype(db, b_dtype), None, None, None, None, None, d_bias, None, None, None, None, None)
 
@@ -375,74 +319,19 @@ def _norm_mul_forward(attn, u, weight, bias, eps, num_heads, linear_dim, concat_
     """One launch of the norm-mul kernel; returns ``(out, mean, rstd)`` (inputs already contiguous in
     their last dimension, weight / bias already of the activation dtype); without ``stats`` the last two
     are None."""
-    rows = attn.shape[0]
-    D = num_heads * linear_dim
-    if group_norm:
-        mult = 3 if (concat_u and concat_x) else 1
-    else:
-        mult = 1 + int(concat_u) + int(concat_x)
-    out = torch.empty((rows, mult * D), dtype=attn.dtype, device=attn.device)
-    groups = num_heads if group_norm else 1
-    mean = torch.empty(rows * groups, dtype=torch.float32, device=attn.device) if stats else None
-    rstd = torch.empty(rows * groups, dtype=torch.float32, device=attn.device) if stats else None
-    a = _cabi.NormMulArgs()
-    a.attn, a.u, a.weight, a.bias = attn.data_ptr(), u.data_ptr(), weight.data_ptr(), bias.data_ptr()
-    a.out = out.data_ptr()
-    if stats:
-        a.mean, a.rstd = mean.data_ptr(), rstd.data_ptr()
-    a.attn_row_stride, a.u_row_stride, a.out_row_stride = attn.stride(0), u.stride(0), out.stride(0)
-    a.rows, a.H, a.V = rows, num_heads, linear_dim
-    a.concat_u, a.concat_x, a.act, a.group_norm = int(concat_u), int(concat_x), act, int(group_norm)
-    a.eps, a.dtype = eps, dtype_code(attn)
-    mask = None
-    if dropout_seed is not None and dropout_ratio > 0.0:
-        a.dropout_ratio, a.dropout_seed = dropout_ratio, dropout_seed.data_ptr()
-        if want_mask and rows > 0:
-            # one bit per output element, for a backward that reads the mask instead of running the
-            # generator again (where the library can store it: 16-bit elements, whole aligned vectors)
-            nbytes = _cabi.lib().b200_hstu_norm_mul_dropout_mask_bytes(a)
-            if nbytes > 0:
-                mask = torch.empty(nbytes, dtype=torch.uint8, device=attn.device)
-                a.dropout_mask = mask.data_ptr()
-    if rows > 0:
-        with on_device(attn.device):
-            _cabi.check(_cabi.lib().b200_hstu_norm_mul_fwd(a, stream_ptr(attn.device)), "b200_hstu_norm_mul_fwd")
-    if want_mask:
-        return out, mean, rstd, mask
-    return out, mean, rstd
+    result = _cabi.host().norm_mul_forward(
+        attn, u, weight, bias, eps, num_heads, linear_dim, concat_u, concat_x, act, group_norm, dropout_ratio, dropout_seed,
+        dtype_code(attn), want_mask, stats)
+    return result if want_mask else result[:3]
 
 
 def _norm_mul_backward(dout, attn, u, weight, bias, mean, rstd, eps, num_heads, linear_dim, concat_u, concat_x, act,
                        group_norm, dropout_ratio, dropout_seed, dropout_mask=None):
     """Backward of the norm-mul kernel; returns ``(dattn, du, dweight, dbias)``.  ``dropout_mask``: the
     bits the forward stored; without them the kernel regenerates the mask from the seed."""
-    rows = attn.shape[0]
-    if dout.stride(-1) != 1:
-        dout = dout.contiguous()
-    dattn = torch.empty((rows, num_heads * linear_dim), dtype=attn.dtype, device=attn.device)
-    du = torch.empty_like(dattn)
-    dw = torch.empty_like(weight)
-    db = torch.empty_like(bias)
-    nbytes = _cabi.lib().b200_hstu_norm_mul_bwd_workspace_bytes(num_heads, linear_dim, int(group_norm))
-    partial = torch.empty(nbytes, dtype=torch.uint8, device=attn.device)
-    a = _cabi.NormMulArgs()
-    a.attn, a.u, a.weight, a.bias = attn.data_ptr(), u.data_ptr(), weight.data_ptr(), bias.data_ptr()
-    a.mean, a.rstd = mean.data_ptr(), rstd.data_ptr()
-    a.dout, a.dattn, a.du = dout.data_ptr(), dattn.data_ptr(), du.data_ptr()
-    a.dweight, a.dbias = dw.data_ptr(), db.data_ptr()
-    a.partial, a.partial_bytes = partial.data_ptr(), nbytes
-    a.attn_row_stride, a.u_row_stride = attn.stride(0), u.stride(0)
-    a.dout_row_stride, a.dattn_row_stride, a.du_row_stride = dout.stride(0), dattn.stride(0), du.stride(0)
-    a.rows, a.H, a.V = rows, num_heads, linear_dim
-    a.concat_u, a.concat_x, a.act, a.group_norm = int(concat_u), int(concat_x), act, int(group_norm)
-    a.eps, a.dtype = eps, dtype_code(attn)
-    if dropout_seed is not None and dropout_ratio > 0.0:   # the forward's mask: stored bits, or regenerated
-        a.dropout_ratio, a.dropout_seed = dropout_ratio, dropout_seed.data_ptr()
-        if dropout_mask is not None and dout.data_ptr() % 16 == 0 and dout.stride(0) % 8 == 0:
-            a.dropout_mask = dropout_mask.data_ptr()
-    with on_device(attn.device):
-        _cabi.check(_cabi.lib().b200_hstu_norm_mul_bwd(a, stream_ptr(attn.device)), "b200_hstu_norm_mul_bwd")
-    return dattn, du, dw, db
+    return _cabi.host().norm_mul_backward(
+        dout, attn, u, weight, bias, mean, rstd, eps, num_heads, linear_dim, concat_u, concat_x, act, group_norm,
+        dropout_ratio, dropout_seed, dropout_mask, dtype_code(attn))
 
 
 # By default the backward of the norm-mul stage regenerates the dropout mask from the seed and nothing
@@ -506,8 +395,7 @@ class _OutputStageFunction(torch.autograd.Function):
         b = as_dtype(bias, attn.dtype).contiguous()
         wo = as_dtype(output_weight, x.dtype)
         cfg = (eps, num_heads, linear_dim, concat_u, concat_x, act, group_norm, dropout_ratio)
-        y, mean, rstd = _norm_mul_forward(attn, u, w, b, *cfg, dropout_seed)
-        out = torch.addmm(x, y, wo)
+        out, mean, rstd = _cabi.host().output_forward(attn, u, x, w, b, wo, *cfg, dropout_seed, dtype_code(attn), True)
         ctx.save_for_backward(attn, u, w, b, wo, mean, rstd, dropout_seed)
         ctx.cfg = cfg
         ctx.dtypes = (weight.dtype, bias.dtype, output_weight.dtype)
@@ -516,13 +404,10 @@ class _OutputStageFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         attn, u, w, b, wo, mean, rstd, dropout_seed = ctx.saved_tensors
-        y, _, _ = _norm_mul_forward(attn, u, w, b, *ctx.cfg, dropout_seed)
         if dout.stride(-1) != 1:
             dout = dout.contiguous()
-        d_wo = y.t() @ dout
-        del y
-        dy = dout @ wo.t()
-        dattn, du, dw, db = _norm_mul_backward(dy, attn, u, w, b, mean, rstd, *ctx.cfg, dropout_seed)
+        dattn, du, dw, db, d_wo = _cabi.host().output_backward(dout, attn, u, w, b, wo, mean, rstd, *ctx.cfg, dropout_seed,
+                                                               dtype_code(attn))
         wdt, bdt, odt = ctx.dtypes
         return (dattn, du, dout, as_dtype(dw, wdt), as_dtype(db, bdt), as_dtype(d_wo, odt), None, None, None, None,
                 None, None, None, None, None)
@@ -622,6 +507,16 @@ def hstu_compute_output(
             return _OutputStageFunction.apply(attn, u, x, norm_weight, norm_bias, output_weight, float(norm_eps),
                                               int(num_heads), int(ld), cu, cx, 0 if g_ else _ACT[mul_u_activation_type],
                                               g_, float(dropout_ratio) if seed is not None else 0.0, seed)
+    drop = training and dropout_ratio > 0.0
+    if (not group_norm and mul_u_activation_type in _ACT and not (drop and dropout_ratio >= 1.0)
+            and outside_autograd(attn, u, x, norm_weight, norm_bias, output_weight)):
+        return _cabi.host().output_forward(
+            attn if attn.stride(-1) == 1 else attn.contiguous(), u if u.stride(-1) == 1 else u.contiguous(), x,
+            as_dtype(norm_weight, attn.dtype).contiguous(), as_dtype(norm_bias, attn.dtype).contiguous(),
+            as_dtype(output_weight, x.dtype), float(norm_eps), int(num_heads),
+            int(linear_dim) if linear_dim > 0 else attn.shape[1] // num_heads, bool(concat_u), bool(concat_x),
+            _ACT[mul_u_activation_type], False, float(dropout_ratio) if drop else 0.0,
+            _draw_dropout_seed(attn.device) if drop else None, dtype_code(attn), False)[0]
     y = hstu_norm_mul_dropout(attn, u, norm_weight, norm_bias, norm_eps, dropout_ratio, training, concat_u, concat_x,
                               mul_u_activation_type, group_norm, num_heads, linear_dim)
     return addmm(x, y, as_dtype(output_weight, x.dtype), kernel)
@@ -668,7 +563,6 @@ def hstu_preprocess_and_attention(
     if (_FUSED_UQVK and x.is_cuda and _fused_uqvk_supported(x, uvqk_weight, hv)
             and attn_dim == hidden_dim and attn_dim in (64, 128)):
         # one autograd node for the stage and the attention (see _FusedPreprocessAttentionFunction)
-        from .hstu_attention import _i32, _index, hstu_attention_fwd
         require_cuda(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias, seq_offsets, num_targets, bias_by_distance)
         inference = outside_autograd(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias, bias_by_distance)
         offs = _index(seq_offsets) if inference else _i32(seq_offsets)
@@ -677,11 +571,16 @@ def hstu_preprocess_and_attention(
             raise RuntimeError("num_targets must have one entry per sequence")
         rab = None if bias_by_distance is None else bias_by_distance.to(torch.float32).reshape(-1).contiguous()
         if inference:
-            u, q, k, v = _fused_uqvk_inference(x, norm_weight, norm_bias, float(norm_eps), uvqk_weight, uvqk_bias,
-                                               num_heads, attn_dim, hidden_dim)
-            attn = hstu_attention_fwd(int(max_seq_len), float(attn_alpha), q, k, v, offs, nt, None,
-                                      int(max_attn_len), int(contextual_seq_len), 0, rab)
-            return u, attn.view(-1, hv), k, v
+            nw, nb, w, b = _stage_parameters(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias)
+            nbytes = _cabi.lib().b200_hstu_ln_linear_workspace_bytes(*w.shape)
+            ws, prepared, remember = _prepared_workspace(nw, nb, w, b, nbytes, x.device, True)
+            result = _cabi.host().uvqk_attention_inference(
+                x, nw, nb, w, b, float(norm_eps), num_heads, attn_dim, hidden_dim, ws, prepared, offs, nt, rab,
+                int(max_seq_len), float(attn_alpha), int(max_attn_len), int(contextual_seq_len),
+                *_attention_switches(x), _attention._CHECK_STATUS)
+            if remember is not None:
+                remember()
+            return result
         u, attn, k, v = _FusedPreprocessAttentionFunction.apply(
             x, norm_weight, norm_bias, float(norm_eps), uvqk_weight, uvqk_bias, num_heads, attn_dim, hidden_dim,
             offs, nt, rab, int(max_seq_len), float(attn_alpha), int(max_attn_len), int(contextual_seq_len),
