@@ -40,6 +40,7 @@ EXPORTS = [
     "b200_hstu_ln_linear_supported",
     "b200_hstu_concat_2d_jagged",
     "b200_hstu_split_2d_jagged",
+    "b200_hstu_append_kv",
     "b200_hstu_add_timestamp_positional_embeddings_fwd",
     "b200_hstu_add_timestamp_positional_embeddings_bwd",
     "b200_hstu_last_error",

@@ -78,6 +78,7 @@ int layer_norm_bwd(const void *dy, int64_t dy_rs, const void *x, int64_t x_rs, c
                    int64_t partial_bytes, int64_t rows, int D, int dtype, cudaStream_t st);
 int64_t stage_bwd_workspace_bytes(int cols);
 int jagged_concat_split(const b200_hstu_jagged_args &j, bool split, cudaStream_t st);
+int append_kv(const b200_hstu_append_kv_args &p, cudaStream_t st);
 int ts_pos_fwd(const b200_hstu_ts_pos_args &p, cudaStream_t st);
 int ts_pos_bwd(const b200_hstu_ts_pos_args &p, cudaStream_t st);
 int ln_linear_fwd(const b200_hstu_ln_linear_args &a, cudaStream_t st);
@@ -230,6 +231,10 @@ int b200_hstu_concat_2d_jagged(const b200_hstu_jagged_args *args, b200_hstu_stre
 int b200_hstu_split_2d_jagged(const b200_hstu_jagged_args *args, b200_hstu_stream_t stream) {
   if (!args) return fail(B200_HSTU_EINVAL, "split_2D_jagged: NULL args");
   return jagged_concat_split(*args, true, (cudaStream_t)stream);
+}
+int b200_hstu_append_kv(const b200_hstu_append_kv_args *args, b200_hstu_stream_t stream) {
+  if (!args) return fail(B200_HSTU_EINVAL, "append_kv: NULL args");
+  return append_kv(*args, (cudaStream_t)stream);
 }
 int b200_hstu_add_timestamp_positional_embeddings_fwd(const b200_hstu_ts_pos_args *args, b200_hstu_stream_t stream) {
   if (!args) return fail(B200_HSTU_EINVAL, "add_timestamp_positional_embeddings: NULL args");

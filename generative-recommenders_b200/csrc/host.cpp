@@ -119,16 +119,17 @@ void check_status(const b200_hstu_attn_args &a, int which, cudaStream_t stream, 
                              "]); the output is incomplete");
 }
 
-// `delta` > 0: cached inference (q holds the last `delta` rows of every sequence); rows that no sequence
-// has are zero.  Returns the output and the scratch (for the backward's plan, and the status words).
+// `delta` > 0: cached inference (q holds the last `delta` rows of every sequence); rows of sequences shorter than
+// that are zero (`long_enough`: there are none).  Returns the output and the scratch (for the backward's plan, and the status words).
 std::tuple<Tensor, MaybeTensor> attention_forward(const Tensor &q, const Tensor &k, const Tensor &v,
                                                   const Tensor &offsets, const MaybeTensor &targets,
                                                   const MaybeTensor &scale, const MaybeTensor &bias,
                                                   int64_t max_seq_len, double alpha, int64_t max_attn_len,
                                                   int64_t contextual_seq_len, int64_t min_full_attn_seq_len,
                                                   int64_t impl, int64_t dtype, bool plan, double dropout,
-                                                  const MaybeTensor &seed, int64_t delta, bool status) {
-  Tensor out = delta > 0 ? at::zeros({q.size(0), q.size(1), v.size(2)}, q.options())
+                                                  const MaybeTensor &seed, int64_t delta, bool long_enough,
+                                                  bool status) {
+  Tensor out = delta > 0 && !long_enough ? at::zeros({q.size(0), q.size(1), v.size(2)}, q.options())
                          : at::empty({q.size(0), q.size(1), v.size(2)}, q.options());
   b200_hstu_attn_args a = {};
   fill_attn(a, q, k, v, offsets, targets, scale, bias,
@@ -392,8 +393,44 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> uvqk_attention_inference(
   const Qkv t = qkv_views(s.uvqk, H, A, V);
   Tensor out = std::get<0>(attention_forward(t.q, t.k, t.v, offsets, targets, std::nullopt, bias, max_seq_len, alpha,
                                              max_attn_len, contextual_seq_len, 0, impl, dtype, false, 0.0, std::nullopt, 0,
-                                             status));
+                                             true, status));
   return {s.u, out.view({x.size(0), H * V}), t.k, t.v};
+}
+
+// Cached inference: uvqk stage on the new rows, their K and V behind the cached ones, attention of the new rows.
+// Returns u, attention output, k, v, offsets of k and v.
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> cached_attention(
+    const Tensor &x, const Tensor &nw, const Tensor &nb, const Tensor &w, const Tensor &b, double eps, int64_t H,
+    int64_t A, int64_t V, const Tensor &workspace, bool prepared, const Tensor &k_cache, const Tensor &v_cache,
+    const Tensor &cache_offsets, const MaybeTensor &targets, int64_t max_seq_len, double alpha, int64_t max_attn_len,
+    int64_t contextual_seq_len, int64_t impl, int64_t dtype) {
+  const int64_t B = cache_offsets.numel() - 1, delta = x.size(0) / B, rows = k_cache.size(0) + x.size(0);
+  const Uvqk s = uvqk_launch(x, nw, nb, w, b, eps, H * V, dtype, true, workspace, prepared);
+  const Qkv t = qkv_views(s.uvqk, H, A, V);
+  Tensor k = empty_like_of({rows, H, A}, x), v = empty_like_of({rows, H, V}, x);
+  Tensor offsets = at::empty({B + 1}, cache_offsets.options());
+  b200_hstu_append_kv_args a = {};
+  a.k_cache = ptr(k_cache);
+  a.v_cache = ptr(v_cache);
+  a.k_new = ptr(t.k);
+  a.v_new = ptr(t.v);
+  a.k = ptr(k);
+  a.v = ptr(v);
+  a.offsets = static_cast<const int64_t *>(cache_offsets.data_ptr());
+  a.full_offsets = static_cast<int64_t *>(offsets.data_ptr());
+  a.k_row_bytes = H * A * x.element_size();
+  a.v_row_bytes = H * V * x.element_size();
+  a.k_new_stride_bytes = t.k.stride(0) * x.element_size();
+  a.v_new_stride_bytes = t.v.stride(0) * x.element_size();
+  a.cached_rows = k_cache.size(0);
+  a.B = (int32_t)B;
+  a.delta = (int32_t)delta;
+  Launch l(x);
+  check(b200_hstu_append_kv(&a, l.stream), "b200_hstu_append_kv");
+  Tensor out = std::get<0>(attention_forward(t.q, k, v, offsets, targets, std::nullopt, std::nullopt, max_seq_len, alpha,
+                                             max_attn_len, contextual_seq_len, 0, impl, dtype, false, 0.0, std::nullopt,
+                                             delta, true, false));
+  return {s.u, out.view({x.size(0), H * V}), k, v, offsets};
 }
 
 // u, attention output, k, v, uvqk, mean, rstd, scratch with the backward's plan
@@ -405,7 +442,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, MaybeTensor> 
   const Uvqk s = uvqk_launch(x, nw, nb, w, b, eps, H * V, dtype, false, std::nullopt, false);
   const Qkv t = qkv_views(s.uvqk, H, A, V);
   auto [out, ws] = attention_forward(t.q, t.k, t.v, offsets, targets, std::nullopt, bias, max_seq_len, alpha, max_attn_len,
-                                     contextual_seq_len, 0, impl, dtype, plan, 0.0, std::nullopt, 0, status);
+                                     contextual_seq_len, 0, impl, dtype, plan, 0.0, std::nullopt, 0, true, status);
   return {s.u, out, t.k, t.v, s.uvqk, *s.mean, *s.rstd, ws};
 }
 
@@ -502,6 +539,7 @@ PYBIND11_MODULE(_host, m) {
   m.def("uvqk_supported", &uvqk_supported, unlocked);
   m.def("uvqk_backward", &uvqk_backward, unlocked);
   m.def("uvqk_attention_inference", &uvqk_attention_inference, unlocked);
+  m.def("cached_attention", &cached_attention, unlocked);
   m.def("uvqk_attention_forward", &uvqk_attention_forward, unlocked);
   m.def("uvqk_attention_backward", &uvqk_attention_backward, unlocked);
 }

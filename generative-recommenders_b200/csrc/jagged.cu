@@ -106,6 +106,74 @@ int launch_jagged(const JaggedArgs &a, bool split, cudaStream_t st) {
   return 0;
 }
 
+// Cached K and V of every sequence followed by its `delta` new rows, both tensors (blockIdx.y) and the
+// offsets of the result in one launch.  The new rows are read where they lie (column blocks of the uvqk
+// buffer: a row stride of their own).  Bound by the copy itself: 32 users, 17 k cached rows of 1 KB, 20 new
+// rows each 11 us, where two concatenations, two copies that made the new rows contiguous and the arithmetic
+// on the offsets took 28 us and seven launches.
+struct AppendKvArgs {
+  const char *cache[2], *fresh[2];
+  char *full[2];
+  int64_t fresh_stride[2], row_bytes[2];   // bytes
+  const int64_t *off;                      // of the cache, [B + 1]
+  int64_t *off_full;                       // of the result, [B + 1]
+  int64_t total;                           // rows of the result
+  int B, delta;
+};
+
+template <typename V>
+__global__ void __launch_bounds__(JAG_THREADS) append_kv_kernel(AppendKvArgs a) {
+  __shared__ const char *source[JAG_ROWS];
+  const bool is_v = blockIdx.y != 0;
+  const char *cache = is_v ? a.cache[1] : a.cache[0], *fresh = is_v ? a.fresh[1] : a.fresh[0];
+  const int64_t fresh_stride = is_v ? a.fresh_stride[1] : a.fresh_stride[0];
+  const int64_t row_bytes = is_v ? a.row_bytes[1] : a.row_bytes[0];
+  const int64_t g0 = (int64_t)blockIdx.x * JAG_ROWS;
+  const int rows = (int)((a.total - g0) < JAG_ROWS ? (a.total - g0) : JAG_ROWS);
+  if (blockIdx.x == 0 && !is_v)
+    for (int b = threadIdx.x; b <= a.B; b += JAG_THREADS) a.off_full[b] = a.off[b] + (int64_t)a.delta * b;
+  if ((int)threadIdx.x < rows) {
+    const int64_t g = g0 + threadIdx.x;
+    int lo = 0, hi = a.B;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (a.off[mid] + (int64_t)a.delta * mid <= g) lo = mid; else hi = mid;
+    }
+    const int64_t start = a.off[lo], len = a.off[lo + 1] - start, pos = g - start - (int64_t)a.delta * lo;
+    const char *src = nullptr;   // a row the offsets do not account for is skipped
+    if (pos >= 0 && pos < len) src = cache + (start + pos) * row_bytes;
+    else if (pos >= len && pos < len + a.delta) src = fresh + ((int64_t)a.delta * lo + pos - len) * fresh_stride;
+    source[threadIdx.x] = src;
+  }
+  __syncthreads();
+  const int per_row = (int)(row_bytes / (int64_t)sizeof(V));
+  const int n = rows * per_row;
+  V *__restrict__ out = (V *)((is_v ? a.full[1] : a.full[0]) + g0 * row_bytes);
+  constexpr int UNROLL = 4;
+  for (int base = threadIdx.x; base < n; base += JAG_THREADS * UNROLL) {
+    V val[UNROLL];
+    bool have[UNROLL];
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      const int i = base + u * JAG_THREADS;
+      const int r = i / per_row;
+      have[u] = i < n && source[r] != nullptr;
+      if (have[u]) val[u] = ((const V *)source[r])[i - r * per_row];
+    }
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u)
+      if (have[u]) out[base + u * JAG_THREADS] = val[u];
+  }
+}
+
+template <typename V>
+int launch_append_kv(const AppendKvArgs &a, cudaStream_t st) {
+  append_kv_kernel<V><<<dim3((unsigned)((a.total + JAG_ROWS - 1) / JAG_ROWS), 2), JAG_THREADS, 0, st>>>(a);
+  count_launch();
+  B200_CHECK_LAUNCH("append_kv_kernel");
+  return 0;
+}
+
 // ---------------------------------------------------------------------------------------
 // timestamp + position embeddings
 // ---------------------------------------------------------------------------------------
@@ -411,6 +479,39 @@ int jagged_concat_split(const b200_hstu_jagged_args &j, bool split, cudaStream_t
   if ((align & 3) == 0) return launch_jagged<uint32_t>(a, split, st);
   if ((align & 1) == 0) return launch_jagged<uint16_t>(a, split, st);
   return launch_jagged<uint8_t>(a, split, st);
+}
+
+int append_kv(const b200_hstu_append_kv_args &p, cudaStream_t st) {
+  if (p.B < 0 || p.delta < 0 || p.cached_rows < 0 || p.k_row_bytes <= 0 || p.v_row_bytes <= 0)
+    return fail(B200_HSTU_EINVAL, "append_kv: negative size");
+  AppendKvArgs a;
+  a.total = p.cached_rows + (int64_t)p.B * p.delta;
+  if (p.B == 0 || a.total == 0) return 0;
+  if (!p.offsets || !p.full_offsets || !p.k || !p.v || (p.cached_rows > 0 && (!p.k_cache || !p.v_cache)) ||
+      (p.delta > 0 && (!p.k_new || !p.v_new)))
+    return fail(B200_HSTU_EINVAL, "append_kv: null tensor");
+  a.cache[0] = (const char *)p.k_cache;
+  a.cache[1] = (const char *)p.v_cache;
+  a.fresh[0] = (const char *)p.k_new;
+  a.fresh[1] = (const char *)p.v_new;
+  a.full[0] = (char *)p.k;
+  a.full[1] = (char *)p.v;
+  a.fresh_stride[0] = p.k_new_stride_bytes;
+  a.fresh_stride[1] = p.v_new_stride_bytes;
+  a.row_bytes[0] = p.k_row_bytes;
+  a.row_bytes[1] = p.v_row_bytes;
+  a.off = p.offsets;
+  a.off_full = p.full_offsets;
+  a.B = p.B;
+  a.delta = p.delta;
+  ProfileScope prof(PROF_JAGGED, st);
+  uintptr_t align = 0;
+  for (int t = 0; t < 2; ++t)
+    align |= (uintptr_t)a.cache[t] | (uintptr_t)a.fresh[t] | (uintptr_t)a.full[t] | (uintptr_t)a.fresh_stride[t] |
+             (uintptr_t)a.row_bytes[t];
+  if ((align & 15) == 0) return launch_append_kv<uint4>(a, st);
+  if ((align & 3) == 0) return launch_append_kv<uint32_t>(a, st);
+  return launch_append_kv<uint8_t>(a, st);
 }
 
 static int fill_ts_pos(const b200_hstu_ts_pos_args &p, TsPosArgs &a) {

@@ -142,7 +142,7 @@ def hstu_attention_fwd(max_seq_len, alpha, q, k, v, seq_offsets, num_targets, at
     out, ws = _cabi.host().attention_forward(
         q, k, v, seq_offsets, num_targets, attn_scale, bias_by_distance, max_seq_len, alpha, max_attn_len,
         contextual_seq_len, min_full_attn_seq_len, _IMPL[_forced_impl], dtype_code(q), plan_for_backward, dropout_pr,
-        dropout_seed, 0, _CHECK_STATUS)
+        dropout_seed, 0, True, _CHECK_STATUS)
     return (out, ws) if plan_for_backward else out
 
 
@@ -334,5 +334,5 @@ def delta_hstu_mha(
     v = last_dim_contiguous(v.detach())
     out, _ = _cabi.host().attention_forward(
         q, k, v, _index(seq_offsets), _index(num_targets), None, None, int(max_seq_len), float(alpha), int(max_attn_len),
-        int(contextual_seq_len), 0, _IMPL[_forced_impl], dtype_code(q), False, 0.0, None, delta, False)
+        int(contextual_seq_len), 0, _IMPL[_forced_impl], dtype_code(q), False, 0.0, None, delta, False, False)
     return out

@@ -281,6 +281,34 @@ def set_fused_uqvk(on: bool) -> None:
     _FUSED_UQVK = bool(on)
 
 
+def hstu_cached_attention(x, norm_weight, norm_bias, norm_eps, num_heads, attn_dim, hidden_dim, uvqk_weight, uvqk_bias,
+                          k_cache, v_cache, cache_offsets, num_targets, max_seq_len, attn_alpha, max_attn_len,
+                          contextual_seq_len):
+    """The uvqk stage on the new rows of every sequence, their K and V behind the cached ones, and the attention
+    of the new rows against both: ``(u, attn [M, H dv], k, v, seq_offsets)``, or None where the separate
+    ops have to do it."""
+    hv, ha, M = hidden_dim * num_heads, attn_dim * num_heads, x.shape[0]
+    B = cache_offsets.numel() - 1
+    if not (_FUSED_UQVK and x.is_cuda and _fused_uqvk_supported(x, uvqk_weight, hv) and B > 0 and M % B == 0
+            and cache_offsets.dtype is torch.int64 and cache_offsets.is_contiguous() and not _attention._CHECK_STATUS
+            and outside_autograd(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias, k_cache, v_cache)):
+        return None
+    for t, width in ((k_cache, ha), (v_cache, hv)):
+        if t.dim() != 2 or t.shape[1] != width or t.dtype is not x.dtype or not t.is_contiguous():
+            return None
+    require_cuda(norm_weight, norm_bias, uvqk_weight, uvqk_bias, k_cache, v_cache, cache_offsets, num_targets)
+    nw, nb, w, b = _stage_parameters(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias)
+    nbytes = _cabi.lib().b200_hstu_ln_linear_workspace_bytes(*w.shape)
+    ws, prepared, remember = _prepared_workspace(nw, nb, w, b, nbytes, x.device, True)
+    result = _cabi.host().cached_attention(
+        x, nw, nb, w, b, float(norm_eps), num_heads, attn_dim, hidden_dim, ws, prepared, k_cache, v_cache,
+        cache_offsets, _index(num_targets), int(max_seq_len), float(attn_alpha), int(max_attn_len),
+        int(contextual_seq_len), *_attention_switches(x))
+    if remember is not None:
+        remember()
+    return result
+
+
 def hstu_compute_uqvk(
     x: torch.Tensor,
     norm_weight: torch.Tensor,

@@ -24,7 +24,8 @@ import torch
 
 from .common import HammerKernel, as_dtype, span
 from .hstu_attention import delta_hstu_mha
-from .hstu_compute import hstu_compute_output, hstu_compute_uqvk, hstu_preprocess_and_attention
+from .hstu_compute import (hstu_cached_attention, hstu_compute_output, hstu_compute_uqvk,
+                           hstu_preprocess_and_attention)
 from .jagged_tensors import concat_2D_jagged, split_2D_jagged
 
 
@@ -183,6 +184,50 @@ class STULayer(torch.nn.Module):
         (reference stu.py:358-424); ``delta_x`` is ``[B * delta_size, D]``."""
         if self._rel_bias_table is not None:
             raise NotImplementedError("cached_forward with a relative bias table")
+        num_targets_ = num_targets if self._target_aware else None
+        fused = None
+        if (self.k_cache is not None and self.v_cache is not None and self.kv_caching_offsets is not None
+                and type(self).construct_full_kv is STULayer.construct_full_kv
+                and delta_x.dim() == 2 and delta_x.shape[0] > 0):
+            delta_size = delta_x.shape[0] // (self.kv_caching_offsets.numel() - 1)
+            max_seq_len = self.max_kv_caching_len + delta_size
+            with span("## delta_hstu_mha ##"):
+                fused = hstu_cached_attention(
+                    delta_x, as_dtype(self._input_norm_weight, delta_x.dtype),
+                    as_dtype(self._input_norm_bias, delta_x.dtype), 1e-6, self._num_heads, self._attention_dim,
+                    self._hidden_dim, as_dtype(self._uvqk_weight, delta_x.dtype),
+                    as_dtype(self._uvqk_beta, delta_x.dtype), self.k_cache, self.v_cache, self.kv_caching_offsets,
+                    num_targets_, max_seq_len, self._attn_alpha, self._max_attn_len, self._contextual_seq_len)
+        if fused is not None:
+            delta_u, delta_attn_output, k, v, seq_offsets = fused
+            self.update_kv_cache(max_seq_len=max_seq_len, seq_offsets=seq_offsets, k=k, v=v,
+                                 max_kv_caching_len=max_kv_caching_len, kv_caching_lengths=kv_caching_lengths)
+        else:
+            delta_u, delta_attn_output = self._cached_attention_of_ops(delta_x, num_targets_, max_kv_caching_len,
+                                                                       kv_caching_lengths)
+        with span("## stu_compute_output ##"):
+            return hstu_compute_output(
+                attn=delta_attn_output,
+                u=delta_u,
+                x=delta_x,
+                norm_weight=as_dtype(self._output_norm_weight, delta_x.dtype),
+                norm_bias=as_dtype(self._output_norm_bias, delta_x.dtype),
+                norm_eps=1e-6,
+                dropout_ratio=self._output_dropout_ratio,
+                output_weight=as_dtype(self._output_weight, delta_x.dtype),
+                group_norm=self._use_group_norm,
+                num_heads=self._num_heads,
+                linear_dim=self._hidden_dim,
+                concat_u=True,
+                concat_x=True,
+                mul_u_activation_type="none",
+                training=self.training,
+                kernel=self._hammer_kernel,
+                recompute_y_in_backward=False,
+            )
+
+    def _cached_attention_of_ops(self, delta_x, num_targets, max_kv_caching_len, kv_caching_lengths):
+        """``(u, attention output)`` of ``cached_forward`` from the separate ops."""
         with span("## stu_compute_uqvk ##"):
             delta_u, delta_q, delta_k, delta_v = hstu_compute_uqvk(
                 x=delta_x,
@@ -210,31 +255,12 @@ class STULayer(torch.nn.Module):
                 k=k,
                 v=v,
                 seq_offsets=seq_offsets,
-                num_targets=num_targets if self._target_aware else None,
+                num_targets=num_targets,
                 max_attn_len=self._max_attn_len,
                 contextual_seq_len=self._contextual_seq_len,
                 kernel=self._hammer_kernel,
             ).view(-1, self._hidden_dim * self._num_heads)
-        with span("## stu_compute_output ##"):
-            return hstu_compute_output(
-                attn=delta_attn_output,
-                u=delta_u,
-                x=delta_x,
-                norm_weight=as_dtype(self._output_norm_weight, delta_x.dtype),
-                norm_bias=as_dtype(self._output_norm_bias, delta_x.dtype),
-                norm_eps=1e-6,
-                dropout_ratio=self._output_dropout_ratio,
-                output_weight=as_dtype(self._output_weight, delta_x.dtype),
-                group_norm=self._use_group_norm,
-                num_heads=self._num_heads,
-                linear_dim=self._hidden_dim,
-                concat_u=True,
-                concat_x=True,
-                mul_u_activation_type="none",
-                training=self.training,
-                kernel=self._hammer_kernel,
-                recompute_y_in_backward=False,
-            )
+        return delta_u, delta_attn_output
 
     def forward(
         self,

@@ -341,6 +341,23 @@ int b200_hstu_concat_2d_jagged(const b200_hstu_jagged_args *args, b200_hstu_stre
 int b200_hstu_split_2d_jagged(const b200_hstu_jagged_args *args, b200_hstu_stream_t stream);
 
 /*
+ * Cached inference (generative_recommenders/modules/stu.py:137-173): k, v [cached_rows + B * delta, .] =
+ * the cached rows of every sequence (k_cache, v_cache, contiguous, jagged over `offsets`, int64 [B + 1])
+ * followed by its `delta` new rows (k_new, v_new [B * delta, .] with row strides of their own);
+ * full_offsets [B + 1] = the offsets of the result.  One launch.
+ */
+typedef struct b200_hstu_append_kv_args {
+  const void *k_cache, *v_cache, *k_new, *v_new;
+  void *k, *v;
+  const int64_t *offsets;
+  int64_t *full_offsets;
+  int64_t k_row_bytes, v_row_bytes, k_new_stride_bytes, v_new_stride_bytes;
+  int64_t cached_rows;
+  int32_t B, delta;
+} b200_hstu_append_kv_args;
+int b200_hstu_append_kv(const b200_hstu_append_kv_args *args, b200_hstu_stream_t stream);
+
+/*
  * add_timestamp_positional_embeddings (generative_recommenders/ops/position.py:40-118; semantics
  * of ops/pytorch/pt_position.py:40-160):
  *   out[t] = alpha * seq_embeddings[t] + (ts_weight[bucket(t)] + pos_weight[index(t)])

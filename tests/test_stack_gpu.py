@@ -261,3 +261,43 @@ def test_calls_without_gradients_equal_the_autograd_path():
         dual = fwad.make_dual(q, torch.ones_like(q))
         with pytest.raises(NotImplementedError, match="jvp"):
             G.hstu_mha(300, 0.1, dual, k, v, offs, num_targets=nt)
+
+
+def _layer(D, H, d, dtype, seed):
+    torch.manual_seed(seed)
+    cfg = G.STULayerConfig(embedding_dim=D, num_heads=H, hidden_dim=d, attention_dim=d, contextual_seq_len=2)
+    layer = G.STULayer(cfg).to(DEV)
+    with torch.no_grad():
+        for p in layer.parameters():
+            if p.dim() == 1:
+                p.add_(0.05 * torch.randn_like(p))
+    return layer.to(dtype).eval()
+
+
+@pytest.mark.parametrize("B, delta, longest", [(1, 1, 0), (5, 7, 60), (33, 130, 200), (3, 64, 128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_cached_rows_and_new_rows_in_one_launch(dtype, B, delta, longest):
+    """The K, V and offsets that ``cached_forward`` builds in one launch are those of ``construct_full_kv``, and its
+    result is that of the separate ops."""
+    layer = _layer(256, 2, 64, dtype, B)
+    g = torch.Generator().manual_seed(delta)
+    lengths = torch.randint(0, longest + 1, (B,), generator=g)
+    if B > 1:
+        lengths[1] = 0
+    offs = torch.cat([torch.zeros(1, dtype=torch.int64), lengths.cumsum(0)]).to(DEV)
+    rows = int(offs[-1])
+    layer.k_cache, layer.v_cache = (torch.randn(rows, 128, generator=g).to(dtype).to(DEV) for _ in range(2))
+    layer.kv_caching_offsets, layer.max_kv_caching_len = offs, longest
+    x = torch.randn(B * delta, 256, generator=g).to(dtype).to(DEV)
+    nt = torch.full((B,), min(delta, 3), device=DEV)
+    HC = G.hstu_compute
+    params = [layer._input_norm_weight, layer._input_norm_bias, layer._uvqk_weight, layer._uvqk_beta]
+    with torch.no_grad():
+        u, q, k, v = G.hstu_compute_uqvk(x, params[0], params[1], 1e-6, 2, 64, 64, params[2], params[3])
+        full_k, full_v, n, full_offs = layer.construct_full_kv(k.flatten(1, 2), v.flatten(1, 2))
+        got = HC.hstu_cached_attention(x, params[0], params[1], 1e-6, 2, 64, 64, params[2], params[3], layer.k_cache,
+                                       layer.v_cache, offs, nt, n, layer._attn_alpha, 0, 2)
+        want, want_attn = layer._cached_attention_of_ops(x, nt, 0, None)
+    assert torch.equal(got[2].flatten(1), full_k) and torch.equal(got[3].flatten(1), full_v)
+    assert torch.equal(got[4], full_offs)
+    assert torch.equal(got[0], want) and torch.equal(got[1], want_attn)
