@@ -289,15 +289,17 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> norm_mul_backward(
 // ---------------------------------------------------------------------------------------
 // output stage: x + norm_mul(attn, u) W
 // ---------------------------------------------------------------------------------------
-std::tuple<Tensor, MaybeTensor, MaybeTensor> output_forward(const Tensor &attn, const Tensor &u, const Tensor &x,
+// `over_x`: the result goes over x.
+std::tuple<Tensor, MaybeTensor, MaybeTensor> output_forward(const Tensor &attn, const Tensor &u, Tensor x,
                                                             const Tensor &weight, const Tensor &bias,
                                                             const Tensor &output_weight, double eps, int64_t H,
                                                             int64_t V, bool concat_u, bool concat_x, int64_t act,
                                                             bool group_norm, double dropout, const MaybeTensor &seed,
-                                                            int64_t dtype, bool stats) {
+                                                            int64_t dtype, bool stats, bool over_x) {
   auto [y, mean, rstd, mask] = norm_mul_forward(attn, u, weight, bias, eps, H, V, concat_u, concat_x, act, group_norm,
                                                 dropout, seed, dtype, false, stats);
-  return {at::addmm(x, y, output_weight), mean, rstd};
+  // (addmm copies x into its result first, a pass over memory: 1.26 ms of the 49 of four layers on 484 k rows of 1024)
+  return {over_x ? x.addmm_(y, output_weight) : at::addmm(x, y, output_weight), mean, rstd};
 }
 
 // dattn, du, d_norm_weight, d_norm_bias, d_output_weight
@@ -395,6 +397,32 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> uvqk_attention_inference(
                                              max_attn_len, contextual_seq_len, 0, impl, dtype, false, 0.0, std::nullopt, 0,
                                              true, status));
   return {s.u, out.view({x.size(0), H * V}), t.k, t.v};
+}
+
+// The same from the separate stages: LayerNorm, library GEMM, SiLU
+std::tuple<Tensor, Tensor, Tensor, Tensor> separate_attention_inference(
+    const Tensor &x, const Tensor &nw, const Tensor &nb, const Tensor &w, const Tensor &b, double eps, int64_t H,
+    int64_t A, int64_t V, const Tensor &offsets, const MaybeTensor &targets, const MaybeTensor &bias,
+    int64_t max_seq_len, double alpha, int64_t max_attn_len, int64_t contextual_seq_len, int64_t impl, int64_t dtype,
+    bool status) {
+  Tensor uvqk, u = empty_like_of({x.size(0), H * V}, x);
+  {
+    Tensor normed = empty_like_of({x.size(0), x.size(1)}, x);
+    Launch l(x);
+    check(b200_hstu_layer_norm_fwd(x.data_ptr(), x.stride(0), nw.data_ptr(), nb.data_ptr(), normed.data_ptr(),
+                                   normed.stride(0), nullptr, nullptr, x.size(0), (int32_t)x.size(1), (float)eps,
+                                   (int32_t)dtype, l.stream),
+          "b200_hstu_layer_norm_fwd");
+    uvqk = at::addmm(b, normed, w);
+    check(b200_hstu_silu_fwd(uvqk.data_ptr(), uvqk.stride(0), u.data_ptr(), u.stride(0), x.size(0), (int32_t)(H * V),
+                             (int32_t)dtype, l.stream),
+          "b200_hstu_silu_fwd");
+  }
+  const Qkv t = qkv_views(uvqk, H, A, V);
+  Tensor out = std::get<0>(attention_forward(t.q, t.k, t.v, offsets, targets, std::nullopt, bias, max_seq_len, alpha,
+                                             max_attn_len, contextual_seq_len, 0, impl, dtype, false, 0.0, std::nullopt, 0,
+                                             true, status));
+  return {u, out.view({x.size(0), H * V}), t.k, t.v};
 }
 
 // Cached inference: uvqk stage on the new rows, their K and V behind the cached ones, attention of the new rows.
@@ -539,6 +567,7 @@ PYBIND11_MODULE(_host, m) {
   m.def("uvqk_supported", &uvqk_supported, unlocked);
   m.def("uvqk_backward", &uvqk_backward, unlocked);
   m.def("uvqk_attention_inference", &uvqk_attention_inference, unlocked);
+  m.def("separate_attention_inference", &separate_attention_inference, unlocked);
   m.def("cached_attention", &cached_attention, unlocked);
   m.def("uvqk_attention_forward", &uvqk_attention_forward, unlocked);
   m.def("uvqk_attention_backward", &uvqk_attention_backward, unlocked);

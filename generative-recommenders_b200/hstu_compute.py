@@ -423,7 +423,8 @@ class _OutputStageFunction(torch.autograd.Function):
         b = as_dtype(bias, attn.dtype).contiguous()
         wo = as_dtype(output_weight, x.dtype)
         cfg = (eps, num_heads, linear_dim, concat_u, concat_x, act, group_norm, dropout_ratio)
-        out, mean, rstd = _cabi.host().output_forward(attn, u, x, w, b, wo, *cfg, dropout_seed, dtype_code(attn), True)
+        out, mean, rstd = _cabi.host().output_forward(attn, u, x, w, b, wo, *cfg, dropout_seed, dtype_code(attn), True,
+                                                          False)
         ctx.save_for_backward(attn, u, w, b, wo, mean, rstd, dropout_seed)
         ctx.cfg = cfg
         ctx.dtypes = (weight.dtype, bias.dtype, output_weight.dtype)
@@ -497,6 +498,48 @@ def hstu_norm_mul_dropout(
     return y
 
 
+def _output_inference(attn, u, x, norm_weight, norm_bias, norm_eps, output_weight, num_heads, linear_dim, concat_u,
+                      concat_x, act, dropout_ratio, over_x=False):
+    """The output stage (LayerNorm flavour) where no gradient is wanted; with ``over_x`` the result goes over
+    x."""
+    return _cabi.host().output_forward(
+        attn if attn.stride(-1) == 1 else attn.contiguous(), u if u.stride(-1) == 1 else u.contiguous(), x,
+        as_dtype(norm_weight, attn.dtype).contiguous(), as_dtype(norm_bias, attn.dtype).contiguous(),
+        as_dtype(output_weight, x.dtype), float(norm_eps), int(num_heads),
+        int(linear_dim) if linear_dim > 0 else attn.shape[1] // num_heads, bool(concat_u), bool(concat_x), act, False,
+        float(dropout_ratio), _draw_dropout_seed(attn.device) if dropout_ratio > 0.0 else None, dtype_code(attn), False,
+        over_x and x.is_contiguous())[0]
+
+
+def _compute_output(attn, u, x, norm_weight, norm_bias, norm_eps, output_weight, num_heads, linear_dim, dropout_ratio,
+                    training, concat_u, concat_x, mul_u_activation_type, group_norm, recompute_y_in_backward, kernel,
+                    over_x=False):
+    """``hstu_compute_output``; ``over_x``: the caller has no use for x any more, the result may go over it."""
+    _require_cuda_backend(kernel)
+    require_cuda(attn, u, x, norm_weight, norm_bias, output_weight)
+    if recompute_y_in_backward and torch.is_grad_enabled() and mul_u_activation_type in _ACT and attn.shape[0] > 0:
+        g_ = bool(group_norm)
+        cu, cx = bool(concat_u), bool(concat_x)
+        if g_ and cu != cx:
+            cu = cx = False
+        drop = training and dropout_ratio > 0.0
+        if not (drop and g_):   # the group-norm variant draws its mask with torch's dropout: kept on the plain path
+            seed = _draw_dropout_seed(attn.device) if (drop and dropout_ratio < 1.0) else None
+            ld = linear_dim if linear_dim > 0 else attn.shape[1] // num_heads
+            return _OutputStageFunction.apply(attn, u, x, norm_weight, norm_bias, output_weight, float(norm_eps),
+                                              int(num_heads), int(ld), cu, cx, 0 if g_ else _ACT[mul_u_activation_type],
+                                              g_, float(dropout_ratio) if seed is not None else 0.0, seed)
+    drop = training and dropout_ratio > 0.0
+    if (not group_norm and mul_u_activation_type in _ACT and not (drop and dropout_ratio >= 1.0)
+            and outside_autograd(attn, u, x, norm_weight, norm_bias, output_weight)):
+        return _output_inference(attn, u, x, norm_weight, norm_bias, norm_eps, output_weight, num_heads, linear_dim,
+                                 concat_u, concat_x, _ACT[mul_u_activation_type], dropout_ratio if drop else 0.0,
+                                 over_x=over_x)
+    y = hstu_norm_mul_dropout(attn, u, norm_weight, norm_bias, norm_eps, dropout_ratio, training, concat_u, concat_x,
+                              mul_u_activation_type, group_norm, num_heads, linear_dim)
+    return addmm(x, y, as_dtype(output_weight, x.dtype), kernel)
+
+
 def hstu_compute_output(
     attn: torch.Tensor,
     u: torch.Tensor,
@@ -521,33 +564,9 @@ def hstu_compute_output(
     generative_recommenders/ops/pytorch/pt_hstu_linear.py:85-120).
     With ``recompute_y_in_backward`` the stage is one autograd node that does not keep the
     concatenated activation (see ``_OutputStageFunction``)."""
-    _require_cuda_backend(kernel)
-    require_cuda(attn, u, x, norm_weight, norm_bias, output_weight)
-    if recompute_y_in_backward and torch.is_grad_enabled() and mul_u_activation_type in _ACT and attn.shape[0] > 0:
-        g_ = bool(group_norm)
-        cu, cx = bool(concat_u), bool(concat_x)
-        if g_ and cu != cx:
-            cu = cx = False
-        drop = training and dropout_ratio > 0.0
-        if not (drop and g_):   # the group-norm variant draws its mask with torch's dropout: kept on the plain path
-            seed = _draw_dropout_seed(attn.device) if (drop and dropout_ratio < 1.0) else None
-            ld = linear_dim if linear_dim > 0 else attn.shape[1] // num_heads
-            return _OutputStageFunction.apply(attn, u, x, norm_weight, norm_bias, output_weight, float(norm_eps),
-                                              int(num_heads), int(ld), cu, cx, 0 if g_ else _ACT[mul_u_activation_type],
-                                              g_, float(dropout_ratio) if seed is not None else 0.0, seed)
-    drop = training and dropout_ratio > 0.0
-    if (not group_norm and mul_u_activation_type in _ACT and not (drop and dropout_ratio >= 1.0)
-            and outside_autograd(attn, u, x, norm_weight, norm_bias, output_weight)):
-        return _cabi.host().output_forward(
-            attn if attn.stride(-1) == 1 else attn.contiguous(), u if u.stride(-1) == 1 else u.contiguous(), x,
-            as_dtype(norm_weight, attn.dtype).contiguous(), as_dtype(norm_bias, attn.dtype).contiguous(),
-            as_dtype(output_weight, x.dtype), float(norm_eps), int(num_heads),
-            int(linear_dim) if linear_dim > 0 else attn.shape[1] // num_heads, bool(concat_u), bool(concat_x),
-            _ACT[mul_u_activation_type], False, float(dropout_ratio) if drop else 0.0,
-            _draw_dropout_seed(attn.device) if drop else None, dtype_code(attn), False)[0]
-    y = hstu_norm_mul_dropout(attn, u, norm_weight, norm_bias, norm_eps, dropout_ratio, training, concat_u, concat_x,
-                              mul_u_activation_type, group_norm, num_heads, linear_dim)
-    return addmm(x, y, as_dtype(output_weight, x.dtype), kernel)
+    return _compute_output(attn, u, x, norm_weight, norm_bias, norm_eps, output_weight, num_heads, linear_dim,
+                           dropout_ratio, training, concat_u, concat_x, mul_u_activation_type, group_norm,
+                           recompute_y_in_backward, kernel)
 
 
 def hstu_preprocess_and_attention(
@@ -614,6 +633,19 @@ def hstu_preprocess_and_attention(
             offs, nt, rab, int(max_seq_len), float(attn_alpha), int(max_attn_len), int(contextual_seq_len),
             bool(recompute_uvqk_in_backward))
         return u, attn.view(-1, hidden_dim * num_heads), k, v
+    if (x.is_cuda and x.shape[0] > 0 and x.stride(1) == 1 and not (_FUSED_UQVK and _fused_uqvk_supported(x, uvqk_weight, hv))
+            and all(t.dtype is x.dtype for t in (norm_weight, norm_bias, uvqk_weight, uvqk_bias))
+            and outside_autograd(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias, bias_by_distance)):
+        # the separate stages in one call
+        require_cuda(norm_weight, norm_bias, uvqk_weight, uvqk_bias, seq_offsets, num_targets, bias_by_distance)
+        offs, nt = _index(seq_offsets), _index(num_targets)
+        if nt is not None and nt.numel() != offs.numel() - 1:
+            raise RuntimeError("num_targets must have one entry per sequence")
+        rab = None if bias_by_distance is None else bias_by_distance.to(torch.float32).reshape(-1).contiguous()
+        return _cabi.host().separate_attention_inference(
+            x, norm_weight.contiguous(), norm_bias.contiguous(), uvqk_weight, uvqk_bias, float(norm_eps), num_heads,
+            attn_dim, hidden_dim, offs, nt, rab, int(max_seq_len), float(attn_alpha), int(max_attn_len),
+            int(contextual_seq_len), *_attention_switches(x), _attention._CHECK_STATUS)
     u, q, k, v = hstu_compute_uqvk(
         x=x, norm_weight=norm_weight, norm_bias=norm_bias, norm_eps=norm_eps, num_heads=num_heads,
         attn_dim=attn_dim, hidden_dim=hidden_dim, uvqk_weight=uvqk_weight, uvqk_bias=uvqk_bias, kernel=kernel,

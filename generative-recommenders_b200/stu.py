@@ -21,10 +21,12 @@ from dataclasses import dataclass
 from typing import List, Optional
 
 import torch
+from torch.compiler import is_compiling
+from torch.nn.modules import module as _module
 
 from .common import HammerKernel, as_dtype, span
 from .hstu_attention import delta_hstu_mha
-from .hstu_compute import (hstu_cached_attention, hstu_compute_output, hstu_compute_uqvk,
+from .hstu_compute import (_compute_output, hstu_cached_attention, hstu_compute_uqvk,
                            hstu_preprocess_and_attention)
 from .jagged_tensors import concat_2D_jagged, split_2D_jagged
 
@@ -182,6 +184,9 @@ class STULayer(torch.nn.Module):
     ) -> torch.Tensor:
         """The layer on the last ``delta_size`` rows of every sequence against the cached K / V
         (reference stu.py:358-424); ``delta_x`` is ``[B * delta_size, D]``."""
+        return self._cached_forward(delta_x, num_targets, max_kv_caching_len, kv_caching_lengths, False)
+
+    def _cached_forward(self, delta_x, num_targets, max_kv_caching_len, kv_caching_lengths, over_x):
         if self._rel_bias_table is not None:
             raise NotImplementedError("cached_forward with a relative bias table")
         num_targets_ = num_targets if self._target_aware else None
@@ -206,7 +211,7 @@ class STULayer(torch.nn.Module):
             delta_u, delta_attn_output = self._cached_attention_of_ops(delta_x, num_targets_, max_kv_caching_len,
                                                                        kv_caching_lengths)
         with span("## stu_compute_output ##"):
-            return hstu_compute_output(
+            return _compute_output(
                 attn=delta_attn_output,
                 u=delta_u,
                 x=delta_x,
@@ -224,6 +229,7 @@ class STULayer(torch.nn.Module):
                 training=self.training,
                 kernel=self._hammer_kernel,
                 recompute_y_in_backward=False,
+                over_x=over_x,
             )
 
     def _cached_attention_of_ops(self, delta_x, num_targets, max_kv_caching_len, kv_caching_lengths):
@@ -272,6 +278,11 @@ class STULayer(torch.nn.Module):
         max_kv_caching_len: int = 0,
         kv_caching_lengths: Optional[torch.Tensor] = None,
     ) -> torch.Tensor:
+        return self._forward(x, x_offsets, max_seq_len, num_targets, max_kv_caching_len, kv_caching_lengths, False)
+
+    def _forward(self, x, x_offsets, max_seq_len, num_targets, max_kv_caching_len, kv_caching_lengths, over_x):
+        """``forward``; ``over_x``: the caller has no use for x any more, the result may go over it where no
+        gradient is wanted."""
         bias = None
         if self._rel_bias_table is not None:
             bias = position_bias_by_distance(self._rel_bias_table, max_seq_len)
@@ -302,7 +313,7 @@ class STULayer(torch.nn.Module):
         self.update_kv_cache(max_seq_len=max_seq_len, seq_offsets=x_offsets, k=k, v=v,
                              max_kv_caching_len=max_kv_caching_len, kv_caching_lengths=kv_caching_lengths)
         with span("## stu_compute_output ##"):
-            return hstu_compute_output(
+            return _compute_output(
                 attn=attn_output,
                 u=u,
                 x=x,
@@ -320,7 +331,16 @@ class STULayer(torch.nn.Module):
                 training=self.training,
                 kernel=self._hammer_kernel,
                 recompute_y_in_backward=self._recompute_y,
+                over_x=over_x,
             )
+
+
+def _unobserved(layer, method) -> bool:
+    """True where ``layer.method`` is this file's and no hook gets to see what goes in or comes out."""
+    return (type(layer) is STULayer and method not in layer.__dict__ and not layer._forward_hooks
+            and not layer._forward_pre_hooks and not layer._backward_hooks and not layer._backward_pre_hooks
+            and layer._compiled_call_impl is None and not _module._has_any_global_hook()
+            and not is_compiling())
 
 
 class STUStack(torch.nn.Module):
@@ -339,10 +359,16 @@ class STUStack(torch.nn.Module):
         max_kv_caching_len: int = 0,
         kv_caching_lengths: Optional[torch.Tensor] = None,
     ) -> torch.Tensor:
+        previous = None
         for layer in self._stu_layers:
-            x = layer(x=x, x_lengths=x_lengths, x_offsets=x_offsets, max_seq_len=max_seq_len,
-                      num_targets=num_targets, max_kv_caching_len=max_kv_caching_len,
-                      kv_caching_lengths=kv_caching_lengths)
+            # what one layer hands to the next is the stack's own: it may be overwritten, unless someone looks on
+            if previous is not None and _unobserved(previous, "forward") and _unobserved(layer, "forward"):
+                x = layer._forward(x, x_offsets, max_seq_len, num_targets, max_kv_caching_len, kv_caching_lengths, True)
+            else:
+                x = layer(x=x, x_lengths=x_lengths, x_offsets=x_offsets, max_seq_len=max_seq_len,
+                          num_targets=num_targets, max_kv_caching_len=max_kv_caching_len,
+                          kv_caching_lengths=kv_caching_lengths)
+            previous = layer
         return x
 
     def cached_forward(
@@ -352,8 +378,14 @@ class STUStack(torch.nn.Module):
         max_kv_caching_len: int = 0,
         kv_caching_lengths: Optional[torch.Tensor] = None,
     ) -> torch.Tensor:
+        previous = None
         for layer in self._stu_layers:
-            delta_x = layer.cached_forward(delta_x=delta_x, num_targets=num_targets,
-                                           max_kv_caching_len=max_kv_caching_len,
-                                           kv_caching_lengths=kv_caching_lengths)
+            if (previous is not None and _unobserved(previous, "cached_forward")
+                    and _unobserved(layer, "cached_forward")):
+                delta_x = layer._cached_forward(delta_x, num_targets, max_kv_caching_len, kv_caching_lengths, True)
+            else:
+                delta_x = layer.cached_forward(delta_x=delta_x, num_targets=num_targets,
+                                               max_kv_caching_len=max_kv_caching_len,
+                                               kv_caching_lengths=kv_caching_lengths)
+            previous = layer
         return delta_x

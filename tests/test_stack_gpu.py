@@ -274,6 +274,29 @@ def _layer(D, H, d, dtype, seed):
     return layer.to(dtype).eval()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("D, H, d", [(768, 6, 128), (1024, 8, 64), (640, 16, 128), (520, 3, 8)])
+def test_layer_without_gradients_equals_the_ops_one_by_one(dtype, D, H, d):
+    """Where the fused uvqk kernel does not apply, a layer without gradients queues its separate stages in one call:
+    the same bits as the public ops one after the other."""
+    if dtype == torch.float32 and H * d > 1024:
+        pytest.skip("wider than a row of 32-bit elements can be")
+    layer = _layer(D, H, d, dtype, D)
+    lengths = torch.tensor([5, 130, 3, 77], device=DEV)
+    offs = torch.cat([lengths.new_zeros(1), lengths.cumsum(0)])
+    x = torch.randn(int(offs[-1]), D, device=DEV).to(dtype)
+    nt = torch.tensor([2, 9, 0, 1], device=DEV)
+    with torch.no_grad():
+        got = layer(x, lengths, offs, 130, nt)
+        cast = lambda t: t.to(dtype)  # noqa: E731
+        u, q, k, v = G.hstu_compute_uqvk(x, cast(layer._input_norm_weight), cast(layer._input_norm_bias), 1e-6, H, d, d,
+                                         cast(layer._uvqk_weight), cast(layer._uvqk_beta))
+        attn = G.hstu_mha(130, layer._attn_alpha, q, k, v, offs, num_targets=nt, contextual_seq_len=2).flatten(1)
+        want = G.hstu_compute_output(attn, u, x, cast(layer._output_norm_weight), cast(layer._output_norm_bias), 1e-6,
+                                     cast(layer._output_weight), H, d, 0.3, False, True, True, "none", False, False)
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("B, delta, longest", [(1, 1, 0), (5, 7, 60), (33, 130, 200), (3, 64, 128)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_cached_rows_and_new_rows_in_one_launch(dtype, B, delta, longest):
@@ -301,3 +324,25 @@ def test_cached_rows_and_new_rows_in_one_launch(dtype, B, delta, longest):
     assert torch.equal(got[2].flatten(1), full_k) and torch.equal(got[3].flatten(1), full_v)
     assert torch.equal(got[4], full_offs)
     assert torch.equal(got[0], want) and torch.equal(got[1], want_attn)
+
+
+@pytest.mark.parametrize("D, H, d", [(256, 2, 64), (768, 6, 128)])
+def test_stack_overwrites_nothing_that_anyone_sees(D, H, d):
+    """Without gradients a layer's result goes over its input where that is the stack's own: the same bits as layer by
+    layer, the caller's input and what a hook sees unchanged."""
+    stack = G.STUStack([_layer(D, H, d, torch.bfloat16, i) for i in range(3)])
+    lengths = torch.tensor([5, 130, 77], device=DEV)
+    offs = torch.cat([lengths.new_zeros(1), lengths.cumsum(0)])
+    x = torch.randn(int(offs[-1]), D, device=DEV).bfloat16()
+    before = x.clone()
+    with torch.no_grad():
+        want = [x]
+        for layer in stack._stu_layers:
+            want.append(layer(want[-1], lengths, offs, 130, None))
+        got = stack(x, lengths, offs, 130, None)
+        assert torch.equal(got, want[-1]) and torch.equal(x, before)
+        seen = []
+        handle = stack._stu_layers[1].register_forward_hook(lambda m, args, out: seen.append(out))
+        assert torch.equal(stack(x, lengths, offs, 130, None), want[-1])
+        handle.remove()
+    assert torch.equal(seen[0], want[2]) and torch.equal(x, before)
