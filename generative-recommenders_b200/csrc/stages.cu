@@ -568,7 +568,8 @@ struct NormMulParams {
 // dependent multiplications and the kernels below run few warps; the round keys are shared as well.
 // Used where it measured faster (rows of 16-bit elements, dropout 0.3, 205 MB a tensor): forward with two
 // vectors per lane (D = 512) 290 -> 270 us, backward with one (D = 256) 480 -> 390 us.  The other forms are
-// bound by instruction issue, not by the chains, and lose by the registers it takes (forward D = 256
+// bound by instruction issue, not by the chains, and lose by the registers it takes (the staged kernels, whose
+// rows are not in registers, always use it; forward D = 256
 // 304 -> 334, D = 1024 300 -> 390; backward D = 512 412 -> 414, D = 1024 427 -> 445): they go call by call.
 template <int N>
 __device__ __forceinline__ void philox_many(uint32_t k0, uint32_t k1, const uint64_t (&g)[N], uint32_t (&o)[N][4]) {

@@ -83,8 +83,6 @@ def _fill_common(a, q, k, v, seq_offsets, num_targets, attn_scale, max_seq_len, 
         a.dropout_seed = dropout_seed.data_ptr()
 
 
-_PLAN_OWN, _PLAN_FOR_BACKWARD, _PLAN_REUSE = 0, 1, 2
-
 # B200_HSTU_CHECK_STATUS=1: after every tensor-core attention launch, wait for it and read the status
 # words of its work lists back; a bounded wait that gave up inside the kernel (which then returned
 # early, leaving its output incomplete) becomes a RuntimeError instead of passing silently.  A
