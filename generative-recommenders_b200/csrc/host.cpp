@@ -556,6 +556,18 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, MaybeTensor> uvqk_attention_b
 }  // namespace
 
 PYBIND11_MODULE(_host, m) {
+  // the exceptions that the torch functions of the same calls raise (an allocation that fails is caught by its type)
+  py::register_local_exception_translator([](std::exception_ptr p) {
+    try {
+      if (p) std::rethrow_exception(p);
+    } catch (const c10::OutOfMemoryError &e) {
+      PyErr_SetString(py::module_::import("torch").attr("OutOfMemoryError").ptr(), e.what_without_backtrace());
+    } catch (const c10::IndexError &e) {
+      PyErr_SetString(PyExc_IndexError, e.what_without_backtrace());
+    } catch (const c10::Error &e) {
+      PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+    }
+  });
   // (as with ctypes, other threads run while launches are queued)
   const auto unlocked = py::call_guard<py::gil_scoped_release>();
   m.def("attention_forward", &attention_forward, unlocked);

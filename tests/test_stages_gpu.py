@@ -169,3 +169,15 @@ def test_bf16_stack_with_relative_bias_runs_and_matches_oracle():
     params16 = {n: p.bfloat16() for n, p in params.items()}
     ref16 = O.stu_layer(x, offs, 512, nt, params16, 2, 128, 128, contextual_seq_len=6, rel_bias=rb)
     PM.check_vs_bf16_reference("bf16_layer_with_bias", y, ref, ref16.float())
+
+
+def test_native_calls_raise_what_torch_raises():
+    """An allocation that fails inside a native call is torch's own exception (on the host's account alone: the size is
+    beyond the device's memory, nothing is launched)."""
+    from generative_recommenders_b200 import _cabi
+    attn = torch.zeros(1, 8, device=DEV, dtype=torch.bfloat16).expand(1 << 40, 8)
+    w = torch.ones(8, device=DEV, dtype=torch.bfloat16)
+    with pytest.raises(torch.OutOfMemoryError):
+        _cabi.host().norm_mul_forward(attn, attn, w, w, 1e-6, 1, 8, True, True, 0, False, 0.0, None, 1, False, False)
+    with pytest.raises(RuntimeError, match="status"):
+        _cabi.host().norm_mul_forward(attn[:1], attn[:1], w, w, 1e-6, 1, 8, True, True, 9, False, 0.0, None, 1, False, False)
