@@ -221,6 +221,18 @@ __device__ __forceinline__ void reduce_columns_to_partial(const Row<E, MAXV> &ac
 }
 
 template <typename E, int MAXV>
+__device__ __forceinline__ void store_columns(const Row<E, MAXV> &acc, float *dst, int D, int lane) {
+  constexpr int EV = VecInfo<E>::EV;
+#pragma unroll
+  for (int k = 0; k < MAXV; ++k)
+#pragma unroll
+    for (int t = 0; t < EV; ++t) {
+      const int e = (k * 32 + lane) * EV + t;
+      if (e < D) dst[e] = acc.v[k][t];
+    }
+}
+
+template <typename E, int MAXV>
 __global__ void __launch_bounds__(WARPS * 32, 2) layer_norm_bwd_kernel(
     const E *__restrict__ dy, int64_t dy_rs, const E *__restrict__ x, int64_t x_rs, const E *__restrict__ w,
     const float *__restrict__ mean_in, const float *__restrict__ rstd_in, E *__restrict__ dx, int64_t dx_rs,
@@ -538,6 +550,18 @@ __device__ __forceinline__ float dact_f(float u, int act) {
     return s * (1.f - s);
   }
   return dsiluf_(u);
+}
+
+// Both from one sigmoid, rounded as the two above round by themselves (left to the compiler, the choice
+// between the two activations moves into the product and the last bit with it).
+__device__ __forceinline__ void act_and_dact(float u, int act, float &a, float &da) {
+  a = u;
+  da = 1.f;
+  if (act != 0) {
+    const float s = sigmoidf_(u), t = 1.f - s;
+    a = act == 1 ? s : u * s;
+    da = act == 1 ? s * t : __fmul_rn(s, __fmaf_rn(u, t, 1.f));
+  }
 }
 
 struct NormMulParams {
@@ -1222,13 +1246,21 @@ __global__ void __launch_bounds__(WARPS * 32) norm_mul_bwd_kernel(NormMulParams 
 // The backward with the forward's mask regenerated, for rows of up to two vectors per lane: bound by HBM and
 // by the issue of the generator's and the row's arithmetic together, so it has to keep both busy.  The rows come
 // through shared memory by asynchronous copies (every lane reads what it has copied itself: no barrier), so
-// that the registers hold the row being worked on only and two CTAs fit an SM - the kernel above, whose
-// next row waits in registers, takes 255 of them and runs with eight warps: 415 -> 372 us on 200 k rows of 512
-// (figures at other sizes where the kernel is chosen).
+// that the registers hold the row being worked on only and twelve warps fit an SM - the kernel above, whose
+// next row waits in registers, takes 255 of them and runs with eight: 415 -> 330 us on 200 k rows of 512, 510 -> 390
+// with SiLU on u (figures at other sizes where the kernel is chosen).
+// The results are the kernel above's to the bit.  That takes its order of the column sums: one sum over every
+// 3552th row, eight of them to a block, 444 blocks (on 148 SMs).  With CTAs of four warps, each of which adds up two
+// of the eight one after the other (HALVES), all 444 are resident, three an SM.  (444 CTAs of eight warps are two
+// an SM and a last wave that is half empty: 399 us where this form took 368, both before the activation and its
+// derivative shared a sigmoid.)  A batch with at most one row per sum takes CTAs of eight warps and leaves out
+// the blocks without a row: 70 rows of 512 12.1 -> 6.8 us.
 // Vector path only (aligned pointers and strides, D a multiple of the vector width, 16-bit elements).
-// Shared memory: [WARPS][STAGES][5][MAXV][32] vectors: attn, u, dout's y, u and x part.
-template <typename E, int MAXV, int STAGES>
-__global__ void __launch_bounds__(WARPS * 32, 2) norm_mul_bwd_staged_kernel(NormMulParams p) {
+// Shared memory: [NW][STAGES][5][MAXV][32] vectors: attn, u, dout's y, u and x part; with two halves
+// [2][NW][D] floats, the first halves' sums.
+template <typename E, int MAXV, int STAGES, int HALVES>
+__global__ void __launch_bounds__(WARPS / HALVES * 32, HALVES == 2 ? 3 : 2) norm_mul_bwd_staged_kernel(NormMulParams p) {
+  constexpr int NW = WARPS / HALVES;
   static_assert(VecInfo<E>::EV == 8, "one generator call for a vector");
   extern __shared__ uint4 ring[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1262,94 +1294,130 @@ __global__ void __launch_bounds__(WARPS * 32, 2) norm_mul_bwd_staged_kernel(Norm
     asm volatile("cp.async.commit_group;" ::: "memory");   // (a group for every row, so that they can be counted)
   };
   const int64_t step = (int64_t)gridDim.x * WARPS;
-  int64_t row = (int64_t)blockIdx.x * WARPS + warp;
-#pragma unroll
-  for (int s = 0; s + 1 < STAGES; ++s) request(row + s * step, s);
-  int stage = 0;
-  for (; row < p.rows; row += step) {
-    request(row + (STAGES - 1) * step, stage == 0 ? STAGES - 1 : stage - 1);   // the slot of the row before
-    const float mean = p.mean[row], rstd = p.rstd[row];
-    const uint64_t base = ((uint64_t)row * (uint64_t)width >> 3) + (uint64_t)lane;   // generator call of the row's first vector
-    uint32_t oy[MAXV][4], ou[MAXV][4], ox[MAXV][4];
-    auto words = [&](int off, uint32_t (&o)[MAXV][4]) {
-      uint64_t g[MAXV];
-#pragma unroll
-      for (int k = 0; k < MAXV; ++k) g[k] = base + (uint64_t)((off >> 3) + k * 32);
-      philox_many<MAXV>(drop.k0, drop.k1, g, o);
-    };
-    words(off_y, oy);
-    if (p.concat_u) words(0, ou);
-    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
-    uint4 *in = mine + stage * (5 * MAXV * 32);
-    E *du_row = (E *)p.du + row * p.du_rs, *dx_row = (E *)p.dattn + row * p.dattn_rs;
-    float c1 = 0.f, c2 = 0.f;
-#pragma unroll
-    for (int k = 0; k < MAXV; ++k) {
-      const int e0 = (k * 32 + lane) * 8;
-      if (e0 >= D) continue;
-      float x[8], u[8], g[8];
-      unpack_vec<E>(in[(0 * MAXV + k) * 32], x);
-      unpack_vec<E>(in[(1 * MAXV + k) * 32], u);
-      unpack_vec<E>(in[(2 * MAXV + k) * 32], g);
-      drop.mask8(g, oy[k]);
-      // (weight and bias come from L1 each time)
-      const uint4 wv = __ldg(reinterpret_cast<const uint4 *>((const E *)p.w + e0));
-      const uint4 bv = __ldg(reinterpret_cast<const uint4 *>((const E *)p.b + e0));
-      const E *pw = reinterpret_cast<const E *>(&wv), *pb = reinterpret_cast<const E *>(&bv);
-      alignas(16) float du[8], gw[8];
-#pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        const float w = to_f32(pw[t]);
-        const float xhat = (x[t] - mean) * rstd;
-        const float ga = g[t] * act_f(u[t], p.act);   // gradient w.r.t. the normalised value
-        du[t] = g[t] * (xhat * w + to_f32(pb[t])) * dact_f(u[t], p.act);
-        dw.v[k][t] += ga * xhat;
-        db.v[k][t] += ga;
-        gw[t] = ga * w;
-        c1 += gw[t] * xhat;
-        c2 += gw[t];
-      }
-      // (over what has been read, until the row's sums are there)
-      in[(1 * MAXV + k) * 32] = *reinterpret_cast<const uint4 *>(&gw[0]);
-      in[(2 * MAXV + k) * 32] = *reinterpret_cast<const uint4 *>(&gw[4]);
-      if (p.concat_u) {
-        float more[8];
-        unpack_vec<E>(in[(3 * MAXV + k) * 32], more);
-        drop.mask8(more, ou[k]);
-#pragma unroll
-        for (int t = 0; t < 8; ++t) du[t] += more[t];
-      }
-      store_vec<E>(du_row + e0, du);
+  const int64_t first = (int64_t)blockIdx.x * WARPS + warp;   // rows first + i step, then (first + NW) + i step
+  int64_t ahead = first;   // the row to be requested next
+  int ahead_half = 0;
+  auto advance = [&]() {
+    ahead += step;
+    if (HALVES == 2 && ahead_half == 0 && ahead >= p.rows) {
+      ahead = first + NW;
+      ahead_half = 1;
     }
-    if (p.concat_x) words(off_x, ox);
-    c1 = warp_sum(c1) * invD;
-    c2 = warp_sum(c2) * invD;
+  };
 #pragma unroll
-    for (int k = 0; k < MAXV; ++k) {
-      const int e0 = (k * 32 + lane) * 8;
-      if (e0 >= D) continue;
-      alignas(16) float x[8], dx[8];
-      unpack_vec<E>(in[(0 * MAXV + k) * 32], x);
-      *reinterpret_cast<uint4 *>(&dx[0]) = in[(1 * MAXV + k) * 32];
-      *reinterpret_cast<uint4 *>(&dx[4]) = in[(2 * MAXV + k) * 32];
-#pragma unroll
-      for (int t = 0; t < 8; ++t) dx[t] = (dx[t] - c2 - (x[t] - mean) * rstd * c1) * rstd;
-      if (p.concat_x) {
-        float more[8];
-        unpack_vec<E>(in[(4 * MAXV + k) * 32], more);
-        drop.mask8(more, ox[k]);
-#pragma unroll
-        for (int t = 0; t < 8; ++t) dx[t] += more[t];
-      }
-      store_vec<E>(dx_row + e0, dx);
-    }
-    stage = stage + 1 == STAGES ? 0 : stage + 1;
+  for (int s = 0; s + 1 < STAGES; ++s) {
+    request(ahead, s);
+    advance();
   }
-  __syncthreads();   // the column sums go over the ring
-  float *smem = reinterpret_cast<float *>(ring);
+  int stage = 0;
+  float *sums = reinterpret_cast<float *>(ring + NW * (STAGES * 5 * MAXV * 32));
+  for (int half = 0; half < HALVES; ++half) {
+    for (int64_t row = first + half * NW; row < p.rows; row += step) {
+      request(ahead, stage == 0 ? STAGES - 1 : stage - 1);   // the slot of the row before
+      advance();
+      const float mean = p.mean[row], rstd = p.rstd[row];
+      const uint64_t base = ((uint64_t)row * (uint64_t)width >> 3) + (uint64_t)lane;   // generator call of the row's first vector
+      uint32_t oy[MAXV][4], ou[MAXV][4], ox[MAXV][4];
+      auto words = [&](int off, uint32_t (&o)[MAXV][4]) {
+        uint64_t g[MAXV];
+#pragma unroll
+        for (int k = 0; k < MAXV; ++k) g[k] = base + (uint64_t)((off >> 3) + k * 32);
+        philox_many<MAXV>(drop.k0, drop.k1, g, o);
+      };
+      words(off_y, oy);
+      if (p.concat_u) words(0, ou);
+      asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+      uint4 *in = mine + stage * (5 * MAXV * 32);
+      E *du_row = (E *)p.du + row * p.du_rs, *dx_row = (E *)p.dattn + row * p.dattn_rs;
+      float c1 = 0.f, c2 = 0.f;
+#pragma unroll
+      for (int k = 0; k < MAXV; ++k) {
+        const int e0 = (k * 32 + lane) * 8;
+        if (e0 >= D) continue;
+        float x[8], u[8], g[8];
+        unpack_vec<E>(in[(0 * MAXV + k) * 32], x);
+        unpack_vec<E>(in[(1 * MAXV + k) * 32], u);
+        unpack_vec<E>(in[(2 * MAXV + k) * 32], g);
+        drop.mask8(g, oy[k]);
+        // (weight and bias come from L1 each time)
+        const uint4 wv = __ldg(reinterpret_cast<const uint4 *>((const E *)p.w + e0));
+        const uint4 bv = __ldg(reinterpret_cast<const uint4 *>((const E *)p.b + e0));
+        const E *pw = reinterpret_cast<const E *>(&wv), *pb = reinterpret_cast<const E *>(&bv);
+        alignas(16) float du[8], gw[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+          const float w = to_f32(pw[t]);
+          const float xhat = (x[t] - mean) * rstd;
+          float act, dact;
+          act_and_dact(u[t], p.act, act, dact);
+          const float ga = g[t] * act;   // gradient w.r.t. the normalised value
+          du[t] = g[t] * (xhat * w + to_f32(pb[t])) * dact;
+          dw.v[k][t] += ga * xhat;
+          db.v[k][t] += ga;
+          gw[t] = ga * w;
+          c1 += gw[t] * xhat;
+          c2 += gw[t];
+        }
+        // (over what has been read, until the row's sums are there)
+        in[(1 * MAXV + k) * 32] = *reinterpret_cast<const uint4 *>(&gw[0]);
+        in[(2 * MAXV + k) * 32] = *reinterpret_cast<const uint4 *>(&gw[4]);
+        if (p.concat_u) {
+          float more[8];
+          unpack_vec<E>(in[(3 * MAXV + k) * 32], more);
+          drop.mask8(more, ou[k]);
+#pragma unroll
+          for (int t = 0; t < 8; ++t) du[t] += more[t];
+        }
+        store_vec<E>(du_row + e0, du);
+      }
+      if (p.concat_x) words(off_x, ox);
+      c1 = warp_sum(c1) * invD;
+      c2 = warp_sum(c2);
+#pragma unroll
+      for (int k = 0; k < MAXV; ++k) {
+        const int e0 = (k * 32 + lane) * 8;
+        if (e0 >= D) continue;
+        alignas(16) float x[8], dx[8];
+        unpack_vec<E>(in[(0 * MAXV + k) * 32], x);
+        *reinterpret_cast<uint4 *>(&dx[0]) = in[(1 * MAXV + k) * 32];
+        *reinterpret_cast<uint4 *>(&dx[4]) = in[(2 * MAXV + k) * 32];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) dx[t] = (__fmaf_rn(-c2, invD, dx[t]) - (x[t] - mean) * rstd * c1) * rstd;
+        if (p.concat_x) {
+          float more[8];
+          unpack_vec<E>(in[(4 * MAXV + k) * 32], more);
+          drop.mask8(more, ox[k]);
+#pragma unroll
+          for (int t = 0; t < 8; ++t) dx[t] += more[t];
+        }
+        store_vec<E>(dx_row + e0, dx);
+      }
+      stage = stage + 1 == STAGES ? 0 : stage + 1;
+    }
+    if (half + 1 < HALVES) {
+      store_columns(dw, sums + warp * D, D, lane);
+      store_columns(db, sums + (NW + warp) * D, D, lane);
+      dw.zero();
+      db.zero();
+    }
+  }
+  __syncthreads();   // the last sums go over the ring
+  float *last = reinterpret_cast<float *>(ring);
+  store_columns(dw, last + warp * D, D, lane);
+  store_columns(db, last + (NW + warp) * D, D, lane);
+  __syncthreads();
   float *prow = p.partial + (int64_t)blockIdx.x * 2 * D;
-  reduce_columns_to_partial(dw, smem, prow, D, lane, warp);
-  reduce_columns_to_partial(db, smem, prow + D, D, lane, warp);
+  for (int e = threadIdx.x; e < 2 * D; e += NW * 32) {
+    const int at = e < D ? e : NW * D + e - D;
+    float s = 0.f;
+    if (HALVES == 2) {
+#pragma unroll
+      for (int wv = 0; wv < NW; ++wv) s += sums[at + wv * D];
+    }
+#pragma unroll
+    for (int wv = 0; wv < NW; ++wv) s += last[at + wv * D];
+    prow[e] = s;
+  }
 }
 
 // The same backward for rows of four vectors per lane (D = 1024 in 16-bit elements), which the kernel
@@ -1745,8 +1813,9 @@ int64_t norm_mul_mask_bytes(const b200_hstu_norm_mul_args &a) {
 // Which dropout kernel: device time in us, dropout 0.3, [u | attn | y], bf16, register-resident / staged rows.
 //   forward    D = 512: 300 rows 4.5 / 3.9, 2000 5.7 / 5.1, 15000 24.9 / 24.1, 30000 46.5 / 47.3, 200003 268 / 291
 //              D = 256: 8000 10.1 / 9.3, 15000 15.5 / 15.1, 30000 27.5 / 28.0, 200003 154 / 175
-//   backward   D = 512: 300 rows 12.5 / 9.8, 15000 45.8 / 38.4, 60000 134 / 120, 200003 415 / 372
-//              D = 256: 300 8.6 / 6.7, 15000 24.5 / 21.2, 60000 69.3 / 68.7, 120000 127 / 129, 200003 204 / 208
+//   backward   D = 512: 300 rows 12.6 / 7.5, 2000 16.3 / 11.1, 15000 45.5 / 34.0, 60000 134 / 107, 200003 415 / 330
+//              D = 256: 300 8.8 / 5.8, 2000 11.3 / 8.1, 15000 24.6 / 20.7, 60000 69.1 / 66.4; above, another form of the
+//              staged kernel was level with the register-resident one (120000 127 / 129, 200003 204 / 208)
 // Few rows are few per warp: what a kernel does before its first row counts, and the staged kernels do little.
 constexpr int64_t STAGED_FWD_ROWS = 20000;
 constexpr int64_t STAGED_BWD_ROWS_ONE_VECTOR = 65536;
@@ -1882,13 +1951,17 @@ int norm_mul_t(const b200_hstu_norm_mul_args &a, bool bwd, cudaStream_t st) {
              (pick_maxv<E>(D) == 2 || a.rows <= STAGED_BWD_ROWS_ONE_VECTOR)) {
     if constexpr (EV == 8) {
       const bool one = pick_maxv<E>(D) == 1;
-      const int stages = one ? 4 : 2;
-      const size_t ring = (size_t)WARPS * stages * 5 * (one ? 1 : 2) * 32 * sizeof(uint4);   // 80 KB, two CTAs an SM
-      auto kern = one ? norm_mul_bwd_staged_kernel<E, 1, 4> : norm_mul_bwd_staged_kernel<E, 2, 2>;
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
+      const int64_t with_rows = (a.rows + WARPS - 1) / WARPS;
+      if (grid > with_rows) grid = (int)with_rows;   // (a block without rows adds zeros)
+      const bool few = grid <= 2 * num_sms();
+      const int stages = one && !few ? 4 : 2, warps = few ? WARPS : WARPS / 2;
+      const size_t ring = (size_t)warps * stages * 5 * (one ? 1 : 2) * 32 * sizeof(uint4);   // 40 or 80 KB
+      const size_t bytes = ring + (few ? 0 : (size_t)warps * 2 * D * sizeof(float));
+      auto kern = few ? (one ? norm_mul_bwd_staged_kernel<E, 1, 2, 1> : norm_mul_bwd_staged_kernel<E, 2, 2, 1>)
+                      : (one ? norm_mul_bwd_staged_kernel<E, 1, 4, 2> : norm_mul_bwd_staged_kernel<E, 2, 2, 2>);
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
       if (e != cudaSuccess) return check_cuda(e, "norm_mul backward smem attribute");
-      if (grid > 2 * num_sms()) grid = 2 * num_sms();
-      kern<<<grid, WARPS * 32, ring, st>>>(p);
+      kern<<<grid, warps * 32, bytes, st>>>(p);
     }
   } else if (dropout && D % EV == 0) {
     DISPATCH_MAXV(pick_maxv<E>(D), {

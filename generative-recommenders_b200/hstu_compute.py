@@ -366,9 +366,9 @@ def _norm_mul_backward(dout, attn, u, weight, bias, mean, rstd, eps, num_heads, 
 # is stored.  Switched on, the forward also writes the mask as bits (6 % of the output's bytes) and the
 # backward reads them.  Measured on B200 at 1965 MHz, 200 k rows of bf16, [u | attn | y], ratio 0.3, forward +
 # backward in us (repeats agree within 1 %): D = 256 156 + 207 regenerating, 169 + 225 stored;
-# D = 512 270 + 372 and 314 + 305; D = 1024 592 + 840 and 803 + 3470 (the kernel for that width, with its
-# accumulators in shared memory, only regenerates).  It pays at D = 512 alone, by 4 % for 6 % more activation
-# memory, so it is off.  With recompute_y the mask is never stored.
+# D = 512 270 + 330 and 314 + 305; D = 1024 592 + 840 and 803 + 3470 (the kernel for that width, with its
+# accumulators in shared memory, only regenerates).  It pays at none of these, so it is off.  With recompute_y the
+# mask is never stored.
 _STORE_DROPOUT_MASK = False
 
 

@@ -281,3 +281,29 @@ def test_dropout_kernels_for_few_and_many_rows_agree(H, V, rows):
         results.append((y,) + torch.autograd.grad(y, leaves, dy[:n]))
     for many, few in zip(*results):
         assert torch.equal(many[:70], few)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("act", [0, 2])
+@pytest.mark.parametrize("H,V,rows", [(4, 128, 1), (4, 128, 70), (3, 104, 2368), (4, 128, 2369), (4, 64, 3553), (3, 104, 8347),
+                                      (1, 8, 8347), (4, 128, 20000)])
+def test_staged_dropout_kernels_have_the_bits_of_the_register_kernels(H, V, rows, act, dtype):
+    """Results, stored statistics and all four gradients.  Rows that start off the 16-byte grid are read by the
+    kernels that hold them in registers; the order of every sum is the same in both."""
+    from generative_recommenders_b200 import hstu_compute as HC
+
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    D = H * V
+    attn, u = (torch.randn(rows, D, generator=g, device=DEV).to(dtype) for _ in range(2))
+    w, b = (torch.randn(D, generator=g, device=DEV).to(dtype) for _ in range(2))
+    dy = torch.randn(rows, 3 * D, generator=g, device=DEV).to(dtype)
+    seed = torch.tensor([77], dtype=torch.int64, device=DEV)
+    elsewhere = torch.empty(rows * D + 1, dtype=dtype, device=DEV)[1:].view(rows, D).copy_(attn)
+    assert attn.data_ptr() % 16 == 0 and elsewhere.data_ptr() % 16 != 0
+    results = []
+    for x in (attn, elsewhere):
+        cfg = (1e-6, H, V, True, True, act, False, 0.3, seed)
+        y, mean, rstd = HC._norm_mul_forward(x, u, w, b, *cfg)
+        results.append((y, mean, rstd) + tuple(HC._norm_mul_backward(dy, x, u, w, b, mean, rstd, *cfg)))
+    for name, one, other in zip(("y", "mean", "rstd", "dattn", "du", "dweight", "dbias"), *results):
+        assert torch.equal(one, other), name
