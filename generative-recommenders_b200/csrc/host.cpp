@@ -34,6 +34,12 @@ struct Launch {
       : guard(t.device()), stream(at::cuda::getCurrentCUDAStream(t.device().index()).stream()) {}
 };
 
+// A kernel walks a buffer by the dtype code of the call: what a GEMM has made has to have that type.
+const Tensor &of_type(const Tensor &t, at::ScalarType type) {
+  TORCH_CHECK(t.scalar_type() == type, "a library GEMM gave ", t.scalar_type(), " where the next kernel reads ", type);
+  return t;
+}
+
 Tensor empty_like_of(at::IntArrayRef shape, const Tensor &t) { return at::empty(shape, t.options()); }
 Tensor floats(int64_t n, const Tensor &t) { return at::empty({n}, t.options().dtype(at::kFloat)); }
 Tensor bytes(int64_t n, const Tensor &t) { return at::empty({n}, t.options().dtype(at::kByte)); }
@@ -413,7 +419,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> separate_attention_inference(
                                    normed.stride(0), nullptr, nullptr, x.size(0), (int32_t)x.size(1), (float)eps,
                                    (int32_t)dtype, l.stream),
           "b200_hstu_layer_norm_fwd");
-    uvqk = at::addmm(b, normed, w);
+    uvqk = of_type(at::addmm(b, normed, w), x.scalar_type());
     check(b200_hstu_silu_fwd(uvqk.data_ptr(), uvqk.stride(0), u.data_ptr(), u.stride(0), x.size(0), (int32_t)(H * V),
                              (int32_t)dtype, l.stream),
           "b200_hstu_silu_fwd");

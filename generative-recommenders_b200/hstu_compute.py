@@ -507,7 +507,7 @@ def _output_inference(attn, u, x, norm_weight, norm_bias, norm_eps, output_weigh
         as_dtype(output_weight, x.dtype), float(norm_eps), int(num_heads),
         int(linear_dim) if linear_dim > 0 else attn.shape[1] // num_heads, bool(concat_u), bool(concat_x), act, False,
         float(dropout_ratio), _draw_dropout_seed(attn.device) if dropout_ratio > 0.0 else None, dtype_code(attn), False,
-        over_x and x.is_contiguous())[0]
+        over_x and x.is_contiguous() and not torch.is_autocast_enabled("cuda"))[0]
 
 
 def _compute_output(attn, u, x, norm_weight, norm_bias, norm_eps, output_weight, num_heads, linear_dim, dropout_ratio,
@@ -634,7 +634,8 @@ def hstu_preprocess_and_attention(
         return u, attn.view(-1, hidden_dim * num_heads), k, v
     if (x.is_cuda and x.shape[0] > 0 and x.stride(1) == 1 and not (_FUSED_UQVK and _fused_uqvk_supported(x, uvqk_weight, hv))
             and all(t.dtype is x.dtype for t in (norm_weight, norm_bias, uvqk_weight, uvqk_bias))
-            and outside_autograd(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias, bias_by_distance)):
+            and outside_autograd(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias, bias_by_distance)
+            and not torch.is_autocast_enabled("cuda")):   # (it changes the type between the stages)
         # the separate stages in one call
         require_cuda(norm_weight, norm_bias, uvqk_weight, uvqk_bias, seq_offsets, num_targets, bias_by_distance)
         offs, nt = _index(seq_offsets), _index(num_targets)

@@ -211,3 +211,43 @@ def test_block_offsets_reach_the_quantiser(fp8, blocks):
     _, _, out = module.quantize_e4m3_block(torch.zeros(300, 1, 64), torch.tensor([0, 100, 300]), blocks)
     assert seen == [[0, 1, 3]]
     assert out is blocks
+
+
+class _OnDevice(torch.Tensor):
+    is_cuda = True
+
+
+@pytest.mark.parametrize("autocast", [False, True])
+def test_separate_stages_go_one_by_one_under_autocast(monkeypatch, autocast):
+    """Autocast changes the type between LayerNorm, linear and attention: each op has to see the tensor it gets.
+    The one native call, whose kernels are all told the type of x, is for calls without it."""
+    D, H, d, M = 24, 2, 4, 6
+    made = [torch.zeros(s).as_subclass(_OnDevice) for s in ((M, D), (D,), (D,), (D, 4 * H * d), (4 * H * d,))]
+    offsets = torch.tensor([0, M]).as_subclass(_OnDevice)
+    taken = []
+
+    class _Host:
+        def separate_attention_inference(self, *args):
+            taken.append("one call")
+            return (made[0],) * 4
+
+    def uqvk(**kwargs):
+        taken.append("uqvk")
+        return (torch.zeros(M, H * d),) + (torch.zeros(M, H, d),) * 3
+
+    def attention(**kwargs):
+        taken.append("attention")
+        return torch.zeros(M, H, d)
+
+    monkeypatch.setattr(HC._cabi, "host", lambda: _Host())
+    monkeypatch.setattr(HC, "hstu_compute_uqvk", uqvk)
+    monkeypatch.setattr(HC, "hstu_mha", attention)
+    before = torch.is_autocast_enabled("cuda")
+    torch.set_autocast_enabled("cuda", autocast)
+    try:
+        with torch.no_grad():
+            HC.hstu_preprocess_and_attention(made[0], made[1], made[2], 1e-6, H, d, d, made[3], made[4], M, offsets, 0.5,
+                                             True, None, 0, 0, False, False, False)
+    finally:
+        torch.set_autocast_enabled("cuda", before)
+    assert taken == (["uqvk", "attention"] if autocast else ["one call"])

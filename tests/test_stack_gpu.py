@@ -346,3 +346,41 @@ def test_stack_overwrites_nothing_that_anyone_sees(D, H, d):
         assert torch.equal(stack(x, lengths, offs, 130, None), want[-1])
         handle.remove()
     assert torch.equal(seen[0], want[2]) and torch.equal(x, before)
+
+
+@pytest.mark.parametrize("D, H, d, dtype, other", [(256, 2, 64, torch.float32, torch.bfloat16),
+                                                   (520, 3, 8, torch.float32, torch.float16),
+                                                   (768, 6, 128, torch.bfloat16, torch.float16)])
+def test_stack_under_autocast_equals_the_ops_one_by_one(D, H, d, dtype, other):
+    """Autocast runs the linears in its own type: without gradients every stage takes the type that reaches it."""
+    stack = G.STUStack([_layer(D, H, d, dtype, i) for i in range(2)])
+    lengths = torch.tensor([5, 130, 3, 77], device=DEV)
+    offs = torch.cat([lengths.new_zeros(1), lengths.cumsum(0)])
+    x = torch.randn(int(offs[-1]), D, device=DEV).to(dtype)
+    with torch.no_grad(), torch.autocast("cuda", other):
+        got = stack(x, lengths, offs, 130, None)
+        want = x
+        for layer in stack._stu_layers:
+            u, q, k, v = G.hstu_compute_uqvk(want, *(p.to(want.dtype) for p in (layer._input_norm_weight, layer._input_norm_bias)),
+                                             1e-6, H, d, d, layer._uvqk_weight.to(want.dtype),
+                                             layer._uvqk_beta.to(want.dtype))
+            assert q.dtype is other
+            attn = G.hstu_mha(130, layer._attn_alpha, q, k, v, offs, contextual_seq_len=2).flatten(1)
+            y = G.hstu_norm_mul_dropout(attn, u, layer._output_norm_weight, layer._output_norm_bias, 1e-6, 0.3, False, True,
+                                        True, "none", False, H, d)
+            want = torch.addmm(want, y, layer._output_weight.to(want.dtype))
+    assert got.dtype is other and torch.equal(got, want)
+
+
+def test_separate_stages_refuse_a_gemm_of_another_type():
+    """The native call stops before a kernel reads a buffer as a type that it has not."""
+    M, D, H, d = 130, 520, 3, 8
+    x, w = torch.randn(M, D, device=DEV), torch.randn(D, 4 * H * d, device=DEV)
+    nw, nb, b = torch.ones(D, device=DEV), torch.zeros(D, device=DEV), torch.zeros(4 * H * d, device=DEV)
+    offs = torch.tensor([0, M], device=DEV)
+    call = lambda: G._cabi.host().separate_attention_inference(  # noqa: E731
+        x, nw, nb, w, b, 1e-6, H, d, d, offs, None, None, M, 0.1, 0, 0, 0, G._cabi.F32, False)
+    with torch.no_grad():
+        call()
+        with torch.autocast("cuda", torch.bfloat16), pytest.raises(RuntimeError, match="library GEMM"):
+            call()
