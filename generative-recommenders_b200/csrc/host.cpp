@@ -6,6 +6,7 @@
 // backward); with one Python call, a ctypes struct and a few tensor objects per launch its host side
 // took 115 and 660 us, and the GPU waited.
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
@@ -32,6 +33,12 @@ struct Launch {
   cudaStream_t stream;
   explicit Launch(const Tensor &t)
       : guard(t.device()), stream(at::cuda::getCurrentCUDAStream(t.device().index()).stream()) {}
+};
+
+// The library GEMMs go through the dispatcher, so under autocast they convert their operands.  The backwards
+// are called with the types that the forward chose and keep them, wherever they are called.
+struct NoAutocast {
+  c10::impl::ExcludeDispatchKeyGuard guard{c10::autocast_dispatch_keyset};
 };
 
 // A kernel walks a buffer by the dtype code of the call: what a GEMM has made has to have that type.
@@ -313,15 +320,18 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> output_backward(
     const Tensor &dout_, const Tensor &attn, const Tensor &u, const Tensor &weight, const Tensor &bias,
     const Tensor &output_weight, const Tensor &mean, const Tensor &rstd, double eps, int64_t H, int64_t V,
     bool concat_u, bool concat_x, int64_t act, bool group_norm, double dropout, const MaybeTensor &seed, int64_t dtype) {
+  const NoAutocast no_autocast;
   Tensor d_wo;
-  const Tensor dout = dout_.stride(-1) != 1 ? dout_.contiguous() : dout_;
+  // (under autocast the forward's result may have another type than what went into it)
+  const at::ScalarType type = attn.scalar_type();
+  const Tensor dout = (dout_.stride(-1) != 1 ? dout_.contiguous() : dout_).to(type), wo = output_weight.to(type);
   {
     Tensor y = std::get<0>(norm_mul_forward(attn, u, weight, bias, eps, H, V, concat_u, concat_x, act, group_norm,
                                             dropout, seed, dtype, false, true));
     d_wo = at::mm(y.t(), dout);
   }
-  const Tensor dy = at::mm(dout, output_weight.t());
-  auto [dattn, du, dw, db] = norm_mul_backward(dy, attn, u, weight, bias, mean, rstd, eps, H, V, concat_u, concat_x,
+  const Tensor dy = at::mm(dout, wo.t());
+  auto [dattn, du, dw, db] = norm_mul_backward(of_type(dy, type), attn, u, weight, bias, mean, rstd, eps, H, V, concat_u, concat_x,
                                                act, group_norm, dropout, seed, std::nullopt, dtype);
   return {dattn, du, dw, db, d_wo};
 }
@@ -488,6 +498,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> uvqk_backward(const Tensor &x
                                                                  const Tensor &mean, const Tensor &rstd, double eps,
                                                                  int64_t hv, const MaybeTensor &du_, const Tensor &d_uvqk,
                                                                  int64_t dtype) {
+  const NoAutocast no_autocast;
   const int64_t M = x.size(0), D = x.size(1);
   const int32_t dt = (int32_t)dtype;
   Launch l(x);
@@ -506,7 +517,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> uvqk_backward(const Tensor &x
   Tensor dw = at::mm(normed.t(), d_uvqk);
   // column sums on the tensor cores: cheaper than a strided reduction over [M, N]
   Tensor db = at::mm(at::ones({1, M}, x.options()), d_uvqk).view(-1);
-  Tensor dnormed = at::mm(d_uvqk, w.t());
+  Tensor dnormed = of_type(at::mm(d_uvqk, w.t()), x.scalar_type());
   Tensor dx = at::empty_like(x);
   Tensor dnw = empty_like_of({D}, x), dnb = empty_like_of({D}, x);
   const int64_t n = b200_hstu_layer_norm_bwd_workspace_bytes((int32_t)D);

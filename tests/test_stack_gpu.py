@@ -384,3 +384,39 @@ def test_separate_stages_refuse_a_gemm_of_another_type():
         call()
         with torch.autocast("cuda", torch.bfloat16), pytest.raises(RuntimeError, match="library GEMM"):
             call()
+
+
+@pytest.mark.parametrize("D, H, d, dtype, forward_type, backward_type", [
+    (256, 2, 64, torch.float16, None, torch.bfloat16),               # fused uvqk stage
+    # (uvqk linear as torch's own node, which takes bfloat16 operands in such a region: 2 ** -8 each)
+    (256, 2, 64, torch.float32, None, torch.bfloat16),
+    (256, 2, 64, torch.float32, torch.bfloat16, torch.bfloat16),
+    (256, 2, 64, torch.float32, torch.bfloat16, None),
+])
+def test_backward_keeps_the_types_of_the_forward(D, H, d, dtype, forward_type, backward_type):
+    """A backward gives the same gradients inside an autocast region and outside, and those of the layer whose output
+    stage is not one node."""
+    import contextlib
+
+    region = lambda t: contextlib.nullcontext() if t is None else torch.autocast("cuda", t)  # noqa: E731
+    layer = _layer(D, H, d, dtype, 5).train()
+    layer._output_dropout_ratio = 0.0
+    lengths = torch.tensor([5, 130, 3, 77], device=DEV)
+    offs = torch.cat([lengths.new_zeros(1), lengths.cumsum(0)])
+    x = torch.randn(int(offs[-1]), D, device=DEV).to(dtype).requires_grad_()
+    dy = torch.randn(int(offs[-1]), D, device=DEV)
+
+    def gradients(recompute, backward):
+        layer._recompute_y = recompute
+        with region(forward_type):
+            y = layer(x, lengths, offs, 130, None)
+        with region(backward):
+            return torch.autograd.grad(y, [x] + list(layer.parameters()), dy.to(y.dtype))
+
+    got, plain, apart = gradients(True, backward_type), gradients(True, None), gradients(False, None)
+    names = ["x"] + [n for n, _ in layer.named_parameters()]
+    torchs_own = dtype is torch.float32 and forward_type is None
+    for name, a, b, c, p in zip(names, got, plain, apart, [x] + list(layer.parameters())):
+        assert a.dtype is p.dtype
+        assert torch.equal(a, b) or (torchs_own and not name.startswith("_output")), name
+        assert O.rel_l2(a, c) < 1e-2, name
