@@ -192,7 +192,7 @@ class STULayer(torch.nn.Module):
         num_targets_ = num_targets if self._target_aware else None
         fused = None
         if (self.k_cache is not None and self.v_cache is not None and self.kv_caching_offsets is not None
-                and type(self).construct_full_kv is STULayer.construct_full_kv
+                and _is_own(self, "construct_full_kv")
                 and delta_x.dim() == 2 and delta_x.shape[0] > 0):
             delta_size = delta_x.shape[0] // (self.kv_caching_offsets.numel() - 1)
             max_seq_len = self.max_kv_caching_len + delta_size
@@ -335,12 +335,22 @@ class STULayer(torch.nn.Module):
             )
 
 
+# What the shortcuts below stand in for.  Whoever replaces one of these, on the class as on a layer, wants the
+# replacement called for every layer.
+_OWN = {name: getattr(STULayer, name) for name in ("__call__", "_call_impl", "forward", "cached_forward", "construct_full_kv")}
+
+
+def _is_own(layer, method) -> bool:
+    return type(layer) is STULayer and method not in layer.__dict__ and getattr(STULayer, method) is _OWN[method]
+
+
 def _unobserved(layer, method) -> bool:
-    """True where ``layer.method`` is this file's and no hook gets to see what goes in or comes out."""
-    return (type(layer) is STULayer and method not in layer.__dict__ and not layer._forward_hooks
-            and not layer._forward_pre_hooks and not layer._backward_hooks and not layer._backward_pre_hooks
-            and layer._compiled_call_impl is None and not _module._has_any_global_hook()
-            and not is_compiling())
+    """True without gradients where ``layer.method`` is this file's and no hook, tracer or dispatch mode gets to
+    see what goes in or comes out."""
+    return (not torch.is_grad_enabled() and not is_compiling() and _is_own(layer, method) and _is_own(layer, "__call__")
+            and _is_own(layer, "_call_impl") and not layer._forward_hooks and not layer._forward_pre_hooks
+            and not layer._backward_hooks and not layer._backward_pre_hooks and layer._compiled_call_impl is None
+            and not _module._has_any_global_hook() and torch._C._len_torch_dispatch_stack() == 0)
 
 
 class STUStack(torch.nn.Module):

@@ -251,3 +251,66 @@ def test_separate_stages_go_one_by_one_under_autocast(monkeypatch, autocast):
     finally:
         torch.set_autocast_enabled("cuda", before)
     assert taken == (["uqvk", "attention"] if autocast else ["one call"])
+
+
+class _Sees(torch.utils._python_dispatch.TorchDispatchMode):
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize("replaced, on_class", [(name, on_class) for name in ("forward", "cached_forward", "construct_full_kv")
+                                               for on_class in (False, True)] + [("__call__", True)])
+def test_replaced_methods_of_a_layer_are_called_for_every_layer(monkeypatch, replaced, on_class):
+    stu = importlib.import_module("generative-recommenders_b200.stu")
+    cfg = G.STULayerConfig(embedding_dim=16, num_heads=1, hidden_dim=16, attention_dim=16)
+    layers = [G.STULayer(cfg) for _ in range(3)]
+    stack = G.STUStack(layers)
+    for layer in layers:
+        layer.k_cache = layer.v_cache = torch.zeros(5, 16)
+        layer.kv_caching_offsets, layer.max_kv_caching_len = torch.tensor([0, 2, 5]), 3
+    taken = []
+    shortcuts = {"forward": "_forward", "cached_forward": "_cached_forward", "__call__": "_forward"}
+    if replaced in shortcuts:
+        monkeypatch.setattr(stu.STULayer, shortcuts[replaced], lambda self, *a, **kw: taken.append("own") or torch.zeros(2, 16))
+    else:
+        monkeypatch.setattr(stu, "hstu_cached_attention", lambda *a: taken.append("own"))
+        monkeypatch.setattr(stu.STULayer, "_cached_attention_of_ops", lambda self, *a: (None, None))
+        monkeypatch.setattr(stu, "_compute_output", lambda **kw: kw["x"])
+
+    def run():
+        taken.clear()
+        with torch.no_grad():
+            if replaced in ("forward", "__call__"):
+                stack(torch.zeros(2, 16), None, None, 2, None)
+            else:
+                stack.cached_forward(torch.zeros(2, 16), None)
+        return list(taken)
+
+    assert run() == ["own"] * 3
+    if replaced == "__call__":
+        own = torch.nn.Module.__call__
+        monkeypatch.setattr(torch.nn.Module, "__call__", lambda self, *a, **kw: (
+            own(self, *a, **kw) if self is stack else taken.append("replaced") or torch.zeros(2, 16)))
+    else:
+        def replacement(*args, **kwargs):
+            taken.append("replaced")
+            return torch.zeros(2, 16)
+        if on_class:
+            monkeypatch.setattr(stu.STULayer, replaced, replacement)
+        else:
+            for layer in layers:
+                setattr(layer, replaced, replacement)
+    if replaced == "construct_full_kv":
+        assert run() == []     # (the ops one by one, which call it)
+    else:
+        assert run() == ["replaced"] * 3
+
+
+def test_layers_are_called_as_modules_where_someone_looks_on():
+    stu = importlib.import_module("generative-recommenders_b200.stu")
+    layer = G.STULayer(G.STULayerConfig(embedding_dim=16, num_heads=1, hidden_dim=16, attention_dim=16))
+    with torch.no_grad():
+        assert stu._unobserved(layer, "forward") and stu._unobserved(layer, "cached_forward")
+        with _Sees():
+            assert not stu._unobserved(layer, "forward")
+    assert not stu._unobserved(layer, "forward")     # (gradients: nothing may be overwritten)
