@@ -44,6 +44,12 @@ def _i32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     return as_dtype(t, torch.int32).contiguous()
 
 
+def _require_target_counts(num_targets: Optional[torch.Tensor], sequences: int) -> None:
+    # (the kernels read one entry of every sequence)
+    if num_targets is not None and num_targets.numel() < sequences:
+        raise RuntimeError("num_targets must have one entry per sequence")
+
+
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None or t.numel() == 0 else t.data_ptr()
 
@@ -324,6 +330,7 @@ def delta_hstu_mha(
     require_cuda(delta_q, k, v, seq_offsets, num_targets)
     if k.dtype != delta_q.dtype or v.dtype != delta_q.dtype:
         raise TypeError("delta_q, k, v must share a dtype")
+    _require_target_counts(num_targets, B)
     delta = L // B
     if L == 0 or k.shape[0] == 0:
         return torch.zeros((L, H, v.shape[2]), dtype=delta_q.dtype, device=delta_q.device)

@@ -12,7 +12,7 @@ import torch
 
 from . import _cabi
 from .common import as_dtype, dtype_code, last_dim_contiguous, on_device, require_cuda, stream_ptr
-from .hstu_attention import _index
+from .hstu_attention import _index, _require_target_counts
 
 BLOCK = 128
 
@@ -71,6 +71,7 @@ def hstu_mha_fp8(
     for t in (q8, k8, v8):
         if t.dtype != torch.float8_e4m3fn or not t.is_contiguous():
             raise TypeError("q8 / k8 / v8 must be contiguous float8_e4m3fn tensors")
+    _require_target_counts(num_targets, seq_offsets.numel() - 1)
     L, H, d = q8.shape
     out = torch.empty((L, H, d), dtype=torch.bfloat16, device=q8.device)
     if L == 0:

@@ -10,7 +10,7 @@ from . import _cabi
 from .common import (HammerKernel, _require_cuda_backend, as_dtype, dtype_code, on_device, outside_autograd,
                      require_cuda, stream_ptr)
 from . import hstu_attention as _attention
-from .hstu_attention import _i32, _index, hstu_mha
+from .hstu_attention import _i32, _index, _require_target_counts, hstu_mha
 from .layer_norm import layer_norm
 from .mm import addmm
 
@@ -297,6 +297,7 @@ def hstu_cached_attention(x, norm_weight, norm_bias, norm_eps, num_heads, attn_d
         if t.dim() != 2 or t.shape[1] != width or t.dtype is not x.dtype or not t.is_contiguous():
             return None
     require_cuda(norm_weight, norm_bias, uvqk_weight, uvqk_bias, k_cache, v_cache, cache_offsets, num_targets)
+    _require_target_counts(num_targets, B)
     nw, nb, w, b = _stage_parameters(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias)
     nbytes = _cabi.lib().b200_hstu_ln_linear_workspace_bytes(*w.shape)
     ws, prepared, remember = _prepared_workspace(nw, nb, w, b, nbytes, x.device, True)

@@ -314,3 +314,41 @@ def test_layers_are_called_as_modules_where_someone_looks_on():
         with _Sees():
             assert not stu._unobserved(layer, "forward")
     assert not stu._unobserved(layer, "forward")     # (gradients: nothing may be overwritten)
+
+
+def _cached_call(monkeypatch, host, targets, k_rows=5, v_rows=5):
+    """``hstu_cached_attention`` of two sequences with one new row each; ``host`` answers the native call."""
+    D = 16
+    on = lambda *s, dtype=torch.bfloat16: torch.zeros(s, dtype=dtype).as_subclass(_OnDevice)  # noqa: E731
+    monkeypatch.setattr(HC, "_fused_uqvk_supported", lambda *a: True)
+    monkeypatch.setattr(HC, "_prepared_workspace", lambda *a: (None, False, None))
+    monkeypatch.setattr(HC._cabi, "lib", lambda: _Library())
+    monkeypatch.setattr(HC._cabi, "host", lambda: host)
+    offsets = torch.tensor([0, 2, 5]).as_subclass(_OnDevice)
+    targets = None if targets is None else torch.ones(targets, dtype=torch.int64).as_subclass(_OnDevice)
+    with torch.no_grad():
+        return HC.hstu_cached_attention(on(2, D), on(D), on(D), 1e-6, 1, D, D, on(D, 4 * D), on(4 * D), on(k_rows, D),
+                                        on(v_rows, D), offsets, targets, 4, 0.1, 0, 0)
+
+
+class _Taken:
+    def cached_attention(self, *args):
+        return "taken"
+
+
+@pytest.mark.parametrize("targets", [None, 2, 3])
+def test_cached_attention_takes_a_target_count_for_every_sequence(monkeypatch, targets):
+    assert _cached_call(monkeypatch, _Taken(), targets) == "taken"
+
+
+def test_attention_of_new_rows_refuses_missing_target_counts(monkeypatch):
+    """The kernels read ``num_targets[b]`` of every sequence."""
+    with pytest.raises(RuntimeError, match="one entry per sequence"):
+        _cached_call(monkeypatch, _Taken(), 1)
+    rows = torch.zeros(2, 1, 16).as_subclass(_OnDevice)
+    offsets, targets = (torch.tensor(t).as_subclass(_OnDevice) for t in ([0, 1, 2], [1]))
+    with pytest.raises(RuntimeError, match="one entry per sequence"):
+        G.delta_hstu_mha(2, 0.1, rows, rows, rows, offsets, targets)
+    q8 = rows.to(torch.float8_e4m3fn).as_subclass(_OnDevice)
+    with pytest.raises(RuntimeError, match="one entry per sequence"):
+        G.hstu_mha_fp8(2, 0.1, q8, q8, q8, rows, rows, rows, offsets, offsets, targets)
