@@ -326,6 +326,7 @@ def delta_hstu_mha(
     torch._assert(k.shape[1] == H, "wrong k shape[1]")
     torch._assert(k.shape[2] == D, "wrong k shape[2]")
     torch._assert(v.dim() == 3, "v must be 3-D")
+    torch._assert(v.shape[0] >= k.shape[0], "wrong v shape[0]")
     torch._assert(v.shape[1] == H, "wrong v shape[1]")
     require_cuda(delta_q, k, v, seq_offsets, num_targets)
     if k.dtype != delta_q.dtype or v.dtype != delta_q.dtype:

@@ -294,7 +294,7 @@ def hstu_cached_attention(x, norm_weight, norm_bias, norm_eps, num_heads, attn_d
             and outside_autograd(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias, k_cache, v_cache)):
         return None
     for t, width in ((k_cache, ha), (v_cache, hv)):
-        if t.dim() != 2 or t.shape[1] != width or t.dtype is not x.dtype or not t.is_contiguous():
+        if t.dim() != 2 or t.shape != (k_cache.shape[0], width) or t.dtype is not x.dtype or not t.is_contiguous():
             return None
     require_cuda(norm_weight, norm_bias, uvqk_weight, uvqk_bias, k_cache, v_cache, cache_offsets, num_targets)
     _require_target_counts(num_targets, B)

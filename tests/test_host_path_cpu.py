@@ -352,3 +352,14 @@ def test_attention_of_new_rows_refuses_missing_target_counts(monkeypatch):
     q8 = rows.to(torch.float8_e4m3fn).as_subclass(_OnDevice)
     with pytest.raises(RuntimeError, match="one entry per sequence"):
         G.hstu_mha_fp8(2, 0.1, q8, q8, q8, rows, rows, rows, offsets, offsets, targets)
+
+
+@pytest.mark.parametrize("k_rows, v_rows", [(5, 5), (5, 4), (5, 6)])
+def test_cached_attention_reads_k_and_v_of_as_many_rows(monkeypatch, k_rows, v_rows):
+    """One launch appends to both and takes one row count; other caches go to the separate ops, and a V of fewer
+    rows than K is refused where both are read together."""
+    assert _cached_call(monkeypatch, _Taken(), None, k_rows, v_rows) == ("taken" if k_rows == v_rows else None)
+    if v_rows < k_rows:
+        rows = torch.zeros(k_rows, 1, 16).as_subclass(_OnDevice)
+        with pytest.raises(AssertionError, match="wrong v shape"):
+            G.delta_hstu_mha(k_rows, 0.1, rows[:1], rows, rows[:v_rows], torch.tensor([0, k_rows]).as_subclass(_OnDevice))
