@@ -155,7 +155,8 @@ std::tuple<Tensor, MaybeTensor> attention_forward(const Tensor &q, const Tensor 
   if (plan && given(ws)) a.plan_mode = B200_HSTU_PLAN_FOR_BACKWARD;
   Launch l(q);
   check(b200_hstu_attn_fwd(&a, l.stream), delta > 0 ? "b200_hstu_attn_fwd (delta)" : "b200_hstu_attn_fwd");
-  if (status && given(ws)) check_status(a, 0, l.stream, "b200_hstu_attn_fwd");
+  if (status && given(ws))
+    check_status(a, 0, l.stream, delta > 0 ? "b200_hstu_attn_fwd (delta)" : "b200_hstu_attn_fwd");
   return {out, ws};
 }
 
@@ -447,7 +448,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> cached_attention(
     const Tensor &x, const Tensor &nw, const Tensor &nb, const Tensor &w, const Tensor &b, double eps, int64_t H,
     int64_t A, int64_t V, const Tensor &workspace, bool prepared, const Tensor &k_cache, const Tensor &v_cache,
     const Tensor &cache_offsets, const MaybeTensor &targets, int64_t max_seq_len, double alpha, int64_t max_attn_len,
-    int64_t contextual_seq_len, int64_t impl, int64_t dtype) {
+    int64_t contextual_seq_len, int64_t impl, int64_t dtype, bool status) {
   const int64_t B = cache_offsets.numel() - 1, delta = x.size(0) / B, rows = k_cache.size(0) + x.size(0);
   const Uvqk s = uvqk_launch(x, nw, nb, w, b, eps, H * V, dtype, true, workspace, prepared);
   const Qkv t = qkv_views(s.uvqk, H, A, V);
@@ -473,7 +474,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> cached_attention(
   check(b200_hstu_append_kv(&a, l.stream), "b200_hstu_append_kv");
   Tensor out = std::get<0>(attention_forward(t.q, k, v, offsets, targets, std::nullopt, std::nullopt, max_seq_len, alpha,
                                              max_attn_len, contextual_seq_len, 0, impl, dtype, false, 0.0, std::nullopt,
-                                             delta, true, false));
+                                             delta, true, status));
   return {s.u, out.view({x.size(0), H * V}), k, v, offsets};
 }
 

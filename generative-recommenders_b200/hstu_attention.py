@@ -340,5 +340,5 @@ def delta_hstu_mha(
     v = last_dim_contiguous(v.detach())
     out, _ = _cabi.host().attention_forward(
         q, k, v, _index(seq_offsets), _index(num_targets), None, None, int(max_seq_len), float(alpha), int(max_attn_len),
-        int(contextual_seq_len), 0, _IMPL[_forced_impl], dtype_code(q), False, 0.0, None, delta, False, False)
+        int(contextual_seq_len), 0, _IMPL[_forced_impl], dtype_code(q), False, 0.0, None, delta, False, _CHECK_STATUS)
     return out

@@ -290,7 +290,7 @@ def hstu_cached_attention(x, norm_weight, norm_bias, norm_eps, num_heads, attn_d
     hv, ha, M = hidden_dim * num_heads, attn_dim * num_heads, x.shape[0]
     B = cache_offsets.numel() - 1
     if not (_FUSED_UQVK and x.is_cuda and _fused_uqvk_supported(x, uvqk_weight, hv) and B > 0 and M % B == 0
-            and cache_offsets.dtype is torch.int64 and cache_offsets.is_contiguous() and not _attention._CHECK_STATUS
+            and cache_offsets.dtype is torch.int64 and cache_offsets.is_contiguous()
             and outside_autograd(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias, k_cache, v_cache)):
         return None
     for t, width in ((k_cache, ha), (v_cache, hv)):
@@ -304,7 +304,7 @@ def hstu_cached_attention(x, norm_weight, norm_bias, norm_eps, num_heads, attn_d
     result = _cabi.host().cached_attention(
         x, nw, nb, w, b, float(norm_eps), num_heads, attn_dim, hidden_dim, ws, prepared, k_cache, v_cache,
         cache_offsets, _index(num_targets), int(max_seq_len), float(attn_alpha), int(max_attn_len),
-        int(contextual_seq_len), *_attention_switches(x))
+        int(contextual_seq_len), *_attention_switches(x), _attention._CHECK_STATUS)
     if remember is not None:
         remember()
     return result

@@ -363,3 +363,25 @@ def test_cached_attention_reads_k_and_v_of_as_many_rows(monkeypatch, k_rows, v_r
         rows = torch.zeros(k_rows, 1, 16).as_subclass(_OnDevice)
         with pytest.raises(AssertionError, match="wrong v shape"):
             G.delta_hstu_mha(k_rows, 0.1, rows[:1], rows, rows[:v_rows], torch.tensor([0, k_rows]).as_subclass(_OnDevice))
+
+
+@pytest.mark.parametrize("on", [False, True])
+def test_status_check_reaches_cached_attention(monkeypatch, on):
+    """Checked or not, the same path runs."""
+    asked = []
+
+    class _Host:
+        def cached_attention(self, *args):
+            asked.append(args[-1])
+            return "taken"
+
+        def attention_forward(self, *args):
+            asked.append(args[-1])
+            return args[0], None
+
+    HA = importlib.import_module("generative-recommenders_b200.hstu_attention")
+    monkeypatch.setattr(HA, "_CHECK_STATUS", on)
+    assert _cached_call(monkeypatch, _Host(), None) == "taken"
+    rows = torch.zeros(2, 1, 16).as_subclass(_OnDevice)
+    G.delta_hstu_mha(2, 0.1, rows, rows, rows, torch.tensor([0, 1, 2]).as_subclass(_OnDevice))
+    assert asked == [on, on]

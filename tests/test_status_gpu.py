@@ -93,3 +93,23 @@ def test_status_check_reports_a_recorded_site():
     assert HA.attention_status(a, 0, q.device) == [301, 0, 0]
     with pytest.raises(RuntimeError, match="bounded wait"):
         HA._raise_on_status(a, 0, q.device, "test")
+
+
+def test_status_check_of_cached_attention():
+    q, k, v, do, offs, nt = _inputs(3)
+    new = q[:3 * 7]
+    want = G.delta_hstu_mha(600, 0.1, new, k, v, offs)
+    torch.manual_seed(0)
+    layer = G.STULayer(G.STULayerConfig(embedding_dim=256, num_heads=2, hidden_dim=128, attention_dim=128)).to(DEV).bfloat16()
+    layer.k_cache, layer.v_cache = k.flatten(1), v.flatten(1)
+    layer.kv_caching_offsets, layer.max_kv_caching_len = offs, 513
+    x = torch.randn(3 * 7, 256, device=DEV).bfloat16()
+    layer.eval()
+    with torch.no_grad():
+        want_layer = layer.cached_forward(x, nt.clamp(max=7))
+        HA.set_status_check(True)
+        try:
+            got, got_layer = G.delta_hstu_mha(600, 0.1, new, k, v, offs), layer.cached_forward(x, nt.clamp(max=7))
+        finally:
+            HA.set_status_check(False)
+    assert torch.equal(got, want) and torch.equal(got_layer, want_layer)
