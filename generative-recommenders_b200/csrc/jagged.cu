@@ -117,7 +117,7 @@ struct AppendKvArgs {
   int64_t fresh_stride[2], row_bytes[2];   // bytes
   const int64_t *off;                      // of the cache, [B + 1]
   int64_t *off_full;                       // of the result, [B + 1]
-  int64_t total;                           // rows of the result
+  int64_t total, cached;                   // rows of the result, of the cache
   int B, delta;
 };
 
@@ -140,8 +140,8 @@ __global__ void __launch_bounds__(JAG_THREADS) append_kv_kernel(AppendKvArgs a) 
       if (a.off[mid] + (int64_t)a.delta * mid <= g) lo = mid; else hi = mid;
     }
     const int64_t start = a.off[lo], len = a.off[lo + 1] - start, pos = g - start - (int64_t)a.delta * lo;
-    const char *src = nullptr;   // a row the offsets do not account for is skipped
-    if (pos >= 0 && pos < len) src = cache + (start + pos) * row_bytes;
+    const char *src = nullptr;   // a row that the offsets do not account for, or that is not there, is skipped
+    if (pos >= 0 && pos < len && (uint64_t)(start + pos) < (uint64_t)a.cached) src = cache + (start + pos) * row_bytes;
     else if (pos >= len && pos < len + a.delta) src = fresh + ((int64_t)a.delta * lo + pos - len) * fresh_stride;
     source[threadIdx.x] = src;
   }
@@ -168,7 +168,8 @@ __global__ void __launch_bounds__(JAG_THREADS) append_kv_kernel(AppendKvArgs a) 
 
 template <typename V>
 int launch_append_kv(const AppendKvArgs &a, cudaStream_t st) {
-  append_kv_kernel<V><<<dim3((unsigned)((a.total + JAG_ROWS - 1) / JAG_ROWS), 2), JAG_THREADS, 0, st>>>(a);
+  const int64_t blocks = (a.total + JAG_ROWS - 1) / JAG_ROWS;
+  append_kv_kernel<V><<<dim3((unsigned)(blocks > 0 ? blocks : 1), 2), JAG_THREADS, 0, st>>>(a);
   count_launch();
   B200_CHECK_LAUNCH("append_kv_kernel");
   return 0;
@@ -486,9 +487,10 @@ int append_kv(const b200_hstu_append_kv_args &p, cudaStream_t st) {
     return fail(B200_HSTU_EINVAL, "append_kv: negative size");
   AppendKvArgs a;
   a.total = p.cached_rows + (int64_t)p.B * p.delta;
-  if (p.B == 0 || a.total == 0) return 0;
-  if (!p.offsets || !p.full_offsets || !p.k || !p.v || (p.cached_rows > 0 && (!p.k_cache || !p.v_cache)) ||
-      (p.delta > 0 && (!p.k_new || !p.v_new)))
+  if ((p.B == 0 || a.total == 0) && (!p.offsets || !p.full_offsets)) return 0;
+  if (p.B == 0) a.total = 0;   // (no sequence has a row; the offsets are written all the same)
+  if (a.total > 0 && (!p.offsets || !p.full_offsets || !p.k || !p.v || (p.cached_rows > 0 && (!p.k_cache || !p.v_cache)) ||
+                      (p.delta > 0 && (!p.k_new || !p.v_new))))
     return fail(B200_HSTU_EINVAL, "append_kv: null tensor");
   a.cache[0] = (const char *)p.k_cache;
   a.cache[1] = (const char *)p.v_cache;
@@ -502,6 +504,7 @@ int append_kv(const b200_hstu_append_kv_args &p, cudaStream_t st) {
   a.row_bytes[1] = p.v_row_bytes;
   a.off = p.offsets;
   a.off_full = p.full_offsets;
+  a.cached = p.cached_rows;
   a.B = p.B;
   a.delta = p.delta;
   ProfileScope prof(PROF_JAGGED, st);

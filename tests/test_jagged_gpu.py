@@ -271,3 +271,48 @@ def test_positional_encoder_module_matches_oracle():
     assert torch.equal(xg.grad.cpu(), xr.grad)
     torch.testing.assert_close(enc._position_embeddings_weight.grad.cpu(), pw.grad, rtol=1e-4, atol=1e-4)
     torch.testing.assert_close(enc._timestamp_embeddings_weight.grad.cpu(), tw.grad, rtol=1e-4, atol=2e-3)
+
+
+def _append_kv(k_cache, v_cache, k_new, v_new, offsets, full_rows):
+    """``b200_hstu_append_kv`` through the C ABI: (k, v, offsets of both), filled with -1 before."""
+    import ctypes
+
+    class Args(ctypes.Structure):
+        _fields_ = ([(n, ctypes.c_void_p) for n in ("k_cache", "v_cache", "k_new", "v_new", "k", "v", "offsets", "full_offsets")]
+                    + [(n, ctypes.c_int64) for n in ("k_row_bytes", "v_row_bytes", "k_new_stride_bytes", "v_new_stride_bytes",
+                                                     "cached_rows")]
+                    + [("B", ctypes.c_int32), ("delta", ctypes.c_int32)])
+
+    B = offsets.numel() - 1
+    full_k, full_v = (torch.full((full_rows, t.shape[1]), -1, dtype=t.dtype, device=DEV) for t in (k_cache, v_cache))
+    full_offsets = torch.full_like(offsets, -1)
+    size = k_cache.element_size()
+    a = Args(*(t.data_ptr() for t in (k_cache, v_cache, k_new, v_new, full_k, full_v, offsets, full_offsets)),
+             k_cache.shape[1] * size, v_cache.shape[1] * size, k_new.stride(0) * size, v_new.stride(0) * size,
+             k_cache.shape[0], B, k_new.shape[0] // max(B, 1))
+    G._cabi.check(G._cabi.lib().b200_hstu_append_kv(ctypes.byref(a), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)),
+                  "b200_hstu_append_kv")
+    torch.cuda.synchronize()
+    return full_k, full_v, full_offsets
+
+
+@pytest.mark.parametrize("width, skip, dtype", [(64, 0, torch.bfloat16), (64, 2, torch.bfloat16), (64, 1, torch.bfloat16),
+                                                (3, 0, torch.float32), (5, 0, torch.int8)])
+@pytest.mark.parametrize("lengths, delta", [([3, 0, 40], 2), ([1], 1), ([0, 0], 0), ([0, 5], 0), ([], 0), ([0, 0, 0], 9)])
+def test_append_kv_at_every_alignment_and_without_rows(width, skip, dtype, lengths, delta):
+    """16-byte, 4-byte and single-byte moves (``skip``: elements before the caches), the new rows with strides of
+    their own; the offsets are written for an empty result too."""
+    g = torch.Generator().manual_seed(width)
+    rows, B = sum(lengths), len(lengths)
+    draw = lambda n, w: torch.randint(-100, 100, (n, w), generator=g).to(dtype).to(DEV)  # noqa: E731
+    k_cache, v_cache = (torch.zeros(skip + rows * w, dtype=dtype, device=DEV)[skip:].view(rows, w).copy_(draw(rows, w))
+                        for w in (width, 2 * width))
+    both = draw(B * delta, 3 * width)
+    k_new, v_new = both[:, :width], both[:, width:]
+    offsets = torch.tensor([0] + lengths, device=DEV).cumsum(0)
+    k, v, full = _append_kv(k_cache, v_cache, k_new, v_new, offsets, rows + B * delta)
+    at = offsets.tolist()
+    for got, cache, new in ((k, k_cache, k_new), (v, v_cache, v_new)):
+        want = [t for b in range(B) for t in (cache[at[b]:at[b + 1]], new[b * delta:(b + 1) * delta])]
+        assert torch.equal(got, torch.cat(want) if want else got[:0])
+    assert full.tolist() == [o + b * delta for b, o in enumerate(at)]
