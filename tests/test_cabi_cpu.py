@@ -206,3 +206,28 @@ def test_backward_tile_rule_leaves_out_what_lies_between_window_and_tail():
             if L - t >= c + 1 and qt * T >= c and c == 0:
                 assert lo // T == int(cols[0]) // T
     assert gaps > 100
+
+
+def test_forward_tile_rule_starts_at_the_first_column_seen_with_a_prefix_too():
+    """Forward and dQ launch with window and full-attention tail (128-row tiles): every visible column is in the range
+    or the diagonal block, and tiles behind the prefix start at the tile of the first column that they see."""
+    lib = _cabi.lib()
+    rng = random.Random(78)
+    T, started = 128, 0
+    for _ in range(200):
+        N = 1500
+        L = rng.randint(1, N)
+        c = rng.choice([0, 1, 5, 127, 128, 129, 300])
+        t = rng.randint(0, max(0, min(L - 1, rng.choice([1, 60, 300]))))
+        W = rng.choice([1, 127, 128, 129, 400])
+        F = rng.choice([0, 1, 100, 128, 129, 700])
+        mask = O.valid_attn_mask(L, t, True, W, c, F)
+        for m0 in range(0, L, T):
+            lo, hi, dg = _range(lib, L, t, N, c, W, F, m0, T)
+            cols = torch.nonzero(mask[m0:m0 + T].any(dim=0)).flatten()
+            held = ((cols >= lo) & (cols < hi)) | ((dg >= 0) & (cols >= dg) & (cols < dg + T))
+            assert bool(held.all()), (L, t, c, W, F, m0, lo, hi, dg)
+            if L - t >= c + 1 and m0 >= c:
+                assert lo // T == int(cols[0]) // T, (L, t, c, W, F, m0, lo, hi, dg)
+                started += lo >= T
+    assert started > 100
