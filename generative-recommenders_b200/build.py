@@ -53,14 +53,17 @@ def _compile(src, obj, verbose):
 
 
 def _build_host(force, verbose):
-    """csrc/host.cpp -> _host.so, an extension module linked against the library beside it."""
-    src, hdr = os.path.join(CSRC, "host.cpp"), os.path.join(ROOT, "include", "b200_hstu.h")
-    if not force and os.path.exists(HOST) and os.path.getmtime(HOST) >= max(os.path.getmtime(src), os.path.getmtime(hdr)):
-        return
+    """csrc/host.cpp -> _host.so, an extension module linked against the library beside it.  It is compiled against
+    torch's headers and the interpreter's, so another of either builds it anew (``build/_host.built_with``)."""
     import sysconfig
 
     import torch
 
+    src, hdr = os.path.join(CSRC, "host.cpp"), os.path.join(ROOT, "include", "b200_hstu.h")
+    stamp, built_with = os.path.join(BUILD, "_host.built_with"), "torch %s, python %s" % (torch.__version__, sys.version)
+    if (not force and os.path.exists(HOST) and os.path.getmtime(HOST) >= max(os.path.getmtime(src), os.path.getmtime(hdr))
+            and os.path.exists(stamp) and open(stamp).read() == built_with):
+        return
     t = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
     includes = [os.path.join(t, "include"), os.path.join(t, "include", "torch", "csrc", "api", "include"),
@@ -74,6 +77,8 @@ def _build_host(force, verbose):
         sys.stderr.write("== host.cpp (exit %d)\n%s\n" % (r.returncode, r.stdout + r.stderr))
     if r.returncode != 0:
         raise RuntimeError("building _host.so failed")
+    with open(stamp, "w") as f:
+        f.write(built_with)
 
 
 def build(force=False, verbose=False):

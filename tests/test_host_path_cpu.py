@@ -385,3 +385,23 @@ def test_status_check_reaches_cached_attention(monkeypatch, on):
     rows = torch.zeros(2, 1, 16).as_subclass(_OnDevice)
     G.delta_hstu_mha(2, 0.1, rows, rows, rows, torch.tensor([0, 1, 2]).as_subclass(_OnDevice))
     assert asked == [on, on]
+
+
+def test_host_module_is_built_anew_for_another_torch(tmp_path, monkeypatch):
+    build = importlib.import_module("generative-recommenders_b200.build")
+    runs = []
+
+    def run(cmd, **kw):
+        runs.append(cmd)
+        (tmp_path / "_host.so").write_text("")
+        return importlib.import_module("subprocess").CompletedProcess(cmd, 0, "", "")
+
+    monkeypatch.setattr(build, "BUILD", str(tmp_path))
+    monkeypatch.setattr(build, "HOST", str(tmp_path / "_host.so"))
+    monkeypatch.setattr(build, "subprocess", type("S", (), {"run": staticmethod(run)}))
+    for expected in (1, 1):
+        build._build_host(False, False)
+        assert len(runs) == expected
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    build._build_host(False, False)
+    assert len(runs) == 2
