@@ -172,6 +172,10 @@ def _fused_uqvk_backward(x, nw, nb, w, uvqk, mean, rstd, eps, hv, du, d_uvqk):
 
 def _stage_parameters(x, norm_weight, norm_bias, weight, bias):
     """The parameters as the fused kernel reads them (a parameter that is so already: itself)."""
+    D, N = weight.shape
+    if x.shape[1] != D or norm_weight.numel() < D or norm_bias.numel() < D or bias.numel() < N:
+        raise RuntimeError("the uvqk stage on rows of %d needs norm parameters of that many entries, a weight of "
+                           "that many rows and a bias of its columns" % x.shape[1])
     return (as_dtype(norm_weight, x.dtype).contiguous(), as_dtype(norm_bias, x.dtype).contiguous(),
             _aligned16(as_dtype(weight, x.dtype).contiguous()), as_dtype(bias, x.dtype).contiguous())
 

@@ -405,3 +405,16 @@ def test_host_module_is_built_anew_for_another_torch(tmp_path, monkeypatch):
     monkeypatch.setattr(torch, "__version__", "0.0.0")
     build._build_host(False, False)
     assert len(runs) == 2
+
+
+@pytest.mark.parametrize("width, norm, rows, bias", [(16, 16, 16, 64), (24, 16, 16, 64), (8, 16, 16, 64), (16, 8, 16, 64),
+                                                     (16, 16, 16, 63)])
+def test_fused_uvqk_stage_refuses_parameters_of_another_width(width, norm, rows, bias):
+    """The kernel reads them, and sizes its workspace, by the width of x."""
+    t = lambda *s: torch.zeros(s, dtype=torch.bfloat16)  # noqa: E731
+    call = lambda: HC._stage_parameters(t(3, width), t(norm), t(norm), t(rows, 64), t(bias))  # noqa: E731
+    if (width, norm, rows, bias) == (16, 16, 16, 64):
+        assert len(call()) == 4
+    else:
+        with pytest.raises(RuntimeError, match="uvqk stage"):
+            call()
