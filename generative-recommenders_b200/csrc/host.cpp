@@ -355,6 +355,9 @@ struct Uvqk {
 Uvqk uvqk_launch(const Tensor &x, const Tensor &nw, const Tensor &nb, const Tensor &w, const Tensor &b, double eps,
                  int64_t hv, int64_t dtype, bool inference, const MaybeTensor &workspace, bool prepared) {
   const int64_t M = x.size(0), D = x.size(1), N = w.size(1);
+  // (the kernel reads them, and sizes its workspace, by the width of x)
+  TORCH_CHECK(w.size(0) == D && nw.numel() >= D && nb.numel() >= D && b.numel() >= N,
+              "uvqk stage: parameters of another width than x");
   Uvqk r;
   r.uvqk = empty_like_of({M, N}, x);
   r.u = empty_like_of({M, hv}, x);
@@ -442,6 +445,19 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> separate_attention_inference(
   return {u, out.view({x.size(0), H * V}), t.k, t.v};
 }
 
+// Whether cached_attention() takes these: one launch appends to K and V, which have the same rows
+bool cached_supported(const Tensor &x, const Tensor &weight, int64_t hv, int64_t ha, const Tensor &k_cache,
+                      const Tensor &v_cache, const Tensor &cache_offsets) {
+  const auto fits = [&](const Tensor &t, int64_t width) {
+    return t.dim() == 2 && t.size(0) == k_cache.size(0) && t.size(1) == width && t.scalar_type() == x.scalar_type() &&
+           t.is_contiguous();
+  };
+  if (x.dim() != 2 || x.size(0) == 0 || (x.scalar_type() != at::kBFloat16 && x.scalar_type() != at::kHalf) ||
+      cache_offsets.scalar_type() != at::kLong || !cache_offsets.is_contiguous() || !fits(k_cache, ha) || !fits(v_cache, hv))
+    return false;
+  return uvqk_supported(x, weight, hv, x.scalar_type() == at::kBFloat16 ? B200_HSTU_BF16 : B200_HSTU_F16);
+}
+
 // Cached inference: uvqk stage on the new rows, their K and V behind the cached ones, attention of the new rows.
 // Returns u, attention output, k, v, offsets of k and v.
 std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> cached_attention(
@@ -450,6 +466,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> cached_attention(
     const Tensor &cache_offsets, const MaybeTensor &targets, int64_t max_seq_len, double alpha, int64_t max_attn_len,
     int64_t contextual_seq_len, int64_t impl, int64_t dtype, bool status) {
   const int64_t B = cache_offsets.numel() - 1, delta = x.size(0) / B, rows = k_cache.size(0) + x.size(0);
+  TORCH_CHECK(!given(targets) || targets->numel() >= B, "num_targets must have one entry per sequence");
   const Uvqk s = uvqk_launch(x, nw, nb, w, b, eps, H * V, dtype, true, workspace, prepared);
   const Qkv t = qkv_views(s.uvqk, H, A, V);
   Tensor k = empty_like_of({rows, H, A}, x), v = empty_like_of({rows, H, V}, x);
@@ -598,6 +615,7 @@ PYBIND11_MODULE(_host, m) {
   m.def("uvqk_backward", &uvqk_backward, unlocked);
   m.def("uvqk_attention_inference", &uvqk_attention_inference, unlocked);
   m.def("separate_attention_inference", &separate_attention_inference, unlocked);
+  m.def("cached_supported", &cached_supported, unlocked);
   m.def("cached_attention", &cached_attention, unlocked);
   m.def("uvqk_attention_forward", &uvqk_attention_forward, unlocked);
   m.def("uvqk_attention_backward", &uvqk_attention_backward, unlocked);

@@ -1253,8 +1253,8 @@ __global__ void __launch_bounds__(WARPS * 32) norm_mul_bwd_kernel(NormMulParams 
 // 3552th row, eight of them to a block, 444 blocks (on 148 SMs).  With CTAs of four warps, each of which adds up two
 // of the eight one after the other (HALVES), all 444 are resident, three an SM.  (444 CTAs of eight warps are two
 // an SM and a last wave that is half empty: 399 us where this form took 368, both before the activation and its
-// derivative shared a sigmoid.)  A batch with at most one row per sum takes CTAs of eight warps and leaves out
-// the blocks without a row: 70 rows of 512 12.1 -> 6.8 us.
+// derivative shared a sigmoid.)  Batches of up to two blocks an SM (one row a sum)
+// take CTAs of eight warps and leave out the blocks without a row: 70 rows of 512 12.1 -> 6.8 us.
 // Vector path only (aligned pointers and strides, D a multiple of the vector width, 16-bit elements).
 // Shared memory: [NW][STAGES][5][MAXV][32] vectors: attn, u, dout's y, u and x part; with two halves
 // [2][NW][D] floats, the first halves' sums.

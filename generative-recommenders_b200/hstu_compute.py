@@ -10,7 +10,7 @@ from . import _cabi
 from .common import (HammerKernel, _require_cuda_backend, as_dtype, dtype_code, on_device, outside_autograd,
                      require_cuda, stream_ptr)
 from . import hstu_attention as _attention
-from .hstu_attention import _i32, _index, _require_target_counts, hstu_mha
+from .hstu_attention import _i32, _index, hstu_mha
 from .layer_norm import layer_norm
 from .mm import addmm
 
@@ -135,6 +135,8 @@ def _fused_uqvk_launch(x, nw, nb, eps, w, b, hv, inference=False):
     and mean and rstd are None."""
     M, D = x.shape
     N = w.shape[1]
+    if w.shape[0] != D or nw.numel() < D or nb.numel() < D or b.numel() < N:   # (the kernel reads them by the width of x)
+        raise RuntimeError("uvqk stage: parameters of another width than x")
     uvqk = torch.empty((M, N), dtype=x.dtype, device=x.device)
     u = torch.empty((M, hv), dtype=x.dtype, device=x.device)
     mean = torch.empty(M, dtype=torch.float32, device=x.device) if not inference else None
@@ -172,10 +174,6 @@ def _fused_uqvk_backward(x, nw, nb, w, uvqk, mean, rstd, eps, hv, du, d_uvqk):
 
 def _stage_parameters(x, norm_weight, norm_bias, weight, bias):
     """The parameters as the fused kernel reads them (a parameter that is so already: itself)."""
-    D, N = weight.shape
-    if x.shape[1] != D or norm_weight.numel() < D or norm_bias.numel() < D or bias.numel() < N:
-        raise RuntimeError("the uvqk stage on rows of %d needs norm parameters of that many entries, a weight of "
-                           "that many rows and a bias of its columns" % x.shape[1])
     return (as_dtype(norm_weight, x.dtype).contiguous(), as_dtype(norm_bias, x.dtype).contiguous(),
             _aligned16(as_dtype(weight, x.dtype).contiguous()), as_dtype(bias, x.dtype).contiguous())
 
@@ -293,15 +291,11 @@ def hstu_cached_attention(x, norm_weight, norm_bias, norm_eps, num_heads, attn_d
     ops have to do it."""
     hv, ha, M = hidden_dim * num_heads, attn_dim * num_heads, x.shape[0]
     B = cache_offsets.numel() - 1
-    if not (_FUSED_UQVK and x.is_cuda and _fused_uqvk_supported(x, uvqk_weight, hv) and B > 0 and M % B == 0
-            and cache_offsets.dtype is torch.int64 and cache_offsets.is_contiguous()
+    if not (_FUSED_UQVK and x.is_cuda and B > 0 and M % B == 0
+            and _cabi.host().cached_supported(x, uvqk_weight, hv, ha, k_cache, v_cache, cache_offsets)
             and outside_autograd(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias, k_cache, v_cache)):
         return None
-    for t, width in ((k_cache, ha), (v_cache, hv)):
-        if t.dim() != 2 or t.shape != (k_cache.shape[0], width) or t.dtype is not x.dtype or not t.is_contiguous():
-            return None
     require_cuda(norm_weight, norm_bias, uvqk_weight, uvqk_bias, k_cache, v_cache, cache_offsets, num_targets)
-    _require_target_counts(num_targets, B)
     nw, nb, w, b = _stage_parameters(x, norm_weight, norm_bias, uvqk_weight, uvqk_bias)
     nbytes = _cabi.lib().b200_hstu_ln_linear_workspace_bytes(*w.shape)
     ws, prepared, remember = _prepared_workspace(nw, nb, w, b, nbytes, x.device, True)

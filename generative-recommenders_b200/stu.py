@@ -192,7 +192,7 @@ class STULayer(torch.nn.Module):
         num_targets_ = num_targets if self._target_aware else None
         fused = None
         if (self.k_cache is not None and self.v_cache is not None and self.kv_caching_offsets is not None
-                and _is_own(self, "construct_full_kv")
+                and "construct_full_kv" not in self.__dict__ and type(self).construct_full_kv is _OWN_FULL_KV
                 and delta_x.dim() == 2 and delta_x.shape[0] > 0):
             delta_size = delta_x.shape[0] // (self.kv_caching_offsets.numel() - 1)
             max_seq_len = self.max_kv_caching_len + delta_size
@@ -335,22 +335,26 @@ class STULayer(torch.nn.Module):
             )
 
 
-# What the shortcuts below stand in for.  Whoever replaces one of these, on the class as on a layer, wants the
-# replacement called for every layer.
-_OWN = {name: getattr(STULayer, name) for name in ("__call__", "_call_impl", "forward", "cached_forward", "construct_full_kv")}
+# What the shortcuts of this file stand in for.  Whoever replaces one of these, on the class as on a layer, wants
+# the replacement called for every layer.
+_OWN_FORWARD, _OWN_CACHED_FORWARD, _OWN_FULL_KV = STULayer.forward, STULayer.cached_forward, STULayer.construct_full_kv
+_OWN_CALL, _OWN_CALL_IMPL = STULayer.__call__, STULayer._call_impl
 
 
-def _is_own(layer, method) -> bool:
-    return type(layer) is STULayer and method not in layer.__dict__ and getattr(STULayer, method) is _OWN[method]
+def _nobody_looks_on() -> bool:
+    """True where a stack's layers may hand tensors on by themselves and over one another: there are no gradients, and
+    no tracer, dispatch mode, hook of all modules or replaced method gets to see them."""
+    return (not torch.is_grad_enabled() and not is_compiling() and not _module._has_any_global_hook()
+            and STULayer.forward is _OWN_FORWARD and STULayer.cached_forward is _OWN_CACHED_FORWARD
+            and STULayer.__call__ is _OWN_CALL and STULayer._call_impl is _OWN_CALL_IMPL
+            and torch._C._len_torch_dispatch_stack() == 0)
 
 
 def _unobserved(layer, method) -> bool:
-    """True without gradients where ``layer.method`` is this file's and no hook, tracer or dispatch mode gets to
-    see what goes in or comes out."""
-    return (not torch.is_grad_enabled() and not is_compiling() and _is_own(layer, method) and _is_own(layer, "__call__")
-            and _is_own(layer, "_call_impl") and not layer._forward_hooks and not layer._forward_pre_hooks
-            and not layer._backward_hooks and not layer._backward_pre_hooks and layer._compiled_call_impl is None
-            and not _module._has_any_global_hook() and torch._C._len_torch_dispatch_stack() == 0)
+    """True where ``layer.method`` is the class's and no hook of the layer gets to see what goes in or comes out."""
+    return (type(layer) is STULayer and method not in layer.__dict__ and not layer._forward_hooks
+            and not layer._forward_pre_hooks and not layer._backward_hooks and not layer._backward_pre_hooks
+            and layer._compiled_call_impl is None)
 
 
 class STUStack(torch.nn.Module):
@@ -369,16 +373,16 @@ class STUStack(torch.nn.Module):
         max_kv_caching_len: int = 0,
         kv_caching_lengths: Optional[torch.Tensor] = None,
     ) -> torch.Tensor:
-        previous = None
+        alone, own = _nobody_looks_on(), False
         for layer in self._stu_layers:
             # what one layer hands to the next is the stack's own: it may be overwritten, unless someone looks on
-            if previous is not None and _unobserved(previous, "forward") and _unobserved(layer, "forward"):
+            handed_on, own = own, alone and _unobserved(layer, "forward")
+            if handed_on and own:
                 x = layer._forward(x, x_offsets, max_seq_len, num_targets, max_kv_caching_len, kv_caching_lengths, True)
             else:
                 x = layer(x=x, x_lengths=x_lengths, x_offsets=x_offsets, max_seq_len=max_seq_len,
                           num_targets=num_targets, max_kv_caching_len=max_kv_caching_len,
                           kv_caching_lengths=kv_caching_lengths)
-            previous = layer
         return x
 
     def cached_forward(
@@ -388,14 +392,13 @@ class STUStack(torch.nn.Module):
         max_kv_caching_len: int = 0,
         kv_caching_lengths: Optional[torch.Tensor] = None,
     ) -> torch.Tensor:
-        previous = None
+        alone, own = _nobody_looks_on(), False
         for layer in self._stu_layers:
-            if (previous is not None and _unobserved(previous, "cached_forward")
-                    and _unobserved(layer, "cached_forward")):
+            handed_on, own = own, alone and _unobserved(layer, "cached_forward")
+            if handed_on and own:
                 delta_x = layer._cached_forward(delta_x, num_targets, max_kv_caching_len, kv_caching_lengths, True)
             else:
                 delta_x = layer.cached_forward(delta_x=delta_x, num_targets=num_targets,
                                                max_kv_caching_len=max_kv_caching_len,
                                                kv_caching_lengths=kv_caching_lengths)
-            previous = layer
         return delta_x

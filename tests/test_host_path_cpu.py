@@ -310,41 +310,43 @@ def test_layers_are_called_as_modules_where_someone_looks_on():
     stu = importlib.import_module("generative-recommenders_b200.stu")
     layer = G.STULayer(G.STULayerConfig(embedding_dim=16, num_heads=1, hidden_dim=16, attention_dim=16))
     with torch.no_grad():
-        assert stu._unobserved(layer, "forward") and stu._unobserved(layer, "cached_forward")
+        assert stu._nobody_looks_on() and stu._unobserved(layer, "forward") and stu._unobserved(layer, "cached_forward")
         with _Sees():
-            assert not stu._unobserved(layer, "forward")
-    assert not stu._unobserved(layer, "forward")     # (gradients: nothing may be overwritten)
+            assert not stu._nobody_looks_on()
+    assert not stu._nobody_looks_on()     # (gradients: nothing may be overwritten)
+    layer.register_forward_hook(lambda *a: None)
+    assert not stu._unobserved(layer, "forward")
 
 
-def _cached_call(monkeypatch, host, targets, k_rows=5, v_rows=5):
-    """``hstu_cached_attention`` of two sequences with one new row each; ``host`` answers the native call."""
+def _cached_call(monkeypatch, host, targets):
+    """``hstu_cached_attention`` of two sequences with one new row each; ``host`` answers the native calls."""
     D = 16
     on = lambda *s, dtype=torch.bfloat16: torch.zeros(s, dtype=dtype).as_subclass(_OnDevice)  # noqa: E731
-    monkeypatch.setattr(HC, "_fused_uqvk_supported", lambda *a: True)
-    monkeypatch.setattr(HC, "_prepared_workspace", lambda *a: (None, False, None))
+    monkeypatch.setattr(HC, "_prepared_workspace", lambda *a: (torch.zeros(4096, dtype=torch.uint8), False, None))
     monkeypatch.setattr(HC._cabi, "lib", lambda: _Library())
     monkeypatch.setattr(HC._cabi, "host", lambda: host)
     offsets = torch.tensor([0, 2, 5]).as_subclass(_OnDevice)
     targets = None if targets is None else torch.ones(targets, dtype=torch.int64).as_subclass(_OnDevice)
     with torch.no_grad():
-        return HC.hstu_cached_attention(on(2, D), on(D), on(D), 1e-6, 1, D, D, on(D, 4 * D), on(4 * D), on(k_rows, D),
-                                        on(v_rows, D), offsets, targets, 4, 0.1, 0, 0)
+        return HC.hstu_cached_attention(on(2, D), on(D), on(D), 1e-6, 1, D, D, on(D, 4 * D), on(4 * D), on(5, D), on(5, D),
+                                        offsets, targets, 4, 0.1, 0, 0)
 
 
-class _Taken:
+class _Native:
+    """The native calls, the choice of path answered by yes."""
+
+    def __init__(self):
+        self.native = G._cabi.host()
+
     def cached_attention(self, *args):
-        return "taken"
+        return self.native.cached_attention(*args)
 
-
-@pytest.mark.parametrize("targets", [None, 2, 3])
-def test_cached_attention_takes_a_target_count_for_every_sequence(monkeypatch, targets):
-    assert _cached_call(monkeypatch, _Taken(), targets) == "taken"
+    def cached_supported(self, *args):
+        return True
 
 
 def test_attention_of_new_rows_refuses_missing_target_counts(monkeypatch):
     """The kernels read ``num_targets[b]`` of every sequence."""
-    with pytest.raises(RuntimeError, match="one entry per sequence"):
-        _cached_call(monkeypatch, _Taken(), 1)
     rows = torch.zeros(2, 1, 16).as_subclass(_OnDevice)
     offsets, targets = (torch.tensor(t).as_subclass(_OnDevice) for t in ([0, 1, 2], [1]))
     with pytest.raises(RuntimeError, match="one entry per sequence"):
@@ -352,17 +354,35 @@ def test_attention_of_new_rows_refuses_missing_target_counts(monkeypatch):
     q8 = rows.to(torch.float8_e4m3fn).as_subclass(_OnDevice)
     with pytest.raises(RuntimeError, match="one entry per sequence"):
         G.hstu_mha_fp8(2, 0.1, q8, q8, q8, rows, rows, rows, offsets, offsets, targets)
+    with pytest.raises(RuntimeError, match="one entry per sequence"):
+        _cached_call(monkeypatch, _Native(), 1)
 
 
 @pytest.mark.parametrize("k_rows, v_rows", [(5, 5), (5, 4), (5, 6)])
-def test_cached_attention_reads_k_and_v_of_as_many_rows(monkeypatch, k_rows, v_rows):
+def test_cached_attention_reads_k_and_v_of_as_many_rows(k_rows, v_rows):
     """One launch appends to both and takes one row count; other caches go to the separate ops, and a V of fewer
     rows than K is refused where both are read together."""
-    assert _cached_call(monkeypatch, _Taken(), None, k_rows, v_rows) == ("taken" if k_rows == v_rows else None)
+    t = lambda *s: torch.zeros(s, dtype=torch.bfloat16)  # noqa: E731
+    offsets = torch.tensor([0, 2, 5])
+    assert G._cabi.host().cached_supported(t(2, 64), t(64, 256), 64, 64, t(k_rows, 64), t(v_rows, 64), offsets) == (
+        k_rows == v_rows)
     if v_rows < k_rows:
         rows = torch.zeros(k_rows, 1, 16).as_subclass(_OnDevice)
         with pytest.raises(AssertionError, match="wrong v shape"):
             G.delta_hstu_mha(k_rows, 0.1, rows[:1], rows, rows[:v_rows], torch.tensor([0, k_rows]).as_subclass(_OnDevice))
+
+
+def test_cached_attention_in_one_call_takes_what_it_can_read():
+    """16-bit rows, contiguous caches of the same type and of the heads' widths, int64 offsets."""
+    t = lambda *s, dtype=torch.bfloat16: torch.zeros(s, dtype=dtype)  # noqa: E731
+    good = {"x": t(2, 64), "w": t(64, 256), "hv": 64, "ha": 64, "k": t(5, 64), "v": t(5, 64), "offsets": torch.tensor([0, 2, 5])}
+    supported = lambda **kw: G._cabi.host().cached_supported(*dict(good, **kw).values())  # noqa: E731
+    assert supported()
+    for name, other in (("x", t(2, 64, dtype=torch.float32)), ("x", t(0, 64)), ("x", t(2, 128)[:, ::2]), ("x", t(2, 1, 64)),
+                        ("k", t(5, 64, dtype=torch.float16)), ("v", t(5, 64, dtype=torch.float32)), ("k", t(5, 63)),
+                        ("v", t(5, 128)[:, :64]), ("v", t(5, 1, 64)), ("k", t(5)),
+                        ("offsets", torch.tensor([0, 2, 5], dtype=torch.int32)), ("offsets", torch.arange(6)[::2])):
+        assert not supported(**{name: other}), name
 
 
 @pytest.mark.parametrize("on", [False, True])
@@ -370,7 +390,7 @@ def test_status_check_reaches_cached_attention(monkeypatch, on):
     """Checked or not, the same path runs."""
     asked = []
 
-    class _Host:
+    class _Host(_Native):
         def cached_attention(self, *args):
             asked.append(args[-1])
             return "taken"
@@ -407,14 +427,13 @@ def test_host_module_is_built_anew_for_another_torch(tmp_path, monkeypatch):
     assert len(runs) == 2
 
 
-@pytest.mark.parametrize("width, norm, rows, bias", [(16, 16, 16, 64), (24, 16, 16, 64), (8, 16, 16, 64), (16, 8, 16, 64),
-                                                     (16, 16, 16, 63)])
+@pytest.mark.parametrize("width, norm, rows, bias", [(24, 16, 16, 64), (8, 16, 16, 64), (16, 8, 16, 64), (16, 16, 16, 63)])
 def test_fused_uvqk_stage_refuses_parameters_of_another_width(width, norm, rows, bias):
     """The kernel reads them, and sizes its workspace, by the width of x."""
     t = lambda *s: torch.zeros(s, dtype=torch.bfloat16)  # noqa: E731
-    call = lambda: HC._stage_parameters(t(3, width), t(norm), t(norm), t(rows, 64), t(bias))  # noqa: E731
-    if (width, norm, rows, bias) == (16, 16, 16, 64):
-        assert len(call()) == 4
-    else:
-        with pytest.raises(RuntimeError, match="uvqk stage"):
-            call()
+    x, nw, w, b, ws = t(2, width), t(norm), t(rows, 64), t(bias), torch.zeros(4096, dtype=torch.uint8)
+    with pytest.raises(RuntimeError, match="another width"):
+        HC._fused_uqvk_launch(x, nw, nw, 1e-6, w, b, 16, True)
+    with pytest.raises(RuntimeError, match="another width"):
+        G._cabi.host().cached_attention(x, nw, nw, w, b, 1e-6, 1, 16, 16, ws, False, t(5, 16), t(5, 16),
+                                        torch.tensor([0, 2, 5]), None, 4, 0.1, 0, 0, 0, G._cabi.BF16, False)
