@@ -341,7 +341,7 @@ void b200_hstu_host_kv_range(int32_t len, int32_t num_targets, int32_t max_seq_l
 /* Host utility: the query tiles (128 rows each) that the backward's K/V-stationary kernel visits
    for kv tile `kt`: tiles [t_lo, t_lo + n_main) plus `extra_tile` when it is >= 0 (with a window and a
    full-attention tail the kernel leaves out some of that range: b200_hstu_host_bwd_q_visits). */
-static TileItem host_kv_item(int32_t len, int32_t num_targets, int32_t max_seq_len, int32_t contextual_seq_len,
+static KvTileItem host_kv_item(int32_t len, int32_t num_targets, int32_t max_seq_len, int32_t contextual_seq_len,
                              int32_t max_attn_len, int32_t min_full_attn_seq_len, int32_t kt) {
   AttnGeomParams g;
   g.seq_offsets = {nullptr, 1};
@@ -353,15 +353,15 @@ static TileItem host_kv_item(int32_t len, int32_t num_targets, int32_t max_seq_l
   g.c = contextual_seq_len;
   g.F = min_full_attn_seq_len;
   g.delta = 0;
-  TileItem it;
-  fill_kv_item(it, g, 0, kt, 0, len, num_targets);
+  KvTileItem it;
+  fill_kv_item<true>(it, g, 0, kt, 0, len, num_targets);
   return it;
 }
 
 void b200_hstu_host_bwd_q_tiles(int32_t len, int32_t num_targets, int32_t max_seq_len, int32_t contextual_seq_len,
                                 int32_t max_attn_len, int32_t min_full_attn_seq_len, int32_t kt, int32_t *t_lo,
                                 int32_t *n_main, int32_t *extra_tile) {
-  const TileItem it = host_kv_item(len, num_targets, max_seq_len, contextual_seq_len, max_attn_len,
+  const KvTileItem it = host_kv_item(len, num_targets, max_seq_len, contextual_seq_len, max_attn_len,
                                    min_full_attn_seq_len, kt);
   *t_lo = it.t_lo;
   *n_main = it.n_main + it.gap;
@@ -372,7 +372,7 @@ void b200_hstu_host_bwd_q_tiles(int32_t len, int32_t num_targets, int32_t max_se
    domain; tile 0 may come once more for the contextual rows). */
 int b200_hstu_host_bwd_q_visits(int32_t len, int32_t num_targets, int32_t max_seq_len, int32_t contextual_seq_len,
                                 int32_t max_attn_len, int32_t min_full_attn_seq_len, int32_t kt, int32_t qt) {
-  const TileItem it = host_kv_item(len, num_targets, max_seq_len, contextual_seq_len, max_attn_len,
+  const KvTileItem it = host_kv_item(len, num_targets, max_seq_len, contextual_seq_len, max_attn_len,
                                    min_full_attn_seq_len, kt);
   int n = 0;
   for (int j = 0; j < it.n_tiles; ++j) n += it.tile_at(j) == qt;

@@ -406,11 +406,16 @@ __device__ __forceinline__ void zero_rows_beyond(uint16_t *base, int64_t rs, int
   }
 }
 
-template <bool DKDV>
-__device__ __forceinline__ void fill_bwd_item(TileItem &it, const AttnGeomParams &g, const ItemDesc &d) {
-  if (DKDV) fill_kv_item(it, g, d.b, d.t, d.start, d.len, d.nt);
-  else fill_q_item(it, g, d.b, d.t, d.start, d.len, d.nt);
+template <bool TAIL>
+__device__ __forceinline__ void fill_bwd_item(KvTileItem &it, const AttnGeomParams &g, const ItemDesc &d) {
+  fill_kv_item<TAIL>(it, g, d.b, d.t, d.start, d.len, d.nt);
 }
+template <bool TAIL>
+__device__ __forceinline__ void fill_bwd_item(TileItem &it, const AttnGeomParams &g, const ItemDesc &d) {
+  fill_q_item<TAIL>(it, g, d.b, d.t, d.start, d.len, d.nt);
+}
+template <bool DKDV>
+using BwdItem = std::conditional_t<DKDV, KvTileItem, TileItem>;
 
 // ---------------------------------------------------------------------------------------
 // Work items travel from the producer warp to the other warps as ready-made geometry (64 bytes
@@ -426,10 +431,10 @@ struct __align__(16) ItemGeom {
   int max_id;
   uint32_t gap;              // of the main range: where it is (upper 16 bits) and how many tiles it leaves out
   int pad[2];
-  // Only items of the kv-stationary launch have a gap, and their extra tile is tile 0.
-  template <bool DKDV>
+  // Only items of the kv-stationary launch with window and tail have a gap, and their extra tile is tile 0.
+  template <bool GAP>
   __device__ __forceinline__ int tile_at(int j, uint32_t gap_) const {
-    if (DKDV) return j < n_main ? t_lo + j + (j >= (int)(gap_ >> 16) ? (int)(gap_ & 0xffffu) : 0) : 0;
+    if (GAP) return j < n_main ? t_lo + j + (j >= (int)(gap_ >> 16) ? (int)(gap_ & 0xffffu) : 0) : 0;
     return j < n_main ? t_lo + j : extra_tile;
   }
 };
@@ -442,7 +447,11 @@ __device__ __forceinline__ void geom_from_item(ItemGeom &g, const TileItem &it, 
   g.start = it.start; g.len = it.len; g.nt = it.nt;
   g.m0 = it.m0; g.n_tiles = it.n_tiles; g.t_lo = it.t_lo; g.n_main = it.n_main;
   g.extra_tile = it.extra_tile; g.L = it.m.L; g.u = it.u; g.regular = it.regular ? 1 : 0;
-  g.max_id = it.m.max_id; g.gap = (uint32_t)it.gap_at << 16 | (uint32_t)it.gap; g.pad[0] = g.pad[1] = 0;
+  g.max_id = it.m.max_id; g.gap = 0; g.pad[0] = g.pad[1] = 0;
+}
+__device__ __forceinline__ void geom_from_item(ItemGeom &g, const KvTileItem &it, int idx) {
+  geom_from_item(g, static_cast<const TileItem &>(it), idx);
+  g.gap = (uint32_t)it.gap_at << 16 | (uint32_t)it.gap;
 }
 // the fields the activation and epilogue code reads (no tile ranges are recomputed)
 __device__ __forceinline__ void item_from_geom(TileItem &it, const ItemGeom &g, const AttnGeomParams &gp) {
@@ -522,12 +531,13 @@ __device__ __forceinline__ void bwd_stage2(uint32_t acc_tmem, uint32_t a_tmem, u
   __syncwarp();
 }
 
-template <int D, bool IS_BF16, bool DKDV, bool BIAS>
+template <int D, bool IS_BF16, bool DKDV, bool BIAS, bool TAIL>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
     hstu_attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                                const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
                                const BwdParams p) {
   using SM = BwdSmem<D>;
+  constexpr bool GAP = DKDV && TAIL;   // items whose tiles have a gap
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -613,8 +623,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
       tr.init(p.trace, 0, true);
       ItemGeom g;
       {
-        TileItem it;
-        fill_bwd_item<DKDV>(it, p.g, load_desc(p.items, blockIdx.x / p.H));
+        BwdItem<DKDV> it;
+        fill_bwd_item<TAIL>(it, p.g, load_desc(p.items, blockIdx.x / p.H));
         geom_from_item(g, it, blockIdx.x);
       }
       ok = geom_publish(wc, sched_ring, sched_full, sched_empty, 0, g);
@@ -633,7 +643,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
         // order of requests = order of first use: X0, Y0(0) feed G1; X1, Y1(0) feed G2
         for (int j = 0; j < g.n_tiles; ++j, ++cnt) {
           const int s0 = cnt % Y0_STAGES, s1 = cnt % Y1_STAGES;
-          const int row = g.start + g.template tile_at<DKDV>(j, g.gap) * TILE;
+          const int row = g.start + g.template tile_at<GAP>(j, g.gap) * TILE;
           if (j == 0) {
             ok = mbar_wait(wc, x_empty, (it_cnt & 1) ^ 1, 401);
             if (!ok) break;
@@ -670,8 +680,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
           if (j == j_geom) {
             ng.idx = nidx;
             if (nidx < num_items) {
-              TileItem ni;
-              fill_bwd_item<DKDV>(ni, p.g, nd);
+              BwdItem<DKDV> ni;
+              fill_bwd_item<TAIL>(ni, p.g, nd);
               geom_from_item(ng, ni, nidx);
             }
             ok = geom_publish(wc, sched_ring, sched_full, sched_empty, it_cnt + 1, ng);
@@ -834,8 +844,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
     tr.init(p.trace, 2, warp == 2 && lane == 0);
     if ((int)blockIdx.x < num_items) {
       ItemGeom g;
-      // (these warps hand an item's slot back when they are through with the item)
-      ok = geom_fetch(wc, sched_ring, sched_full, sched_empty, 0, g, false);
+      // (with a gap to read these warps hand an item's slot back when they are through with the item)
+      ok = geom_fetch(wc, sched_ring, sched_full, sched_empty, 0, g, !GAP && lane == 0);
       while (ok && g.idx < num_items) {
         TileItem it;
         item_from_geom(it, g, p.g);
@@ -853,9 +863,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
           if (DKDV) ci = col_interval(it, own_j); else ri = row_interval(it, own_j);
           // (the gap is read from the item's slot each time: this loop has no register to keep it in)
           const uint32_t gap =
-              DKDV ? reinterpret_cast<const volatile ItemGeom *>(sched_ring + (item_no % GEOM_SLOTS) * GEOM_SLOT_BYTES)->gap
+              GAP ? reinterpret_cast<const volatile ItemGeom *>(sched_ring + (item_no % GEOM_SLOTS) * GEOM_SLOT_BYTES)->gap
                    : 0u;
-          const int o0 = g.template tile_at<DKDV>(j, gap) * TILE;  // first position of the streamed tile
+          const int o0 = g.template tile_at<GAP>(j, gap) * TILE;  // first position of the streamed tile
           const int c0 = o0 + wg * 64;  // first streamed position of this thread's 64 columns
           ActTile at;
           at.tS = tS;
@@ -894,9 +904,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
           }
         }
         if (!ok) break;
-        if (lane == 0) mbar_arrive(sched_empty + 8 * (item_no % GEOM_SLOTS));
+        if (GAP && lane == 0) mbar_arrive(sched_empty + 8 * (item_no % GEOM_SLOTS));
         ++item_no;
-        ok = geom_fetch(wc, sched_ring, sched_full, sched_empty, item_no, g, false);
+        ok = geom_fetch(wc, sched_ring, sched_full, sched_empty, item_no, g, !GAP && lane == 0);
       }
     }
   } else {
@@ -1044,6 +1054,7 @@ int launch_bwd_tc(const b200_hstu_attn_args &a, cudaStream_t st) {
   ulonglong2 *trace_buf = nullptr;
   if (want_trace != nullptr && a.plan_mode != B200_HSTU_PLAN_REUSE && a.workspace_bytes >= eb + 2 * one + TRACE_BYTES)
     trace_buf = reinterpret_cast<ulonglong2 *>(reinterpret_cast<uint8_t *>(a.workspace) + eb + 2 * one);
+  const bool tail = leaves_tiles_out(p.g);
   const int64_t upper = (int64_t)max_items * a.H;
   const int grid = (int)(upper < device_sm_count() ? upper : device_sm_count());
   // own scratch: [bias table | kv list | q list]; planned by the forward: [bias table | forward
@@ -1058,7 +1069,9 @@ int launch_bwd_tc(const b200_hstu_attn_args &a, cudaStream_t st) {
   if (!reuse) {
     {
       ProfileScope prof(PROF_PLAN, st);
-      attn_plan2_kernel<PLAN_KV_TILE, PLAN_Q_TILE><<<2, PLAN_THREADS, 0, st>>>(
+      const auto plan = tail ? attn_plan2_kernel<PLAN_KV_TILE, PLAN_Q_TILE, true>
+                             : attn_plan2_kernel<PLAN_KV_TILE, PLAN_Q_TILE, false>;
+      plan<<<2, PLAN_THREADS, 0, st>>>(
           p.g, hdr_kv, reinterpret_cast<ItemDesc *>(hdr_kv + 1), hdr_q, reinterpret_cast<ItemDesc *>(hdr_q + 1),
           max_items, grid, bt);
     }
@@ -1066,7 +1079,8 @@ int launch_bwd_tc(const b200_hstu_attn_args &a, cudaStream_t st) {
     B200_CHECK_LAUNCH("attention plan (backward)");
   }
   {
-    auto kern = hstu_attn_bwd_sm100_kernel<D, IS_BF16, true, BIAS>;
+    auto kern = tail ? hstu_attn_bwd_sm100_kernel<D, IS_BF16, true, BIAS, true>
+                     : hstu_attn_bwd_sm100_kernel<D, IS_BF16, true, BIAS, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::DYN_BYTES);
     if (e != cudaSuccess) return check_cuda(e, "backward smem attribute");
     BwdParams pk = p;
@@ -1084,7 +1098,8 @@ int launch_bwd_tc(const b200_hstu_attn_args &a, cudaStream_t st) {
     B200_CHECK_LAUNCH("tcgen05 attention backward (dk, dv)");
   }
   {
-    auto kern = hstu_attn_bwd_sm100_kernel<D, IS_BF16, false, BIAS>;
+    auto kern = tail ? hstu_attn_bwd_sm100_kernel<D, IS_BF16, false, BIAS, true>
+                     : hstu_attn_bwd_sm100_kernel<D, IS_BF16, false, BIAS, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::DYN_BYTES);
     if (e != cudaSuccess) return check_cuda(e, "backward smem attribute");
     BwdParams pq = p;

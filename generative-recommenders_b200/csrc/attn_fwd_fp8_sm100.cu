@@ -193,6 +193,7 @@ struct __align__(16) PairGeom {
 };
 constexpr int GEOM_INTS = 29;
 
+template <bool TAIL>
 __device__ __forceinline__ void geom_from_pair(PairGeom &g, const PairItem &pr, int idx, int delta) {
   g.idx = idx;
   g.start = pr.A.start; g.len = pr.A.len; g.nt = pr.A.nt;
@@ -201,7 +202,7 @@ __device__ __forceinline__ void geom_from_pair(PairGeom &g, const PairItem &pr, 
   g.n_main = pr.n_main; g.extra0 = pr.extra0; g.extra1 = pr.extra1;
   g.a_lo = pr.A.t_lo; g.a_hi = pr.A.t_lo + pr.A.n_main; g.a_x = pr.A.extra_tile; g.a_n = pr.A.n_tiles;
   g.b_lo = pr.B.t_lo; g.b_hi = pr.B.t_lo + pr.B.n_main; g.b_x = pr.B.extra_tile; g.b_n = pr.B.n_tiles;
-  const FullRange fa = full_tile_range(pr.A), fb = full_tile_range(pr.B);
+  const FullRange fa = full_tile_range<TAIL>(pr.A), fb = full_tile_range<TAIL>(pr.B);
   g.fa_lo = fa.lo; g.fa_hi = fa.hi; g.fb_lo = fb.lo; g.fb_hi = fb.hi;
   // cached inference: q / out hold `delta` rows per sequence; otherwise they are jagged like k / v
   g.q_row = delta > 0 ? pr.A.b * delta + pr.A.mt * TILE : pr.A.start + pr.A.m0;
@@ -233,7 +234,7 @@ __device__ __forceinline__ bool geom_fetch(const WaitCtx &wc, const uint8_t *rin
   return true;
 }
 
-template <int D>
+template <int D, bool TAIL>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
     hstu_attn_fwd_fp8_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                                    const __grid_constant__ CUtensorMap tmap_v, const Fp8Params p) {
@@ -313,8 +314,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
       {
         const ItemDesc d = load_desc(p.items, blockIdx.x / p.H);
         PairItem pr;
-        fill_pair_item(pr, p.g, d.b, d.t, d.start, d.len, d.nt);
-        geom_from_pair(g, pr, blockIdx.x, p.g.delta);
+        fill_pair_item<TAIL>(pr, p.g, d.b, d.t, d.start, d.len, d.nt);
+        geom_from_pair<TAIL>(g, pr, blockIdx.x, p.g.delta);
       }
       ok = geom_publish(wc, sched_ring, sched_full, sched_empty, 0, g);
       while (g.idx < num_items && ok) {
@@ -374,8 +375,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
             ng.idx = nidx;
             if (nidx < num_items) {
               PairItem np;
-              fill_pair_item(np, p.g, nd.b, nd.t, nd.start, nd.len, nd.nt);
-              geom_from_pair(ng, np, nidx, p.g.delta);
+              fill_pair_item<TAIL>(np, p.g, nd.b, nd.t, nd.start, nd.len, nd.nt);
+              geom_from_pair<TAIL>(ng, np, nidx, p.g.delta);
             }
             ok = geom_publish(wc, sched_ring, sched_full, sched_empty, it_cnt + 1, ng);
             if (!ok) break;
@@ -847,15 +848,17 @@ int attn_tc_fwd_fp8(const b200_hstu_attn_fp8_args &fa, cudaStream_t st) {
   p.bias_ext = nullptr;
   p.wide_stores = (reinterpret_cast<uintptr_t>(a.out) & 31) == 0 && a.o_row_stride % 16 == 0 && a.o_head_stride % 16 == 0;
   const int max_items = (int)plan_max_items(a.total_L, a.B);
+  const bool tail = leaves_tiles_out(p.g);
   const int64_t upper = (int64_t)max_items * a.H;
   const int grid = (int)(upper < device_sm_count() ? upper : device_sm_count());
   {
     ProfileScope prof(PROF_PLAN, st);
-    attn_plan_kernel<PLAN_Q_PAIR><<<1, PLAN_THREADS, 0, st>>>(p.g, hdr, items, max_items, grid, BiasTable{nullptr, 0, nullptr, 0});
+    const auto plan = tail ? attn_plan_kernel<PLAN_Q_PAIR, true> : attn_plan_kernel<PLAN_Q_PAIR, false>;
+    plan<<<1, PLAN_THREADS, 0, st>>>(p.g, hdr, items, max_items, grid, BiasTable{nullptr, 0, nullptr, 0});
   }
   count_launch();
   B200_CHECK_LAUNCH("attention plan");
-  auto kern = hstu_attn_fwd_fp8_sm100_kernel<D>;
+  auto kern = tail ? hstu_attn_fwd_fp8_sm100_kernel<D, true> : hstu_attn_fwd_fp8_sm100_kernel<D, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::DYN_BYTES);
   if (e != cudaSuccess) return check_cuda(e, "fp8 forward smem attribute");
   {

@@ -199,6 +199,7 @@ struct __align__(16) PairGeom {
 };
 constexpr int GEOM_INTS = 28;
 
+template <bool TAIL>
 __device__ __forceinline__ void geom_from_pair(PairGeom &g, const PairItem &pr, int idx, int delta) {
   g.idx = idx;
   g.start = pr.A.start; g.len = pr.A.len; g.nt = pr.A.nt;
@@ -207,7 +208,7 @@ __device__ __forceinline__ void geom_from_pair(PairGeom &g, const PairItem &pr, 
   g.n_main = pr.n_main; g.extra0 = pr.extra0; g.extra1 = pr.extra1;
   g.a_lo = pr.A.t_lo; g.a_hi = pr.A.t_lo + pr.A.n_main; g.a_x = pr.A.extra_tile; g.a_n = pr.A.n_tiles;
   g.b_lo = pr.B.t_lo; g.b_hi = pr.B.t_lo + pr.B.n_main; g.b_x = pr.B.extra_tile; g.b_n = pr.B.n_tiles;
-  const FullRange fa = full_tile_range(pr.A), fb = full_tile_range(pr.B);
+  const FullRange fa = full_tile_range<TAIL>(pr.A), fb = full_tile_range<TAIL>(pr.B);
   g.fa_lo = fa.lo; g.fa_hi = fa.hi; g.fb_lo = fb.lo; g.fb_hi = fb.hi;
   // cached inference: q / out hold `delta` rows per sequence; otherwise they are jagged like k / v
   g.q_row = delta > 0 ? pr.A.b * delta + pr.A.mt * TILE : pr.A.start + pr.A.m0;
@@ -278,7 +279,7 @@ __device__ __noinline__ void masked_tile(uint32_t tS, int wg, float half_alpha, 
   tmem_st16(tS + wg * 64 + 16, p1);
 }
 
-template <int D, bool IS_BF16, bool ONE_PATH, bool BIAS>
+template <int D, bool IS_BF16, bool ONE_PATH, bool BIAS, bool TAIL>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
     hstu_attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                                const __grid_constant__ CUtensorMap tmap_v, const FwdParams p) {
@@ -358,8 +359,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
       {
         const ItemDesc d = load_desc(p.items, blockIdx.x / p.H);
         PairItem pr;
-        fill_pair_item(pr, p.g, d.b, d.t, d.start, d.len, d.nt);
-        geom_from_pair(g, pr, blockIdx.x, p.g.delta);
+        fill_pair_item<TAIL>(pr, p.g, d.b, d.t, d.start, d.len, d.nt);
+        geom_from_pair<TAIL>(g, pr, blockIdx.x, p.g.delta);
       }
       ok = geom_publish(wc, sched_ring, sched_full, sched_empty, 0, g);
       while (g.idx < num_items && ok) {
@@ -419,8 +420,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
             ng.idx = nidx;
             if (nidx < num_items) {
               PairItem np;
-              fill_pair_item(np, p.g, nd.b, nd.t, nd.start, nd.len, nd.nt);
-              geom_from_pair(ng, np, nidx, p.g.delta);
+              fill_pair_item<TAIL>(np, p.g, nd.b, nd.t, nd.start, nd.len, nd.nt);
+              geom_from_pair<TAIL>(ng, np, nidx, p.g.delta);
             }
             ok = geom_publish(wc, sched_ring, sched_full, sched_empty, it_cnt + 1, ng);
             if (!ok) break;
@@ -846,6 +847,7 @@ int launch_fwd_tc(const b200_hstu_attn_args &a, cudaStream_t st) {
   p.g.c = a.contextual_seq_len;
   p.g.F = a.min_full_attn_seq_len;
   p.g.delta = a.delta_size;
+  const bool tail = leaves_tiles_out(p.g);
   const int64_t eb = bias_table_bytes(a.bias_by_distance, a.max_seq_len);
   uint8_t *lists = reinterpret_cast<uint8_t *>(a.workspace) + eb;
   BiasTable bt{a.bias_by_distance, a.bias_numel, reinterpret_cast<float *>(a.workspace), a.max_seq_len};
@@ -888,15 +890,18 @@ int launch_fwd_tc(const b200_hstu_attn_args &a, cudaStream_t st) {
                     (long long)(eb + 3 * one), (long long)a.workspace_bytes);
       PlanHeader *hdr_kv = reinterpret_cast<PlanHeader *>(lists + one);
       PlanHeader *hdr_q = reinterpret_cast<PlanHeader *>(lists + 2 * one);
-      attn_plan3_kernel<PLAN_Q_PAIR><<<3, PLAN_THREADS, 0, st>>>(p.g, hdr, items, hdr_kv, reinterpret_cast<ItemDesc *>(hdr_kv + 1),
+      const auto plan = tail ? attn_plan3_kernel<PLAN_Q_PAIR, true> : attn_plan3_kernel<PLAN_Q_PAIR, false>;
+      plan<<<3, PLAN_THREADS, 0, st>>>(p.g, hdr, items, hdr_kv, reinterpret_cast<ItemDesc *>(hdr_kv + 1),
                                                     hdr_q, reinterpret_cast<ItemDesc *>(hdr_q + 1), max_items, grid, bt);
     } else {
-      attn_plan_kernel<PLAN_Q_PAIR><<<1, PLAN_THREADS, 0, st>>>(p.g, hdr, items, max_items, grid, bt);
+      const auto plan = tail ? attn_plan_kernel<PLAN_Q_PAIR, true> : attn_plan_kernel<PLAN_Q_PAIR, false>;
+      plan<<<1, PLAN_THREADS, 0, st>>>(p.g, hdr, items, max_items, grid, bt);
     }
   }
   count_launch();
   B200_CHECK_LAUNCH("attention plan");
-  auto kern = hstu_attn_fwd_sm100_kernel<D, IS_BF16, ONE_PATH, BIAS>;
+  auto kern = tail ? hstu_attn_fwd_sm100_kernel<D, IS_BF16, ONE_PATH, BIAS, true>
+                   : hstu_attn_fwd_sm100_kernel<D, IS_BF16, ONE_PATH, BIAS, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::DYN_BYTES);
   if (e != cudaSuccess) return check_cuda(e, "forward smem attribute");
   {

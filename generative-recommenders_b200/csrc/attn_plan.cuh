@@ -48,6 +48,17 @@ __host__ __device__ __forceinline__ int q_tiles_of(const AttnGeomParams &g, int 
   return ((g.delta > 0 ? g.delta : L) + 127) / 128;
 }
 
+// Which launches take the rules that look between window and tail (TAIL below): those whose sequences may have tiles
+// there.  On all launches these rules cost the others: in microseconds of a launch with its planning, rules
+// nowhere / everywhere / as chosen here, forward of 400 sequences of 20 - 300 rows with targets (d = 128) 84.1 / 86.2 /
+// 84.4, of 600 of 20 - 128 rows (d = 64) 54.4 / 55.4 / 54.4; with window 100 and tail 50, 600 of 100 - 250 rows, forward
+// 115.6 / 120.8 / 115.6, backward 272 / 284 / 274.  Where the line lies: window and tail 100 on 171 - 480 rows backward 204
+// without, 208 with them; window 200, tail 100 on 171 - 800 rows 176 and 173; window 517, tail 100 on 37 - 3001 rows
+// 319 and 236, forward 128 and 96.
+inline bool leaves_tiles_out(const AttnGeomParams &g) {
+  return g.W > 0 && g.F > 0 && (int64_t)g.max_seq_len >= (int64_t)g.W + g.F + 3 * TILE;
+}
+
 struct TileItem {
   int b, mt;              // sequence, tile index inside the sequence
   int start, len, nt;     // first token row, untruncated length, number of targets
@@ -55,10 +66,13 @@ struct TileItem {
   SeqMask m;
   int t_lo, n_main;       // opposite-side tiles [t_lo, t_lo + n_main)
   int extra_tile;         // >= 0: one more tile outside the main range
-  int gap_at, gap;        // the main range leaves out `gap` tiles after its first `gap_at` (kv items only; 16 bits)
   int n_tiles;
   int u;                  // first target position
   bool regular;           // closed-form row intervals / tile classification are valid
+};
+// What the kv-stationary launch walks: its main range leaves out `gap` tiles after its first `gap_at` (16 bits each).
+struct KvTileItem : TileItem {
+  int gap_at, gap;
   __host__ __device__ __forceinline__ int tile_at(int j) const {
     return j < n_main ? t_lo + j + (j >= gap_at ? gap : 0) : extra_tile;
   }
@@ -75,23 +89,24 @@ __host__ __device__ __forceinline__ void fill_common(TileItem &it, const AttnGeo
   it.m0 = t * TILE + (g.delta > 0 ? it.m.L - g.delta : 0);
   it.u = len - nt;
   it.regular = (it.u >= g.c + 1) && (nt >= 0) && (len <= it.m.L);
-  it.gap_at = it.gap = 0;
 }
 
 // The last row of a query tile (rows [m0, rows_end)) that sees a window instead of everything before it, as
 // a position (a target stands where the history ends); below m0 when the tile has none.
+template <bool TAIL>
 __host__ __device__ __forceinline__ int last_windowed_row(const TileItem &it, int rows_end) {
   const SeqMask &m = it.m;
   const int last = rows_end - 1;
-  if (m.F > 0) return last < it.u - m.F - 1 ? last : it.u - m.F - 1;
+  if (TAIL && m.F > 0) return last < it.u - m.F - 1 ? last : it.u - m.F - 1;
   return last < it.u ? last : it.u;
 }
 
 // kv tiles that the query tile `mt` of a sequence visits
+template <bool TAIL>
 __host__ __device__ __forceinline__ void fill_q_item(TileItem &it, const AttnGeomParams &g, int b, int mt, int start,
                                                      int len, int nt) {
   fill_common(it, g, b, mt, start, len, nt);
-  KvRange r = kv_range_for_q_tile(it.m, it.len, it.nt, it.m0, TILE);
+  KvRange r = kv_range_for_q_tile<TAIL>(it.m, it.len, it.nt, it.m0, TILE);
   it.t_lo = r.lo / TILE;
   int t_hi = (r.hi + TILE - 1) / TILE;
   if (t_hi <= it.t_lo) t_hi = it.t_lo + 1;
@@ -123,7 +138,7 @@ __host__ __device__ __forceinline__ bool tile_pair_is_full(const TileItem &it, i
   int lim = it.m0 < it.u ? it.m0 : it.u;
   if (n0 + TILE > lim) return false;
   if (m.W > 0) {
-    const int last = last_windowed_row(it, it.m0 + TILE < m.L ? it.m0 + TILE : m.L);
+    const int last = last_windowed_row<true>(it, it.m0 + TILE < m.L ? it.m0 + TILE : m.L);
     if ((m.F == 0 || last >= it.m0) && last - n0 > m.W) return false;
   }
   return true;
@@ -134,6 +149,7 @@ __host__ __device__ __forceinline__ bool tile_pair_is_full(const TileItem &it, i
 struct FullRange {
   int lo, hi;
 };
+template <bool TAIL>
 __host__ __device__ __forceinline__ FullRange full_tile_range(const TileItem &it) {
   FullRange r = {0, 0};
   if (!it.regular) return r;
@@ -142,9 +158,10 @@ __host__ __device__ __forceinline__ FullRange full_tile_range(const TileItem &it
   const int lim = it.m0 < it.u ? it.m0 : it.u;
   int lo = m.c > 0 ? (m.c + TILE - 1) / TILE : 0;
   if (m.W > 0) {
-    const int last = last_windowed_row(it, it.m0 + TILE < m.L ? it.m0 + TILE : m.L);
+    if (!TAIL && m.F > 0) return r;
+    const int last = last_windowed_row<TAIL>(it, it.m0 + TILE < m.L ? it.m0 + TILE : m.L);
     const int first = last - m.W;   // n0 >= first
-    if (first > 0 && (m.F == 0 || last >= it.m0)) {
+    if (first > 0 && (!TAIL || m.F == 0 || last >= it.m0)) {
       const int t = (first + TILE - 1) / TILE;
       lo = t > lo ? t : lo;
     }
@@ -161,9 +178,11 @@ __host__ __device__ __forceinline__ FullRange full_tile_range(const TileItem &it
 // then the tail and the targets.  (23 sequences of 37 - 3001 rows, window 517, tail 100, 6 heads of 64: with
 // every tile from the diagonal on visited and masked 183 us, now 139; forward and dQ launch, whose query
 // tiles outside the tail now start at their window: 151 -> 109 and 157 -> 114.)
-__host__ __device__ __forceinline__ void fill_kv_item(TileItem &it, const AttnGeomParams &g, int b, int kt, int start,
-                                                      int len, int nt) {
+template <bool TAIL>
+__host__ __device__ __forceinline__ void fill_kv_item(KvTileItem &it, const AttnGeomParams &g, int b, int kt,
+                                                      int start, int len, int nt) {
   fill_common(it, g, b, kt, start, len, nt);
+  it.gap_at = it.gap = 0;
   const int L = it.m.L;
   const int ntiles = (L + TILE - 1) / TILE;
   int t_lo = kt, t_hi = ntiles;
@@ -175,7 +194,7 @@ __host__ __device__ __forceinline__ void fill_kv_item(TileItem &it, const AttnGe
     if (n0 >= it.u) {
       // only target columns: each is seen by its own row alone
       t_hi = kt + 1;
-    } else if (g.W > 0) {
+    } else if (g.W > 0 && (TAIL || g.F == 0)) {
       // history rows i see j >= i - W; target rows see j >= u - W.  Last history row that can
       // still see a column of this tile: n1 - 1 + W.
       int last_row = n1 - 1 + g.W;
@@ -192,7 +211,7 @@ __host__ __device__ __forceinline__ void fill_kv_item(TileItem &it, const AttnGe
         int hist_end = L - 1 < last_row ? L - 1 : last_row;
         t_hi = hist_end / TILE + 1;
       }
-      if (g.F > 0) {
+      if (TAIL && g.F > 0) {
         const int w_end = (it.u - 1 < last_row ? it.u - 1 : last_row) / TILE + 1;   // behind the windowed rows
         const int tail = it.u - g.F > n0 ? (it.u - g.F) / TILE : kt;
         t_hi = ntiles;
@@ -217,7 +236,7 @@ __host__ __device__ __forceinline__ void fill_kv_item(TileItem &it, const AttnGe
   }
   it.t_lo = t_lo;
   it.n_main = t_hi - t_lo - it.gap;
-  if (it.gap > 0) it.gap_at -= t_lo;
+  if (TAIL && it.gap > 0) it.gap_at -= t_lo;
   if (it.n_main < 0) it.n_main = 0;
   it.n_tiles = it.n_main + (it.extra_tile >= 0 ? 1 : 0);
 }
@@ -237,6 +256,7 @@ struct PairItem {
   }
 };
 
+template <bool TAIL>
 __host__ __device__ __forceinline__ void fill_pair_item(PairItem &p, const AttnGeomParams &g, int b, int pair,
                                                         int start, int len, int nt) {
   // With an odd number of query tiles the tile left without a partner is the FIRST one (a single
@@ -246,11 +266,11 @@ __host__ __device__ __forceinline__ void fill_pair_item(PairItem &p, const AttnG
   const int ntiles = q_tiles_of(g, L);
   const bool odd = (ntiles & 1) != 0;
   const int first = odd ? (pair == 0 ? 0 : 2 * pair - 1) : 2 * pair;
-  fill_q_item(p.A, g, b, first, start, len, nt);
+  fill_q_item<TAIL>(p.A, g, b, first, start, len, nt);
   p.hasB = !(odd && pair == 0) && (first + 1) < ntiles;
   int lo = p.A.t_lo, hi = p.A.t_lo + p.A.n_main;
   if (p.hasB) {
-    fill_q_item(p.B, g, b, first + 1, start, len, nt);
+    fill_q_item<TAIL>(p.B, g, b, first + 1, start, len, nt);
     lo = p.B.t_lo < lo ? p.B.t_lo : lo;
     int bh = p.B.t_lo + p.B.n_main;
     hi = bh > hi ? bh : hi;
@@ -362,25 +382,25 @@ __host__ __device__ __forceinline__ uint32_t col_mask_bits(const ColInterval &r,
   return bits & low_bits(L - base);
 }
 
-template <int KIND>
+template <int KIND, bool TAIL>
 __host__ __device__ __forceinline__ int item_cost(const AttnGeomParams &g, int b, int t, int len, int nt) {
   if (KIND == PLAN_Q_PAIR) {
     PairItem p;
-    fill_pair_item(p, g, b, t, 0, len, nt);
+    fill_pair_item<TAIL>(p, g, b, t, 0, len, nt);
     // a query tile without a partner takes about 1.6x as long per kv tile
     return p.hasB ? p.A.n_tiles + p.B.n_tiles : (p.A.n_tiles * 8 + 4) / 5;
   } else if (KIND == PLAN_Q_TILE) {
     TileItem it;
-    fill_q_item(it, g, b, t, 0, len, nt);
+    fill_q_item<TAIL>(it, g, b, t, 0, len, nt);
     return it.n_tiles;
   } else {
-    TileItem it;
-    fill_kv_item(it, g, b, t, 0, len, nt);
+    KvTileItem it;
+    fill_kv_item<TAIL>(it, g, b, t, 0, len, nt);
     return it.n_tiles;
   }
 }
 
-template <int KIND>
+template <int KIND, bool TAIL>
 __device__ __forceinline__ void plan_body(const AttnGeomParams &g, PlanHeader *hdr, ItemDesc *items, int max_items,
                                           int first_dynamic) {
   static_assert(PLAN_BUCKETS == PLAN_THREADS, "one bucket per thread in the scan");
@@ -412,7 +432,7 @@ __device__ __forceinline__ void plan_body(const AttnGeomParams &g, PlanHeader *h
         if (first && pass == 1 && kept_bucket >= 0) {
           bucket = kept_bucket;
         } else {
-          int cost = item_cost<KIND>(g, b, t, len, nt);
+          int cost = item_cost<KIND, TAIL>(g, b, t, len, nt);
           cost = cost < PLAN_BUCKETS - 1 ? cost : PLAN_BUCKETS - 1;
           bucket = PLAN_BUCKETS - 1 - cost;  // expensive first
           if (first && pass == 0) kept_bucket = bucket;
@@ -506,32 +526,32 @@ __device__ __forceinline__ void build_bias_table(const BiasTable &t) {
   }
 }
 
-template <int KIND>
+template <int KIND, bool TAIL>
 __global__ void __launch_bounds__(PLAN_THREADS) attn_plan_kernel(AttnGeomParams g, PlanHeader *hdr, ItemDesc *items,
                                                                  int max_items, int first_dynamic, BiasTable bt) {
   build_bias_table(bt);
   // the attention kernel that follows may already set itself up; it waits for this grid to
   // finish before it reads the list
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  plan_body<KIND>(g, hdr, items, max_items, first_dynamic);
+  plan_body<KIND, TAIL>(g, hdr, items, max_items, first_dynamic);
 }
 
 // two work lists in one launch (one CTA each): the backward's K/V-tile and query-tile lists
-template <int KIND0, int KIND1>
+template <int KIND0, int KIND1, bool TAIL>
 __global__ void __launch_bounds__(PLAN_THREADS) attn_plan2_kernel(AttnGeomParams g, PlanHeader *hdr0, ItemDesc *items0,
                                                                   PlanHeader *hdr1, ItemDesc *items1, int max_items,
                                                                   int first_dynamic, BiasTable bt) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (blockIdx.x == 0) build_bias_table(bt);
   if (blockIdx.x == 0)
-    plan_body<KIND0>(g, hdr0, items0, max_items, first_dynamic);
+    plan_body<KIND0, TAIL>(g, hdr0, items0, max_items, first_dynamic);
   else
-    plan_body<KIND1>(g, hdr1, items1, max_items, first_dynamic);
+    plan_body<KIND1, TAIL>(g, hdr1, items1, max_items, first_dynamic);
 }
 
 // all three work lists of a training step in one launch (one CTA each): forward, then the
 // backward's K/V-tile and query-tile lists
-template <int KIND0>
+template <int KIND0, bool TAIL>
 __global__ void __launch_bounds__(PLAN_THREADS) attn_plan3_kernel(AttnGeomParams g, PlanHeader *hdr0, ItemDesc *items0,
                                                                   PlanHeader *hdr1, ItemDesc *items1, PlanHeader *hdr2,
                                                                   ItemDesc *items2, int max_items, int first_dynamic,
@@ -539,11 +559,11 @@ __global__ void __launch_bounds__(PLAN_THREADS) attn_plan3_kernel(AttnGeomParams
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (blockIdx.x == 0) build_bias_table(bt);
   if (blockIdx.x == 0)
-    plan_body<KIND0>(g, hdr0, items0, max_items, first_dynamic);
+    plan_body<KIND0, TAIL>(g, hdr0, items0, max_items, first_dynamic);
   else if (blockIdx.x == 1)
-    plan_body<PLAN_KV_TILE>(g, hdr1, items1, max_items, first_dynamic);
+    plan_body<PLAN_KV_TILE, TAIL>(g, hdr1, items1, max_items, first_dynamic);
   else
-    plan_body<PLAN_Q_TILE>(g, hdr2, items2, max_items, first_dynamic);
+    plan_body<PLAN_Q_TILE, TAIL>(g, hdr2, items2, max_items, first_dynamic);
 }
 
 __device__ __forceinline__ ItemDesc load_desc(const ItemDesc *items, int idx) {

@@ -146,6 +146,10 @@ struct KvRange {
   int diag_lo;     // >= 0: an extra block [diag_lo, diag_lo + T) outside the main range
 };
 
+// TAIL: with a window and a full-attention tail, look which tiles lie between the two; without TAIL such a launch
+// visits everything.  (The shorter rules count: a producer works an item out between two requests, and sequences of one
+// or two tiles wait for it.  See leaves_tiles_out().)
+template <bool TAIL = true>
 __host__ __device__ __forceinline__ KvRange kv_range_for_q_tile(const SeqMask &m, int len, int num_targets, int m0,
                                                                 int T) {
   KvRange r;
@@ -169,7 +173,7 @@ __host__ __device__ __forceinline__ KvRange kv_range_for_q_tile(const SeqMask &m
   int lo = 0;
   // a tile that reaches into the full-attention tail (its last `F` history rows, and then the targets) has
   // rows that see everything before them
-  if (m.W > 0 && !(m.F > 0 && m1 > u - m.F)) {
+  if (m.W > 0 && (m.F == 0 || (TAIL && m1 <= u - m.F))) {
     lo = first - m.W;
     if (lo < m.c) lo = 0;  // first - W <= c - 1: the row also sees the contextual prefix
   }

@@ -687,3 +687,30 @@ def test_window_with_full_tail_over_many_tiles(impl, case):
     out, grads = _run(q, k, v, offs, N, 1.0 / d ** 0.5, nt, Wn, ctx, F, dout)
     ref, rgrads = _oracle(q, k, v, offs, N, 1.0 / d ** 0.5, nt, Wn, ctx, F, dout)
     _check_all(("gap", impl, case), out, grads, ref, rgrads, offs)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("ctx, targets, bias", [(0, 0, False), (5, 20, False), (130, 1, True)])
+def test_launches_that_look_for_tiles_between_window_and_tail_and_those_that_do_not(d, ctx, targets, bias):
+    """Whether a launch leaves out the tiles between window and tail is decided by max_seq_len (584 on, for 100 and
+    100).  It also divides the result: twice as large a power of two halves everything exactly."""
+    g = torch.Generator().manual_seed(d + ctx)
+    lengths = torch.tensor([512, 511, 385, 384, 257, 136])
+    offs = torch.cat([lengths.new_zeros(1), lengths.cumsum(0)]).cuda()
+    nt = torch.tensor([targets, 0, targets, 1, 0, targets]).clamp(max=targets).cuda()
+    q, k, v, dout = (torch.randn(int(offs[-1]), 2, d, generator=g).bfloat16().cuda() for _ in range(4))
+    table = torch.randn(512, generator=g).cuda() * 0.1 if bias else None
+    results = []
+    for N in (512, 1024):
+        leaves = [t.clone().requires_grad_() for t in (q, k, v)]
+        out = G.hstu_mha(N, 1.0 / d, *leaves, offs, num_targets=nt, max_attn_len=100, contextual_seq_len=ctx,
+                         min_full_attn_seq_len=100, bias_by_distance=table)
+        results.append((out.detach(),) + torch.autograd.grad(out, leaves, dout))
+    for short, long in zip(*results):
+        assert torch.equal(short, 2 * long)
+    if d == 128 and not bias:
+        quantised = [G.quantize_e4m3_block(t, offs) for t in (q, k, v)]
+        fp8 = [G.hstu_mha_fp8(N, 1.0 / d, *(t[0] for t in quantised), *(t[1] for t in quantised), quantised[0][2], offs,
+                              num_targets=nt, max_attn_len=100, contextual_seq_len=ctx, min_full_attn_seq_len=100)
+               for N in (512, 1024)]
+        assert torch.equal(fp8[0], 2 * fp8[1])
